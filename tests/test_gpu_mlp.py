@@ -75,3 +75,23 @@ def test_mlp_training_learns_a_separable_rule(ctx, rtr):
     assert losses[-1] < 0.5 * losses[0], losses
     acc = ((m.score(_dev(X)).cpu().numpy() > 0.5) == (y > 0.5)).mean()
     assert acc > 0.9, acc
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 1025, 2047, 2048, 5003])
+def test_mlp_gradient_at_block_and_slab_edges(ctx, rtr, n):
+    """Rows per block (32) and rows per slab of the weight gradients (from
+    1,024: one slab below 2,048 rows, then several), ragged ends included.
+    FP32 sums of n terms in chains of at most ~300: far below 1e-5 of the
+    gradient's norm."""
+    theta = OM.init_params(n)
+    X, y = _data(n + 1, n)
+    m = rtr.Mlp(ctx, theta)
+    loss, g = m.loss_grad(_dev(X), _dev(y))
+    rl, rg = OM.loss_and_grad(theta, X, y)
+    g = g.cpu().numpy().astype(np.float64)
+    assert abs(float(loss.item()) - rl) <= 1e-5 * max(1.0, abs(rl))
+    o = 0
+    for name, shape in OM.SIZES:
+        k = int(np.prod(shape))
+        assert np.linalg.norm(g[o:o + k] - rg[o:o + k]) <= 1e-5 * np.linalg.norm(rg), name
+        o += k
