@@ -48,3 +48,19 @@ def test_tdf_batch_many_keypoints(ctx):
     out = out.cpu().numpy()
     for k in range(64):
         assert np.array_equal(out[k], O.tdf(occ[offs[k]:offs[k + 1]], 30)), k
+
+
+@pytest.mark.parametrize("n_keys,dim", [(1, 32), (37, 30), (38, 30), (3, 31), (40, 9), (70000, 1)])
+def test_tdf_batch_row_split_edges(ctx, n_keys, dim):
+    """Both row splits (whole rows from two CTAs per SM on, quarters below),
+    the largest grid edge, keypoints beyond the launch grid's y limit, and
+    occupied voxels outside the grid, near and far."""
+    import torch
+    rng = np.random.default_rng(n_keys + dim)
+    per = 1 if n_keys > 1000 else 50
+    occ = rng.integers(-40, dim + 40, size=(n_keys * per, 3)).astype(np.int32)
+    occ[::7] *= 100
+    offs = (np.arange(n_keys + 1) * per).astype(np.int32)
+    out = ctx.tdf_batch(torch.from_numpy(occ).cuda(), torch.from_numpy(offs).cuda(), dim).cpu().numpy()
+    for k in range(n_keys) if n_keys < 1000 else (0, 1, 65534, 65535, 65536, n_keys - 1):
+        assert np.array_equal(out[k], O.tdf(occ[k * per:(k + 1) * per], dim)), k
