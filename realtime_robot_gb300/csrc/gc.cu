@@ -115,14 +115,14 @@ __global__ void k_gcg_setup(GcGrid* gg, const GridMeta* __restrict__ mbox, float
   float lo[3], hi[3];
   double diag2 = 0.0, mag = 0.0;
   for (int a = 0; a < 3; ++a) {
-    lo[a] = n > 0 ? ordered_to_float(m.bmin[a]) : 0.f;
-    hi[a] = n > 0 ? ordered_to_float(m.bmax[a]) : 0.f;
+    lo[a] = n > 0 ? box_lo(&m, a) : 0.f;
+    hi[a] = n > 0 ? box_hi(&m, a) : 0.f;
     if (!isfinite(lo[a]) || !isfinite(hi[a]) || !(hi[a] >= lo[a])) {
       lo[a] = isfinite(lo[a]) ? lo[a] : (isfinite(hi[a]) ? hi[a] : 0.f);
       hi[a] = isfinite(hi[a]) && hi[a] >= lo[a] ? hi[a] : lo[a];
     }
-    const float ml = n > 0 ? ordered_to_float(mbox->bmin[a]) : 0.f;
-    const float mh = n > 0 ? ordered_to_float(mbox->bmax[a]) : 0.f;
+    const float ml = n > 0 ? box_lo(mbox, a) : 0.f;
+    const float mh = n > 0 ? box_hi(mbox, a) : 0.f;
     gg->mlo[a] = ml;
     gg->mhi[a] = mh;
     const double e = (double)mh - (double)ml;
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
     // largest model-side distance: the diagonal of the endpoints' box
     float d2 = 0.f;
     for (int k = 0; k < 3; ++k) {
-      const float e = ordered_to_float(c.mbox->bmax[k]) - ordered_to_float(c.mbox->bmin[k]);
+      const float e = box_hi(c.mbox, k) - box_lo(c.mbox, k);
       d2 += e * e;
     }
     const float R = (sqrtf(d2) + g.gc) * 1.0001f + 1.0e-5f;
@@ -909,7 +909,9 @@ __global__ void k_gc_poses(const float4* __restrict__ pm, const float4* __restri
 #pragma unroll
   for (int k = 0; k < 9; ++k) H[k] = __shfl_sync(0xffffffffu, H[k], 0);
   double R[9];
-  umeyama_rotation_warp(H, R);
+  const double r = umeyama_rotation_warp(pick9(H, lane < 9 ? lane : 8));
+#pragma unroll
+  for (int k = 0; k < 9; ++k) R[k] = __shfl_sync(0xffffffffu, r, k);
   if (lane == 0) {
     double* T = poses + (size_t)c * 16;
     for (int r = 0; r < 3; ++r) {
@@ -1098,11 +1100,11 @@ static rtr_status gc_launch(rtr_context* ctx, Scratch& s, const float* d_model_k
   RTR_CUDA(cudaMemsetAsync(b.misc, 0, sizeof(int) * 16, st));
   RTR_CUDA(cudaMemsetAsync(b.arrive, 0, sizeof(unsigned), st));
   GcDev g{b.pm, b.ps, C, d_C, gc_size, b.taken, b.set_size, b.set_mem, gc_set_stride(C)};
-  bbox_build(b.mbox, b.pm, C, d_C, st);
+  RTR_TRY(bbox_build(b.mbox, b.pm, C, d_C, st));
   pso.end();
   // the coarse grid over the scene endpoints (seed-test pruning)
   ProfScope pgr(ctx, st, "gc_grid");
-  bbox_build(&b.sg->m, b.ps, C, d_C, st);
+  RTR_TRY(bbox_build(&b.sg->m, b.ps, C, d_C, st));
   k_gcg_setup<<<1, 32, 0, st>>>(b.sg, b.mbox, gc_size, C, d_C);
   k_gcg_keys<<<nb, 256, 0, st>>>(b.ps, C, d_C, b.sg, b.gk0);
   uint32_t *gks, *gvs;  // gks unused: the cell order is all the seed tests need

@@ -1,10 +1,11 @@
-// grid.cuh — radix-sorted uniform grid (build on device, exact searches).
+// grid.cuh — uniform grid (built on device, exact searches) and radix sort.
 //
-// A grid over n points with cell edge h: points are sorted by the linear index
-// of their cell (x fastest) with a stable LSD radix sort, and a dense table
-// gives each cell its [start, end) range in the sorted order.  Every size and
-// every bound is computed on the device, so a build can sit inside a captured
-// CUDA graph; capacities come from the host.
+// A grid over n points with cell edge h keeps the points in the order of the
+// linear index of their cell (x fastest) and one table of ncells + 1 starts:
+// cell c holds points [starts[c], starts[c + 1]), and a run of cells along x
+// is one contiguous run of points.  Every size and every bound is computed on
+// the device, so a build can sit inside a captured CUDA graph; capacities
+// come from the host.
 #pragma once
 #include "common.cuh"
 
@@ -14,25 +15,33 @@ struct GridMeta {
   int nx, ny, nz;
   int n;                 // points in the grid
   unsigned ncells;       // nx*ny*nz
-  unsigned bmin[3];      // bounding box as order-preserving unsigned
+  // bounding box as order-preserving unsigned, the lower corner complemented
+  // so that both start at zero (cleared by a memset); see box_lo, box_hi
+  unsigned nmin[3];
   unsigned bmax[3];
+  unsigned ticket;       // blocks of the box reduction that are done
 };
 
 struct GridDev {
   const GridMeta* meta;  // device
-  const float4* pts;     // points sorted by cell; w = original index (int bits)
-  const int* idx;        // original index of each sorted point
-  const uint2* cells;    // per cell {start, end}
+  const float4* pts;     // points in cell order; w = original index (int bits)
+  const uint32_t* starts;  // [ncells + 1]
 };
+
+#ifdef __CUDACC__
+__device__ __forceinline__ float box_lo(const GridMeta* m, int a) { return ordered_to_float(~m->nmin[a]); }
+__device__ __forceinline__ float box_hi(const GridMeta* m, int a) { return ordered_to_float(m->bmax[a]); }
+#endif
 
 namespace rtr {
 
 struct GridBufs {
-  GridMeta* meta;
+  GridMeta* meta;        // followed by the table in one allocation
+  uint32_t* starts;      // [cell_cap + 1]
+  uint32_t* tiles;       // tile sums of the table's scan
   float4* pts;
-  int* idx;
-  uint2* cells;
-  uint32_t *k0, *v0, *k1, *v1, *hist;
+  uint32_t *k0, *v0;     // cell of each point, and its rank there
+  uint32_t *k1, *v1, *hist;  // ordered builds only
   int n_cap;
   unsigned cell_cap;
 };
@@ -45,18 +54,20 @@ void radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, ui
                       int n_cap, int n_host, const int* d_n, int bits, bool vals_iota,
                       cudaStream_t st, uint32_t** k_out, uint32_t** v_out);
 
-void grid_plan(ScratchPlan& plan, int n_cap, unsigned cell_cap);
-bool grid_take(Scratch& s, int n_cap, unsigned cell_cap, GridBufs* b);
+// ordered: the points of a cell in ascending original index (a stable sort by
+// cell); otherwise in any order (counted into place, a quarter of the time).
+void grid_plan(ScratchPlan& plan, int n_cap, unsigned cell_cap, bool ordered = false);
+bool grid_take(Scratch& s, int n_cap, unsigned cell_cap, GridBufs* b, bool ordered = false);
 // Build the grid over pts[0..n) (n = *d_n when d_n != NULL).  h_req is the
 // requested cell edge; if the bounding box needs more than cell_cap cells the
 // edge grows until it fits (searches stay exact, only slower).
-void grid_build(const GridBufs& b, const float4* pts, int n_host, const int* d_n, float h_req,
-                cudaStream_t st);
-// Bounding box only (fills m->bmin / m->bmax).
-void bbox_build(GridMeta* m, const float4* pts, int n, cudaStream_t st);
+rtr_status grid_build(const GridBufs& b, const float4* pts, int n_host, const int* d_n, float h_req, cudaStream_t st,
+                      bool ordered = false);
+// Bounding box only (box_lo, box_hi).
+rtr_status bbox_build(GridMeta* m, const float4* pts, int n, cudaStream_t st);
 // Same over the first *d_n (<= n_cap) points.
-void bbox_build(GridMeta* m, const float4* pts, int n_cap, const int* d_n, cudaStream_t st);
-inline GridDev grid_dev(const GridBufs& b) { return GridDev{b.meta, b.pts, b.idx, b.cells}; }
+rtr_status bbox_build(GridMeta* m, const float4* pts, int n_cap, const int* d_n, cudaStream_t st);
+inline GridDev grid_dev(const GridBufs& b) { return GridDev{b.meta, b.pts, b.starts}; }
 inline unsigned default_cell_cap(int n) {
   unsigned c = (unsigned)n * 8u;
   return c < (1u << 18) ? (1u << 18) : c;

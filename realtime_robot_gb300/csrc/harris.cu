@@ -64,10 +64,9 @@ __device__ int hr_gather(const HrArgs& a, const GridView& g, float4 q, int* list
   const HrBox bb = hr_box(g, q, a.r);
   int cnt = 0;
   for (int z = bb.z0; z <= bb.z1; ++z)
-    for (int y = bb.y0; y <= bb.y1; ++y)
-      for (int x = bb.x0; x <= bb.x1; ++x) {
-        const uint2 c = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
-        for (unsigned j0 = c.x; j0 < c.y; j0 += 32) {
+    for (int y = bb.y0; y <= bb.y1; ++y) {
+      const uint2 c = row_span(g, bb.x0, bb.x1, y, z);
+      for (unsigned j0 = c.x; j0 < c.y; j0 += 32) {
           const unsigned j = j0 + (unsigned)lane;
           bool in = false;
           int id = 0;
@@ -205,9 +204,8 @@ __global__ void __launch_bounds__(HR_WARPS * 32) k_hr_select(HrArgs a, const flo
       const float4 q = a.pts[i];
       const HrBox bb = hr_box(g, q, a.r);
       for (int z = bb.z0; z <= bb.z1 && ok; ++z)
-        for (int y = bb.y0; y <= bb.y1 && ok; ++y)
-          for (int x = bb.x0; x <= bb.x1 && ok; ++x) {
-            const uint2 c = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
+        for (int y = bb.y0; y <= bb.y1 && ok; ++y) {
+            const uint2 c = row_span(g, bb.x0, bb.x1, y, z);
             bool larger = false;
             for (unsigned j = c.x + (unsigned)lane; j < c.y; j += 32) {
               const float4 p = g.pts[j];
@@ -356,7 +354,7 @@ rtr_status rtr_harris3d(rtr_context* ctx, const float* d_pts, int n, const rtr_h
   int* err = reinterpret_cast<int*>(s.base + o_e);
   ProfScope ps(ctx, st, "harris3d");
   const float4* pts = reinterpret_cast<const float4*>(d_pts);
-  grid_build(gb, pts, n, nullptr, prm->radius, st);
+  RTR_TRY(grid_build(gb, pts, n, nullptr, prm->radius, st));
   RTR_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
   HrArgs a{grid_dev(gb), pts, n, prm->radius, prm->radius * prm->radius, err};
   const int nb = hr_blocks(n);

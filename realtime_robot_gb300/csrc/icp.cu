@@ -1,15 +1,16 @@
 // icp.cu — persistent point-to-point ICP (replaces the PCL
 // IterativeClosestPoint used by keyPointICP, function.h:111-148).
 //
-// One cooperative launch runs every iteration.  Per iteration each thread
-// transforms its source points with the FP32 pose, finds the exact 1-NN in the
-// target grid within max_corr_dist (rejection), and accumulates the centred
-// sums (dp, dq, dp dq^T, d^2) in FP32 Kahan–Babuška accumulators; warps and
-// the block combine them with TwoSum-compensated shuffles into one (hi, lo)
-// pair per value per block.  The last block to arrive reduces the block pairs
-// in FP64 (fixed order), solves the pose in FP64 (pose.cuh) and releases the
-// others through a generation word.  Every wait is bounded by a clock64
-// budget; a block that runs out writes RTR_ERR_TIMEOUT and leaves.
+// One cooperative launch runs every iteration.  Per iteration the source
+// points are transformed with the FP32 pose and matched to their exact 1-NN
+// in the target grid within max_corr_dist (rejection; most points only show
+// that their last neighbour still is the nearest, see k_icp), and each thread
+// accumulates the centred sums (dp, dq, dp dq^T, d^2) in FP32 Kahan–Babuška
+// accumulators; warps and the block combine them with TwoSum-compensated
+// shuffles into one (hi, lo) pair per value per block.  The last block to
+// arrive reduces the block pairs (fixed order, FP64 closing), solves the pose
+// in FP64 (pose.cuh) and publishes it to the others.  Every wait is bounded by
+// a clock64 budget; a block that runs out writes RTR_ERR_TIMEOUT and leaves.
 #include <math.h>
 #include <atomic>
 #include <string.h>
@@ -24,7 +25,7 @@ namespace rtr {
 constexpr int ICP_THREADS = 256;
 constexpr int ICP_WARPS = ICP_THREADS / 32;
 constexpr int ICP_NV = 16;  // dp(3) dq(3) dp*dq^T(9) d^2(1)
-
+constexpr int ICP_CHUNK = 2048;  // points a block matches between two barriers
 
 __device__ __forceinline__ unsigned long long icp_timer() {
   unsigned long long t;
@@ -32,23 +33,65 @@ __device__ __forceinline__ unsigned long long icp_timer() {
   return t;
 }
 
+// Between iterations nothing may cost the SM its L1: an acquire or a full
+// fence invalidates it, and every load of the next iteration (points, table,
+// the matching state, all of them hits otherwise) would go to L2.  So a block
+// arrives with a release alone, and the new pose is published as twelve
+// 64-bit words that carry the iteration beside the value: whoever reads the
+// right iteration has the value, in any order.  Only the block that arrives
+// last fences, to read the others' sums.  (Two 20k chairs 1583 -> 1387 us,
+// the room's recognition 4284 -> 4116 us.)
+__device__ __forceinline__ unsigned icp_arrive(unsigned* p) {
+  unsigned v;
+  asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 __device__ __forceinline__ float centre_of(const GridMeta* m, int a) {
-  return 0.5f * (ordered_to_float(m->bmin[a]) + ordered_to_float(m->bmax[a]));
+  return 0.5f * (box_lo(m, a) + box_hi(m, a));
 }
 
 // One launch serves many problems: block b works on problem blk2prob[b]
 // together with that problem's other nblk - 1 blocks; problems never wait on
 // one another.
+//
+// Matching.  The search that found a point's neighbour also found how far away
+// every other target point was ("room").  As long as the distance the source
+// point has moved since then, subtracted from the room, leaves more than the
+// distance to the neighbour as it is now, the neighbour is still the nearest,
+// and the point needs no search (for a point without a neighbour: more than
+// the bound).  Both sides carry a margin far above their rounding, so the
+// correspondences are those of a search from scratch.  Each iteration runs
+//   1. a thread per point: is the last answer still certain?  The others
+//      queue up in shared memory;
+//   2. G lanes per queued point: the search (grid_nn1_from), starting from
+//      the last neighbour; a queue keeps every lane busy where single points
+//      scattered over the warps would hold up 32 lanes each;
+//   3. a thread per point: the sums.
+// A search per point and iteration, each from the full bound, was over half of
+// the kernel.  Per iteration of block 0, matching and sums before and now: two
+// 20k chairs 25 and 8 us; 102k points against a 285k-point frame 35 and 10 us;
+// 16 refinements of a 9.2k-voxel model in a room 24 and 10 us.
 template <int G>  // lanes cooperating on one source point's 1-NN search
-__global__ void __launch_bounds__(ICP_THREADS) k_icp(const IcpDev* __restrict__ probs,
-                                                     const int* __restrict__ blk2prob) {
+__global__ void __launch_bounds__(ICP_THREADS, 2) k_icp(const IcpDev* __restrict__ probs,
+                                                        const int* __restrict__ blk2prob) {
   const IcpDev& a = probs[blk2prob[blockIdx.x]];
   const int lb = (int)blockIdx.x - a.blk0;
   __shared__ float s_red[ICP_WARPS][ICP_NV][2];
   __shared__ int s_cnt[ICP_WARPS];
   __shared__ double s_sum[ICP_NV];
-  __shared__ double s_P[16], s_D[16], s_H[9];
-  __shared__ long long s_n;
+  __shared__ float s_T[12];
+  __shared__ int s_pos[ICP_CHUNK];             // matched position of each point of the chunk (-1: none)
+  __shared__ unsigned short s_queue[ICP_CHUNK];  // points to search
+  __shared__ int s_qn;
   __shared__ int s_last, s_stop;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -63,16 +106,22 @@ __global__ void __launch_bounds__(ICP_THREADS) k_icp(const IcpDev* __restrict__ 
     return;
   }
   const int B = a.nblk;
-  const GridView g = load_view(a.grid);
-  const bool near27 = grid_near27_ok(g, a.r2max);  // every match within the 27 cells around a query
+  const BoxView bv = box_view(a.grid);
+  const GridView& g = bv.g;
+  const float r = sqrt_up(a.r2max);
   // Centring: target terms about the target box centre c, source terms about
   // the source box centre moved by the current pose (cp), so the FP32 products
   // stay small even while the clouds are far apart.
   const float c[3] = {centre_of(a.grid.meta, 0), centre_of(a.grid.meta, 1), centre_of(a.grid.meta, 2)};
   const float4 cs = make_float4(centre_of(a.src_meta, 0), centre_of(a.src_meta, 1), centre_of(a.src_meta, 2), 0.f);
-  constexpr int QPB = ICP_THREADS / G;  // source points per block per pass
-  constexpr int NVL = ICP_NV / G;        // sums kept per lane
-  const unsigned stride = (unsigned)B * QPB;
+  float mag = 0.f;  // the size of the source's coordinates
+#pragma unroll
+  for (int k = 0; k < 3; ++k) mag += fmaxf(fabsf(box_lo(a.src_meta, k)), fabsf(box_hi(a.src_meta, k)));
+  // point l of this block: groups of 8 points (whole lines) dealt out to the
+  // blocks in turn, which mixes regions with and without neighbours
+  const int groups = (a.n_src + 7) / 8;
+  const int n_loc = lb < groups ? ((groups - lb + B - 1) / B) * 8 : 0;
+  auto point_of = [&](int l) { return ((l >> 3) * B + lb) * 8 + (l & 7); };
   const int lg = lane & (G - 1);
   const unsigned gmask = ((1u << G) - 1u) << (lane & ~(G - 1));
 
@@ -80,241 +129,319 @@ __global__ void __launch_bounds__(ICP_THREADS) k_icp(const IcpDev* __restrict__ 
   unsigned long long t_it = 0, t_arr = 0;
   for (int it = 0; it < a.max_it; ++it) {
     if (prof0) t_it = icp_timer();
+    if (it == 0) {  // later poses arrive in s_T
+      if (tid < 12) s_T[tid] = __double2float_rn(a.init[tid]);
+      __syncthreads();
+    }
     float T[12];
-    if (it == 0) {
 #pragma unroll
-      for (int k = 0; k < 12; ++k) T[k] = __double2float_rn(a.init[k]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 12; ++k) T[k] = __ldcg(a.posef + k);
-    }
+    for (int k = 0; k < 12; ++k) T[k] = s_T[k];
     const float4 cp = xform_exact(T, cs);
-    // The G lanes of a group share the 16 sums of their points: lane lg keeps
-    // values lg*NVL .. lg*NVL+NVL-1 (dp 0-2, dq 3-5, dp dq^T 6-14, d^2 15),
-    // each over the group's points in order, as one lane holding all 16 would.
-    KSum acc[NVL];
-#pragma unroll
-    for (int k = 0; k < NVL; ++k) acc[k].init();
-    int cnt = 0;
-    for (unsigned i = (unsigned)lb * QPB + tid / G; i < (unsigned)a.n_src; i += stride) {
-      const float4 p = xform_exact(T, a.src[i]);
-      float d2;
-      int j, pos;
-      if (near27)  // the group agrees on (d2, j, pos)
-        grid_nn1_near<G>(g, p, a.r2max, lg, gmask, d2, j, pos);
-      else
-        grid_nn1_group<G, true>(g, p, a.r2max, lg, gmask, d2, j, pos);
-      if (j >= 0) {
-        const float4 q = g.pts[pos];
-        const float dp[3] = {__fsub_rn(p.x, cp.x), __fsub_rn(p.y, cp.y), __fsub_rn(p.z, cp.z)};
-        const float dq[3] = {__fsub_rn(q.x, c[0]), __fsub_rn(q.y, c[1]), __fsub_rn(q.z, c[2])};
-#pragma unroll
-        for (int k = 0; k < NVL; ++k) {
-          const int v = lg * NVL + k;
-          float x;
-          if (v < 3)
-            x = v == 0 ? dp[0] : (v == 1 ? dp[1] : dp[2]);
-          else if (v < 6)
-            x = v == 3 ? dq[0] : (v == 4 ? dq[1] : dq[2]);
-          else if (v < 15) {
-            const int r = (v - 6) / 3, kk = (v - 6) % 3;
-            x = __fmul_rn(r == 0 ? dp[0] : (r == 1 ? dp[1] : dp[2]), kk == 0 ? dq[0] : (kk == 1 ? dq[1] : dq[2]));
-          } else
-            x = d2;
-          acc[k].add(x);
+    // rounding of the search, and of a point's position then and now
+    const float margin = bv.margin + 2.0e-6f * (mag + fabsf(T[3]) + fabsf(T[7]) + fabsf(T[11]));
+    float run_s = 0.f, run_c = 0.f;  // thread v < 16: the block's sum of value v so far
+    int run_n = 0;
+    for (int c0 = 0; c0 < n_loc; c0 += ICP_CHUNK) {
+      const int cn = min(ICP_CHUNK, n_loc - c0);
+      if (c0 > 0) __syncthreads();  // the last chunk's places are free
+      if (tid == 0) s_qn = 0;
+      __syncthreads();
+      // 1. still certain?  (loop bound rounded up: the ballots need whole warps)
+      for (int l = tid; l < ((cn + 31) & ~31); l += ICP_THREADS) {
+        const int i = l < cn ? point_of(c0 + l) : a.n_src;
+        bool search = false;
+        int pos = -1;
+        if (i < a.n_src) {
+          search = true;
+          if (it > 0 && a.anchor) {
+            const float4 was = a.anchor[i], p = xform_exact(T, a.src[i]);
+            pos = a.last[i];
+            float reach = r;
+            if (pos >= 0) {
+              const float d2 = dist2_exact(p, g.pts[pos]);
+              reach = d2 <= a.r2max ? sqrt_up(d2) : __int_as_float(0x7f800000);
+            }
+            search = !(reach + margin < was.w - sqrt_up(dist2_exact(p, was)));
+          }
         }
-        ++cnt;
+        if (l < cn) s_pos[l] = pos;
+        const unsigned bal = __ballot_sync(0xffffffffu, search);
+        int base = 0;
+        if (lane == 0 && bal) base = atomicAdd(&s_qn, __popc(bal));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (search) s_queue[base + __popc(bal & lanemask_lt())] = (unsigned short)l;
       }
-      if (a.trace_corr && lg == 0)
-        a.trace_corr[(size_t)it * (size_t)a.n_src + (size_t)(a.src_idx ? a.src_idx[i] : (int)i)] = j;
+      __syncthreads();
+      // 2. the searches.  A box is widened by what the point moved since its
+      // last search, up to half the neighbour's distance (its next nearest
+      // is about that much farther) or a fraction of the bound.
+      const int qn = s_qn;
+      for (int k = tid / G; k < qn; k += ICP_THREADS / G) {
+        const int l = s_queue[k], i = point_of(c0 + l), was = s_pos[l];
+        const float4 p = xform_exact(T, a.src[i]);
+        float extra = 0.f, room;
+        if (it > 0 && a.anchor) {
+          const float m = 4.f * sqrt_up(dist2_exact(p, a.anchor[i]));
+          if (was >= 0)
+            extra = fminf(m, fmaxf(0.5f * fminf(sqrt_up(dist2_exact(p, g.pts[was])), r), 0.1f * g.h));
+          else
+            extra = m < 0.4f * r ? fminf(m, 0.3f * r) : 0.f;
+        }
+        const int pos = grid_nn1_from<G>(bv, p, a.r2max, r, was, extra, lg, gmask, &room);
+        if (lg == 0) {
+          s_pos[l] = pos;
+          if (a.anchor) {
+            a.anchor[i] = make_float4(p.x, p.y, p.z, room);
+            a.last[i] = pos;
+          }
+        }
+      }
+      __syncthreads();
+      // 3. the sums: dp 0-2, dq 3-5, dp dq^T 6-14, d^2 15
+      KSum acc[ICP_NV];
+#pragma unroll
+      for (int k = 0; k < ICP_NV; ++k) acc[k].init();
+      int cnt = 0;
+      for (int l = tid; l < cn; l += ICP_THREADS) {
+        const int i = point_of(c0 + l), pos = s_pos[l];
+        if (i >= a.n_src) continue;
+        if (pos >= 0) {
+          const float4 p = xform_exact(T, a.src[i]), q = g.pts[pos];
+          const float dp[3] = {__fsub_rn(p.x, cp.x), __fsub_rn(p.y, cp.y), __fsub_rn(p.z, cp.z)};
+          const float dq[3] = {__fsub_rn(q.x, c[0]), __fsub_rn(q.y, c[1]), __fsub_rn(q.z, c[2])};
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            acc[k].add(dp[k]);
+            acc[3 + k].add(dq[k]);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) acc[6 + 3 * k + m].add(__fmul_rn(dp[k], dq[m]));
+          }
+          acc[15].add(dist2_exact(p, q));
+          ++cnt;
+        }
+        if (a.trace_corr)
+          a.trace_corr[(size_t)it * (size_t)a.n_src + (size_t)(a.src_idx ? a.src_idx[i] : i)] =
+              pos >= 0 ? pt_index(g.pts[pos]) : -1;
+      }
+      // compensated sums over the warp, halving the values a lane
+      // holds with each exchange (lane bit 4 keeps values 0-7 or 8-15, ...), so
+      // 16 combinations a lane instead of 80; lane l ends with value l / 2
+      {
+        float s[ICP_NV], e[ICP_NV];
+#pragma unroll
+        for (int k = 0; k < ICP_NV; ++k) {
+          s[k] = acc[k].s;
+          e[k] = acc[k].c;
+        }
+#pragma unroll
+        for (int off = 16, nv = ICP_NV / 2; off >= 2; off >>= 1, nv >>= 1) {
+          const bool up = (lane & off) != 0;
+#pragma unroll
+          for (int k = 0; k < nv; ++k) {
+            const float ks = up ? s[k + nv] : s[k], ke = up ? e[k + nv] : e[k];
+            const float os = __shfl_xor_sync(0xffffffffu, up ? s[k] : s[k + nv], off);
+            const float oe = __shfl_xor_sync(0xffffffffu, up ? e[k] : e[k + nv], off);
+            float t, err;
+            two_sum(ks, os, t, err);
+            s[k] = t;
+            e[k] = __fadd_rn(__fadd_rn(ke, oe), err);
+          }
+        }
+        const float os = __shfl_xor_sync(0xffffffffu, s[0], 1), oe = __shfl_xor_sync(0xffffffffu, e[0], 1);
+        float t, err;
+        two_sum(s[0], os, t, err);
+        if ((lane & 1) == 0) {
+          s_red[warp][lane >> 1][0] = t;
+          s_red[warp][lane >> 1][1] = __fadd_rn(__fadd_rn(e[0], oe), err);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+      if (lane == 0) s_cnt[warp] = cnt;
+      __syncthreads();
+      if (tid < ICP_NV) {
+        for (int w = 0; w < ICP_WARPS; ++w) {
+          float t, e;
+          two_sum(run_s, s_red[w][tid][0], t, e);
+          run_s = t;
+          run_c = __fadd_rn(__fadd_rn(run_c, s_red[w][tid][1]), e);
+        }
+      }
+      if (tid == 0)
+        for (int w = 0; w < ICP_WARPS; ++w) run_n += s_cnt[w];
     }
-    // block partial: compensated sums over the warp's groups (offsets >= G,
-    // the same tree a single lane per group would meet), then across warps
-#pragma unroll
-    for (int k = 0; k < NVL; ++k) {
-      float s = acc[k].s, cc = acc[k].c;
-#pragma unroll
-      for (int off = 16; off >= G; off >>= 1) {
-        const float s2 = __shfl_down_sync(0xffffffffu, s, off);
-        const float c2 = __shfl_down_sync(0xffffffffu, cc, off);
-        float t, e;
-        two_sum(s, s2, t, e);
-        s = t;
-        cc = __fadd_rn(__fadd_rn(cc, c2), e);
-      }
-      if (lane < G) {
-        s_red[warp][lane * NVL + k][0] = s;
-        s_red[warp][lane * NVL + k][1] = cc;
-      }
-    }
-    cnt = lg == 0 ? cnt : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if (lane == 0) s_cnt[warp] = cnt;
-    __syncthreads();
     if (tid < ICP_NV) {
-      float s = s_red[0][tid][0], cc = s_red[0][tid][1];
-      for (int w = 1; w < ICP_WARPS; ++w) {
-        float t, e;
-        two_sum(s, s_red[w][tid][0], t, e);
-        s = t;
-        cc = __fadd_rn(__fadd_rn(cc, s_red[w][tid][1]), e);
-      }
-      a.partial[lb * 32 + tid] = s;
-      a.partial[lb * 32 + 16 + tid] = cc;
+      a.partial[lb * 32 + tid] = run_s;
+      a.partial[lb * 32 + ICP_NV + tid] = run_c;
     }
-    if (tid == 0) {
-      int tot = 0;
-      for (int w = 0; w < ICP_WARPS; ++w) tot += s_cnt[w];
-      a.pcount[lb] = tot;
-    }
+    if (tid == 0) a.pcount[lb] = run_n;
     __syncthreads();
     if (tid == 0) {
       if (prof0) {
         t_arr = icp_timer();
         atomicAdd(a.prof + 0, t_arr - t_it);
       }
-      __threadfence();
-      const unsigned t = atomicAdd(a.arrive, 1u);
+      const unsigned t = icp_arrive(a.arrive);
       s_last = (t == (unsigned)(it + 1) * (unsigned)B - 1u) ? 1 : 0;
+      if (s_last) __threadfence();
     }
     __syncthreads();
     if (s_last) {
       const unsigned long long t_s0 = a.prof && tid == 0 ? icp_timer() : 0ull;
-      __threadfence();
-      // current pose (FP64) fetched early, used after the solve
-      if (tid < 16) {
-        const double pk = it == 0 ? a.init[tid] : __ldcg(a.pose64 + tid);
-        s_P[tid] = pk;
-        if (it == 0 && a.trace_pose) a.trace_pose[tid] = pk;
-      }
+      // warp 0 lane k: entry k of the current pose (FP64), fetched early
+      const double pk = warp != 0 || lane > 15 ? 0.0 : (it == 0 ? a.init[lane] : __ldcg(a.pose64 + lane));
       // Cross-block reduction.  GB300 issues one FP64 warp-instruction per ~16
       // SM cycles, so the tree runs on compensated FP32 pairs (TwoSum, ~48-bit
       // significand) and FP64 closes it: one (double)hi + (double)lo per value.
-      // Warp w reduces values 2w and 2w + 1 (lanes stride over the blocks in
-      // a fixed order), so no thread holds all sixteen pairs.
-      static_assert(ICP_WARPS * 2 == ICP_NV, "two values per warp");
+      // Thread (k, v) adds value v of blocks k, k + 16, ... (in that order, ten
+      // blocks' loads in flight, whole lines), then k is reduced away.
       {
-        float hs0 = 0.f, ls0 = 0.f, hs1 = 0.f, ls1 = 0.f;
+        constexpr int KG = ICP_THREADS / ICP_NV;
+        const int v = tid & (ICP_NV - 1), kg = tid / ICP_NV;
+        float hs = 0.f, ls = 0.f;
         int nloc = 0;
-        const int v0 = 2 * warp;
-        for (int b = lane; b < B; b += 32) {
-          const float2 h = __ldcg(reinterpret_cast<const float2*>(a.partial + b * 32 + v0));
-          const float2 l = __ldcg(reinterpret_cast<const float2*>(a.partial + b * 32 + 16 + v0));
-          if (warp == 0) nloc += __ldcg(a.pcount + b);
-          float t, e;
-          two_sum(hs0, h.x, t, e);
-          hs0 = t;
-          ls0 = __fadd_rn(__fadd_rn(ls0, l.x), e);
-          two_sum(hs1, h.y, t, e);
-          hs1 = t;
-          ls1 = __fadd_rn(__fadd_rn(ls1, l.y), e);
-        }
-        warp_ksum(hs0, ls0);
-        warp_ksum(hs1, ls1);
+        for (int b0 = kg; b0 < B; b0 += 10 * KG) {
+          float h[10], l[10];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nloc += __shfl_down_sync(0xffffffffu, nloc, o);
-        if (lane == 0) {
-          s_sum[v0] = (double)hs0 + (double)ls0;
-          s_sum[v0 + 1] = (double)hs1 + (double)ls1;
-          if (warp == 0) s_n = nloc;
+          for (int u = 0; u < 10; ++u) {
+            const int b = b0 + KG * u;
+            h[u] = b < B ? __ldcg(a.partial + b * 32 + v) : 0.f;
+            l[u] = b < B ? __ldcg(a.partial + b * 32 + ICP_NV + v) : 0.f;
+            if (v == 0 && b < B) nloc += __ldcg(a.pcount + b);
+          }
+#pragma unroll
+          for (int u = 0; u < 10; ++u) {
+            float t, e;
+            two_sum(hs, h[u], t, e);
+            hs = t;
+            ls = __fadd_rn(__fadd_rn(ls, l[u]), e);
+          }
         }
+        {
+          const float os = __shfl_xor_sync(0xffffffffu, hs, 16), ol = __shfl_xor_sync(0xffffffffu, ls, 16);
+          float t, e;
+          two_sum(hs, os, t, e);
+          hs = t;
+          ls = __fadd_rn(__fadd_rn(ls, ol), e);
+        }
+        nloc += __shfl_xor_sync(0xffffffffu, nloc, 16);
+        if (lane < ICP_NV) {
+          s_red[warp][lane][0] = hs;
+          s_red[warp][lane][1] = ls;
+        }
+        if (lane == 0) s_cnt[warp] = nloc;
       }
       __syncthreads();
+      if (warp == 0) {
+        float hs = s_red[0][lane & (ICP_NV - 1)][0], ls = s_red[0][lane & (ICP_NV - 1)][1];
+        for (int w = 1; w < ICP_WARPS; ++w) {
+          float t, e;
+          two_sum(hs, s_red[w][lane & (ICP_NV - 1)][0], t, e);
+          hs = t;
+          ls = __fadd_rn(__fadd_rn(ls, s_red[w][lane & (ICP_NV - 1)][1]), e);
+        }
+        if (lane < ICP_NV) s_sum[lane] = (double)hs + (double)ls;
+        __syncwarp();
+      }
       if (a.prof && tid == 0) atomicAdd(a.prof + 4, icp_timer() - t_s0);
-      // centred cross-covariance, one element per lane
-      if (tid < 9 && s_n >= 3) {
-        const double inv = 1.0 / (double)s_n;
-        const int r = tid / 3, k = tid % 3;
-        s_H[tid] = s_sum[6 + tid] - (double)s_n * (s_sum[r] * inv) * (s_sum[3 + k] * inv);
-      }
-      __syncthreads();
-      if (warp == 0) {  // the pose solve: warp 0, FP64 products spread over its lanes
-        const long long n = s_n;
-        int stop = 0, converged = 1;
-        double fitness = 0.0;
-        double D[12] = {1.0, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0};
+      if (warp == 0) {
+        // the pose solve and the new pose, on warp 0 without a block barrier:
+        // 3-vectors, 3x3 and 4x4 matrices are spread over the lanes (FP64 is
+        // charged per warp instruction) and operands come by shuffle
+        const unsigned full = 0xffffffffu;
+        int n = 0;
+#pragma unroll
+        for (int w = 0; w < ICP_WARPS; ++w) n += s_cnt[w];
+        int stop = it + 1 >= a.max_it ? 1 : 0, converged = 1;
+        double fitness = 0.0, np = pk;
+        if (it == 0 && a.trace_pose && lane < 16) a.trace_pose[lane] = pk;
         if (n < 3) {
           stop = 1;
           converged = 0;
         } else {
-          const double inv = 1.0 / (double)n;
-          double mdp[3], mdq[3], H[9], R[9];
-          for (int k = 0; k < 3; ++k) {
-            mdp[k] = s_sum[k] * inv;
-            mdq[k] = s_sum[3 + k] * inv;
-          }
+          // 1 / n: the FP32 reciprocal and two Newton steps
+          const double dn = (double)n;
+          double inv = (double)__frcp_rn((float)n);
+          inv = fma(inv, fma(-dn, inv, 1.0), inv);
+          inv = fma(inv, fma(-dn, inv, 1.0), inv);
+          // centred cross-covariance, entry e in lane e; the rotation likewise
+          const int e = lane < 9 ? lane : 8;
+          const double r = umeyama_rotation_warp(fma(-(s_sum[e / 3] * inv), s_sum[3 + e % 3], s_sum[6 + e]));
+          // lanes 0-2: source mean, 3-5: target mean; then lane i: t_i
+          const int v = lane < 6 ? lane : 5;
+          const float off = v == 0 ? cp.x : (v == 1 ? cp.y : (v == 2 ? cp.z : (v == 3 ? c[0] : (v == 4 ? c[1] : c[2]))));
+          const double mean = fma(s_sum[v], inv, (double)off);
+          const int i3 = lane < 3 ? lane : 2;
+          double t = __shfl_sync(full, mean, 3 + i3);
 #pragma unroll
-          for (int k = 0; k < 9; ++k) H[k] = s_H[k];
-          umeyama_rotation_warp(H, R);
-          double mp[3], mq[3], t[3];
-          for (int k = 0; k < 3; ++k) {
-            mp[k] = mdp[k] + (double)(k == 0 ? cp.x : (k == 1 ? cp.y : cp.z));
-            mq[k] = mdq[k] + (double)c[k];
-          }
-          for (int r = 0; r < 3; ++r) t[r] = mq[r] - (R[r * 3 + 0] * mp[0] + R[r * 3 + 1] * mp[1] + R[r * 3 + 2] * mp[2]);
+          for (int k = 0; k < 3; ++k)
+            t = fma(-__shfl_sync(full, r, 3 * i3 + k), __shfl_sync(full, mean, k), t);
+          // pose <- [r t] pose, entry (lane / 4, lane % 4) in lanes 0-11; its last row stays
+          const int ar = lane < 12 ? lane >> 2 : 2, bc = lane & 3;
+          double acc = __shfl_sync(full, t, ar) * __shfl_sync(full, pk, 12 + bc);
 #pragma unroll
-          for (int r = 0; r < 3; ++r) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) D[r * 4 + k] = R[r * 3 + k];
-            D[r * 4 + 3] = t[r];
-          }
+          for (int k = 0; k < 3; ++k)
+            acc = fma(__shfl_sync(full, r, 3 * ar + k), __shfl_sync(full, pk, 4 * k + bc), acc);
+          if (lane < 12) np = acc;
           fitness = s_sum[15] * inv;
-          const double cosang = 0.5 * (R[0] + R[4] + R[8] - 1.0);
-          const double tsq = t[0] * t[0] + t[1] * t[1] + t[2] * t[2];
-          if (a.eps_t > 0.0 && tsq < a.eps_t && (a.eps_r <= 0.0 || cosang > a.eps_r)) stop = 1;
+          if (a.eps_t > 0.0) {
+            const double t0 = __shfl_sync(full, t, 0), t1 = __shfl_sync(full, t, 1), t2 = __shfl_sync(full, t, 2);
+            const double tr = __shfl_sync(full, r, 0) + __shfl_sync(full, r, 4) + __shfl_sync(full, r, 8);
+            if (t0 * t0 + t1 * t1 + t2 * t2 < a.eps_t && (a.eps_r <= 0.0 || 0.5 * (tr - 1.0) > a.eps_r)) stop = 1;
+          }
         }
-        if (it + 1 >= a.max_it) stop = 1;
+        if (lane < 16) {
+          a.pose64[lane] = np;
+          if (lane < 12) {
+            const float f = __double2float_rn(np);
+            s_T[lane] = f;
+            st_relaxed(a.posew + lane, ((unsigned long long)((unsigned)(it + 1) | (stop ? 0x80000000u : 0u)) << 32) |
+                                           __float_as_uint(f));
+          }
+          if (a.trace_pose) a.trace_pose[(size_t)(it + 1) * 16 + lane] = np;
+          a.result->pose[lane] = np;
+        }
         if (lane == 0) {
-#pragma unroll
-          for (int k = 0; k < 16; ++k) s_D[k] = k < 12 ? D[k] : (k == 15 ? 1.0 : 0.0);
           a.result->fitness = fitness;
           a.result->iterations = it + 1;
           a.result->converged = converged;
-          a.result->n_corr = (int)n;
+          a.result->n_corr = n;
           a.result->status = RTR_OK;
           s_stop = stop;
           if (a.prof) atomicAdd(a.prof + 5, icp_timer() - t_s0);
         }
-      }
-      __syncthreads();
-      // pose <- dT * pose, one element per thread
-      if (tid < 16) {
-        const int r = tid >> 2, cidx = tid & 3;
-        const double pk = s_D[r * 4 + 0] * s_P[0 * 4 + cidx] + s_D[r * 4 + 1] * s_P[1 * 4 + cidx] +
-                          s_D[r * 4 + 2] * s_P[2 * 4 + cidx] + s_D[r * 4 + 3] * s_P[3 * 4 + cidx];
-        a.pose64[tid] = pk;
-        if (tid < 12) a.posef[tid] = __double2float_rn(pk);
-        if (a.trace_pose) a.trace_pose[(size_t)(it + 1) * 16 + tid] = pk;
-        a.result->pose[tid] = pk;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        __threadfence();
-        st_release_gpu(a.gen, (unsigned)(it + 1) | (s_stop ? 0x80000000u : 0u));
-        if (a.prof) {
+        if (lane == 0 && a.prof) {
           atomicAdd(a.prof + 1, icp_timer() - t_s0);
           atomicAdd(a.prof + 3, 1ull);
         }
       }
       __syncthreads();
     } else {
-      if (tid == 0) {
+      if (tid < 32) {
         const long long t0 = clock64();
-        unsigned gv;
+        unsigned long long w = 0;
+        bool here = lane >= 12, late = false;
         for (;;) {
-          gv = ld_acquire_gpu(a.gen);
-          if ((gv & 0x7fffffffu) >= (unsigned)(it + 1)) break;
-          if (clock64() - t0 > a.budget) {
+          if (!here) {
+            w = ld_relaxed(a.posew + lane);
+            here = (unsigned)((w >> 32) & 0x7fffffffu) >= (unsigned)(it + 1);
+          }
+          if (__all_sync(0xffffffffu, here)) break;
+          late = __any_sync(0xffffffffu, clock64() - t0 > a.budget);
+          if (late) break;
+          __nanosleep(32);
+        }
+        if (late) {
+          if (lane == 0) {
             atomicExch(a.status, (int)RTR_ERR_TIMEOUT);
             a.result->status = RTR_ERR_TIMEOUT;
             a.result->converged = 0;
-            gv = 0x80000000u;
-            break;
+            s_stop = 1;
           }
-          __nanosleep(64);
+        } else {
+          if (lane < 12) s_T[lane] = __uint_as_float((unsigned)w);
+          if (lane == 0) s_stop = (int)(w >> 63);
         }
-        s_stop = (gv >> 31) ? 1 : 0;
         if (prof0) atomicAdd(a.prof + 2, icp_timer() - t_arr);
       }
       __syncthreads();
@@ -371,17 +498,18 @@ int icp_max_blocks(rtr_context* ctx) {
   return v;
 }
 
-// Lanes per source point: the tuning override when set, else the most lanes
-// (8, 4, 2) with which the launch needs at most four passes over its points
-// (measured on GB300: a 20k-point ICP on the ring search is fastest at 8, two
-// passes; sixteen 9.2k-point refinements on the 27-cell search at 2, 3.8
-// passes: 1.40 ms against 1.48 at 4 and 1.75 at 8).
+// Lanes per searched source point: the tuning override when set, else by the
+// points a block has to match.  Few points leave lanes idle and wait on the
+// latency of single searches: 8 lanes; many keep the block busy, and what
+// counts is instructions: 4, then 2.  Measured (8 / 4 / 2 lanes): two 20k
+// chairs, 66 points a block, 1332 / 1352 / 1871 us; 16 refinements of 9.2k
+// points, 484 a block, the room's recognition 4196 / 4074 / 4140 us; a batch of
+// 64 pairs, thousands a block, 32.8 / 31.2 / 31.2 ms.
 int icp_pick_group(const rtr_context* ctx, long long total_pts, int blocks) {
   const int t = ctx->tune_icp_group;
   if (t == 2 || t == 4 || t == 8) return t;
-  const long long lanes = (long long)blocks * ICP_THREADS;
-  if (total_pts * 8 <= 4 * lanes) return 8;
-  return total_pts * 4 <= 4 * lanes ? 4 : 2;
+  const long long per_block = total_pts / (blocks > 0 ? blocks : 1);
+  return per_block <= 128 ? 8 : (per_block <= 1024 ? 4 : 2);
 }
 
 static rtr_status launch_icp(int G, const IcpDev* d_probs, const int* d_blk2prob, int blocks, cudaStream_t st) {
@@ -427,18 +555,20 @@ __global__ void k_icp_setup(IcpSetup s, IcpDev* __restrict__ probs, int* __restr
       for (int i = 0; i < 16; ++i) d.init[i] = s.init_dev[k][i];
     probs[pid] = d;
     d.arrive[0] = 0u;
-    d.gen[0] = 0u;
+    for (int i = 0; i < 12; ++i) d.posew[i] = 0ull;
   }
 }
 
-void icp_multi_plan(ScratchPlan& p, int n_probs, int max_blocks) {
+void icp_multi_plan(ScratchPlan& p, int n_probs, int max_blocks, size_t n_state) {
   p.add<IcpDev>(n_probs);
   p.add<int>(max_blocks);
   p.add<double>((size_t)n_probs * 16);
-  p.add<float>((size_t)n_probs * 16);
+  p.add<unsigned long long>((size_t)n_probs * 16);
   p.add<float>((size_t)max_blocks * 32);
   p.add<int>(max_blocks);
-  p.add<unsigned>((size_t)n_probs * 2);
+  p.add<unsigned>(n_probs);
+  p.add<float4>(n_state);
+  p.add<int>(n_state);
 }
 
 rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, cudaStream_t st) {
@@ -452,11 +582,19 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
   IcpDev* d_probs = s.take<IcpDev>(M);
   int* d_b2p = s.take<int>(maxb);
   double* pose64 = s.take<double>((size_t)M * 16);
-  float* posef = s.take<float>((size_t)M * 16);
+  unsigned long long* posew = s.take<unsigned long long>((size_t)M * 16);
   float* partial = s.take<float>((size_t)maxb * 32);
   int* pcount = s.take<int>(maxb);
-  unsigned* sync = s.take<unsigned>((size_t)M * 2);
+  unsigned* sync = s.take<unsigned>(M);
   if (!sync) return fail(RTR_ERR_CAPACITY, "icp: scratch carve");
+  // the matching state, when the scratch at hand holds it (the plans of the
+  // single-cloud entry points include it; a recognition's stages leave far
+  // more): without it every point is searched in every iteration
+  size_t n_state = 0;
+  for (int i = 0; i < M; ++i) n_state += (size_t)specs[i].dev.n_src;
+  float4* anchor = s.take<float4>(n_state);
+  int* last = s.take<int>(n_state);
+  if (!last) anchor = nullptr;
   // apportion blocks: want_i = ceil(n_i * G / threads), scaled to fit
   long long want_total = 0;
   std::vector<long long> want(M);
@@ -478,11 +616,16 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
     d.blk0 = blk;
     d.nblk = nblk[i];
     d.pose64 = pose64 + 16 * i;
-    d.posef = posef + 16 * i;
+    d.posew = posew + 16 * i;
     d.partial = partial + (size_t)blk * 32;
     d.pcount = pcount + blk;
-    d.arrive = sync + 2 * i;
-    d.gen = sync + 2 * i + 1;
+    d.arrive = sync + i;
+    d.anchor = anchor;
+    d.last = last;
+    if (anchor) {
+      anchor += d.n_src;
+      last += d.n_src;
+    }
     d.status = ctx->d_status;
     d.budget = ctx->wait_budget_cycles;
     d.prof = i == 0 ? reinterpret_cast<unsigned long long*>(ctx->d_status + 32) : nullptr;
@@ -548,7 +691,7 @@ rtr_status rtr_icp(rtr_context* ctx, const float* d_src, int n_src, const float*
   for (int i = 0; i < 4; ++i) plan.add<uint32_t>(n_src);
   plan.add<uint32_t>(radix_hist_entries(n_src));
   plan.add<GridMeta>(1);
-  icp_multi_plan(plan, 1, maxb);
+  icp_multi_plan(plan, 1, maxb, n_src);
   Scratch s;
   RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
   GridBufs gb;
@@ -567,14 +710,14 @@ rtr_status rtr_icp(rtr_context* ctx, const float* d_src, int n_src, const float*
   if (!(h > 0.f)) h = params->max_corr_dist > 0.f ? 0.5f * params->max_corr_dist : -1.f;
   {
     ProfScope ps(ctx, st, "grid_build");
-    grid_build(gb, reinterpret_cast<const float4*>(d_tgt), n_tgt, nullptr, h, st);
+    RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_tgt), n_tgt, nullptr, h, st));
   }
 
   IcpDev a;
   memset(&a, 0, sizeof(a));
   a.grid = grid_dev(gb);
   a.src_meta = src_meta;
-  bbox_build(src_meta, reinterpret_cast<const float4*>(d_src), n_src, st);
+  RTR_TRY(bbox_build(src_meta, reinterpret_cast<const float4*>(d_src), n_src, st));
   a.src = src_sorted;
   a.src_idx = src_idx;
   a.n_src = n_src;
@@ -624,7 +767,7 @@ rtr_status rtr_icp_multi(rtr_context* ctx, const float* d_src, int n_src, const 
   ScratchPlan plan;
   grid_plan(plan, n_tgt, cell_cap);
   plan.add<GridMeta>(1);
-  icp_multi_plan(plan, n_problems, maxb);
+  icp_multi_plan(plan, n_problems, maxb, (size_t)n_problems * n_src);
   Scratch s;
   RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
   GridBufs gb;
@@ -634,8 +777,8 @@ rtr_status rtr_icp_multi(rtr_context* ctx, const float* d_src, int n_src, const 
   float h = params->cell_size;
   if (!(h > 0.f)) h = params->max_corr_dist > 0.f ? 0.5f * params->max_corr_dist : -1.f;
   ProfScope ps(ctx, st, "icp_multi");
-  grid_build(gb, reinterpret_cast<const float4*>(d_tgt), n_tgt, nullptr, h, st);
-  bbox_build(src_meta, reinterpret_cast<const float4*>(d_src), n_src, st);
+  RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_tgt), n_tgt, nullptr, h, st));
+  RTR_TRY(bbox_build(src_meta, reinterpret_cast<const float4*>(d_src), n_src, st));
   std::vector<IcpSpec> specs((size_t)n_problems);
   const float r = params->max_corr_dist;
   for (int k = 0; k < n_problems; ++k) {

@@ -12,16 +12,17 @@ struct IcpDev {
   const float4* src;          // source points (any order; sorted by target cell is faster)
   const int* src_idx;         // original index of each source point (NULL: identity)
   int n_src;
+  float4* anchor;             // [n_src] where the point was last searched from, w = its room there; or NULL
+  int* last;                  // [n_src] sorted position of its neighbour then, or -1
   int max_it;
   float r2max;
   double eps_t, eps_r;
   double init[16];
   double* pose64;             // [16]
-  float* posef;               // [12]
-  float* partial;             // [nblk][32]
+  unsigned long long* posew;  // [12] the FP32 pose: value, iteration << 32, bit 63 = last
+  float* partial;             // [nblk][32]: a block's sums, 16 high parts, then the low ones
   int* pcount;                // [nblk]
   unsigned* arrive;
-  unsigned* gen;
   rtr_icp_result* result;
   double* trace_pose;
   int* trace_corr;
@@ -44,7 +45,8 @@ struct IcpSpec {
 
 int icp_max_blocks(rtr_context* ctx);
 int icp_pick_group(const rtr_context* ctx, long long total_pts, int blocks);
-void icp_multi_plan(ScratchPlan& p, int n_probs, int max_blocks);
+// n_state: source points over all problems (0: no room planned for their matching state)
+void icp_multi_plan(ScratchPlan& p, int n_probs, int max_blocks, size_t n_state);
 // Runs every problem; specs are completed (blocks, state buffers) in place.
 rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, cudaStream_t st);
 

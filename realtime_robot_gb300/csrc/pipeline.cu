@@ -157,8 +157,7 @@ __global__ void __launch_bounds__(256, 4) k_hv_count(GridDev gd, const float4* _
   const int h = blockIdx.x / bph, part = blockIdx.x - h * bph;
   if (d_nhyp) n_hyp = min(*d_nhyp, n_hyp);
   if (h >= n_hyp) return;
-  const GridView g = load_view(gd);
-  const bool near27 = grid_near27_ok(g, r2);  // every inlier within the 27 cells around a point
+  const BoxView g = box_view(gd);
   float T[12];
 #pragma unroll
   for (int k = 0; k < 12; ++k) T[k] = __double2float_rn(poses[(size_t)h * 16 + k]);
@@ -171,15 +170,7 @@ __global__ void __launch_bounds__(256, 4) k_hv_count(GridDev gd, const float4* _
   const int i1 = min(total, (part + 1) * HV_PPB);
   for (int i = part * HV_PPB + threadIdx.x / HV_G; i < i1; i += blockDim.x / HV_G) {
     const float4 p = xform_exact(T, model[(size_t)i * stride]);
-    bool in;
-    if (near27) {
-      in = grid_any_near<HV_G>(g, p, r2, lg, gmask);
-    } else {
-      float d2;
-      int bi, bp;
-      grid_nn1_group<HV_G, true>(g, p, r2, lg, gmask, d2, bi, bp);
-      in = bi >= 0;
-    }
+    const bool in = grid_any_within<HV_G>(g, p, r2, lg, gmask);
     if (lg == 0 && in) ++cnt;
   }
 #pragma unroll
@@ -427,7 +418,8 @@ rtr_status rtr_model_create(rtr_context* ctx, const float* d_pts, int n, const r
   r = shot_dev(ctx, sd, m->vox, m->nrm, V, nullptr, m->keys, K, nullptr, prm->descriptor_r, m->desc, nullptr, st);
   if (r != RTR_OK) return cleanup(r);
   k_gather_kp<<<nblocks(K), 256, 0, st>>>(m->vox, m->keys, d_cnt + 1, K, m->kp);
-  bbox_build(m->vox_meta, m->vox, V, st);
+  r = bbox_build(m->vox_meta, m->vox, V, st);
+  if (r != RTR_OK) return cleanup(r);
   RTR_LAUNCHED(1);
   if (cudaMalloc(&m->db_hi, match_tc_bf16_bytes(K)) != cudaSuccess ||
       cudaMalloc(&m->db_lo, match_tc_bf16_bytes(K)) != cudaSuccess ||
@@ -639,7 +631,7 @@ static size_t stage_bytes(int n, const rtr_recog_params* q, bool learned) {
   stage = gc_scratch_bytes(n, q->max_clusters) > stage ? gc_scratch_bytes(n, q->max_clusters) : stage;
   {
     ScratchPlan t;
-    icp_multi_plan(t, q->refine_top, 152 * 16);
+    icp_multi_plan(t, q->refine_top, 152 * 16, 0);
     stage = t.bytes > stage ? t.bytes : stage;
   }
   {
@@ -686,14 +678,14 @@ static rtr_status scene_stages(rtr_context* ctx, const Scratch& stage, SceneBufs
   }
   {
     ProfScope ps(ctx, ax, "shot_grid");
-    grid_build(b.shot_grid, b.sv, n, dV, q->descriptor_r, ax);
+    RTR_TRY(grid_build(b.shot_grid, b.sv, n, dV, q->descriptor_r, ax));
   }
   RTR_CUDA(cudaEventRecord(ctx->ev_side[1], ax));
   {
     ProfScope ps(ctx, ax, "scene_grid");
     // 1.5 x the ICP distance measured fastest for refinement and verification
     const float cell = ctx->tune_scene_grid_mm > 0 ? 1e-3f * (float)ctx->tune_scene_grid_mm : 1.5f * q->icp_max_dist;
-    grid_build(b.grid, b.sv, n, dV, cell, ax);
+    RTR_TRY(grid_build(b.grid, b.sv, n, dV, cell, ax));
   }
   RTR_CUDA(cudaEventRecord(ctx->ev_side[2], ax));
   {
@@ -1104,7 +1096,7 @@ rtr_status rtr_pose_inliers(rtr_context* ctx, const float* d_model, int n_model,
   if (!score) return fail(RTR_ERR_CAPACITY, "rtr_pose_inliers: scratch");
   ProfScope ps(ctx, st, "pose_inliers");
   // a cell 1.5 x the radius: the counts take the 27-cell existence search
-  grid_build(gb, reinterpret_cast<const float4*>(d_scene), n_scene, nullptr, 1.5f * radius, st);
+  RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_scene), n_scene, nullptr, 1.5f * radius, st));
   RTR_TRY(hv_score(grid_dev(gb), reinterpret_cast<const float4*>(d_model), n_model, 1, d_poses, n_poses, nullptr,
                    radius * radius, d_counts, score, st));
   RTR_CUDA(cudaGetLastError());

@@ -442,37 +442,28 @@ __device__ __forceinline__ void shot_bins(float pos, int nb, bool circular, int&
 
 #define SHOT_FOR_SUPPORT(...)                                                                     \
   for (int z = max(cz - 1, 0); z <= min(cz + 1, g.nz - 1); ++z)                                  \
-    for (int y = max(cy - 1, 0); y <= min(cy + 1, g.ny - 1); ++y)                                \
-      for (int x = max(cx - 1, 0); x <= min(cx + 1, g.nx - 1); ++x) {                            \
-        const uint2 c_ = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x]; \
-        for (unsigned j_ = c_.x + (unsigned)lane; j_ < c_.y; j_ += 32) {                         \
-          const float4 q = g.pts[j_];                                                            \
-          const int qi = pt_index(q);                                                            \
-          const float d2 = dist2_exact(kp, q);                                                   \
-          if (!(d2 <= R2)) continue;                                                             \
-          const float4 qn = nrm[qi];                                                             \
-          const float facing = dot3_exact(qn.x, qn.y, qn.z, nk.x, nk.y, nk.z);                   \
-          if (!(facing >= SHOT_FACING)) continue;                                                \
-          const float dx = __fsub_rn(q.x, kp.x), dy = __fsub_rn(q.y, kp.y), dz = __fsub_rn(q.z, kp.z); \
-          __VA_ARGS__                                                                             \
-        }                                                                                        \
-      }
+    for (int y = max(cy - 1, 0); y <= min(cy + 1, g.ny - 1); ++y) {                              \
+      const uint2 c_ = row_span(g, max(cx - 1, 0), min(cx + 1, g.nx - 1), y, z);                 \
+      for (unsigned j_ = c_.x + (unsigned)lane; j_ < c_.y; j_ += 32) {                           \
+        const float4 q = g.pts[j_];                                                              \
+        const int qi = pt_index(q);                                                              \
+        const float d2 = dist2_exact(kp, q);                                                     \
+        if (!(d2 <= R2)) continue;                                                               \
+        const float4 qn = nrm[qi];                                                               \
+        const float facing = dot3_exact(qn.x, qn.y, qn.z, nk.x, nk.y, nk.z);                     \
+        if (!(facing >= SHOT_FACING)) continue;                                                  \
+        const float dx = __fsub_rn(q.x, kp.x), dy = __fsub_rn(q.y, kp.y), dz = __fsub_rn(q.z, kp.z); \
+        __VA_ARGS__                                                                               \
+      }                                                                                          \
+    }
 
 // The support is gathered once, in pass 1, into a per-warp list in shared
 // memory (SHOT_CAP entries: the offset from the keypoint with its squared
-// length, and the normal); passes 2 and 3 read the list.  Cells whose box
-// lies beyond R are not walked.  A keypoint with more support points than
+// length, and the normal); passes 2 and 3 read the list.  A row of cells along
+// x is one run of points, cut to the cells within R.  A keypoint with more support points than
 // the list holds walks the cells again in passes 2 and 3 (the fixed-point
 // sums make the order irrelevant).
 constexpr int SHOT_CAP = 176;  // with the histograms: 56 KB a block, four blocks an SM
-
-__device__ __forceinline__ float shot_cell_d2(const GridView& g, float4 q, int x, int y, int z) {
-  const float lx = g.ox + (float)x * g.h, ly = g.oy + (float)y * g.h, lz = g.oz + (float)z * g.h;
-  const float dx = fmaxf(fmaxf(lx - q.x, q.x - (lx + g.h)), 0.f);
-  const float dy = fmaxf(fmaxf(ly - q.y, q.y - (ly + g.h)), 0.f);
-  const float dz = fmaxf(fmaxf(lz - q.z, q.z - (lz + g.h)), 0.f);
-  return dx * dx + dy * dy + dz * dz;
-}
 
 // One support point's contribution to the histogram (16 interpolated bins,
 // fixed-point votes, scale hs, added by shared-memory atomics).  (dx, dy,
@@ -526,7 +517,7 @@ __global__ void __launch_bounds__(SHOT_WARPS * 32, 4) k_shot(GridDev gd, const f
   const int nk_total = cnt_of(nk_host, d_nk);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const float R2 = __fmul_rn(R, R);
-  const float cell_r2 = R2 * 1.0001f + 1e-12f;  // a cell is walked when its box is within R (with a margin)
+  const float cell_r2 = R2 * 1.0001f + 1e-12f;  // cells within R are walked (with a margin)
   const int e_cov = 30 - shot_exp2_above(__fmul_rn(R2, R)), e_z = 30 - shot_exp2_above(R);
   const float cov_scale = pow2f(e_cov), cov_unscale = pow2f(-e_cov), z_scale = pow2f(e_z);
   unsigned* H = hist[wid];
@@ -543,10 +534,17 @@ __global__ void __launch_bounds__(SHOT_WARPS * 32, 4) k_shot(GridDev gd, const f
     long long m0 = 0, m1 = 0, m2 = 0, m3 = 0, m4 = 0, m5 = 0;
     int ns = 0;
     for (int z = max(cz - 1, 0); z <= min(cz + 1, g.nz - 1); ++z)
-      for (int y = max(cy - 1, 0); y <= min(cy + 1, g.ny - 1); ++y)
-        for (int x = max(cx - 1, 0); x <= min(cx + 1, g.nx - 1); ++x) {
-          if (shot_cell_d2(g, kp, x, y, z) > cell_r2) continue;
-          const uint2 c = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
+      for (int y = max(cy - 1, 0); y <= min(cy + 1, g.ny - 1); ++y) {
+          const float ly = g.oy + (float)y * g.h, lz = g.oz + (float)z * g.h;
+          const float ry = fmaxf(fmaxf(ly - kp.y, kp.y - (ly + g.h)), 0.f);
+          const float rz = fmaxf(fmaxf(lz - kp.z, kp.z - (lz + g.h)), 0.f);
+          const float rest = cell_r2 - (ry * ry + rz * rz);
+          if (rest < 0.f) continue;
+          const float rx = sqrtf(rest) * 1.0001f;
+          const int x0 = max(max(q_cell(kp.x - rx, g.ox, g.inv_h), cx - 1), 0);
+          const int x1 = min(min(q_cell(kp.x + rx, g.ox, g.inv_h), cx + 1), g.nx - 1);
+          if (x0 > x1) continue;
+          const uint2 c = row_span(g, x0, x1, y, z);
           for (unsigned j0 = c.x; j0 < c.y; j0 += 32) {
             const unsigned j = j0 + (unsigned)lane;
             bool in = false;
@@ -689,7 +687,7 @@ rtr_status normals_dev(rtr_context* ctx, Scratch& s, const float4* pts, int n_ca
   GridBufs gb;
   const unsigned cap = default_cell_cap(n_cap);
   if (!grid_take(s, n_cap, cap, &gb)) return fail(RTR_ERR_CAPACITY, "normals: scratch");
-  grid_build(gb, pts, n_cap, d_n, cell, st);
+  RTR_TRY(grid_build(gb, pts, n_cap, d_n, cell, st));
   const int nb = blocks_for(n_cap, 128);
   if (k <= 8)
     k_normals<8><<<nb, 128, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], out);
@@ -720,7 +718,7 @@ rtr_status shot_dev(rtr_context* ctx, Scratch& s, const float4* pts, const float
   GridBufs gb;
   const unsigned cap = default_cell_cap(n_cap);
   if (!grid_take(s, n_cap, cap, &gb)) return fail(RTR_ERR_CAPACITY, "shot: scratch");
-  grid_build(gb, pts, n_cap, d_n, R, st);
+  RTR_TRY(grid_build(gb, pts, n_cap, d_n, R, st));
   return shot_on_grid(gb, pts, nrm, keys, nk_cap, d_nk, R, desc, lrf, st);
 }
 

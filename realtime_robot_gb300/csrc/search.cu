@@ -1,4 +1,4 @@
-// search.cu — rtr_knn1 / rtr_knn entry points over the radix-sorted grid.
+// search.cu — rtr_knn1 / rtr_knn entry points over the uniform grid.
 #include <string.h>
 
 #include <mutex>
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128) k_knn(GridDev gd, const float4* __restric
 // least 1.01 x the reach, so the cube of cells around the query's reach
 // (widened by a rounding margin) spans at most 3 cells per axis: lane k
 // owns cells k and k + 32 of that cube.  A cell's points are stored in
-// ascending original index (the grid's sort is stable), so the warp merges
+// ascending original index (an ordered grid), so the warp merges
 // the cells' hit sequences by repeated minimum: the output comes out sorted
 // and a cut at max_per_query keeps the lowest indices.  A cube of more than
 // 64 cells (coordinates so large that the margin exceeds the cell's slack)
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) k_range(GridDev gd, const float4* __restr
     const int nc = (finite_q && ex > 0 && ey > 0 && ez > 0) ? ex * ey * ez : 0;
     auto cell_range = [&](int k) -> uint2 {
       const int x = x0 + k % ex, y = y0 + (k / ex) % ey, z = z0 + k / (ex * ey);
-      return g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
+      return cell_span(g, x, y, z);
     };
     // the true count
     int cnt = 0;
@@ -174,14 +174,14 @@ static rtr_status range_search(rtr_context* ctx, const char* who, bool box, cons
   RTR_CHECK_ARG(d_target != nullptr, "%s: NULL target", who);
   const unsigned cap = default_cell_cap(n_target);
   ScratchPlan plan;
-  grid_plan(plan, n_target, cap);
+  grid_plan(plan, n_target, cap, true);
   Scratch s;
   RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
   GridBufs gb;
-  if (!grid_take(s, n_target, cap, &gb)) return fail(RTR_ERR_CAPACITY, "%s: scratch", who);
+  if (!grid_take(s, n_target, cap, &gb, true)) return fail(RTR_ERR_CAPACITY, "%s: scratch", who);
   // cell edge 1.01 x the reach (the table's size limit may widen it)
   const float h = reach > 0.f ? 1.01f * reach : 1.0e-3f;
-  grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr, h, st);
+  RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr, h, st, true));
   const float4* q = reinterpret_cast<const float4*>(d_query);
   int nb = (n_query + 3) / 4;
   if (nb > 152 * 16) nb = 152 * 16;
@@ -251,8 +251,8 @@ rtr_status rtr_knn1(rtr_context* ctx, const float* d_query, int n_query, const f
   GridBufs gb;
   if (!grid_take(s, n_target, cap, &gb)) return fail(RTR_ERR_CAPACITY, "rtr_knn1: scratch");
   const bool bounded = max_dist > 0.f && max_dist < 1e18f;
-  grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr,
-             bounded ? 0.5f * max_dist : -1.f, st);
+  RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr,
+                     bounded ? 0.5f * max_dist : -1.f, st));
   ProfScope ps(ctx, st, "knn1");
   RTR_LAUNCHED(1);
   k_knn1<<<search_blocks(n_query * KNN1_G), 128, 0, st>>>(grid_dev(gb), reinterpret_cast<const float4*>(d_query),
@@ -317,8 +317,8 @@ rtr_status rtr_knn1_static(const float* d_query, int n_query, const float* d_tar
   GridBufs gb;
   if (!grid_take(s, n_target, cap, &gb)) return fail(RTR_ERR_CAPACITY, "rtr_knn1_static: scratch");
   const bool bounded = max_dist > 0.f && max_dist < 1e18f;
-  grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr,
-             bounded ? 0.5f * max_dist : -1.f, st);
+  RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr,
+                     bounded ? 0.5f * max_dist : -1.f, st));
   RTR_LAUNCHED(1);
   k_knn1<<<search_blocks(n_query * KNN1_G), 128, 0, st>>>(grid_dev(gb), reinterpret_cast<const float4*>(d_query),
                                                  n_query, bounded ? max_dist * max_dist : __builtin_inff(),
@@ -347,7 +347,7 @@ rtr_status rtr_knn(rtr_context* ctx, const float* d_query, int n_query, const fl
   RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
   GridBufs gb;
   if (!grid_take(s, n_target, cap, &gb)) return fail(RTR_ERR_CAPACITY, "rtr_knn: scratch");
-  grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr, -1.f, st);
+  RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_target), n_target, nullptr, -1.f, st));
   const float4* q = reinterpret_cast<const float4*>(d_query);
   const int nb = search_blocks(n_query);
   ProfScope ps(ctx, st, "knn");

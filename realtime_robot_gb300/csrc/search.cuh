@@ -21,7 +21,7 @@ struct GridView {
   float ox, oy, oz, h, inv_h;
   int nx, ny, nz;
   const float4* __restrict__ pts;
-  const uint2* __restrict__ cells;
+  const uint32_t* __restrict__ starts;
 };
 
 __device__ __forceinline__ GridView load_view(const GridDev& g) {
@@ -36,9 +36,16 @@ __device__ __forceinline__ GridView load_view(const GridDev& g) {
   v.ny = m->ny;
   v.nz = m->nz;
   v.pts = g.pts;
-  v.cells = g.cells;
+  v.starts = g.starts;
   return v;
 }
+
+// Points of cell (x, y, z), and of the run of cells x0 .. x1 of row (y, z).
+__device__ __forceinline__ uint2 row_span(const GridView& g, int x0, int x1, int y, int z) {
+  const unsigned r = ((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx;
+  return make_uint2(__ldg(g.starts + r + (unsigned)x0), __ldg(g.starts + r + (unsigned)x1 + 1u));
+}
+__device__ __forceinline__ uint2 cell_span(const GridView& g, int x, int y, int z) { return row_span(g, x, x, y, z); }
 
 __device__ __forceinline__ int pt_index(float4 p) { return __float_as_int(p.w); }
 
@@ -140,38 +147,6 @@ __device__ __forceinline__ void nn_take(float4 p, unsigned j, float4 q, float& b
   }
 }
 
-// Exact 1-NN with d^2 <= r2max (r2max = +inf: unbounded), one thread per
-// query.  Returns the original index (or -1) and the sorted position.
-__device__ __forceinline__ void grid_nn1(const GridView& g, float4 q, float r2max, float& bd, int& bi,
-                                         int& bpos) {
-  bd = r2max;
-  bi = INT_MAX;
-  bpos = -1;
-  const int cx = q_cell(q.x, g.ox, g.inv_h), cy = q_cell(q.y, g.oy, g.inv_h),
-            cz = q_cell(q.z, g.oz, g.inv_h);
-  // nothing of the grid within the bound: done before walking any ring
-  if (beyond(grid_box_dist(g, q), search_margin(g, q, 0), r2max)) {
-    bi = -1;
-    bd = __int_as_float(0x7f800000);
-    return;
-  }
-  for (int k = first_ring(g, cx, cy, cz);; ++k) {
-    const float margin = search_margin(g, q, k);
-    RTR_FOR_RING(g, cx, cy, cz, k, {
-      const uint2 c = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
-      if (c.x < c.y && !beyond(cell_box_dist(g, q, x, y, z), margin, bd))
-        for (unsigned j = c.x; j < c.y; ++j) nn_take(g.pts[j], j, q, bd, bi, bpos);
-    })
-    if (ring_covers(g, cx, cy, cz, k)) break;
-    if (beyond(ring_bound(g, q, cx, cy, cz, k), margin, bd)) break;
-  }
-  if (bi == INT_MAX) {
-    bi = -1;
-    bpos = -1;
-    bd = __int_as_float(0x7f800000);
-  }
-}
-
 // Group reduction of (bd, bi, bpos) over the G lanes in gmask.
 template <int G>
 __device__ __forceinline__ void group_best(unsigned gmask, float& bd, int& bi, int& bpos) {
@@ -196,10 +171,9 @@ __device__ __forceinline__ void group_best(unsigned gmask, float& bd, int& bi, i
 // every ring the group agrees on the best (d^2, index), so the ring loop is
 // uniform inside the group.  A lane skips a cell only when the cell is beyond
 // its own best, which is never better than the group's.
-// CP (cell-parallel): each lane scans its own candidate cells of a chunk,
-// with the first two points of all four issued as independent loads, instead
-// of the group scanning one candidate cell after another.  Same result.
-template <int G, bool CP = false>
+// Exact 1-NN with d^2 <= r2max (r2max = +inf: unbounded); the original index
+// (or -1) and the sorted position.
+template <int G>
 __device__ __forceinline__ void grid_nn1_group(const GridView& g, float4 q, float r2max, int lg,
                                                unsigned gmask, float& bd, int& bi, int& bpos) {
   bd = r2max;
@@ -235,45 +209,27 @@ __device__ __forceinline__ void grid_nn1_group(const GridView& g, float4 q, floa
             // the cell's box first: a cell beyond the current best is not fetched
             if (max(max(abs(x - cx), abs(y - cy)), abs(z - cz)) == k &&
                 !beyond(cell_box_dist(g, q, x, y, z), margin, bd)) {
-              cc[s] = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
+              cc[s] = cell_span(g, x, y, z);
               cand[s] = cc[s].x < cc[s].y;
             }
           }
         }
-        if (CP) {
-          float4 p0[4], p1[4];
 #pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const unsigned a = cc[s].x, e = cc[s].y;
-            p0[s] = (cand[s] && a < e) ? g.pts[a] : q;
-            p1[s] = (cand[s] && a + 1 < e) ? g.pts[a + 1] : q;
-          }
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            if (!cand[s]) continue;
-            const unsigned a = cc[s].x, e = cc[s].y;
-            if (a < e) nn_take(p0[s], a, q, bd, bi, bpos);
-            if (a + 1 < e) nn_take(p1[s], a + 1, q, bd, bi, bpos);
-            for (unsigned j = a + 2; j < e; ++j) nn_take(g.pts[j], j, q, bd, bi, bpos);
-          }
-        } else {
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            unsigned bal = __ballot_sync(gmask, cand[s]) >> gbase;
-            while (bal) {
-              const int src = __ffs(bal) - 1;
-              bal &= bal - 1;
-              const unsigned b0 = __shfl_sync(gmask, cc[s].x, gbase + src);
-              const unsigned b1 = __shfl_sync(gmask, cc[s].y, gbase + src);
-              for (unsigned j = b0 + (unsigned)lg; j < b1; j += G) nn_take(g.pts[j], j, q, bd, bi, bpos);
-            }
+        for (int s = 0; s < 4; ++s) {
+          unsigned bal = __ballot_sync(gmask, cand[s]) >> gbase;
+          while (bal) {
+            const int src = __ffs(bal) - 1;
+            bal &= bal - 1;
+            const unsigned b0 = __shfl_sync(gmask, cc[s].x, gbase + src);
+            const unsigned b1 = __shfl_sync(gmask, cc[s].y, gbase + src);
+            for (unsigned j = b0 + (unsigned)lg; j < b1; j += G) nn_take(g.pts[j], j, q, bd, bi, bpos);
           }
         }
       }
     } else {
       // large rings: walk only the shell, all lanes on the same cell
       RTR_FOR_RING(g, cx, cy, cz, k, {
-        const uint2 c = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
+        const uint2 c = cell_span(g, x, y, z);
         if (c.x < c.y && !beyond(cell_box_dist(g, q, x, y, z), margin, bd))
           for (unsigned j = c.x + (unsigned)lg; j < c.y; j += G) nn_take(g.pts[j], j, q, bd, bi, bpos);
       })
@@ -289,132 +245,282 @@ __device__ __forceinline__ void grid_nn1_group(const GridView& g, float4 q, floa
   }
 }
 
-// True when every point within sqrt(r2max) of any query lies in the 3x3x3
-// cells around the query's cell: the cell edge exceeds the radius by 1 % and
-// the grid is small enough (<= 4096 cells per axis) that the rounding of a
-// cell index stays far below that slack.
-__device__ __forceinline__ bool grid_near27_ok(const GridView& g, float r2max) {
-  const float r = sqrtf(r2max);
-  return r2max >= 0.f && isfinite(r) && g.h >= 1.01f * r && g.nx <= 4096 && g.ny <= 4096 && g.nz <= 4096;
-}
-
-// Offsets (-1, 0, +1 as bits 0, 1, 2) along one axis that stay in the grid
-// (0 <= c + d < n) and, for d != 0, whose face lies within reach (squared
-// face distance <= thr2).
-__device__ __forceinline__ unsigned near_axis_mask(int c, int n, float fm2, float fp2, float thr2) {
-  unsigned m = 0u;
-  if (c - 1 >= 0 && c - 1 < n && !(fm2 > thr2)) m |= 1u;
-  if (c >= 0 && c < n) m |= 2u;
-  if (c + 1 >= 0 && c + 1 < n && !(fp2 > thr2)) m |= 4u;
-  return m;
-}
-// Offset of the k-th set bit (k < popc(m)) of a 3-bit axis mask.
-__device__ __forceinline__ int near_axis_pick(unsigned m, int k) {
-  const int b0 = (int)(m & 1u), b1 = (int)((m >> 1) & 1u);
-  return k < b0 ? -1 : (k < b0 + b1 ? 0 : 1);
-}
-
-// The query's position relative to its cell: squared distances to the six
-// faces (clamped at 0; underestimates under rounding).
-struct NearCell {
-  int cx, cy, cz;
-  float xm2, xp2, ym2, yp2, zm2, zp2;
+// Box searches, for many queries against one grid: what does not depend on
+// the query is computed once.  The rounding of a search is covered by the
+// margin of the grid plus the query's own part (box_margin).
+struct BoxView {
+  GridView g;
+  float margin;
+  float nxm, nym, nzm;  // last cell of each axis
+  float hx, hy, hz;     // upper corner
 };
-__device__ __forceinline__ NearCell near_cell(const GridView& g, float4 q) {
-  NearCell c;
-  c.cx = q_cell(q.x, g.ox, g.inv_h);
-  c.cy = q_cell(q.y, g.oy, g.inv_h);
-  c.cz = q_cell(q.z, g.oz, g.inv_h);
-  const float xl = g.ox + (float)c.cx * g.h, yl = g.oy + (float)c.cy * g.h, zl = g.oz + (float)c.cz * g.h;
-  const float fxm = fmaxf(q.x - xl, 0.f), fxp = fmaxf(xl + g.h - q.x, 0.f);
-  const float fym = fmaxf(q.y - yl, 0.f), fyp = fmaxf(yl + g.h - q.y, 0.f);
-  const float fzm = fmaxf(q.z - zl, 0.f), fzp = fmaxf(zl + g.h - q.z, 0.f);
-  c.xm2 = fxm * fxm;
-  c.xp2 = fxp * fxp;
-  c.ym2 = fym * fym;
-  c.yp2 = fyp * fyp;
-  c.zm2 = fzm * fzm;
-  c.zp2 = fzp * fzp;
+__device__ __forceinline__ BoxView box_view(const GridDev& gd) {
+  BoxView b;
+  b.g = load_view(gd);
+  const GridView& g = b.g;
+  b.nxm = (float)(g.nx - 1);
+  b.nym = (float)(g.ny - 1);
+  b.nzm = (float)(g.nz - 1);
+  b.hx = g.ox + (float)g.nx * g.h;
+  b.hy = g.oy + (float)g.ny * g.h;
+  b.hz = g.oz + (float)g.nz * g.h;
+  float s = fmaxf(fmaxf(fabsf(g.ox), fabsf(g.oy)), fabsf(g.oz));
+  s = fmaxf(s, fmaxf(fmaxf(fabsf(b.hx), fabsf(b.hy)), fabsf(b.hz)));
+  b.margin = 8.0e-6f * (1.0f + s + (float)(max(max(g.nx, g.ny), g.nz) + 3) * g.h);
+  return b;
+}
+__device__ __forceinline__ float box_margin(const BoxView& b, float4 q) {
+  return b.margin + 8.0e-6f * fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
+}
+
+__device__ __forceinline__ float sqrt_up(float x) {  // >= sqrt(x), by a few parts in 10^6
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r * 1.00001f;
+}
+
+// The cells meeting the box q -+ t (t > 0 includes the margin), in cell units.
+struct CellBox {
+  float uy, uz, tc2;
+  int x0, x1, y0, y1, z0, z1;
+};
+__device__ __forceinline__ CellBox cell_box(const BoxView& v, float4 q, float t) {
+  const GridView& g = v.g;
+  const float ux = (q.x - g.ox) * g.inv_h;
+  CellBox c;
+  c.uy = (q.y - g.oy) * g.inv_h;
+  c.uz = (q.z - g.oz) * g.inv_h;
+  const float tc = t * g.inv_h;
+  c.tc2 = tc * tc * 1.00001f;
+  c.x0 = __float2int_rd(fminf(fmaxf(ux - tc, 0.f), v.nxm));
+  c.x1 = __float2int_rd(fminf(fmaxf(ux + tc, 0.f), v.nxm));
+  c.y0 = __float2int_rd(fminf(fmaxf(c.uy - tc, 0.f), v.nym));
+  c.y1 = __float2int_rd(fminf(fmaxf(c.uy + tc, 0.f), v.nym));
+  c.z0 = __float2int_rd(fminf(fmaxf(c.uz - tc, 0.f), v.nzm));
+  c.z1 = __float2int_rd(fminf(fmaxf(c.uz + tc, 0.f), v.nzm));
   return c;
 }
 
-// The neighbour cells a query must visit: every (dx, dy, dz) != 0 from the
-// per-axis masks whose box is within reach; entry k (k = lg, lg + G, ...) of
-// that list for lane lg.  thr2 must be the same in every lane of the group
-// (the lists then agree).  Calls body(x, y, z) for each of the lane's cells.
+// Calls body(span) for the rows of the box along x, each one contiguous run of
+// points, four rows' spans in flight; a row farther from q than t (by its y
+// and z extent) is skipped.  body returns true to stop (after its four rows).
+template <typename F>
+__device__ __forceinline__ void box_rows(const BoxView& v, const CellBox& c, F body) {
+  const int rows = (c.y1 - c.y0 + 1) * (c.z1 - c.z0 + 1);
+  int y = c.y0, z = c.z0;
+  for (int r0 = 0; r0 < rows; r0 += 4) {
+    uint2 s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s[u] = make_uint2(0u, 0u);
+      if (r0 + u < rows) {
+        const float fy = (float)y, fz = (float)z;
+        const float dy = fmaxf(fmaxf(fy - c.uy, c.uy - (fy + 1.f)), 0.f);
+        const float dz = fmaxf(fmaxf(fz - c.uz, c.uz - (fz + 1.f)), 0.f);
+        if (!(dy * dy + dz * dz > c.tc2)) s[u] = row_span(v.g, c.x0, c.x1, y, z);
+        if (++y > c.y1) {
+          y = c.y0;
+          ++z;
+        }
+      }
+    }
+    bool stop = false;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) stop |= body(s[u]);
+    if (stop) return;
+  }
+}
+
+// The two nearest of the points seen: the best by (d^2, index) and the
+// squared distance of the second.
+struct Near2 {
+  float bd, sd;
+  int bi, bpos;
+};
+__device__ __forceinline__ void near2_take(float4 p, unsigned j, float4 q, Near2& n) {
+  const float d2 = dist2_exact(q, p);
+  const int id = pt_index(p);
+  // a point at infinite (or NaN) d^2 is never a neighbour
+  const bool better = d2 < n.bd || (d2 == n.bd && id < n.bi && d2 < __int_as_float(0x7f800000));
+  n.sd = fminf(n.sd, better ? n.bd : d2);
+  if (better) {
+    n.bd = d2;
+    n.bi = id;
+    n.bpos = (int)j;
+  }
+}
+
+// Calls take(p, j) for the points of the box's rows, spread over the G lanes
+// of the group.  Up to 4 lanes walk the rows one after another, striding
+// through each row's points: fewest instructions, for kernels with enough
+// queries in flight to hide that every row is a dependent load.  With 8 lanes
+// and more each lane fetches one row's span, a prefix sum over the rows
+// numbers their points, and the lanes stride through the numbers, four loads
+// in flight each: a few round trips in all, for kernels whose queries are few
+// and wait on one another.  Uniform in the group.
 template <int G, typename F>
-__device__ __forceinline__ void near_neighbours(const GridView& g, const NearCell& c, float thr2, int lg, F body) {
-  const unsigned mx = near_axis_mask(c.cx, g.nx, c.xm2, c.xp2, thr2);
-  const unsigned my = near_axis_mask(c.cy, g.ny, c.ym2, c.yp2, thr2);
-  const unsigned mz = near_axis_mask(c.cz, g.nz, c.zm2, c.zp2, thr2);
-  const int nxo = __popc(mx), nyo = __popc(my), nzo = __popc(mz);
-  const int total = nxo * nyo * nzo;
-  for (int k = lg; k < total; k += G) {
-    const int ix = k % nxo, iy = (k / nxo) % nyo, iz = k / (nxo * nyo);
-    const int dx = near_axis_pick(mx, ix), dy = near_axis_pick(my, iy), dz = near_axis_pick(mz, iz);
-    if ((dx | dy | dz) == 0) continue;  // the own cell
-    const float b2 = (dx < 0 ? c.xm2 : (dx > 0 ? c.xp2 : 0.f)) + (dy < 0 ? c.ym2 : (dy > 0 ? c.yp2 : 0.f)) +
-                     (dz < 0 ? c.zm2 : (dz > 0 ? c.zp2 : 0.f));
-    if (b2 > thr2) continue;  // an edge or corner cell beyond reach
-    body(c.cx + dx, c.cy + dy, c.cz + dz);
+__device__ __forceinline__ void box_points(const BoxView& v, const CellBox& c, int lg, unsigned gmask, F take) {
+  if (G <= 4) {
+    box_rows(v, c, [&](uint2 s) {
+      unsigned j = s.x + (unsigned)lg;
+      for (; j + G < s.y; j += 2 * G) {
+        const float4 p0 = v.g.pts[j], p1 = v.g.pts[j + G];
+        take(p0, j);
+        take(p1, j + G);
+      }
+      if (j < s.y) take(v.g.pts[j], j);
+      return false;
+    });
+    return;
+  }
+  const int ey = c.y1 - c.y0 + 1, rows = ey * (c.z1 - c.z0 + 1);
+  for (int r0 = 0; r0 < rows; r0 += G) {
+    const int r = r0 + lg;
+    uint2 s = make_uint2(0u, 0u);
+    if (r < rows) {
+      const int zi = r / ey, y = c.y0 + r - zi * ey, z = c.z0 + zi;
+      const float fy = (float)y, fz = (float)z;
+      const float dy = fmaxf(fmaxf(fy - c.uy, c.uy - (fy + 1.f)), 0.f);
+      const float dz = fmaxf(fmaxf(fz - c.uz, c.uz - (fz + 1.f)), 0.f);
+      if (!(dy * dy + dz * dz > c.tc2)) s = row_span(v.g, c.x0, c.x1, y, z);
+    }
+    unsigned incl = s.y - s.x;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+      const unsigned t = __shfl_up_sync(gmask, incl, o, G);
+      if (lg >= o) incl += t;
+    }
+    const unsigned total = __shfl_sync(gmask, incl, G - 1, G);
+    const unsigned off = s.y - incl;  // point k of the numbering lies at off + k of its row
+    for (unsigned k0 = 0; k0 < total; k0 += 4 * G) {
+      unsigned j[4];
+      float4 p[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const unsigned k = k0 + u * G + (unsigned)lg;
+        int row = 0;  // the first row whose points go past k
+#pragma unroll
+        for (int step = G / 2; step > 0; step >>= 1)
+          if (k >= __shfl_sync(gmask, incl, row + step - 1, G)) row += step;
+        j[u] = __shfl_sync(gmask, off, row, G) + k;
+        if (k < total) p[u] = v.g.pts[j[u]];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k0 + u * G + (unsigned)lg < total) take(p[u], j[u]);
+    }
   }
 }
 
-// Exact 1-NN with d^2 <= r2max over the 27 cells around the query's cell
-// (precondition: grid_near27_ok), G lanes per query as grid_nn1_group; same
-// result.  The query's own cell is scanned first and the group agrees on its
-// best; then only the neighbours whose box, measured through the query's
-// distances to its own cell's faces (an underestimate), is within that best
-// plus the rounding margin are fetched, spread over the group.  No ring
-// bookkeeping and no square root per cell.
+// Whether the cells of the box hold no point; the group's lanes share the rows.
 template <int G>
-__device__ __forceinline__ void grid_nn1_near(const GridView& g, float4 q, float r2max, int lg, unsigned gmask,
-                                              float& bd, int& bi, int& bpos) {
-  bd = r2max;
-  bi = INT_MAX;
-  bpos = -1;
-  const NearCell c = near_cell(g, q);
-  if (c.cx >= 0 && c.cx < g.nx && c.cy >= 0 && c.cy < g.ny && c.cz >= 0 && c.cz < g.nz) {
-    const uint2 e = g.cells[((unsigned)c.cz * (unsigned)g.ny + (unsigned)c.cy) * (unsigned)g.nx + (unsigned)c.cx];
-    for (unsigned j = e.x + (unsigned)lg; j < e.y; j += G) nn_take(g.pts[j], j, q, bd, bi, bpos);
+__device__ __forceinline__ bool box_empty(const BoxView& v, const CellBox& c, int lg, unsigned gmask) {
+  const int ey = c.y1 - c.y0 + 1, rows = ey * (c.z1 - c.z0 + 1);
+  bool any = false;
+#pragma unroll 4
+  for (int r = lg; r < rows; r += G) {
+    const int zi = r / ey;
+    const uint2 s = row_span(v.g, c.x0, c.x1, c.y0 + r - zi * ey, c.z0 + zi);
+    any |= s.x < s.y;
   }
-  group_best<G>(gmask, bd, bi, bpos);
-  const float t = search_margin(g, q, 1) + sqrtf(bd * 1.000001f + 1e-30f);
-  const float thr2 = t * t * 1.00001f;
-  near_neighbours<G>(g, c, thr2, lg, [&](int x, int y, int z) {
-    const uint2 e = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
-    for (unsigned j = e.x; j < e.y; ++j) nn_take(g.pts[j], j, q, bd, bi, bpos);
-  });
-  group_best<G>(gmask, bd, bi, bpos);
-  if (bi == INT_MAX) {
-    bi = -1;
-    bpos = -1;
-    bd = __int_as_float(0x7f800000);
-  }
+  return !__any_sync(gmask, any);
 }
 
-// Whether any point lies within sqrt(r2) of q (d^2 <= r2, finite), over the
-// 27 cells around q's cell (precondition: grid_near27_ok(g, r2)), G lanes
-// per query; the same answer as grid_nn1_group finding a neighbour.  The own
-// cell first, then the neighbours within reach; every lane stops once the
-// group has found one.
+// Exact 1-NN with d^2 <= r2max (r >= its root), G lanes per query (see
+// grid_nn1_group; the same neighbour), for queries that come again and move
+// little.  cand: the sorted position of any grid point, by choice the last
+// answer, or -1.  With a candidate one box of its distance is scanned: where
+// it is the answer or close to it, a few rows.  Without one the box grows
+// from one cell edge, doubling up to the bound, until something is found, and
+// then covers what was found.  *room: every point of the grid but the answer
+// (every point, when there is none) is at least that far away.  extra widens
+// the last box, so that room comes out useful; and where the bound holds
+// nothing, boxes up to eight times it are tried for emptiness (spans only, no
+// points), so that a query in the open is told it need not come back soon.  Returns the answer's
+// sorted position or -1; uniform in the group.
 template <int G>
-__device__ __forceinline__ bool grid_any_near(const GridView& g, float4 q, float r2, int lg, unsigned gmask) {
-  const NearCell c = near_cell(g, q);
+__device__ __forceinline__ int grid_nn1_from(const BoxView& v, float4 q, float r2max, float r, int cand, float extra,
+                                             int lg, unsigned gmask, float* room) {
+  const GridView& g = v.g;
+  const float inf = __int_as_float(0x7f800000);
+  Near2 n;
+  const float far = r + extra, margin = box_margin(v, q);
+  float tr = 0.f, t;
+  if (cand >= 0) {
+    t = fminf(sqrt_up(dist2_exact(q, g.pts[cand])), r) + extra + margin;
+  } else {
+    const float dx = fmaxf(fmaxf(g.ox - q.x, q.x - v.hx), 0.f), dy = fmaxf(fmaxf(g.oy - q.y, q.y - v.hy), 0.f),
+                dz = fmaxf(fmaxf(g.oz - q.z, q.z - v.hz), 0.f);
+    const float d0 = sqrt_up(dx * dx + dy * dy + dz * dz);  // to the grid's box
+    if (d0 * 0.9999f > r + margin) {  // nothing of the grid within the bound
+      *room = d0 * 0.9999f - margin;
+      return -1;
+    }
+    tr = fminf(far, d0 + g.h);
+    t = tr + margin;
+  }
+  bool whole;
+  for (;;) {
+    const CellBox c = cell_box(v, q, t);
+    n = Near2{inf, inf, INT_MAX, -1};
+    box_points<G>(v, c, lg, gmask, [&](float4 p, unsigned j) { near2_take(p, j, q, n); });
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const float od = __shfl_xor_sync(gmask, n.bd, o), os = __shfl_xor_sync(gmask, n.sd, o);
+      const int oi = __shfl_xor_sync(gmask, n.bi, o), op = __shfl_xor_sync(gmask, n.bpos, o);
+      const bool better = od < n.bd || (od == n.bd && oi < n.bi);
+      n.sd = fminf(fminf(n.sd, os), better ? n.bd : od);
+      if (better) {
+        n.bd = od;
+        n.bi = oi;
+        n.bpos = op;
+      }
+    }
+    whole = c.x0 == 0 && c.y0 == 0 && c.z0 == 0 && c.x1 == g.nx - 1 && c.y1 == g.ny - 1 && c.z1 == g.nz - 1;
+    if (cand >= 0 || whole) break;
+    if (n.bpos >= 0) {
+      const float need = margin + fminf(sqrt_up(n.bd), far);
+      if (need <= t) break;  // all within the answer's distance, or the bound, has been seen
+      t = need + extra;
+      cand = n.bpos;  // the last box
+    } else {
+      if (tr >= far) break;
+      tr = fminf(far, 2.f * tr);
+      t = tr + margin;
+    }
+  }
+  float seen = whole ? inf : t - margin;  // every point closer than this has been seen
+  const bool hit = n.bd <= r2max && n.bpos >= 0;
+  if (n.bpos < 0 && !whole && seen < 1.0e30f) {
+    for (int k = 0; k < 5; ++k) {  // 1.5^5 = 7.6
+      const CellBox c = cell_box(v, q, 1.5f * seen + margin);
+      if (!box_empty<G>(v, c, lg, gmask)) break;
+      seen *= 1.5f;
+    }
+  }
+  *room = fminf(sqrt_up(hit ? n.sd : n.bd) * 0.9999f, seen);
+  return hit ? n.bpos : -1;
+}
+
+// Whether any point lies within sqrt(r2) of q (d^2 <= r2, finite r2), G lanes
+// per query; the same answer as grid_nn1_group finding a neighbour.  Every
+// lane stops once the group has found one.
+template <int G>
+__device__ __forceinline__ bool grid_any_within(const BoxView& v, float4 q, float r2, int lg, unsigned gmask) {
+  const GridView& g = v.g;
+  const float r = sqrt_up(r2) + box_margin(v, q);
+  if (g.ox - q.x > r || q.x - v.hx > r || g.oy - q.y > r || q.y - v.hy > r || g.oz - q.z > r || q.z - v.hz > r)
+    return false;
   bool found = false;
-  if (c.cx >= 0 && c.cx < g.nx && c.cy >= 0 && c.cy < g.ny && c.cz >= 0 && c.cz < g.nz) {
-    const uint2 e = g.cells[((unsigned)c.cz * (unsigned)g.ny + (unsigned)c.cy) * (unsigned)g.nx + (unsigned)c.cx];
-    for (unsigned j = e.x + (unsigned)lg; j < e.y && !found; j += G) found = dist2_exact(q, g.pts[j]) <= r2;
-  }
-  if (__any_sync(gmask, found)) return true;
-  const float t = search_margin(g, q, 1) + sqrtf(r2 * 1.000001f + 1e-30f);
-  const float thr2 = t * t * 1.00001f;
-  near_neighbours<G>(g, c, thr2, lg, [&](int x, int y, int z) {
-    if (found) return;
-    const uint2 e = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
-    for (unsigned j = e.x; j < e.y && !found; ++j) found = dist2_exact(q, g.pts[j]) <= r2;
+  int left = 4;
+  box_rows(v, cell_box(v, q, r), [&](uint2 s) {
+    for (unsigned j = s.x + (unsigned)lg; j < s.y && !found; j += G) found = dist2_exact(q, g.pts[j]) <= r2;
+    if (--left > 0) return false;
+    left = 4;
+    found = G > 1 ? __any_sync(gmask, found) != 0 : found;
+    return found;
   });
-  return __any_sync(gmask, found);
+  return found;
 }
 
 // Exact K-NN (K compile-time), sorted by (d^2, index).  The K nearest by that
@@ -449,7 +555,7 @@ __device__ __forceinline__ void grid_knn(const GridView& g, float4 q, float (&bd
   for (int k = first_ring(g, cx, cy, cz);; ++k) {
     const float margin = search_margin(g, q, k);
     RTR_FOR_RING(g, cx, cy, cz, k, {
-      const uint2 c = g.cells[((unsigned)z * (unsigned)g.ny + (unsigned)y) * (unsigned)g.nx + (unsigned)x];
+      const uint2 c = cell_span(g, x, y, z);
       if (c.x < c.y && !beyond(cell_box_dist(g, q, x, y, z), margin, bd[K - 1])) {
         for (unsigned j = c.x; j < c.y; ++j) {
           const float4 p = g.pts[j];

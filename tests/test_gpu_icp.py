@@ -160,3 +160,70 @@ def test_pose_inliers_equals_oracle(ctx, rtr):
         frac = g.inlier_fraction(src, 1, poses.reshape(-1, 16), r)
         g.close()
         assert np.array_equal(cnt, np.rint(frac * src.shape[0]).astype(np.int32)), (cnt, frac)
+
+
+@pytest.mark.parametrize("n_src,n_tgt,max_dist,cell,shift", [
+    (7, 50, 0.05, 0.0, 0.0),        # one group of 8 points, most blocks idle
+    (4099, 3001, 0.02, 0.03, 0.03),  # most points without a neighbour at first
+    (4099, 3001, 0.3, 0.0, 0.1),    # a bound far beyond the neighbours' distance
+    (2500, 2500, 0.0, 0.0, 0.0),    # no bound
+    (2500, 2500, 0.0, 0.0, 40.0),   # no bound, and the clouds far apart
+    (5000, 5000, 0.05, 0.004, 0.02),  # boxes of many cells
+])
+def test_icp_kept_neighbours_equal_a_search_from_scratch(ctx, rtr, n_src, n_tgt, max_dist, cell, shift):
+    """Every iteration's correspondences, whether the point was searched or
+    its last answer kept, equal the oracle's search; two points of the source
+    and one of the target are not finite."""
+    src, tgt, _ = rtr.config0_pair(n_src, max(n_src, n_tgt))
+    src, tgt = src[:n_src].copy(), tgt[:n_tgt].copy()
+    src[:, 0] += np.float32(shift)
+    if n_src > 100:
+        src[5, 1], src[17, 2], tgt[9, 0] = np.nan, np.inf, np.nan
+    import torch
+    res, tp, tc = ctx.icp(_dev(src), _dev(tgt), 25, max_dist, cell_size=cell, trace=True)
+    r = ctx.parse_icp_result(res)
+    n_it = r["iterations"]
+    poses, corr = tp.cpu().numpy(), tc.cpu().numpy()
+    for k in range(n_it):
+        q = O.transform_f32(poses[k].reshape(4, 4), src)
+        ri, _ = O.nn1(q, tgt, max_dist, "brute")
+        assert np.array_equal(corr[k], ri), k
+
+
+def test_icp_many_problems_share_a_block_each(ctx, rtr):
+    """More points per block than one chunk of the matching (2,048): 300
+    problems on the GPU's blocks give what one problem alone gives."""
+    src, tgt, T = rtr.config0_pair(8, 9001)
+    inits = np.array([T, np.eye(4), T])
+    inits[2][:3, 3] += 0.01
+    alone = [ctx.parse_icp_result(ctx.icp(_dev(src), _dev(tgt), 12, 0.03, init=i, cell_size=0.02)[0]) for i in inits]
+    many = ctx.icp_multi(_dev(src), _dev(tgt), inits[np.arange(300) % 3], 12, 0.03, cell_size=0.02)
+    for k, m in enumerate(many):
+        a = alone[k % 3]
+        assert m["status"] == 0 and m["n_corr"] == a["n_corr"]
+        np.testing.assert_allclose(m["pose"], a["pose"], rtol=0, atol=1e-9)
+
+
+def test_recognition_refines_alike_without_room_for_the_matching_state(rtr):
+    """A scene of a few points and a large model: the recognition's scratch
+    need not hold the refinement's matching state, which then searches every
+    point in every iteration.  Same instances and poses as with a larger
+    arena."""
+    prm = rtr.recog_default_params(scene_outward=1)
+    model = rtr.synth_shape(rtr.SOFA, 60000, 3)
+    scene = rtr.synth_transform_noise(rtr.synth_shape(rtr.SOFA, 2000, 4), rtr.synth_rigid(5, 20.0, 0.2), 0.002, 6)
+    out = []
+    for reserve in (0, 1 << 30):
+        c = rtr.Context(0)
+        m = rtr.Model(c, _dev(model), prm)
+        if reserve:
+            c.reserve(reserve)
+        out.append(rtr.parse_recog_result(rtr.recognize(c, m, _dev(scene), prm)))
+        c.check()
+        m.close()
+        c.close()
+    a, b = out
+    assert a["n_clusters"] == b["n_clusters"] and len(a["instances"]) == len(b["instances"])
+    for x, y in zip(a["instances"], b["instances"]):
+        assert x["hypothesis"] == y["hypothesis"] and x["score"] == y["score"]
+        np.testing.assert_allclose(x["pose"], y["pose"], rtol=0, atol=1e-9)

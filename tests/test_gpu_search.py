@@ -123,3 +123,29 @@ def test_box_search_at_keypoints_of_main_scan(ctx):
     oidx, ocnt = O.range_search(keys, scan, 0.1, True, 4096)
     assert np.array_equal(cnt.cpu().numpy(), ocnt) and ocnt.max() < 4096
     assert np.array_equal(idx.cpu().numpy(), oidx)
+
+
+@pytest.mark.parametrize("kind", ["one_cell", "one_point", "line", "clusters"])
+def test_grid_counted_into_place_on_uneven_clouds(ctx, kind):
+    """Cells holding the whole cloud, duplicates, a degenerate box and a few
+    dense clusters, with points that are not finite: 1-NN and k-NN as brute
+    force finds them."""
+    rng = np.random.default_rng(3)
+    n = 5003
+    t = _rand(rng, n, 0.001)
+    if kind == "one_point":
+        t[:, :3] = 0.25
+    elif kind == "line":
+        t[:, 1:3] = 0.5
+    elif kind == "clusters":
+        t[:, :3] += rng.integers(0, 3, (n, 1)).astype(np.float32) * 5
+    t[11, 0], t[12, 1] = np.nan, np.inf
+    q = np.concatenate([t[:400] + np.float32(1e-4), _rand(rng, 300, 1.0)])
+    q[:, 3] = 0
+    for md in (0.0, 0.004, 2.0):
+        idx, _ = ctx.knn1(_dev(q), _dev(t), md)
+        ri, _ = O.nn1(q, t, md, "brute")
+        assert np.array_equal(idx.cpu().numpy(), ri), md
+    ki, _ = ctx.knn(_dev(q[:50]), _dev(t), 8)
+    first = O.nn1(q[:50], t, 0.0, "brute")[0]
+    assert np.array_equal(ki.cpu().numpy()[:, 0], first)
