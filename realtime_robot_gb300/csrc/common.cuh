@@ -96,6 +96,7 @@ struct rtr_context {
   size_t io_bytes = 0;
   cudaStream_t host_stream = nullptr;  // stream of the host-pointer entry points
   int* h_pin = nullptr;                // 64 pinned ints for small device->host reads
+  void* plane_host = nullptr;          // page-locked words of the plane segmentation (planes.cu)
   int tune_icp_group = 0;              // lanes per ICP source point (0: automatic)
   size_t scratch_limit = 0;            // largest scratch arena this context may hold (0: no limit)
   int tune_batch_workers = 0;          // workers of rtr_recognize_batch (0: automatic)

@@ -235,6 +235,7 @@ rtr_status rtr_context_destroy(rtr_context* ctx) {
   if (ctx->io) cudaFree(ctx->io);
   if (ctx->host_stream) cudaStreamDestroy(ctx->host_stream);
   if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
+  if (ctx->plane_host) cudaFreeHost(ctx->plane_host);
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->d_sync) cudaFree(ctx->d_sync);
   delete ctx;

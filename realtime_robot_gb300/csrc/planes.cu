@@ -5,27 +5,34 @@
 // through PCL's SACSegmentation, ExtractIndices and ConvexHull.
 //
 // One call extracts planes one after another from the points still
-// unclaimed (the reference's loop, while more than 15 % remain):
-//   RANSAC   sample slots in batches of 64: one thread per slot draws three
-//            positions in the remaining list (SplitMix64 of seed, round,
-//            slot) and forms the plane (float); every thread of the grid
-//            then tests its points against the 64 planes (the planes in
-//            shared memory, counts per block, one atomic per slot and block);
-//            the host walks the slots in order with the adaptive stop rule
-//            (99 % confidence, at most max_iterations valid samples);
-//   refit    one 1024-thread block sums the best plane's inliers in FP64,
-//            thread t over positions t, t + 1024, ... in order, then a
-//            pairwise tree in shared memory (a fixed order, the oracle's);
-//            the host solves the 3x3 eigenproblem (planes_host.cpp);
-//   select   the refitted plane's inliers (float test) flagged and scanned;
-//   hull     the inliers projected onto the plane (float); the 8 points
-//            extreme along u, v, u+v and u-v bound an octagon, and a point
-//            strictly inside it (exact double orientation tests) cannot be
-//            a hull vertex and is dropped; the rest are sorted by (u, v)
-//            with two stable radix passes and one thread runs Andrew's
-//            monotone chain (exact orientation tests); the host measures
-//            the hull's area and perimeter;
-//   remove   the inliers leave the remaining list (stable compaction).
+// unclaimed (the reference's loop, while more than 15 % remain).  What bounds
+// it at the clouds' sizes (thousands to a few 100k points) is not work but
+// the length of the chain: launches, host round trips, and steps that ran on
+// one thread or one block.  So a round is five launches and three waits, and
+// results reach the host through page-locked memory that the last block of a
+// kernel writes:
+//   RANSAC   192 sample slots at a time (the walk usually ends in the first):
+//            each block forms the planes of the batch itself (SplitMix64 of
+//            seed, round, slot draws three positions; float) and counts its
+//            points within each, one ballot per warp and plane; the host
+//            walks the slots in order with the adaptive stop rule (99 %
+//            confidence, at most max_iterations valid samples);
+//   refit    the best plane's inliers summed in FP64: partial t over positions
+//            t, t + 1024, ... in order, each of the nine sums by threads of
+//            its own over 36 blocks, then a pairwise tree in the last block (a
+//            fixed order, the oracle's); the host solves the 3x3
+//            eigenproblem (planes_host.cpp);
+//   select   the refitted plane's inliers (float test), projected onto the
+//            plane (float), and the extreme points along 16 directions;
+//   rest     the others close up in order; inliers strictly inside the polygon
+//            of the extremes (exact orientation tests) cannot be hull
+//            vertices and are dropped;
+//   hull     one block sorts what is left by (u, v) in shared memory and runs
+//            Andrew's monotone chain (orientation in float where its error
+//            bound decides, else exact); more than PL_HULL_CAP points, or
+//            PL_HULL_OUT vertices, take the radix sort and one thread's chain
+//            from memory; the host measures the hull's area and perimeter.
+// A 20k-point chair, 5 planes: 4.38 ms before, 0.55 ms now.
 // Everything that decides which points are inliers is computed exactly as
 // in the CPU oracle (oracle/planes.c), so planes, inlier sets and hulls are
 // bit-identical to it.
@@ -36,11 +43,32 @@
 
 #include "grid.cuh"
 #include "planes_host.h"
-#include "scan.cuh"
 
 namespace rtr {
 
-constexpr int PL_SLOTS = 64;        // RANSAC samples scored per batch
+constexpr int PL_SLOTS = 192;       // RANSAC samples scored per batch
+constexpr int PL_HULL_CAP = 2048;   // points the hull kernel sorts in shared memory
+constexpr int PL_HULL_OUT = 1024;   // hull vertices returned through page-locked memory
+constexpr int PL_TILE = 1024;       // points per block of the ordered compaction
+
+// What kernels tell the host, in page-locked memory.
+struct PlHost {
+  int valid[PL_SLOTS], count[PL_SLOTS];
+  float4 coef[PL_SLOTS];
+  double sums[9];
+  int n_fit;
+  int m_rest;     // points that remain
+  int n_left;     // inliers not dropped by the polygon
+  int hull;       // hull vertices (-1: too many points or vertices for the hull kernel)
+  float2 uv[PL_HULL_OUT];
+};
+// Device words that start at zero and are reset by whoever reads them last.
+struct PlDev {
+  int count[PL_SLOTS];
+  unsigned ticket_score, ticket_refit;
+  int n_in, n_left;            // inliers projected, inliers left by the polygon
+  unsigned long long ext[16];  // extreme of each direction: ordered value << 32 | position in uv
+};
 constexpr int PL_PARTIALS = 1024;   // strided FP64 partial sums of the refit
 
 __device__ __forceinline__ uint64_t pl_mix(uint64_t z) {
@@ -60,26 +88,12 @@ __device__ __forceinline__ bool pl_within(float4 c, float4 p, float thr) {
   return fabsf(s) <= thr;
 }
 
-__device__ __forceinline__ bool finite3(float4 p) { return isfinite(p.x) && isfinite(p.y) && isfinite(p.z); }
+// Position j of the list (the whole cloud when rem is NULL).
+__device__ __forceinline__ int pl_at(const int* rem, int j) { return rem ? rem[j] : j; }
 
-__global__ void k_pl_finite(const float4* __restrict__ pts, int n, uint32_t* __restrict__ flags) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    flags[i] = finite3(pts[i]) ? 1u : 0u;
-}
-
-// out[pos[i]] = i (or src[i]) where flags[i] (== want)
-__global__ void k_pl_compact(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ pos,
-                             const int* __restrict__ src, int n, uint32_t want, int* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (flags[i] == want) out[pos[i]] = src ? src[i] : i;
-}
-
-// one thread per slot of the batch: three positions and their plane
-__global__ void k_pl_slots(const float4* __restrict__ pts, const int* __restrict__ rem, int m, uint64_t seed,
-                           int round, int slot0, int n_slots, float4* __restrict__ coef, int* __restrict__ valid) {
-  const int s = threadIdx.x;
-  if (s >= n_slots) return;
-  const int gs = slot0 + s;
+// one sample slot: three positions and their plane
+__device__ __forceinline__ int pl_slot(const float4* __restrict__ pts, const int* __restrict__ rem, int m,
+                                       uint64_t seed, int round, int gs, float4* out) {
   const int i0 = pl_pick(seed, round, gs, 0, m), i1 = pl_pick(seed, round, gs, 1, m), i2 = pl_pick(seed, round, gs, 2, m);
   int ok = i0 != i1 && i0 != i2 && i1 != i2;
   float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -101,138 +115,190 @@ __global__ void k_pl_slots(const float4* __restrict__ pts, const int* __restrict
                       -__fadd_rn(__fadd_rn(__fmul_rn(nx, p0.x), __fmul_rn(ny, p0.y)), __fmul_rn(nz, p0.z)));
     }
   }
-  coef[s] = c;
-  valid[s] = ok;
+  *out = c;
+  return ok;
 }
 
-// inlier counts of the batch's planes over the remaining points
-__global__ void __launch_bounds__(256) k_pl_count(const float4* __restrict__ pts, const int* __restrict__ rem, int m,
-                                                  const float4* __restrict__ coef, const int* __restrict__ valid,
-                                                  int n_slots, float thr, int* __restrict__ count) {
+// The batch's planes and their inlier counts over the remaining points.  A
+// lane keeps the counts of planes lane, lane + 32, ...; the last block hands
+// everything to the host.
+__global__ void __launch_bounds__(256) k_pl_score(const float4* __restrict__ pts, const int* __restrict__ rem, int m,
+                                                  uint64_t seed, int round, int slot0, int n_slots, float thr,
+                                                  PlDev* __restrict__ dev, PlHost* __restrict__ host) {
   __shared__ float4 sc[PL_SLOTS];
   __shared__ int sv[PL_SLOTS], cnt[PL_SLOTS];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31;
   for (int s = threadIdx.x; s < PL_SLOTS; s += blockDim.x) {
-    sc[s] = s < n_slots ? coef[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-    sv[s] = s < n_slots ? valid[s] : 0;
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+    sv[s] = s < n_slots ? pl_slot(pts, rem, m, seed, round, slot0 + s, &c) : 0;
+    sc[s] = c;
     cnt[s] = 0;
   }
   __syncthreads();
-  // a thread holds up to 4 points and walks the planes; per plane one
-  // warp-aggregated add into the block's counter
-  for (int base = blockIdx.x * blockDim.x * 4; base < m; base += gridDim.x * blockDim.x * 4) {
-    float4 p[4];
-    bool live[4];
+  int mine[PL_SLOTS / 32];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int j = base + r * blockDim.x + threadIdx.x;
-      live[r] = j < m;
-      p[r] = live[r] ? pts[rem[j]] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    for (int s = 0; s < n_slots; ++s) {
-      if (!sv[s]) continue;
-      const float4 c = sc[s];
-      int h = 0;
+  for (int k = 0; k < PL_SLOTS / 32; ++k) mine[k] = 0;
+  for (int base = blockIdx.x * blockDim.x; base < m; base += gridDim.x * blockDim.x) {
+    const int j = base + threadIdx.x;
+    const bool live = j < m;
+    const float4 p = live ? pts[rem[j]] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) h += (live[r] && pl_within(c, p[r], thr)) ? 1 : 0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-      if ((threadIdx.x & 31) == 0 && h) atomicAdd(&cnt[s], h);
-    }
+    for (int k = 0; k < PL_SLOTS / 32; ++k)
+#pragma unroll 4
+      for (int q = 0; q < 32; ++q) {
+        const unsigned b = __ballot_sync(0xffffffffu, live && pl_within(sc[32 * k + q], p, thr));
+        if (lane == q) mine[k] += __popc(b);
+      }
   }
+#pragma unroll
+  for (int k = 0; k < PL_SLOTS / 32; ++k)
+    if (mine[k] && sv[32 * k + lane]) atomicAdd(&cnt[32 * k + lane], mine[k]);
   __syncthreads();
-  for (int s = threadIdx.x; s < n_slots; s += blockDim.x)
-    if (cnt[s]) atomicAdd(&count[s], cnt[s]);
+  for (int s = threadIdx.x; s < PL_SLOTS; s += blockDim.x)
+    if (cnt[s]) atomicAdd(&dev->count[s], cnt[s]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&dev->ticket_score, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int s = threadIdx.x; s < PL_SLOTS; s += blockDim.x) {
+    host->valid[s] = sv[s];
+    host->count[s] = __ldcg(&dev->count[s]);
+    host->coef[s] = sc[s];
+    dev->count[s] = 0;
+  }
+  if (threadIdx.x == 0) dev->ticket_score = 0u;
 }
 
-// FP64 sums of the inliers of plane c in the oracle's fixed order
-__global__ void __launch_bounds__(PL_PARTIALS) k_pl_refit(const float4* __restrict__ pts, const int* __restrict__ rem,
-                                                           int m, float4 c, float thr, double* __restrict__ sums,
-                                                           int* __restrict__ n_out) {
-  extern __shared__ double part[];  // [PL_PARTIALS][9]
-  __shared__ int cnt[PL_PARTIALS];
-  const int t = threadIdx.x;
-  double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+// FP64 sums of the inliers of plane c in the oracle's fixed order: block b has
+// sum b / 4 (x, y, z, xx, xy, xz, yy, yz, zz) of partials 256 (b % 4) ..., a
+// thread per partial; the last block adds the partials pairwise.
+constexpr int PL_REFIT_BLOCKS = 36;
+__global__ void __launch_bounds__(256) k_pl_refit(const float4* __restrict__ pts, const int* __restrict__ rem, int m,
+                                                  float4 c, float thr, double* __restrict__ part,
+                                                  int* __restrict__ part_n, PlDev* __restrict__ dev,
+                                                  PlHost* __restrict__ host) {
+  extern __shared__ double sp[];  // [PL_PARTIALS][9], the last block's
+  __shared__ int sn[PL_PARTIALS];
+  __shared__ int s_last;
+  const int k = blockIdx.x >> 2, t = (blockIdx.x & 3) * 256 + threadIdx.x;
+  double a = 0.0;
   int n = 0;
+#pragma unroll 4
   for (int j = t; j < m; j += PL_PARTIALS) {
     const float4 p = pts[rem[j]];
     if (!pl_within(c, p, thr)) continue;
     const double x = p.x, y = p.y, z = p.z;
-    a[0] = __dadd_rn(a[0], x);
-    a[1] = __dadd_rn(a[1], y);
-    a[2] = __dadd_rn(a[2], z);
-    a[3] = __dadd_rn(a[3], __dmul_rn(x, x));
-    a[4] = __dadd_rn(a[4], __dmul_rn(x, y));
-    a[5] = __dadd_rn(a[5], __dmul_rn(x, z));
-    a[6] = __dadd_rn(a[6], __dmul_rn(y, y));
-    a[7] = __dadd_rn(a[7], __dmul_rn(y, z));
-    a[8] = __dadd_rn(a[8], __dmul_rn(z, z));
+    double v = k == 0 ? x : (k == 1 ? y : z);
+    if (k >= 3) v = __dmul_rn(k < 6 ? x : (k < 8 ? y : z), k == 3 ? x : ((k == 4 || k == 6) ? y : z));
+    a = __dadd_rn(a, v);
     ++n;
   }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) part[t * 9 + k] = a[k];
-  cnt[t] = n;
+  part[k * PL_PARTIALS + t] = a;
+  if (k == 0) part_n[t] = n;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&dev->ticket_refit, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < 9 * PL_PARTIALS; i += 256) sp[i] = __ldcg(part + i);
+  for (int i = threadIdx.x; i < PL_PARTIALS; i += 256) sn[i] = __ldcg(part_n + i);
   __syncthreads();
   for (int width = PL_PARTIALS / 2; width >= 1; width >>= 1) {
-    if (t < width) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) part[t * 9 + k] = __dadd_rn(part[t * 9 + k], part[(t + width) * 9 + k]);
-      cnt[t] += cnt[t + width];
+    for (int i = threadIdx.x; i < 9 * width; i += 256) {
+      const int q = i / width, e = i - q * width;
+      double* P = sp + q * PL_PARTIALS;
+      P[e] = __dadd_rn(P[e], P[e + width]);
     }
+    for (int e = threadIdx.x; e < width; e += 256) sn[e] += sn[e + width];
     __syncthreads();
   }
-  if (t < 9) sums[t] = part[t];
-  if (t == 0) *n_out = cnt[0];
-}
-
-__global__ void k_pl_select(const float4* __restrict__ pts, const int* __restrict__ rem, int m, float4 c, float thr,
-                            uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    const bool w = pl_within(c, pts[rem[j]], thr);
-    in[j] = w ? 1u : 0u;
-    out[j] = w ? 0u : 1u;
+  if (threadIdx.x < 9) host->sums[threadIdx.x] = sp[threadIdx.x * PL_PARTIALS];
+  if (threadIdx.x == 0) {
+    host->n_fit = sn[0];
+    dev->ticket_refit = 0u;
   }
 }
 
-// (u, v) of the inliers, in their order; -0 becomes +0 so that the sort
-// keys order as the float comparisons do
-__global__ void k_pl_project(const float4* __restrict__ pts, const int* __restrict__ rem, int m,
-                             const uint32_t* __restrict__ in, const uint32_t* __restrict__ pos, float4 e1, float4 e2,
-                             float2* __restrict__ uv) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    if (!in[j]) continue;
-    const float4 p = pts[rem[j]];
-    float u = __fadd_rn(__fadd_rn(__fmul_rn(p.x, e1.x), __fmul_rn(p.y, e1.y)), __fmul_rn(p.z, e1.z));
-    float v = __fadd_rn(__fadd_rn(__fmul_rn(p.x, e2.x), __fmul_rn(p.y, e2.y)), __fmul_rn(p.z, e2.z));
-    uv[pos[j]] = make_float2(__fadd_rn(u, 0.f), __fadd_rn(v, 0.f));
-  }
+__device__ __forceinline__ bool finite3(float4 p) { return isfinite(p.x) && isfinite(p.y) && isfinite(p.z); }
+
+// The directions of the extreme points, by angle.
+__device__ __forceinline__ float pl_dir(int d, float u, float v) {
+  const int q = d >> 2, r = d & 3;  // quadrant: (u, v) turned back by q quarter turns
+  const float a = q == 0 ? u : (q == 1 ? v : (q == 2 ? -u : -v)), b = q == 0 ? v : (q == 1 ? -u : (q == 2 ? -v : u));
+  return r == 0 ? a : (r == 1 ? __fadd_rn(__fmul_rn(2.f, a), b) : (r == 2 ? __fadd_rn(a, b) : __fadd_rn(a, __fmul_rn(2.f, b))));
 }
 
-// the 8 extreme points: keys (ordered value << 32) | ~index, largest wins
-// (ties to the lowest index); directions u, u+v, v, v-u, -u, -u-v, -v, u-v
-__global__ void k_pl_extremes(const float2* __restrict__ uv, const int* __restrict__ d_n,
-                              unsigned long long* __restrict__ ext) {
-  const int n = *d_n;
-  unsigned long long best[8];
+// Whether point p of the list stays: finite (FIRST), or off the plane.
+template <bool FIRST>
+__device__ __forceinline__ bool pl_stays(float4 p, float4 c, float thr) {
+  return FIRST ? finite3(p) : !pl_within(c, p, thr);
+}
+
+// Per tile the number of points that stay; the others (inliers) are projected
+// into uv, in any order (-0 becomes +0, so that sort keys order as the float
+// comparisons do), and the extremes are taken.
+template <bool FIRST>
+__global__ void __launch_bounds__(256) k_pl_select(const float4* __restrict__ pts, const int* __restrict__ rem, int m,
+                                                   float4 c, float thr, float4 e1, float4 e2,
+                                                   int* __restrict__ tile_cnt, float2* __restrict__ uv,
+                                                   PlDev* __restrict__ dev) {
+  __shared__ int s_stay;
+  __shared__ unsigned long long s_ext[16];
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_stay = 0;
+  if (threadIdx.x < 16) s_ext[threadIdx.x] = 0ull;
+  __syncthreads();
+  unsigned long long best[16];
 #pragma unroll
-  for (int d = 0; d < 8; ++d) best[d] = 0ull;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float u = uv[i].x, v = uv[i].y;
-    const float val[8] = {u, __fadd_rn(u, v), v, __fsub_rn(v, u), -u, -__fadd_rn(u, v), -v, __fsub_rn(u, v)};
+  for (int d = 0; d < 16; ++d) best[d] = 0ull;
+  int stay_cnt = 0;
 #pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      const unsigned long long k = ((unsigned long long)float_to_ordered(val[d]) << 32) | (unsigned)(~(unsigned)i);
-      best[d] = k > best[d] ? k : best[d];
+  for (int r = 0; r < PL_TILE / 256; ++r) {
+    const int j = blockIdx.x * PL_TILE + r * 256 + threadIdx.x;
+    const bool live = j < m;
+    const float4 p = live ? pts[pl_at(rem, j)] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool stay = live && pl_stays<FIRST>(p, c, thr);
+    stay_cnt += __popc(__ballot_sync(0xffffffffu, stay));
+    if (FIRST) continue;
+    const bool in = live && !stay;
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (!b) continue;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&dev->n_in, __popc(b));
+    base = __shfl_sync(0xffffffffu, base, 0) + __popc(b & lanemask_lt());
+    if (in) {
+      float u = __fadd_rn(__fadd_rn(__fmul_rn(p.x, e1.x), __fmul_rn(p.y, e1.y)), __fmul_rn(p.z, e1.z));
+      float v = __fadd_rn(__fadd_rn(__fmul_rn(p.x, e2.x), __fmul_rn(p.y, e2.y)), __fmul_rn(p.z, e2.z));
+      u = __fadd_rn(u, 0.f);
+      v = __fadd_rn(v, 0.f);
+      uv[base] = make_float2(u, v);
+#pragma unroll
+      for (int d = 0; d < 16; ++d) {
+        const unsigned long long key =
+            ((unsigned long long)float_to_ordered(pl_dir(d, u, v)) << 32) | (unsigned)base;
+        best[d] = key > best[d] ? key : best[d];
+      }
     }
   }
+  if (lane == 0 && stay_cnt) atomicAdd(&s_stay, stay_cnt);
+  if (!FIRST) {
 #pragma unroll
-  for (int d = 0; d < 8; ++d) {
+    for (int d = 0; d < 16; ++d) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long x = __shfl_xor_sync(0xffffffffu, best[d], o);
-      best[d] = x > best[d] ? x : best[d];
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, best[d], o);
+        best[d] = x > best[d] ? x : best[d];
+      }
+      if (lane == 0 && best[d]) atomicMax(&s_ext[d], best[d]);
     }
-    if ((threadIdx.x & 31) == 0 && best[d]) atomicMax(ext + d, best[d]);
   }
+  __syncthreads();
+  if (threadIdx.x == 0) tile_cnt[blockIdx.x] = s_stay;
+  if (!FIRST && threadIdx.x < 16 && s_ext[threadIdx.x]) atomicMax(&dev->ext[threadIdx.x], s_ext[threadIdx.x]);
 }
 
 __device__ __forceinline__ double pl_cross(float2 o, float2 a, float2 b) {
@@ -241,65 +307,216 @@ __device__ __forceinline__ double pl_cross(float2 o, float2 a, float2 b) {
   return __dsub_rn(__dmul_rn(ax, by), __dmul_rn(ay, bx));
 }
 
-// keep[i] = 0 when point i is strictly inside the octagon of the extreme
-// points (then it is no hull vertex), 1 otherwise
-__global__ void k_pl_filter(const float2* __restrict__ uv, const int* __restrict__ d_n,
-                            const unsigned long long* __restrict__ ext, uint32_t* __restrict__ keep) {
-  const int n = *d_n;
-  float2 E[8];
-  int ne = 0;
-  if (n > 0) {
-    for (int d = 0; d < 8; ++d) {
-      const float2 p = uv[~(unsigned)(ext[d] & 0xffffffffull)];
-      if (ne == 0 || p.x != E[ne - 1].x || p.y != E[ne - 1].y) E[ne++] = p;
+// Whether o, a, b turn left (cross > 0): the float cross where its error bound
+// decides (a few parts in 10^7 of its two products), else the exact one.  sign
+// 0 stands for a cross of exactly 0 (collinear).
+__device__ __forceinline__ int pl_turn(float2 o, float2 a, float2 b) {
+  const float l = (a.x - o.x) * (b.y - o.y), r = (a.y - o.y) * (b.x - o.x);
+  const float d = l - r, e = 1.0e-6f * (fabsf(l) + fabsf(r)) + 1.0e-30f;
+  if (d > e) return 1;
+  if (d < -e) return -1;
+  const double x = pl_cross(o, a, b);
+  return x > 0.0 ? 1 : (x < 0.0 ? -1 : 0);
+}
+
+// The points that stay close up in order (offset: the tiles before, then the
+// tile's own ranks); and of the inliers those not strictly inside the polygon
+// of the extreme points are appended to su, in any order.
+template <bool FIRST>
+__global__ void __launch_bounds__(256) k_pl_rest(const float4* __restrict__ pts, const int* __restrict__ rem, int m,
+                                                 float4 c, float thr, const int* __restrict__ tile_cnt,
+                                                 int* __restrict__ out, const float2* __restrict__ uv,
+                                                 float2* __restrict__ su, PlDev* __restrict__ dev,
+                                                 PlHost* __restrict__ host) {
+  constexpr int R = PL_TILE / 256;
+  __shared__ int s_cnt[R][8], s_before[8];
+  __shared__ float2 E[16];
+  __shared__ int s_ne;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int before = 0;
+  for (int t = threadIdx.x; t < blockIdx.x; t += 256) before += tile_cnt[t];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (lane == 0) s_before[warp] = before;
+  int id[R];
+  unsigned bal[R];
+  bool stay[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int j = blockIdx.x * PL_TILE + r * 256 + threadIdx.x;
+    const bool live = j < m;
+    id[r] = live ? pl_at(rem, j) : 0;
+    stay[r] = live && pl_stays<FIRST>(pts[id[r]], c, thr);
+    bal[r] = __ballot_sync(0xffffffffu, stay[r]);
+    if (lane == 0) s_cnt[r][warp] = __popc(bal[r]);
+  }
+  if (!FIRST && warp == 0) {  // the polygon, duplicate corners left out
+    const bool any = dev->n_in > 0;
+    if (any && lane < 16) E[lane] = uv[(unsigned)(dev->ext[lane] & 0xffffffffull)];
+    __syncwarp();
+    if (lane == 0) {
+      int ne = 0;
+      for (int d = 0; any && d < 16; ++d) {
+        const float2 p = E[d];
+        if (ne == 0 || p.x != E[ne - 1].x || p.y != E[ne - 1].y) E[ne++] = p;
+      }
+      while (ne > 1 && E[ne - 1].x == E[0].x && E[ne - 1].y == E[0].y) --ne;
+      s_ne = ne;
     }
-    while (ne > 1 && E[ne - 1].x == E[0].x && E[ne - 1].y == E[0].y) --ne;
   }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  __syncthreads();
+  int off = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) off += s_before[w];
+  int at = off;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    int o = at;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      o += w < warp ? s_cnt[r][w] : 0;
+      at += s_cnt[r][w];
+    }
+    if (stay[r]) out[o + __popc(bal[r] & lanemask_lt())] = id[r];
+  }
+  total = at;
+  if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) host->m_rest = total;
+  if (FIRST) return;
+  const int n = dev->n_in, ne = s_ne;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ((n + 31) & ~31); i += gridDim.x * blockDim.x) {
+    const float2 p = i < n ? uv[i] : make_float2(0.f, 0.f);
     bool inside = ne >= 3;
-    const float2 p = uv[i];
-    for (int e = 0; e < ne && inside; ++e) inside = pl_cross(E[e], E[(e + 1) % ne], p) > 0.0;
-    keep[i] = inside ? 0u : 1u;
+    for (int e = 0; e < ne && inside; ++e) inside = pl_turn(E[e], E[e + 1 < ne ? e + 1 : 0], p) > 0;
+    const bool keep = i < n && !inside;
+    const unsigned b = __ballot_sync(0xffffffffu, keep);
+    if (!b) continue;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&dev->n_left, __popc(b));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (keep) su[base + __popc(b & lanemask_lt())] = p;
   }
 }
 
-__global__ void k_pl_gather_uv(const float2* __restrict__ uv, const uint32_t* __restrict__ keep,
-                               const uint32_t* __restrict__ pos, const int* __restrict__ d_n, float2* __restrict__ out) {
-  const int n = *d_n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (keep[i]) out[pos[i]] = uv[i];
+// Half of Andrew's monotone chain (one thread): the left-turning chain over
+// at(0), ..., at(n - 1) into H; returns its length.  The last two vertices are
+// held in registers.  H may be where at reads from: the chain is never longer
+// than what has been read.
+template <typename F, typename G>
+__device__ __forceinline__ int pl_half(int n, F at, G put_get) {
+  int h = 0;
+  float2 p1 = make_float2(0.f, 0.f), p2 = p1;  // H[h - 1], H[h - 2]
+  for (int i = 0; i < n; ++i) {
+    const float2 p = at(i);
+    while (h >= 2 && pl_turn(p2, p1, p) <= 0) {
+      --h;
+      p1 = p2;
+      if (h >= 2) p2 = *put_get(h - 2);
+    }
+    *put_get(h) = p;
+    ++h;
+    p2 = p1;
+    p1 = p;
+  }
+  return h;
+}
+// The hull from its halves, the lower one from left to right and the upper
+// one from right to left: each but its last point (the other's first).  A
+// single point is its own hull.
+__device__ __forceinline__ int pl_join(int lower, int upper) {
+  const int h = lower + upper - 1;
+  return h > 1 ? h - 1 : h;
 }
 
-// radix keys: the survivors' v, then (second pass) their u in that order
-__global__ void k_pl_keys_v(const float2* __restrict__ su, const int* __restrict__ d_n, uint32_t* __restrict__ k) {
-  const int n = *d_n;
+// Hull of at most PL_HULL_CAP points: a bitonic sort by (u, v) in shared
+// memory; then 32 lanes each reduce a run of the points to its own half chain
+// (a point off the hull of its run is off the hull), and one thread chains
+// what is left; warp 0 does the lower half and warp 1 the upper.  One thread
+// chaining all of a few hundred points took 53 us, this 22 us.  Resets the
+// round's device words.
+__global__ void __launch_bounds__(512) k_pl_hull(const float2* __restrict__ su, PlDev* __restrict__ dev,
+                                                 PlHost* __restrict__ host) {
+  __shared__ unsigned long long key[PL_HULL_CAP];
+  __shared__ float2 s_half[2][PL_HULL_CAP];
+  __shared__ int s_h[2];
+  const int n = dev->n_left, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncthreads();  // everyone has it: it is reset below
+  if (threadIdx.x < 16) dev->ext[threadIdx.x] = 0ull;
+  if (threadIdx.x == 0) {
+    dev->n_in = dev->n_left = 0;
+    host->n_left = n;
+    if (n > PL_HULL_CAP) host->hull = -1;
+  }
+  if (n > PL_HULL_CAP) return;
+  int P = 32;
+  while (P < n) P <<= 1;
+  for (int i = threadIdx.x; i < P; i += blockDim.x)
+    key[i] = i < n ? ((unsigned long long)float_to_ordered(su[i].x) << 32) | float_to_ordered(su[i].y) : ~0ull;
+  __syncthreads();
+  for (int k = 2; k <= P; k <<= 1)
+    for (int jj = k >> 1; jj > 0; jj >>= 1) {
+      for (int t = threadIdx.x; t < (P >> 1); t += blockDim.x) {
+        const int i = ((t & ~(jj - 1)) << 1) | (t & (jj - 1)), l = i | jj;
+        const unsigned long long x = key[i], y = key[l];
+        if ((x > y) == ((i & k) == 0)) {
+          key[i] = y;
+          key[l] = x;
+        }
+      }
+      __syncthreads();
+    }
+  if (warp < 2) {
+    float2* half = s_half[warp];
+    const int run = (n + 31) / 32, b = min(n, lane * run), len = min(n - b, run);
+    auto at = [&](int i) {  // the upper half goes from right to left
+      const unsigned long long x = key[warp == 0 ? i : n - 1 - i];
+      return make_float2(ordered_to_float((unsigned)(x >> 32)), ordered_to_float((unsigned)x));
+    };
+    const int h = pl_half(len, [&](int i) { return at(b + i); }, [&](int i) { return half + b + i; });
+    // close the runs up (a lane writes at or before its own run, after every
+    // lane before it has read)
+    int to = h;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, to, o);
+      if (lane >= o) to += t;
+    }
+    const int total = __shfl_sync(0xffffffffu, to, 31);
+    to -= h;
+    for (int l = 0; l < 32; ++l) {
+      const int lh = __shfl_sync(0xffffffffu, h, l), lb = min(n, l * run), lt = __shfl_sync(0xffffffffu, to, l);
+      for (int i0 = 0; i0 < lh; i0 += 32) {
+        const float2 v = half[lb + min(i0 + lane, lh - 1)];
+        __syncwarp();
+        if (i0 + lane < lh) half[lt + i0 + lane] = v;
+        __syncwarp();
+      }
+    }
+    if (lane == 0) s_h[warp] = pl_half(total, [&](int i) { return half[i]; }, [&](int i) { return half + i; });
+  }
+  __syncthreads();
+  const int lower = s_h[0], h = n > 0 ? pl_join(lower, s_h[1]) : 0;
+  for (int i = threadIdx.x; i < min(h, PL_HULL_OUT); i += blockDim.x)
+    host->uv[i] = i < lower ? s_half[0][i] : s_half[1][i - lower + 1];
+  if (threadIdx.x == 0) host->hull = h > PL_HULL_OUT ? -1 : h;
+}
+
+// radix keys of a larger set: the points' v, then (second pass) their u in
+// that order
+__global__ void k_pl_keys_v(const float2* __restrict__ su, int n, uint32_t* __restrict__ k) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) k[i] = float_to_ordered(su[i].y);
 }
-__global__ void k_pl_keys_u(const float2* __restrict__ su, const uint32_t* __restrict__ order, const int* __restrict__ d_n,
+__global__ void k_pl_keys_u(const float2* __restrict__ su, const uint32_t* __restrict__ order, int n,
                             uint32_t* __restrict__ k) {
-  const int n = *d_n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     k[i] = float_to_ordered(su[order[i]].x);
 }
-
-// Andrew's monotone chain over the survivors in (u, v) order (one thread)
-__global__ void k_pl_chain(const float2* __restrict__ su, const uint32_t* __restrict__ order, const int* __restrict__ d_n,
-                           float2* __restrict__ H, int* __restrict__ h_out) {
+__global__ void k_pl_chain(const float2* __restrict__ su, const uint32_t* __restrict__ order, int n,
+                           float2* __restrict__ H, PlHost* __restrict__ host) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int n = *d_n;
-  int h = 0;
-  for (int i = 0; i < n; ++i) {
-    const float2 p = su[order[i]];
-    while (h >= 2 && pl_cross(H[h - 2], H[h - 1], p) <= 0.0) --h;
-    H[h++] = p;
-  }
-  for (int i = n - 2, lo = h + 1; i >= 0; --i) {
-    const float2 p = su[order[i]];
-    while (h >= lo && pl_cross(H[h - 2], H[h - 1], p) <= 0.0) --h;
-    H[h++] = p;
-  }
-  if (h > 1) --h;
-  *h_out = h;
+  const int lower = pl_half(n, [&](int i) { return su[order[i]]; }, [&](int i) { return H + i; });
+  float2* U = H + lower - 1;  // starts at the lower half's last point, the same
+  const int upper = pl_half(n, [&](int i) { return su[order[n - 1 - i]]; }, [&](int i) { return U + i; });
+  host->hull = pl_join(lower, upper);
 }
 
 // get_Vector3D for each keypoint over the kept surfaces, in list order
@@ -342,11 +559,8 @@ static int pl_blocks(int n) {
   return b < 1 ? 1 : b;
 }
 
-static rtr_status pl_read(cudaStream_t st, void* h, const void* d, size_t bytes) {
-  RTR_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, st));
-  RTR_CUDA(cudaStreamSynchronize(st));
-  return RTR_OK;
-}
+// Tiles of the ordered compaction of m points.
+static int pl_tiles(int m) { return m > 0 ? (m + PL_TILE - 1) / PL_TILE : 1; }
 
 }  // namespace rtr
 
@@ -376,32 +590,29 @@ rtr_status rtr_plane_segment(rtr_context* ctx, const float* d_pts, int n, const 
   if (n == 0) return RTR_OK;
   cudaStream_t st = (cudaStream_t)stream;
   RTR_CUDA(cudaSetDevice(ctx->device));
-  const int nc = n + 1;
+  // page-locked words that the kernels write, kept by the context
+  if (!ctx->plane_host && cudaMallocHost(&ctx->plane_host, sizeof(PlHost)) != cudaSuccess) {
+    (void)cudaGetLastError();
+    ctx->plane_host = nullptr;
+    return fail(RTR_ERR_OOM, "rtr_plane_segment: page-locked words");
+  }
+  PlHost* const host = static_cast<PlHost*>(ctx->plane_host);
   ScratchPlan plan;
-  const size_t o_f = plan.add<uint32_t>(nc), o_g = plan.add<uint32_t>(nc), o_p = plan.add<uint32_t>(nc),
-               o_q = plan.add<uint32_t>(nc), o_t = plan.add<uint32_t>(scan_tiles(nc));
-  const size_t o_rem = plan.add<int>(nc), o_rem2 = plan.add<int>(nc);
-  const size_t o_coef = plan.add<float4>(PL_SLOTS), o_valid = plan.add<int>(PL_SLOTS), o_cnt = plan.add<int>(PL_SLOTS);
-  const size_t o_sums = plan.add<double>(16), o_ints = plan.add<int>(16), o_ext = plan.add<unsigned long long>(8);
-  const size_t o_uv = plan.add<float2>(nc), o_su = plan.add<float2>(nc), o_hull = plan.add<float2>(2 * (size_t)nc + 2);
-  const size_t o_k0 = plan.add<uint32_t>(nc), o_v0 = plan.add<uint32_t>(nc), o_k1 = plan.add<uint32_t>(nc),
-               o_v1 = plan.add<uint32_t>(nc), o_hist = plan.add<uint32_t>(radix_hist_entries(nc));
+  const size_t o_dev = plan.add<PlDev>(1), o_tile = plan.add<int>(pl_tiles(n));
+  const size_t o_rem = plan.add<int>(n), o_rem2 = plan.add<int>(n);
+  const size_t o_part = plan.add<double>(9 * PL_PARTIALS), o_pn = plan.add<int>(PL_PARTIALS);
+  const size_t o_uv = plan.add<float2>(n), o_su = plan.add<float2>(n), o_hull = plan.add<float2>(2 * (size_t)n + 4);
+  const size_t o_k0 = plan.add<uint32_t>(n), o_v0 = plan.add<uint32_t>(n), o_k1 = plan.add<uint32_t>(n),
+               o_v1 = plan.add<uint32_t>(n), o_hist = plan.add<uint32_t>(radix_hist_entries(n));
   Scratch s;
   RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
   char* B = s.base;
-  uint32_t* flags = reinterpret_cast<uint32_t*>(B + o_f);
-  uint32_t* flags2 = reinterpret_cast<uint32_t*>(B + o_g);
-  uint32_t* pos = reinterpret_cast<uint32_t*>(B + o_p);
-  uint32_t* pos2 = reinterpret_cast<uint32_t*>(B + o_q);
-  uint32_t* tiles = reinterpret_cast<uint32_t*>(B + o_t);
+  PlDev* dev = reinterpret_cast<PlDev*>(B + o_dev);
+  int* tile_cnt = reinterpret_cast<int*>(B + o_tile);
   int* rem = reinterpret_cast<int*>(B + o_rem);
   int* rem2 = reinterpret_cast<int*>(B + o_rem2);
-  float4* coef = reinterpret_cast<float4*>(B + o_coef);
-  int* valid = reinterpret_cast<int*>(B + o_valid);
-  int* cnt = reinterpret_cast<int*>(B + o_cnt);
-  double* sums = reinterpret_cast<double*>(B + o_sums);
-  int* ints = reinterpret_cast<int*>(B + o_ints);  // [0] remaining, [1] refit n, [2] inliers, [3] kept out, [4] survivors, [5] hull
-  unsigned long long* ext = reinterpret_cast<unsigned long long*>(B + o_ext);
+  double* part = reinterpret_cast<double*>(B + o_part);
+  int* part_n = reinterpret_cast<int*>(B + o_pn);
   float2* uv = reinterpret_cast<float2*>(B + o_uv);
   float2* su = reinterpret_cast<float2*>(B + o_su);
   float2* hull = reinterpret_cast<float2*>(B + o_hull);
@@ -416,88 +627,83 @@ rtr_status rtr_plane_segment(rtr_context* ctx, const float* d_pts, int n, const 
   // attribute belongs to the current device)
   RTR_CUDA(cudaFuncSetAttribute(k_pl_refit, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(PL_PARTIALS * 9 * sizeof(double))));
+  RTR_CUDA(cudaMemsetAsync(dev, 0, sizeof(PlDev), st));
 
   // the finite points, in index order
-  k_pl_finite<<<pl_blocks(n), 256, 0, st>>>(pts, n, flags);
-  scan_exclusive(flags, pos, tiles, nc, n, nullptr, reinterpret_cast<uint32_t*>(ints), st);
-  k_pl_compact<<<pl_blocks(n), 256, 0, st>>>(flags, pos, nullptr, n, 1u, rem);
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  k_pl_select<true><<<pl_tiles(n), 256, 0, st>>>(pts, nullptr, n, zero4, 0.f, zero4, zero4, tile_cnt, nullptr, dev);
+  k_pl_rest<true><<<pl_tiles(n), 256, 0, st>>>(pts, nullptr, n, zero4, 0.f, tile_cnt, rem, nullptr, nullptr, dev, host);
   RTR_LAUNCHED(2);
-  int m = 0;
-  RTR_TRY(pl_read(st, &m, ints, sizeof(int)));
+  RTR_CUDA(cudaGetLastError());
+  RTR_CUDA(cudaStreamSynchronize(st));
+  int m = host->m_rest;
   const int nr_points = m;
   const int max_slots = 11 * prm->max_iterations;
   int np = 0;
   for (int round = 0; (double)m > prm->remain_frac * (double)nr_points && m >= 3; ++round) {
     // RANSAC, batch by batch until the walk ends
     PlaneWalk w;
-    float4 bc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 bc = zero4;
     for (int base = 0; base < max_slots && !w.done; base += PL_SLOTS) {
       const int ns = max_slots - base < PL_SLOTS ? max_slots - base : PL_SLOTS;
-      RTR_CUDA(cudaMemsetAsync(cnt, 0, PL_SLOTS * sizeof(int), st));
-      k_pl_slots<<<1, PL_SLOTS, 0, st>>>(pts, rem, m, prm->seed, round, base, ns, coef, valid);
-      k_pl_count<<<pl_blocks((m + 3) / 4), 256, 0, st>>>(pts, rem, m, coef, valid, ns, prm->distance, cnt);
-      RTR_LAUNCHED(2);
-      int hv[PL_SLOTS], hc[PL_SLOTS];
-      float4 hcoef[PL_SLOTS];
-      RTR_CUDA(cudaMemcpyAsync(hv, valid, ns * sizeof(int), cudaMemcpyDeviceToHost, st));
-      RTR_CUDA(cudaMemcpyAsync(hc, cnt, ns * sizeof(int), cudaMemcpyDeviceToHost, st));
-      RTR_CUDA(cudaMemcpyAsync(hcoef, coef, ns * sizeof(float4), cudaMemcpyDeviceToHost, st));
+      k_pl_score<<<pl_blocks(m), 256, 0, st>>>(pts, rem, m, prm->seed, round, base, ns, prm->distance, dev, host);
+      RTR_LAUNCHED(1);
+      RTR_CUDA(cudaGetLastError());
       RTR_CUDA(cudaStreamSynchronize(st));
       w.slot = 0;
       w.base = base;
       const int prev_best = w.best;
-      plane_ransac_walk(hv, hc, ns, m, prm->max_iterations, &w);
-      if (w.best != prev_best && w.best >= base) bc = hcoef[w.best - base];
+      plane_ransac_walk(host->valid, host->count, ns, m, prm->max_iterations, &w);
+      if (w.best != prev_best && w.best >= base) bc = host->coef[w.best - base];
     }
     if (w.best < 0) break;
     // least-squares refit over the best sample's inliers
-    k_pl_refit<<<1, PL_PARTIALS, PL_PARTIALS * 9 * sizeof(double), st>>>(pts, rem, m, bc, prm->distance, sums, ints + 1);
+    k_pl_refit<<<PL_REFIT_BLOCKS, 256, PL_PARTIALS * 9 * sizeof(double), st>>>(pts, rem, m, bc, prm->distance, part,
+                                                                             part_n, dev, host);
     RTR_LAUNCHED(1);
-    double h_sums[9];
-    int n_fit = 0;
-    RTR_CUDA(cudaMemcpyAsync(h_sums, sums, sizeof(h_sums), cudaMemcpyDeviceToHost, st));
-    RTR_CUDA(cudaMemcpyAsync(&n_fit, ints + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    RTR_CUDA(cudaGetLastError());
     RTR_CUDA(cudaStreamSynchronize(st));
     float c_in[4] = {bc.x, bc.y, bc.z, bc.w}, c[4];
     int flat = 1;
-    plane_refit(h_sums, n_fit, c_in, c, &flat);
+    plane_refit(host->sums, host->n_fit, c_in, c, &flat);
     const float4 cf = make_float4(c[0], c[1], c[2], c[3]);
     float e1[3], e2[3];
     plane_basis(c, e1, e2);
-    // the refitted plane's inliers, their projections, the rest
-    k_pl_select<<<pl_blocks(m), 256, 0, st>>>(pts, rem, m, cf, prm->distance, flags, flags2);
-    scan_exclusive(flags, pos, tiles, nc, m, nullptr, reinterpret_cast<uint32_t*>(ints + 2), st);
-    scan_exclusive(flags2, pos2, tiles, nc, m, nullptr, reinterpret_cast<uint32_t*>(ints + 3), st);
-    k_pl_project<<<pl_blocks(m), 256, 0, st>>>(pts, rem, m, flags, pos, make_float4(e1[0], e1[1], e1[2], 0.f),
-                                               make_float4(e2[0], e2[1], e2[2], 0.f), uv);
-    // hull: octagon filter, (u, v) sort, monotone chain
-    RTR_CUDA(cudaMemsetAsync(ext, 0, 8 * sizeof(unsigned long long), st));
-    k_pl_extremes<<<pl_blocks(m), 256, 0, st>>>(uv, ints + 2, ext);
-    k_pl_filter<<<pl_blocks(m), 256, 0, st>>>(uv, ints + 2, ext, k0);
-    scan_exclusive(k0, k1, tiles, nc, m, ints + 2, reinterpret_cast<uint32_t*>(ints + 4), st);
-    k_pl_gather_uv<<<pl_blocks(m), 256, 0, st>>>(uv, k0, k1, ints + 2, su);
-    k_pl_keys_v<<<pl_blocks(m), 256, 0, st>>>(su, ints + 4, k0);
-    uint32_t *ks, *vs;
-    radix_sort_pairs(k0, v0, k1, v1, hist, nc, m, ints + 4, 32, true, st, &ks, &vs);
-    // second, stable pass by u over the first pass's order
-    uint32_t* ka = ks == k0 ? k1 : k0;
-    uint32_t* va = vs == v0 ? v1 : v0;
-    k_pl_keys_u<<<pl_blocks(m), 256, 0, st>>>(su, vs, ints + 4, ka);
-    RTR_CUDA(cudaMemcpyAsync(va, vs, sizeof(uint32_t) * (size_t)m, cudaMemcpyDeviceToDevice, st));
-    uint32_t *ks2, *vs2;
-    radix_sort_pairs(ka, va, ka == k0 ? k1 : k0, va == v0 ? v1 : v0, hist, nc, m, ints + 4, 32, false, st, &ks2,
-                     &vs2);
-    k_pl_chain<<<1, 32, 0, st>>>(su, vs2, ints + 4, hull, ints + 5);
-    RTR_LAUNCHED(8);
-    int hi[6];
-    RTR_CUDA(cudaMemcpyAsync(hi, ints, sizeof(hi), cudaMemcpyDeviceToHost, st));
+    // the refitted plane's inliers, what remains, the hull
+    k_pl_select<false><<<pl_tiles(m), 256, 0, st>>>(pts, rem, m, cf, prm->distance, make_float4(e1[0], e1[1], e1[2], 0.f),
+                                                    make_float4(e2[0], e2[1], e2[2], 0.f), tile_cnt, uv, dev);
+    k_pl_rest<false><<<pl_tiles(m), 256, 0, st>>>(pts, rem, m, cf, prm->distance, tile_cnt, rem2, uv, su, dev, host);
+    k_pl_hull<<<1, 512, 0, st>>>(su, dev, host);
+    RTR_LAUNCHED(3);
+    RTR_CUDA(cudaGetLastError());
     RTR_CUDA(cudaStreamSynchronize(st));
-    const int ni = hi[2], nk = hi[3], nh = hi[5];
+    const int nk = host->m_rest, ni = m - nk;
     if (ni == 0) break;
-    std::vector<float> hv((size_t)2 * (nh > 0 ? nh : 1));
-    if (nh > 0) RTR_TRY(pl_read(st, hv.data(), hull, sizeof(float2) * (size_t)nh));
+    std::vector<float2> far_uv;
+    if (host->hull < 0) {  // too many points, or vertices, for the hull kernel
+      const int nl = host->n_left;
+      k_pl_keys_v<<<pl_blocks(nl), 256, 0, st>>>(su, nl, k0);
+      uint32_t *ks, *vs;
+      radix_sort_pairs(k0, v0, k1, v1, hist, nl, nl, nullptr, 32, true, st, &ks, &vs);
+      // second, stable pass by u over the first pass's order
+      uint32_t* ka = ks == k0 ? k1 : k0;
+      uint32_t* va = vs == v0 ? v1 : v0;
+      k_pl_keys_u<<<pl_blocks(nl), 256, 0, st>>>(su, vs, nl, ka);
+      RTR_CUDA(cudaMemcpyAsync(va, vs, sizeof(uint32_t) * (size_t)nl, cudaMemcpyDeviceToDevice, st));
+      uint32_t *ks2, *vs2;
+      radix_sort_pairs(ka, va, ka == k0 ? k1 : k0, va == v0 ? v1 : v0, hist, nl, nl, nullptr, 32, false, st, &ks2,
+                       &vs2);
+      k_pl_chain<<<1, 32, 0, st>>>(su, vs2, nl, hull, host);
+      RTR_LAUNCHED(3);
+      RTR_CUDA(cudaGetLastError());
+      RTR_CUDA(cudaStreamSynchronize(st));
+      far_uv.resize((size_t)host->hull);
+      RTR_CUDA(cudaMemcpyAsync(far_uv.data(), hull, sizeof(float2) * far_uv.size(), cudaMemcpyDeviceToHost, st));
+      RTR_CUDA(cudaStreamSynchronize(st));
+    }
+    const int nh = host->hull;
     double area = 0.0, perim = 0.0;
-    hull_measure(hv.data(), nh, &area, &perim);
+    hull_measure(reinterpret_cast<const float*>(far_uv.empty() ? host->uv : far_uv.data()), nh, &area, &perim);
     if (np < max_surfaces) {
       rtr_surface& S = h_surfaces[np];
       memset(&S, 0, sizeof(S));
@@ -511,15 +717,11 @@ rtr_status rtr_plane_segment(rtr_context* ctx, const float* d_pts, int n, const 
       S.kept = S.is_vertical >= 0 && area >= prm->min_area;
     }
     ++np;
-    // the rest stays, in order
-    k_pl_compact<<<pl_blocks(m), 256, 0, st>>>(flags2, pos2, rem, m, 1u, rem2);
-    RTR_LAUNCHED(1);
     int* t = rem;
     rem = rem2;
     rem2 = t;
     m = nk;
   }
-  RTR_CUDA(cudaStreamSynchronize(st));
   *h_n_surfaces = np < max_surfaces ? np : max_surfaces;
   if (np > max_surfaces)
     return fail(RTR_ERR_CAPACITY, "rtr_plane_segment: %d planes extracted, room for %d", np, max_surfaces);

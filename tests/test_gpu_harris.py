@@ -38,3 +38,19 @@ def test_harris_on_shapes_and_main_clouds(ctx, rtr, flags):
 def test_harris_on_the_room(ctx, rtr):
     scene, _, _ = rtr.synth_room(1)
     assert _check(ctx, rtr, scene) > 0
+
+
+@pytest.mark.parametrize("n,tile", [(1, 1), (33, 1), (1023, 1), (1025, 1), (131072, 45), (131073, 45)])
+def test_harris_bitmap_edges(ctx, rtr, n, tile):
+    """Clouds at the edges of the bitmap's words and of its largest size (the
+    next size lists and sorts instead): a chair, or a lattice of chairs far
+    apart so that no neighbourhood overflows."""
+    if tile == 1:
+        pts = rtr.synth_shape(rtr.CHAIR, n, 5)
+    else:
+        pts = np.concatenate([rtr.synth_shape(rtr.CHAIR, -(-n // tile), 5 + k) for k in range(tile)])[:n].copy()
+        k = np.arange(n) // -(-n // tile)
+        pts[:, 0] += (2 * (k % 7)).astype(np.float32)
+        pts[:, 1] += (2 * (k // 7)).astype(np.float32)
+        pts = pts[np.random.default_rng(1).permutation(n)]
+    _check(ctx, rtr, pts)

@@ -80,3 +80,25 @@ def test_vector3d_and_area_gate_equal_oracle(ctx, rtr):
     rpi = O.ref_correspond(km, mn.cpu().numpy(), ks, sn.cpu().numpy(), sc.cpu().numpy(), mv3=mv3.cpu().numpy(),
                            sv3=sv3.cpu().numpy())
     assert np.array_equal(pi.cpu().numpy(), rpi)
+
+
+def test_plane_hulls_at_their_limits_equal_oracle(ctx, rtr):
+    """A disc whose rim keeps more points than the hull kernel sorts (2,048)
+    and more hull vertices than come back through page-locked memory (1,024);
+    a rectangle of lattice points, whose edges are collinear runs; tiny and
+    duplicate-laden clouds."""
+    rng = np.random.default_rng(5)
+    a = np.sort(rng.uniform(0, 2 * np.pi, 40000))
+    disc = np.zeros((60000, 4), np.float32)
+    disc[:40000, 0], disc[:40000, 1] = 50 * np.cos(a), 50 * np.sin(a)
+    rad, b = 49 * np.sqrt(rng.uniform(0, 1, 20000)), rng.uniform(0, 2 * np.pi, 20000)
+    disc[40000:, 0], disc[40000:, 1] = rad * np.cos(b), rad * np.sin(b)
+    g = np.stack(np.meshgrid(np.arange(40), np.arange(30), indexing="ij"), -1).reshape(-1, 2) * 0.0625
+    lattice = np.zeros((g.shape[0], 4), np.float32)
+    lattice[:, :2] = g
+    lattice[:, 2] = 1.0
+    tiny = np.zeros((3, 4), np.float32)
+    tiny[1, 0] = tiny[2, 1] = 1.0
+    for pts in (disc, lattice, tiny, np.repeat(tiny, 700, 0), np.zeros((64, 4), np.float32), lattice[:1025]):
+        ref, _ = O.plane_segment(pts)
+        _same(ctx.plane_segment(_dev(pts)), ref)
