@@ -75,9 +75,10 @@ const char* rtr_version(void);
  *                    set that lost a member is recomputed by a new round
  *                    instead of in place by the walk (same clusters;
  *                    slower; 0 restores the default);
- *   "gc_inline"      sets the grouping walk recomputes in place per round
- *                    before it hands the rest of the window back to the
- *                    parallel phase (1..4096; default 16);
+ *   "gc_inline"      times per round the grouping walk recomputes sets in
+ *                    place (up to eight at once) before it hands the rest of
+ *                    the window back to the parallel phase (1..4096;
+ *                    default 8);
  *   "scene_grid_mm"  cell edge (mm) of the recognition's scene grid, used by
  *                    verification and ICP refinement (default: 1.5 x the ICP
  *                    distance; the table's size limit may widen it);

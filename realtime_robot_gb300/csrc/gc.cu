@@ -16,8 +16,8 @@
 // window of upcoming seeds under the current taken state, then one warp walks
 // the seeds in order and commits.  A stored set stays exact while none of its
 // members is taken (removing rejected candidates never changes a greedy
-// walk); the walk stops at the first seed whose set lost a member and the
-// next window starts there.  No host round trip inside the grouping.
+// walk); the walk recomputes a set that lost a member in place, or stops there
+// and the next window starts with it.  No host round trip inside the grouping.
 #include "common.cuh"
 #include "pose.cuh"
 #include "grid.cuh"
@@ -51,7 +51,7 @@ struct GcDev {
 
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 
@@ -79,6 +79,19 @@ __device__ __forceinline__ bool gc_consistent(float4 am, float4 as, float4 bm, f
   if (diff > gc + tol) return false;
   if (diff < gc - tol) return true;
   return !(fabsf(__fsub_rn(__fsqrt_rn(u), __fsqrt_rn(v))) > gc);
+}
+
+// The same test without a branch: 1 or 0 where the cheap forms are certain,
+// -1 where only the exact one (below) answers.
+__device__ __forceinline__ int gc_consistent_fast(float4 am, float4 as, float4 bm, float4 bs, float gc, float r2max) {
+  const float v = dist2_exact(as, bs), u = dist2_exact(am, bm);
+  const float a = sqrt_approx(u), b = sqrt_approx(v);
+  const float diff = fabsf(a - b);
+  const float tol = 1.0e-5f * (a + b) + 1.0e-6f;
+  return (v > r2max || diff > gc + tol) ? 0 : (diff < gc - tol ? 1 : -1);
+}
+__device__ __forceinline__ bool gc_consistent_exact(float4 am, float4 as, float4 bm, float4 bs, float gc) {
+  return !(fabsf(__fsub_rn(__fsqrt_rn(dist2_exact(am, bm)), __fsqrt_rn(dist2_exact(as, bs)))) > gc);
 }
 
 // Spatial pruning of the seed tests.  A candidate b passes seed a only if
@@ -242,6 +255,8 @@ struct GcCoop {
   const GridMeta* mbox;  // bounding box of the model endpoints
   int* need;           // [win] seeds whose set is computed this round
   unsigned* mask;      // [win][nwp] seed-test pass bits, one row per needed seed
+  unsigned* summ;      // [win][nsp] bit w of a row: word w of the seed's mask row is not zero
+  int nsp;             // words per summary row
   int win;             // seeds in the first window
   int win_max;         // seeds a window may grow to (the need/mask capacity)
   int nwp;             // words per mask row (C/32 rounded up to a multiple of 4)
@@ -304,6 +319,98 @@ __device__ __forceinline__ float4 shfl4(float4 v, int src) {
 constexpr int GC_PEND = 64;  // candidates staged per warp before admission
 constexpr int GC_PREF = 7;   // mask loads in flight per lane during admission
 
+// Greedy admission of a whole pass list held by the warp: lane l has entries
+// l, l + 32, ... (endpoints in cm and cs, sorted position in cm.w; bit k of
+// alive: entry 32 k + l takes part).  Member 0, the seed, every entry has
+// passed.  The lowest entry alive joins, put(count, position) on its lane, and
+// all others are tested against it at once: the same set as taking the entries
+// in order and testing each against all members so far, in as many steps as
+// the set has members (taking 32 entries at a time against every member cost
+// 3.3 us a list of 140).  Once at most 32 entries are alive they move to one
+// per lane (through tmp).  Stops early when those alive cannot bring the set
+// to thresh members: what has joined until then is the start of the set, and
+// as long as none of it is taken the set stays too small.
+constexpr int GC_FAST = 256;  // longest list taken this way
+constexpr int GC_FK = GC_FAST / 32;
+template <typename Put>
+__device__ __forceinline__ int gc_greedy(float4 (&cm)[GC_FK], float4 (&cs)[GC_FK], unsigned alive, int thresh, float gc,
+                                         float r2max, float4* tmp_m, float4* tmp_s, Put put) {
+  const int lane = threadIdx.x & 31;
+  int cnt = 1;
+  int left = __reduce_add_sync(0xffffffffu, (unsigned)__popc(alive));
+  while (left > 32) {
+    if (cnt + left < thresh) return cnt;
+    const unsigned f = __reduce_min_sync(0xffffffffu, alive ? (unsigned)(__ffs(alive) - 1) * 32u + (unsigned)lane : ~0u);
+    const int src = (int)(f & 31u);
+    // entry f of its lane, by masks: a branch or a select over k would become
+    // an index, and an index would put cm and cs in local memory
+    unsigned e[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int k = 0; k < GC_FK; ++k) {
+      const unsigned here = (f >> 5) == (unsigned)k ? ~0u : 0u;
+      e[0] |= here & __float_as_uint(cm[k].x);
+      e[1] |= here & __float_as_uint(cm[k].y);
+      e[2] |= here & __float_as_uint(cm[k].z);
+      e[3] |= here & __float_as_uint(cm[k].w);
+      e[4] |= here & __float_as_uint(cs[k].x);
+      e[5] |= here & __float_as_uint(cs[k].y);
+      e[6] |= here & __float_as_uint(cs[k].z);
+    }
+    float4 m = make_float4(__uint_as_float(e[0]), __uint_as_float(e[1]), __uint_as_float(e[2]), __uint_as_float(e[3]));
+    float4 t = make_float4(__uint_as_float(e[4]), __uint_as_float(e[5]), __uint_as_float(e[6]), 0.f);
+    if (lane == src) {
+      put(cnt, __float_as_int(m.w));
+      alive &= alive - 1;
+    }
+    ++cnt;
+    m = shfl4(m, src);
+    t = shfl4(t, src);
+    unsigned fail = 0u, unsure = 0u;
+#pragma unroll
+    for (int k = 0; k < GC_FK; ++k) {
+      const int r = gc_consistent_fast(m, t, cm[k], cs[k], gc, r2max);
+      fail |= r == 0 ? 1u << k : 0u;
+      unsure |= r < 0 ? 1u << k : 0u;
+    }
+    alive &= ~fail;
+    if (__any_sync(0xffffffffu, alive & unsure)) {
+#pragma unroll
+      for (int k = 0; k < GC_FK; ++k)
+        if ((alive & unsure & (1u << k)) && !gc_consistent_exact(m, t, cm[k], cs[k], gc)) alive &= ~(1u << k);
+    }
+    left = __reduce_add_sync(0xffffffffu, (unsigned)__popc(alive));
+  }
+  // one entry per lane, in order
+  int base = 0;
+#pragma unroll
+  for (int k = 0; k < GC_FK; ++k) {
+    const bool a = (alive >> k) & 1u;
+    const unsigned b = __ballot_sync(0xffffffffu, a);
+    if (a) {
+      const int at = base + __popc(b & lanemask_lt());
+      tmp_m[at] = cm[k];
+      tmp_s[at] = cs[k];
+    }
+    base += __popc(b);
+  }
+  __syncwarp();
+  bool in = lane < left;
+  const float4 em = in ? tmp_m[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 es = in ? tmp_s[lane] : em;
+  __syncwarp();
+  for (;;) {
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (!b || cnt + __popc(b) < thresh) return cnt;
+    const int f = __ffs(b) - 1;
+    if (lane == f) put(cnt, __float_as_int(em.w));
+    ++cnt;
+    const float4 m = shfl4(em, f), t = shfl4(es, f);
+    const int r = gc_consistent_fast(m, t, em, es, gc, r2max);
+    in = in && lane > f && r != 0;
+    if (in && r < 0) in = gc_consistent_exact(m, t, em, es, gc);
+  }
+}
+
 // Greedy admission of the n (<= 32) staged candidates, in slot order, into
 // the warp's set (members in mem_m/mem_s; member 0 is the seed, which every
 // staged candidate already passed).  Lane k tests candidate k against the
@@ -364,16 +471,40 @@ __device__ __forceinline__ void gc_admit(const GcDev& g, int a, const int* slot,
 // it was computed; a superset of the ones not taken now): greedy admission in
 // list order, candidates taken since skipped, each candidate tested against
 // every member so far (member 0 is the seed).  Members go to rec[]
-// (positions) and mem_m/mem_s.  Returns the member count, or -1 when the set
-// would exceed cap (the caller falls back to a recompute in the next round).
+// (positions), the first 8 also to first[]; mem_m/mem_s are scratch.  Returns the member count (of a set
+// below thresh possibly only its start), or -1 when the set would exceed cap
+// (the caller falls back to a recompute in the next round).
 __device__ __forceinline__ int gc_inline_set(const GcDev& g, int a, const float4* lm, const float4* ls, int nl,
-                                             const unsigned* taken, float4* mem_m, float4* mem_s, int* rec, int cap,
-                                             float r2max) {
+                                             const unsigned* taken, float4* mem_m, float4* mem_s, int* first, int* rec,
+                                             int cap, int thresh, float r2max) {
   const int lane = threadIdx.x & 31;
+  if (nl <= GC_FAST) {
+    float4 cm[GC_FK], cs[GC_FK];
+    unsigned alive = 0u;
+#pragma unroll
+    for (int k = 0; k < GC_FK; ++k) {
+      const int e = 32 * k + lane;
+      cm[k] = cs[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (e < nl) {
+        cm[k] = __ldcg(lm + e);
+        cs[k] = __ldcg(ls + e);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < GC_FK; ++k)
+      if (32 * k + lane < nl && !sbit(taken, __float_as_int(cm[k].w))) alive |= 1u << k;
+    if (lane == 0) rec[0] = first[0] = a;
+    const int cnt = gc_greedy(cm, cs, alive, thresh, g.gc, r2max, mem_m, mem_s, [&](int c, int pos) {
+      if (c < cap) rec[c] = pos;
+      if (c < 8) first[c] = pos;
+    });
+    __syncwarp();
+    return cnt <= cap ? cnt : -1;
+  }
   if (lane == 0) {
     mem_m[0] = __ldg(g.pm + a);
     mem_s[0] = __ldg(g.ps + a);
-    rec[0] = a;
+    rec[0] = first[0] = a;
   }
   __syncwarp();
   int cnt = 1;
@@ -403,6 +534,7 @@ __device__ __forceinline__ int gc_inline_set(const GcDev& g, int a, const float4
         mem_m[cnt] = cm;
         mem_s[cnt] = cs;
         rec[cnt] = b;
+        if (cnt < 8) first[cnt] = b;
       }
       ++cnt;
       if (lane > f && pass) pass = gc_consistent(fm, fs, cm, cs, g.gc, r2max);
@@ -419,15 +551,24 @@ __device__ __forceinline__ int gc_inline_set(const GcDev& g, int a, const float4
 //     not taken and has no set yet, or whose set lost a member to a commit,
 //     joins this round's list;
 //  A1. seed tests of every listed seed against every candidate, spread over
-//     all warps (a warp stages 32 candidates once and tests them against
-//     its group's 32 seeds, one seed per lane); the results are pass
+//     all warps (a warp holds 32 candidates, one per lane, and tests them
+//     against the seeds of its group in reach); the results are pass
 //     bitmasks in candidate order;
 //  A2. one warp per listed seed admits the passing candidates in ascending
 //     order, greedily, against the members so far;
 //  B.  warp 0 of block 0 walks the seeds in order from pos: taken seeds are
-//     skipped, a seed whose set lost a member ends the round (recomputed in
-//     the next one), a set of >= thresh members commits.  The walk also ends
+//     skipped, a set of >= thresh members commits, a seed whose set lost a
+//     member has it recomputed from its pass list, up to eight such sets of
+//     the batch at once by the block's warps; inline_max times a round, then
+//     it ends the round (recomputed in the next one).  The walk also ends
 //     at the window's end, at the last seed, or at max_clusters.
+// What bounds it: dependent steps, not arithmetic or memory.  Room scene
+// (111k correspondences, 3,293 seeds reached; microseconds in P / A1 / A2 / B):
+// 51 / 275 / 213 / 665 in 8 rounds with one set recomputed at a time and
+// branching tests, 44 / 188 / 95 / 332 in 8 rounds now.  In A1 the tests were
+// issue-bound (~100 instructions a seed and chunk: nine exchanges and
+// branches); seeds read from shared memory and tests without branches halve
+// it.
 // A stored set stays exact while none of its members is taken (removing
 // rejected candidates never changes a greedy walk).  Every round advances the
 // walk by at least one seed (the seed at pos is exact when B starts).
@@ -439,8 +580,10 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
   extern __shared__ unsigned s_taken[];  // copy of the taken bitset
   __shared__ float4 mem_m[GC_WARPS][GC_MAXS], mem_s[GC_WARPS][GC_MAXS];
   __shared__ int s_slot[GC_WARPS][GC_PEND];
-  __shared__ int s_rec[GC_MAXS];  // walk: members of a set recomputed in place
-  __shared__ int s_pf[3][32][9];  // walk: sizes and first 8 members of the next batches (cp.async ring)
+  // walk: sets recomputed in place, one per warp: seed, pass list, its length
+  // (then the members found) and the first 8 members
+  __shared__ int s_job[GC_WARPS][11], s_njob;
+  __shared__ int s_pf[3][32][11];  // walk: first 8 members, sizes and pass lists of the next batches (cp.async ring)
   __shared__ int s_pos, s_done, s_ok, s_win;
   __shared__ float s_r2max;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -465,6 +608,7 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
   __syncthreads();
   const float r2max = s_r2max;
   unsigned target = 0;
+  int rows_clean = 0;  // rows of the masks that have been in use
   unsigned long long ph[4] = {0, 0, 0, 0}, tp = 0;
   const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
   if (timer) tp = gtimer();
@@ -509,66 +653,111 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
         c.seed_s[slot] = make_float4(as.x, as.y, as.z, R);
         c.seed_m[slot] = am;
       }
-      // the seed tests only set bits: its mask row starts clear
+      // the seed tests only set bits: its rows start clear (admission leaves
+      // the rows it has used clear)
       slot = __shfl_sync(0xffffffffu, slot, 0);
-      if (need) {
+      if (need && slot >= rows_clean) {
         uint4* row = reinterpret_cast<uint4*>(c.mask + (size_t)slot * c.nwp);
         for (int v = lane; v < (nwp >> 2); v += 32) row[v] = make_uint4(0u, 0u, 0u, 0u);
+        for (int v = lane; v < c.nsp; v += 32) c.summ[(size_t)slot * c.nsp + v] = 0u;
       }
     }
     target += gridDim.x;
     if (!gc_barrier(c, target, &s_ok)) return;
     GC_PHASE(0)
     const int nneed = __ldcg(c.ctl + 6);
-    // ---- A1: seed tests -> pass bitmasks.  Items are (chunk of 32
-    // candidates in cell order, group of 32 listed seeds), spread over all
-    // warps (a chunk near many seeds is shared by as many warps as it has
-    // seed groups).  Lane k holds candidate k of the chunk and seed k of the
-    // group; the group's seeds whose reach meets the chunk's box are taken in
-    // turn, and every lane tests its candidate against each, setting its pass
-    // bit in the seed's row.
+    rows_clean = max(rows_clean, nneed);
+    // ---- A1: seed tests -> pass bitmasks.  A warp takes one group of 32
+    // listed seeds (lane k holds seed k, for the whole phase) and every
+    // so-many-th chunk of 32 candidates in cell order (lane k holds candidate
+    // k, the next chunk's loads in flight); the warps of a group share its
+    // chunks.  The group's seeds whose reach meets the chunk's box are taken
+    // in turn, and every lane tests its candidate against each, setting its
+    // pass bit in the seed's row.
     if (nneed > 0) {
       const int nchunks = (g.C + 31) >> 5;
       const int ngroups = (nneed + 31) >> 5;
-      const long long items = (long long)nchunks * ngroups;
-      for (long long it = gw; it < items; it += nwarps) {
-        const int ch = (int)(it / ngroups);
-        const int s0 = (int)(it - (long long)ch * ngroups) * 32;
-        const int i = ch * 32 + lane, k = s0 + lane;
-        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), bm = q, sa = q, sm = q;
+      // warps of a group; those that its chunks leave over share the seeds of
+      // a chunk (nsl warps, every nsl-th seed each)
+      const int per0 = max(nwarps / ngroups, 1);
+      int nsl = 1;
+      while (nsl < 8 && 2 * nsl * nchunks <= per0) nsl *= 2;
+      const int per = per0 / nsl, used = min(ngroups, nwarps);
+      const int slice = (gw / used) % nsl;
+      const unsigned mine = (nsl == 1 ? 0xffffffffu : nsl == 2 ? 0x55555555u : nsl == 4 ? 0x11111111u : 0x01010101u) << slice;
+      for (int grp = gw % used; grp < ngroups && gw < per * nsl * used; grp += nwarps) {
+        const int s0 = grp * 32, k = s0 + lane;
+        float4 sa = make_float4(0.f, 0.f, 0.f, 0.f), sm = sa;
         int sa_i = -1;
-        if (i < g.C) {
-          q = __ldg(c.cpts + i);
-          bm = __ldg(c.cpm + i);
-        }
         if (k < nneed) {
           sa = __ldcg(c.seed_s + k);
           sm = __ldcg(c.seed_m + k);
           sa_i = __ldcg(c.need + k);
         }
-        const float4 blo = __ldg(c.cbox + 2 * ch), bhi = __ldg(c.cbox + 2 * ch + 1);
-        const int b = i < g.C ? __float_as_int(q.w) : -1;
-        const bool ok = b >= 0 && !sbit(s_taken, b);
-        if (!__any_sync(0xffffffffu, ok)) continue;
-        bool hit = false;
-        if (k < nneed) {
-          const float dx = fmaxf(fmaxf(blo.x - sa.x, sa.x - bhi.x), 0.f);
-          const float dy = fmaxf(fmaxf(blo.y - sa.y, sa.y - bhi.y), 0.f);
-          const float dz = fmaxf(fmaxf(blo.z - sa.z, sa.z - bhi.z), 0.f);
-          hit = blo.w != 0.f || !(dx * dx + dy * dy + dz * dz > sa.w);  // NaN distance: not skipped
-        }
-        const unsigned bit = 1u << (b & 31);
-        const int word = b >> 5;
-        unsigned hits = __ballot_sync(0xffffffffu, hit);
-        while (hits) {
-          const int f = __ffs(hits) - 1;
-          hits &= hits - 1;
-          const float4 fa = shfl4(sa, f), fm = shfl4(sm, f);
-          const int a = __shfl_sync(0xffffffffu, sa_i, f);
-          const bool pass = ok && b != a && gc_consistent(fm, fa, bm, q, g.gc, r2max);
-          const unsigned pb = __ballot_sync(0xffffffffu, pass);
-          if (pass) atomicOr(c.mask + (size_t)(s0 + f) * c.nwp + word, bit);
-          if (lane == 0 && pb) atomicAdd(c.pcnt + s0 + f, __popc(pb));
+        __syncwarp();
+        mem_s[wid][lane] = sa;  // the seeds for the tests: two broadcast reads a seed
+        mem_m[wid][lane] = make_float4(sm.x, sm.y, sm.z, __int_as_float(sa_i));
+        __syncwarp();
+        int ch = gw / used / nsl;
+        float4 nq = make_float4(0.f, 0.f, 0.f, 0.f), nbm = nq, nlo = nq, nhi = nq;
+        auto fetch = [&](int cc) {
+          const int i = cc * 32 + lane;
+          nq = __ldg(c.cpts + min(i, g.C - 1));
+          nbm = __ldg(c.cpm + min(i, g.C - 1));
+          nlo = __ldg(c.cbox + 2 * cc);
+          nhi = __ldg(c.cbox + 2 * cc + 1);
+        };
+        if (ch < nchunks) fetch(ch);
+        for (; ch < nchunks; ch += per) {
+          const float4 q = nq, bm = nbm, blo = nlo, bhi = nhi;
+          if (ch + per < nchunks) fetch(ch + per);
+          bool hit = false;
+          if (k < nneed) {
+            const float dx = fmaxf(fmaxf(blo.x - sa.x, sa.x - bhi.x), 0.f);
+            const float dy = fmaxf(fmaxf(blo.y - sa.y, sa.y - bhi.y), 0.f);
+            const float dz = fmaxf(fmaxf(blo.z - sa.z, sa.z - bhi.z), 0.f);
+            hit = blo.w != 0.f || !(dx * dx + dy * dy + dz * dz > sa.w);  // NaN distance: not skipped
+          }
+          unsigned hits = __ballot_sync(0xffffffffu, hit) & mine;
+          if (!hits) continue;
+          const int b = ch * 32 + lane < g.C ? __float_as_int(q.w) : -1;
+          const bool ok = b >= 0 && !sbit(s_taken, b);
+          unsigned passed = 0u;  // bit f: this lane's candidate passes the group's seed f
+          int npass = 0;         // candidates of the chunk that pass this lane's seed
+          while (hits) {
+            // four seeds at a time (the last one repeats when fewer are
+            // left): their reads and tests are independent
+            int f[4], sure[4];
+            bool unsure = false;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              f[j] = hits ? __ffs(hits) - 1 : f[j ? j - 1 : 0];
+              hits &= hits - 1;
+              const float4 fa = mem_s[wid][f[j]], fm = mem_m[wid][f[j]];
+              const int r = gc_consistent_fast(fm, fa, bm, q, g.gc, r2max);
+              sure[j] = ok && __float_as_int(fm.w) != b ? r : 0;
+              unsure |= sure[j] < 0;
+            }
+            if (__any_sync(0xffffffffu, unsure)) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (sure[j] < 0) sure[j] = gc_consistent_exact(mem_m[wid][f[j]], mem_s[wid][f[j]], bm, q, g.gc);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const unsigned pb = __ballot_sync(0xffffffffu, sure[j] != 0);
+              if (sure[j]) passed |= 1u << f[j];
+              if (lane == f[j]) npass = __popc(pb);
+            }
+          }
+          const unsigned bit = 1u << (b & 31);
+          const int word = b >> 5;
+          for (unsigned pl = passed; pl; pl &= pl - 1) {
+            const int f = s0 + __ffs(pl) - 1;
+            atomicOr(c.mask + (size_t)f * c.nwp + word, bit);
+            atomicOr(c.summ + (size_t)f * c.nsp + (word >> 5), 1u << (word & 31));
+          }
+          if (npass) atomicAdd(c.pcnt + s0 + lane, npass);
         }
       }
     }
@@ -595,17 +784,116 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
       }
       n_list = __shfl_sync(0xffffffffu, n_list, 0);
       off = __shfl_sync(0xffffffffu, off, 0);
+      if (off >= 0 && n_list <= GC_FAST) {
+        // a list that the warp can hold: the words that are not zero come from
+        // the summary, their bits give the positions, in order (both listed
+        // in the warp's shared memory); the endpoints go to the pool and stay
+        // in registers for the admission
+        unsigned* wid_list = reinterpret_cast<unsigned*>(mem_m[wid]);
+        int* pos_list = reinterpret_cast<int*>(mem_s[wid]);
+        unsigned* row = c.mask + (size_t)slot * c.nwp;
+        unsigned* sum = c.summ + (size_t)slot * c.nsp;
+        const int ns = (nwords + 31) >> 5;
+        int nw = 0;
+        for (int v0 = 0; v0 < ns; v0 += 128) {
+          unsigned sw[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int v = v0 + 32 * j + lane;
+            sw[j] = v < ns ? __ldcg(sum + v) : 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int v = v0 + 32 * j + lane, mine = __popc(sw[j]);
+            if (!__any_sync(0xffffffffu, mine)) continue;
+            int incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int y = __shfl_up_sync(0xffffffffu, incl, o);
+              if (lane >= o) incl += y;
+            }
+            int at = nw + incl - mine;
+            for (unsigned w = sw[j]; w; w &= w - 1) wid_list[at++] = (unsigned)v * 32u + (unsigned)(__ffs(w) - 1);
+            if (mine) sum[v] = 0u;
+            nw += __shfl_sync(0xffffffffu, incl, 31);
+          }
+        }
+        __syncwarp();
+        unsigned bits[GC_FK], wat[GC_FK];
+#pragma unroll
+        for (int k = 0; k < GC_FK; ++k) {
+          const int e = 32 * k + lane;
+          wat[k] = e < nw ? wid_list[e] : 0u;
+          bits[k] = e < nw ? __ldcg(row + wat[k]) : 0u;
+        }
+        int np = 0;
+#pragma unroll
+        for (int k = 0; k < GC_FK; ++k) {
+          if (32 * k >= nw) break;
+          const int mine = __popc(bits[k]);
+          int incl = mine;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+          }
+          int at = np + incl - mine;
+          for (unsigned w = bits[k]; w; w &= w - 1) pos_list[at++] = (int)wat[k] * 32 + __ffs(w) - 1;
+          if (mine) row[wat[k]] = 0u;
+          np += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        __syncwarp();
+        float4 cm[GC_FK], cs[GC_FK];
+        unsigned alive = 0u;
+#pragma unroll
+        for (int k = 0; k < GC_FK; ++k) {
+          const int e = 32 * k + lane;
+          cm[k] = cs[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (e < n_list) {
+            const int pj = pos_list[e];
+            cm[k] = __ldg(g.pm + pj);
+            cs[k] = __ldg(g.ps + pj);
+            cm[k].w = __int_as_float(pj);
+            alive |= 1u << k;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < GC_FK; ++k) {
+          const int e = 32 * k + lane;
+          if (e < n_list) {
+            c.pool_m[off + e] = cm[k];
+            c.pool_s[off + e] = cs[k];
+          }
+        }
+        __syncwarp();  // the lists have been read: the admission reuses their memory
+        int* out = g.set_mem + (size_t)a * maxs;
+        cnt = gc_greedy(cm, cs, alive, c.thresh, g.gc, r2max, mem_m[wid], mem_s[wid], [&](int n, int pos) {
+          if (n < maxs) out[n] = pos;
+        });
+        if (lane == 0) {
+          c.plist_off[a] = off;
+          c.plist_cnt[a] = n_list;
+          g.set_size[a] = cnt;
+          c.computed[a] = 1;
+          atomicAdd(c.ctl + 5, 1);
+          atomicAdd(c.ctl + 7, n_list);
+        }
+        __syncwarp();
+        continue;
+      }
       int nemit = 0;
       float4* lmp = off >= 0 ? c.pool_m + off : nullptr;
       float4* lsp = off >= 0 ? c.pool_s + off : nullptr;
-      const uint4* row = reinterpret_cast<const uint4*>(c.mask + (size_t)slot * c.nwp);
+      uint4* row = reinterpret_cast<uint4*>(c.mask + (size_t)slot * c.nwp);
       const int nv = nwp >> 2;
+      for (int v = lane; v < c.nsp; v += 32) c.summ[(size_t)slot * c.nsp + v] = 0u;
       for (int v0 = 0; v0 < nv; v0 += 32 * GC_PREF) {
         uint4 buf[GC_PREF];
 #pragma unroll
         for (int j = 0; j < GC_PREF; ++j) {
           const int idx = v0 + j * 32 + lane;
           buf[j] = idx < nv ? __ldcg(row + idx) : make_uint4(0u, 0u, 0u, 0u);
+          if (idx < nv) row[idx] = make_uint4(0u, 0u, 0u, 0u);
         }
 #pragma unroll
         for (int j = 0; j < GC_PREF; ++j) {
@@ -667,8 +955,9 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
     // p + l (taken? lost a member?) in parallel; only events (a commit or a
     // stale set) are handled in order, and after a commit the later lanes
     // evaluate again.
-    if (blockIdx.x == 0 && wid == 0) {
-      int ncl = __ldcg(c.ctl + 1), err = 0, n_inline = 0;
+    if (blockIdx.x == 0) {
+      int ncl = 0, err = 0, n_inline = 0;
+      if (wid == 0) ncl = __ldcg(c.ctl + 1);
       bool done = false, stop = false;
       int p = pos;
       const int wend = min(pos + win, g.C);
@@ -688,125 +977,166 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
           asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32_gc(&s_pf[slot][lane][8])),
                        "l"(g.set_size + pb + lane)
                        : "memory");
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32_gc(&s_pf[slot][lane][9])),
+                       "l"(c.plist_off + pb + lane)
+                       : "memory");
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32_gc(&s_pf[slot][lane][10])),
+                       "l"(c.plist_cnt + pb + lane)
+                       : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
       };
-      int ring = 0;
-      prefetch(p, 0);
-      prefetch(p + 32, 1);
-      while (p < wend && !stop) {
-        const int nb = min(32, wend - p);
-        const int my = p + lane;
-        prefetch(p + 64, (ring + 2) % 3);
-        asm volatile("cp.async.wait_group 2;" ::: "memory");  // this batch's copies are in
-        __syncwarp();
-        const bool have = lane < nb;
-        const int n_l = have ? s_pf[ring][lane][8] : 0;
-        int m_cur[8];
+      int ring = 0, nb = 0, cursor = 0;
+      bool in_batch = false;
+      int n_l = 0, off_l = -1, nl_l = 0, job_l = -1, m_cur[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) m_cur[k] = s_pf[ring][lane][k];
-        ring = ring == 2 ? 0 : ring + 1;
-        const int ns_l = min(n_l, maxs);
-        int cursor = 0;
-        for (;;) {
-          bool taken_l = true, stale_l = false;
-          if (lane >= cursor && lane < nb) {
-            taken_l = sbit(s_taken, my);
-            if (!taken_l) {
-              // the first 8 members' taken bits in one round of independent
-              // shared-memory loads (a slot past the set reads the seed's own
-              // bit: clear)
-              unsigned acc = 0u;
-#pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const int mb = k < ns_l ? m_cur[k] : my;
-                acc |= s_taken[mb >> 5] >> (mb & 31);
-              }
-              stale_l = (acc & 1u) != 0u;
-              // a longer set: its other members eight independent loads at a time
-              for (int k0 = 8; k0 < ns_l && !stale_l; k0 += 8) {
-                int mbk[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                  mbk[j] = k0 + j < ns_l ? __ldcg(g.set_mem + (size_t)my * maxs + k0 + j) : my;
-                unsigned a2 = 0u;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) a2 |= s_taken[mbk[j] >> 5] >> (mbk[j] & 31);
-                stale_l = (a2 & 1u) != 0u;
-              }
-            }
-          }
-          const unsigned ev = __ballot_sync(0xffffffffu, !taken_l && (stale_l || n_l >= c.thresh));
-          if (!ev) {
-            p += nb;
-            break;
-          }
-          const int f = __ffs(ev) - 1;
-          const bool f_stale = __shfl_sync(0xffffffffu, stale_l, f);
-          const int nf = __shfl_sync(0xffffffffu, n_l, f);
-          if (f_stale) {
-            // lost a member: recompute in place from the pass list, or
-            // (no list kept, or too many members) end the round here
-            const int sa = p + f;
-            const int off = n_inline < c.inline_max ? __ldcg(c.plist_off + sa) : -1;
-            const int ns = off < 0 ? -1
-                                   : gc_inline_set(g, sa, c.pool_m + off, c.pool_s + off, __ldcg(c.plist_cnt + sa),
-                                                   s_taken, mem_m[0], mem_s[0], s_rec, min(GC_MAXS, maxs), r2max);
-            ++n_inline;
-            if (ns < 0) {
-              p += f;
-              stop = true;
-              break;
-            }
-            if (lane == 0) atomicAdd(c.ctl + 5, 1);
-            if (ns >= c.thresh) {
-              for (int k = lane; k < ns; k += 32) {
-                const int mb = s_rec[k];
-                atomicOr(&s_taken[mb >> 5], 1u << (mb & 31));
-                c.cl_members[(size_t)ncl * maxs + k] = mb;
-              }
-              if (lane == 0) c.cl_sizes[ncl] = ns;
+      for (int k = 0; k < 8; ++k) m_cur[k] = 0;
+      if (wid == 0) {
+        prefetch(p, 0);
+        prefetch(p + 32, 1);
+      }
+      for (;;) {
+        if (wid == 0) {
+          int njob = 0;
+          while (!stop) {
+            if (!in_batch) {
+              if (p >= wend) break;
+              nb = min(32, wend - p);
+              prefetch(p + 64, (ring + 2) % 3);
+              asm volatile("cp.async.wait_group 2;" ::: "memory");  // this batch's copies are in
               __syncwarp();
-              ++ncl;
-              if (ncl >= c.max_clusters) {
-                done = stop = true;
-                p += f + 1;
+              const bool have = lane < nb;
+              n_l = have ? s_pf[ring][lane][8] : 0;
+              off_l = have ? s_pf[ring][lane][9] : -1;
+              nl_l = have ? s_pf[ring][lane][10] : 0;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) m_cur[k] = s_pf[ring][lane][k];
+              ring = ring == 2 ? 0 : ring + 1;
+              cursor = 0;
+              in_batch = true;
+            }
+            const int my = p + lane;
+            const int ns_l = min(n_l, maxs);
+            bool taken_l = true, stale_l = false;
+            if (lane >= cursor && lane < nb) {
+              taken_l = sbit(s_taken, my);
+              if (!taken_l) {
+                // the first 8 members' taken bits in one round of independent
+                // shared-memory loads (a slot past the set reads the seed's own
+                // bit: clear)
+                unsigned acc = 0u;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                  const int mb = k < ns_l ? m_cur[k] : my;
+                  acc |= s_taken[mb >> 5] >> (mb & 31);
+                }
+                stale_l = (acc & 1u) != 0u || off_l == -2;
+                // a longer set: its other members eight independent loads at a time
+                for (int k0 = 8; k0 < ns_l && !stale_l; k0 += 8) {
+                  int mbk[8];
+#pragma unroll
+                  for (int j = 0; j < 8; ++j)
+                    mbk[j] = k0 + j < ns_l ? __ldcg(g.set_mem + (size_t)my * maxs + k0 + j) : my;
+                  unsigned a2 = 0u;
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) a2 |= s_taken[mbk[j] >> 5] >> (mbk[j] & 31);
+                  stale_l = (a2 & 1u) != 0u;
+                }
+              }
+            }
+            const unsigned ev = __ballot_sync(0xffffffffu, !taken_l && (stale_l || n_l >= c.thresh));
+            if (!ev) {
+              p += nb;
+              in_batch = false;
+              continue;
+            }
+            const int f = __ffs(ev) - 1;
+            if (__shfl_sync(0xffffffffu, stale_l, f)) {
+              // lost a member: recompute in place from the pass list, together
+              // with the batch's next stale ones, a warp each, or (no list
+              // kept, or too many members) end the round here
+              if (n_inline >= c.inline_max || __shfl_sync(0xffffffffu, off_l, f) < 0) {
+                p += f;
+                stop = true;
                 break;
               }
+              ++n_inline;
+              const bool want = stale_l && off_l >= 0;
+              const unsigned jb = __ballot_sync(0xffffffffu, want);
+              njob = min(__popc(jb), GC_WARPS);
+              job_l = __popc(jb & lanemask_lt());
+              job_l = want && job_l < GC_WARPS ? job_l : -1;
+              if (job_l >= 0) {
+                s_job[job_l][0] = my;
+                s_job[job_l][1] = off_l;
+                s_job[job_l][2] = nl_l;
+              }
+              break;
+            }
+            const int nf = __shfl_sync(0xffffffffu, n_l, f);
+            if (nf > maxs) {
+              err = (int)RTR_ERR_CAPACITY;
+              done = stop = true;
+              p += f;
+              break;
+            }
+            // the committing seed's first 8 members from lane f's registers
+            int mine = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const int v = __shfl_sync(0xffffffffu, m_cur[k], f);
+              if (lane == k) mine = v;
+            }
+            for (int k = lane; k < nf; k += 32) {
+              const int mb = k < 8 ? mine : __ldcg(g.set_mem + (size_t)(p + f) * maxs + k);
+              atomicOr(&s_taken[mb >> 5], 1u << (mb & 31));
+              c.cl_members[(size_t)ncl * maxs + k] = mb;
+            }
+            if (lane == 0) c.cl_sizes[ncl] = nf;
+            __syncwarp();
+            ++ncl;
+            if (ncl >= c.max_clusters) {
+              done = stop = true;
+              p += f + 1;
+              break;
             }
             cursor = f + 1;
-            continue;
           }
-          if (nf > maxs) {
-            err = (int)RTR_ERR_CAPACITY;
-            done = stop = true;
-            p += f;
-            break;
+          if (lane == 0) {
+            s_njob = njob;
+            if (njob) atomicAdd(c.ctl + 5, njob);
           }
-          // the committing seed's first 8 members from lane f's registers
-          int mine = 0;
+        }
+        __syncthreads();
+        if (s_njob == 0) break;
+        if (wid < s_njob) {
+          // the new set takes the stored one's place: exact under the bits
+          // taken now, so the next round need not list its seed
+          const int a = s_job[wid][0], off = s_job[wid][1], nl = s_job[wid][2];
+          int* first = &s_job[wid][3];
+          const int ns = gc_inline_set(g, a, c.pool_m + off, c.pool_s + off, nl, s_taken, mem_m[wid], mem_s[wid],
+                                       first, g.set_mem + (size_t)a * maxs, min(GC_MAXS, maxs), c.thresh, r2max);
+          if (lane == 0) {
+            s_job[wid][2] = ns;
+            if (ns >= 0) g.set_size[a] = ns;
+            else c.computed[a] = 0;  // too long to keep here: a round computes it
+          }
+        }
+        __syncthreads();
+        if (wid == 0 && job_l >= 0) {
+          const int ns = s_job[job_l][2];
+          if (ns < 0) {
+            off_l = -2;  // stale from here on: the round ends at its turn
+          } else {
+            n_l = ns;
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int v = __shfl_sync(0xffffffffu, m_cur[k], f);
-            if (lane == k) mine = v;
+            for (int k = 0; k < 8; ++k) m_cur[k] = s_job[job_l][3 + k];
           }
-          for (int k = lane; k < nf; k += 32) {
-            const int mb = k < 8 ? mine : __ldcg(g.set_mem + (size_t)(p + f) * maxs + k);
-            atomicOr(&s_taken[mb >> 5], 1u << (mb & 31));
-            c.cl_members[(size_t)ncl * maxs + k] = mb;
-          }
-          if (lane == 0) c.cl_sizes[ncl] = nf;
-          __syncwarp();
-          ++ncl;
-          if (ncl >= c.max_clusters) {
-            done = stop = true;
-            p += f + 1;
-            break;
-          }
-          cursor = f + 1;
+          job_l = -1;
         }
         __syncwarp();
       }
+      if (wid == 0) {
       asm volatile("cp.async.wait_all;" ::: "memory");  // no copy left in flight into the ring
       if (p >= g.C) done = true;
       __syncwarp();
@@ -824,6 +1154,7 @@ __global__ void __launch_bounds__(GC_WARPS * 32, 2) k_gc_coop(GcDev g, GcCoop c)
         c.ctl[6] = 0;
       }
       __syncwarp();
+      }
     }
     target += gridDim.x;
     if (!gc_barrier(c, target, &s_ok)) return;
@@ -953,6 +1284,7 @@ struct GcBufs {
   GridMeta* mbox;
   int* need;
   unsigned* mask;
+  unsigned* summ;
   GcGrid* sg;
   uint32_t *gk0, *gv0, *gk1, *gv1;
   float4 *cpts, *cpm;
@@ -963,8 +1295,9 @@ struct GcBufs {
 };
 
 // Window of the walk and the width of a pass-mask row.
-constexpr int GC_WIN = 512;      // first window (room scene: 1.21 ms at 512, 1.27 at 256, 1.25 at 128); results identical
+constexpr int GC_WIN = 512;      // first window (room scene: 894 us at 512, 931 at 256 and at 1,024); results identical
 constexpr int GC_WIN_MAX = 2048;  // a window grows to this while the walk keeps using whole windows
+static int gc_nsp(int C) { return ((C > 0 ? C : 1) + 1023) / 1024; }
 static int gc_nwp(int C) { return (((C > 0 ? C : 1) + 31) / 32 + 3) & ~3; }
 static int gc_win(int C, int want = 0) {
   const size_t row = (size_t)gc_nwp(C) * 4;
@@ -982,8 +1315,10 @@ static int gc_pool_cap(int C) {
   const long long want = (long long)(C > 0 ? C : 1) * 64;
   return (int)(want < (1 << 18) ? (1 << 18) : (want > (4 << 20) ? (4 << 20) : want));
 }
-// Sets the walk recomputes in place per round (measured on the room scene).
-constexpr int GC_INLINE_MAX = 16;
+// Times per round the walk recomputes sets in place (room scene: 894 us at 8,
+// 966 at 4, 905 at 16, 879 at 32; the 12k-point segment's recognition 2.46 ms
+// at 8, 2.53 at 4, 2.47 at 16, 2.48 at 32).
+constexpr int GC_INLINE_MAX = 8;
 
 static void gc_plan(ScratchPlan& p, int C, int max_clusters, int max_members) {
   const int n = C > 0 ? C : 1;
@@ -1003,6 +1338,7 @@ static void gc_plan(ScratchPlan& p, int C, int max_clusters, int max_members) {
   p.add<GridMeta>(1);
   p.add<int>(gc_win(C, GC_WIN_MAX));
   p.add<unsigned>((size_t)gc_win(C, GC_WIN_MAX) * gc_nwp(C));
+  p.add<unsigned>((size_t)gc_win(C, GC_WIN_MAX) * gc_nsp(C));
   p.add<GcGrid>(1);
   for (int i = 0; i < 4; ++i) p.add<uint32_t>(n);
   p.add<float4>(n);
@@ -1038,6 +1374,7 @@ static bool gc_take(Scratch& s, int C, int max_clusters, int max_members, GcBufs
   b->mbox = s.take<GridMeta>(1);
   b->need = s.take<int>(gc_win(C, GC_WIN_MAX));
   b->mask = s.take<unsigned>((size_t)gc_win(C, GC_WIN_MAX) * gc_nwp(C));
+  b->summ = s.take<unsigned>((size_t)gc_win(C, GC_WIN_MAX) * gc_nsp(C));
   b->sg = s.take<GcGrid>(1);
   b->gk0 = s.take<uint32_t>(n);
   b->gv0 = s.take<uint32_t>(n);
@@ -1113,7 +1450,7 @@ static rtr_status gc_launch(rtr_context* ctx, Scratch& s, const float* d_model_k
   RTR_LAUNCHED(3);
   pgr.end();
   GcCoop c{b.misc, b.arrive, b.computed, b.members, b.sizes, gc_thresh, max_clusters,
-           ctx->wait_budget_cycles, ctx->d_status, b.mbox, b.need, b.mask,
+           ctx->wait_budget_cycles, ctx->d_status, b.mbox, b.need, b.mask, b.summ, gc_nsp(C),
            gc_win(C, ctx->tune_gc_window > 0 ? ctx->tune_gc_window : 0), gc_win(C, GC_WIN_MAX), gc_nwp(C),
            b.sg, b.cpts, b.cpm, b.cbox, b.seed_s, b.seed_m, b.pcnt, b.plist_off, b.plist_cnt, b.pool_m, b.pool_s,
            ctx->tune_gc_no_lists ? 0 : gc_pool_cap(C),

@@ -176,3 +176,35 @@ def test_gc_nonfinite_scene_endpoints(ctx):
     assert np.array_equal(sizes, rsizes) and len(sizes) > 0
     for k in range(len(sizes)):
         assert set(mem[k][: sizes[k]].tolist()) == set(np.nonzero(clus == k)[0].tolist()), k
+
+
+@pytest.mark.parametrize("n", [1, 33, 255, 257, 258, 700])
+def test_gc_long_pass_lists_and_sets_recomputed_together(rtr, n):
+    """One rigid cluster of n with noise near the consistency bound, so that
+    pass lists are about n long (held by a warp up to 256 entries, else read
+    in chunks) while sets stay smaller and keep losing members to commits:
+    many stale sets a batch, recomputed by up to eight warps at once."""
+    rng = np.random.default_rng(n)
+    T = rtr.synth_rigid(3, 70.0, 1.0)
+    mk = np.zeros((n, 4), np.float32)
+    mk[:, :3] = rng.uniform(-0.2, 0.2, (n, 3))
+    sk = O.transform_f32(T, mk).astype(np.float32)
+    sk[:, :3] += rng.uniform(-0.006, 0.006, (n, 3)).astype(np.float32)
+    cm = rng.permutation(n).astype(np.int32)
+    cs = cm.copy()
+    cs[::7] = rng.integers(0, n, len(cs[::7]))  # and some wrong ones
+    cd = rng.uniform(0, 0.3, n).astype(np.float32)
+    clus, _, rsizes = O.gc_group(mk, sk, cm, cs, cd, 0.01, 3, 256)
+    c = rtr.Context(0)
+    try:
+        for lists, inline in ((0, 0), (0, 1), (1, 0)):
+            c.set_tuning("gc_pass_lists", lists)
+            c.set_tuning("gc_inline", inline)
+            mem, sizes, _ = c.gc_group(_dev(mk), _dev(sk), _dev(cm, np.int32), _dev(cs, np.int32), _dev(cd),
+                                       0.01, 3, 256, 512)
+            mem, sizes = mem.cpu().numpy(), sizes.cpu().numpy()
+            assert np.array_equal(sizes, rsizes)
+            for k in range(len(sizes)):
+                assert set(mem[k][: sizes[k]].tolist()) == set(np.nonzero(clus == k)[0].tolist()), k
+    finally:
+        c.close()
