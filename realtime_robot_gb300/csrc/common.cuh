@@ -149,6 +149,9 @@ struct Scratch {
 // Ensure the arena holds `bytes`; grows (synchronising) unless `stream` is
 // being captured, in which case RTR_ERR_CAPACITY is returned.
 rtr_status ensure_scratch(rtr_context* ctx, size_t bytes, cudaStream_t stream, Scratch* out);
+// Whether ensure_scratch may be asked for `bytes`: held already, or free to
+// grow (no capture, within the caller's limit).  For what a call can do without.
+bool scratch_obtainable(const rtr_context* ctx, size_t bytes, cudaStream_t stream);
 
 bool stream_is_capturing(cudaStream_t s);
 

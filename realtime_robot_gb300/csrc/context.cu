@@ -69,6 +69,11 @@ rtr_status side_stream_ready(rtr_context* ctx) {
   return RTR_OK;
 }
 
+bool scratch_obtainable(const rtr_context* ctx, size_t bytes, cudaStream_t stream) {
+  return bytes <= ctx->arena_bytes ||
+         (!stream_is_capturing(stream) && (!ctx->scratch_limit || bytes <= ctx->scratch_limit));
+}
+
 rtr_status ensure_scratch(rtr_context* ctx, size_t bytes, cudaStream_t stream, Scratch* out) {
   if (bytes > ctx->arena_bytes) {
     if (stream_is_capturing(stream))

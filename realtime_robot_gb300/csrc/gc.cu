@@ -1296,7 +1296,8 @@ struct GcBufs {
 
 // Window of the walk and the width of a pass-mask row.
 constexpr int GC_WIN = 512;      // first window (room scene: 894 us at 512, 931 at 256 and at 1,024); results identical
-constexpr int GC_WIN_MAX = 2048;  // a window grows to this while the walk keeps using whole windows
+constexpr int GC_WIN_MAX = 1984;  // a window grows to this while the walk keeps using whole windows (the masks'
+                                  // summaries take the 64 rows to 2,048)
 static int gc_nsp(int C) { return ((C > 0 ? C : 1) + 1023) / 1024; }
 static int gc_nwp(int C) { return (((C > 0 ? C : 1) + 31) / 32 + 3) & ~3; }
 static int gc_win(int C, int want = 0) {

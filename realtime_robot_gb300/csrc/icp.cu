@@ -691,9 +691,11 @@ rtr_status rtr_icp(rtr_context* ctx, const float* d_src, int n_src, const float*
   for (int i = 0; i < 4; ++i) plan.add<uint32_t>(n_src);
   plan.add<uint32_t>(radix_hist_entries(n_src));
   plan.add<GridMeta>(1);
+  ScratchPlan least = plan;  // without the matching state
+  icp_multi_plan(least, 1, maxb, 0);
   icp_multi_plan(plan, 1, maxb, n_src);
   Scratch s;
-  RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
+  RTR_TRY(ensure_scratch(ctx, scratch_obtainable(ctx, plan.bytes, st) ? plan.bytes : least.bytes, st, &s));
   GridBufs gb;
   if (!grid_take(s, n_tgt, cell_cap, &gb)) return fail(RTR_ERR_CAPACITY, "rtr_icp: scratch carve");
   float4* src_sorted = s.take<float4>(n_src);
@@ -767,9 +769,11 @@ rtr_status rtr_icp_multi(rtr_context* ctx, const float* d_src, int n_src, const 
   ScratchPlan plan;
   grid_plan(plan, n_tgt, cell_cap);
   plan.add<GridMeta>(1);
+  ScratchPlan least = plan;  // without the matching state
+  icp_multi_plan(least, n_problems, maxb, 0);
   icp_multi_plan(plan, n_problems, maxb, (size_t)n_problems * n_src);
   Scratch s;
-  RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
+  RTR_TRY(ensure_scratch(ctx, scratch_obtainable(ctx, plan.bytes, st) ? plan.bytes : least.bytes, st, &s));
   GridBufs gb;
   if (!grid_take(s, n_tgt, cell_cap, &gb)) return fail(RTR_ERR_CAPACITY, "rtr_icp_multi: scratch carve");
   GridMeta* src_meta = s.take<GridMeta>(1);
