@@ -28,8 +28,8 @@
 // All double and float arithmetic that has to agree with the oracle uses the
 // _rn intrinsics, so nothing is contracted into an FMA.
 //
-// Kernels (one CTA per keypoint or per pair; the work is gather- and
-// latency-bound, the pair kernel's inner loop runs from registers and a
+// Kernels (one CTA per keypoint, a warp or a CTA per pair; the work is gather-
+// and issue-bound, the pair kernels' inner loops run from registers and a
 // 4 KB shared bitmap):
 //   k_ref_occ        box search over the cloud, occupied-leaf count (Number),
 //                    ordered append of the box's point indices;
@@ -39,7 +39,10 @@
 //                    deduplicated in a 32^3 bitmap around the cloud, the
 //                    field read per leaf, the leaves sorted into tree order
 //                    and their squared values added in float one by one
-//                    (the reference's running score), pair transform;
+//                    (the reference's running score), pair transform: a CTA
+//                    per pair, for clouds above 512 points and pairs that
+//   k_ref_distance_warp leaves (a warp per pair, fixed point; its tables come
+//                    from k_ref_keybox);
 //   k_ref_gates / k_ref_scatter   the kept pairs in loop order;
 //   k_ref_ransac / k_ref_argmax   inliers of every kept pair's transform.
 #include <math.h>
@@ -55,6 +58,7 @@ constexpr int REF_VOL = REF_DIM * REF_DIM * REF_DIM;
 constexpr int REF_MAX_DEPTH = 21;
 constexpr int REF_PPT = 8;        // cloud points per thread in k_ref_distance
 constexpr int REF_WIN = 32;       // leaves per axis of the distance kernel's bitmap window
+constexpr unsigned REFW_REDO = 0x7fc0beefu;  // last entry of a transform that the warp form leaves to k_ref_distance
 constexpr int REF_OCC_DEPTH = 5;  // cube depth the occupancy and field kernels hold in a bitmap
 constexpr double REF_FLT_EPS = 1.1920928955078125e-07;  // FLT_EPSILON
 
@@ -456,9 +460,6 @@ __device__ __forceinline__ float leaf_running_score(float dtf, const float* val,
   return __fdiv_rn(dtf, div);
 }
 
-struct WarpSync {
-  __device__ void operator()() const { __syncwarp(); }
-};
 struct BlockSync {
   __device__ void operator()() const { __syncthreads(); }
 };
@@ -487,7 +488,7 @@ __global__ void __launch_bounds__(NT) k_ref_distance(const float4* __restrict__ 
                                                      const int* __restrict__ pair_m,
                                                      const int* __restrict__ pair_s, float res, float half,
                                                      RefRot rot, float* __restrict__ score, float* __restrict__ Tout,
-                                                     int* __restrict__ err) {
+                                                     int* __restrict__ err, int warp_max_points) {
   constexpr int NW = NT / 32;
   constexpr int CAP = NT * REF_PPT;  // distinct leaves <= points
   __shared__ RefShared<NT> sh;
@@ -499,6 +500,8 @@ __global__ void __launch_bounds__(NT) k_ref_distance(const float4* __restrict__ 
   const int s = pair_s ? pair_s[p] : (int)(p % ns);
   const float4 km = mkeys[m], ks = skeys[s];
   float* To = Tout + 16 * p;
+  // smaller clouds: only the pairs that the warp form has left
+  if (moff[m + 1] - moff[m] <= warp_max_points && __float_as_uint(To[15]) != REFW_REDO) return;
   if (!(isfinite(km.x) && isfinite(km.y) && isfinite(km.z) && isfinite(ks.x) && isfinite(ks.y) &&
         isfinite(ks.z))) {
     if (tid == 0) {
@@ -677,221 +680,626 @@ __global__ void __launch_bounds__(NT) k_ref_distance(const float4* __restrict__ 
   for (int i = 0; i < 16; ++i) To[i] = A[i];
 }
 
-// get_Distance, one warp per pair, for occupancy clouds of up to 256 points
-// (8 per lane): the same steps as k_ref_distance with every reduction a
-// shuffle, the growth's point broadcast by shuffle, and the warp's own 4 KB
-// bitmap cleared by the points that set it.
-constexpr int REFW_PPT = 8;
+// get_Distance, one warp per pair, for occupancy clouds of up to 512 points
+// (Q rows of 32; 4 KB of shared memory and less a warp).
+//
+// What bounds it: issue (and the shuffle / shared-memory pipe next to it):
+// about 120 instructions per point and rotation, no FP64 among them.  The
+// chip's FP64 rate is low enough that a dozen double operations a rotation
+// cost more than everything else, so the cubes are kept in fixed point
+// (units of 2^-40 m), where the reference's double arithmetic is exact:
+//  - the bounds of a keypoint's field cube, the leaf edge and FLT_EPSILON are
+//    multiples of the unit and below 2^13 m, so every sum and difference of
+//    the growth rule has at most 53 bits and the doubles are never rounded
+//    (k_ref_keybox checks it; keypoints that fail, and clouds beyond
+//    REFW_RANGE leaves of the origin, are left to k_ref_distance);
+//  - a float p >= c (c a whole number of units) exactly when floor(p) >= c;
+//  - a leaf key is floor((p - min) / res): from a float estimate where that is
+//    farther from a whole number than its error, else from whole-number
+//    remainders (a quotient that is not whole is more than a double's rounding
+//    away from it).
+// Per rotation: points turned; the cloud's box (four reductions; z does not
+// change) grows the cube (lane a % 3 holds axis a); keys; the leaves' tree
+// order as an 18-bit code: 15 Morton bits of the keys' low five bits, and a
+// bit per axis for a cloud that crosses a multiple of 32 leaves there, these
+// ordered by the highest bit that the crossing changes; codes with the point's
+// index sorted in registers (bitonic); equal neighbours dropped; the field
+// values, squared, put in that order in shared memory and added one by one.
+// Main's clouds (340 x 573 keypoints, clouds of 90 points on average): 62.0 ms
+// with double arithmetic per rotation, a bitonic sort of 64-bit Morton codes in
+// shared memory and a 32^3 bitmap; 12.0 ms with the growth in whole units and
+// a 32-bit sort in registers; 7.0 ms with the growth in leaves, one row of 32
+// more per size class instead of powers of two, and no sort where no value is
+// read (half the rotations there).
 constexpr int REFW_WARPS = 4;
+constexpr int REFW_MAX = 512;                 // points of the largest cloud taken
+constexpr float REFW_RANGE = 16384.f;         // leaves; coordinates also below 256 m
 
-__global__ void __launch_bounds__(32 * REFW_WARPS, 4)
+struct RefKeyBox {
+  long long mn[3], mx[3];  // the field cube, 2^-40 m
+  float M[6];              // the yaw step about the keypoint: x and y rows, columns 0, 1, 3
+  int J[3];                // field coordinate of key k: k + J, truncated toward zero
+  int depth, ok, table;    // table: J is not certain, coordinates come from doubles
+};
+
+__device__ __forceinline__ long long to_fix(float x) { return __float2ll_rd(x * 0x1p40f); }
+__device__ __forceinline__ float from_fix_rn(long long v) { return __ll2float_rn(v) * 0x1p-40f; }
+__device__ __forceinline__ float from_fix_ru(long long v) { return __ll2float_ru(v) * 0x1p-40f; }
+
+__device__ __forceinline__ float warp_min(float x) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float x) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Size classes of the warp form: rows of 32 points.  The last two take the
+// clouds whose field coordinates come from a table.
+constexpr int REFW_CLASSES = 11;
+__host__ __device__ constexpr int refw_rows(int c) {
+  constexpr int rows[REFW_CLASSES] = {1, 2, 3, 4, 5, 6, 8, 12, 16, 8, 16};
+  return rows[c];
+}
+__host__ __device__ constexpr int refw_blocks(int c) {  // resident blocks wanted an SM
+  return refw_rows(c) <= 2 ? 8 : (refw_rows(c) <= 5 ? 6 : (refw_rows(c) <= 8 ? 5 : 2));
+}
+__device__ __forceinline__ int refw_class(int n, bool table) {  // n <= REFW_MAX
+  int c = table ? 9 : 0;
+  while (n > 32 * refw_rows(c)) ++c;
+  return c;
+}
+
+// Field cube, yaw step and field offsets of every model keypoint; the keys of
+// each size class into list[class][n], their number into cls[class].
+__global__ void k_ref_keybox(const float4* __restrict__ mkeys, const int* __restrict__ moff, int n, float res,
+                             float half, RefRot rot, RefKeyBox* __restrict__ out, int* __restrict__ list,
+                             int* __restrict__ cls) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= n) return;
+  const int np = moff[m + 1] - moff[m];
+  const float4 km = mkeys[m];
+  RefKeyBox k;
+  const double dres = (double)res;
+  const float lim = fminf(res * REFW_RANGE, 256.f);
+  bool ok = res <= 0.25f && res >= 1.0e-4f && half <= lim && fabsf(km.x) <= lim && fabsf(km.y) <= lim &&
+            fabsf(km.z) <= lim;  // false for NaN
+  const long long r64 = ok ? to_fix(res) : 1;
+  ok = ok && from_fix_rn(r64) == res;
+  const float lo[3] = {__fsub_rn(km.x, half), __fsub_rn(km.y, half), __fsub_rn(km.z, half)};
+  const float hi[3] = {__fadd_rn(km.x, half), __fadd_rn(km.y, half), __fadd_rn(km.z, half)};
+  OctBox b;
+  b.depth = 0;
+  if (ok) oct_define(b, lo, hi, dres);
+  k.table = 0;
+  for (int a = 0; a < 3; ++a) {
+    k.mn[a] = k.mx[a] = 0;
+    k.J[a] = 0;
+    if (!ok) continue;
+    k.mn[a] = __double2ll_rd(b.mn[a] * 0x1p40);
+    k.mx[a] = __double2ll_rd(b.mx[a] * 0x1p40);
+    ok = ok && (double)k.mn[a] * 0x1p-40 == b.mn[a] && (double)k.mx[a] * 0x1p-40 == b.mx[a] &&
+         from_fix_rn(to_fix(lo[a])) == lo[a] && llabs(k.mx[a] - k.mn[a] - (r64 << b.depth)) <= 1ll << 17;
+    // the field coordinate (centre of leaf k - lo) / res = k + num / (2 res):
+    // its whole part is certain while the fraction stays clear of 0 and 1
+    // (rounding moves it by less than 0.05 at REFW_RANGE)
+    const long long num = 2 * (k.mn[a] - to_fix(lo[a])) + r64, den = 2 * r64;
+    long long q = num / den;
+    if (q * den > num) --q;
+    const long long fr = num - q * den;
+    if (fr * 20 < den * 3 || fr * 20 > den * 17) k.table = 1;
+    k.J[a] = (int)q;
+  }
+  float T1[16], T3[16], M[16], Rs[16];
+  eye4(T1);
+  T1[3] = -km.x, T1[7] = -km.y;
+  eye4(T3);
+  T3[3] = km.x, T3[7] = km.y;
+  eye4(Rs);
+  Rs[0] = rot.c1, Rs[4] = rot.s1, Rs[1] = -rot.s1, Rs[5] = rot.c1;
+  mm4(T3, Rs, M);
+  mm4(M, T1, M);
+  // a turn about a vertical axis: z stays, and x and y take nothing from it
+  ok = ok && M[2] == 0.f && M[6] == 0.f && M[8] == 0.f && M[9] == 0.f && M[10] == 1.f && M[11] == 0.f;
+  k.M[0] = M[0], k.M[1] = M[1], k.M[2] = M[3], k.M[3] = M[4], k.M[4] = M[5], k.M[5] = M[7];
+  k.depth = b.depth;
+  k.ok = ok;
+  out[m] = k;
+  if (np <= REFW_MAX) {
+    const int c = refw_class(np, k.table != 0);
+    list[(size_t)c * n + atomicAdd(cls + c, 1)] = m;
+  }
+}
+
+// floor((p - mn) / res) as the reference's doubles give it; est is within a
+// few of it.  p lies in the cube.
+__device__ __forceinline__ int ref_key_exact(float p, long long mn, long long r64, double dres, int est) {
+  const long long P = to_fix(p);
+  if (from_fix_rn(P) == p) {
+    long long r = P - mn - (long long)est * r64;
+    while (r < 0) --est, r += r64;
+    while (r >= r64) ++est, r -= r64;
+    return est;
+  }
+  return (int)__double2uint_rz(__ddiv_rn(__dsub_rn((double)p, (double)mn * 0x1p-40), dres));
+}
+
+// Ascending sort of 32 Q words, word i = lane * Q + q: runs of Q sorted in
+// each lane, then merged pairwise five times.  A merge compares the runs head
+// to tail (lower lanes keep the smaller words), halves the bitonic rest lane
+// against lane, and sorts the bitonic Q left in each lane; the halving needs
+// only even lengths, so Q need not be a power of two.
+__device__ __forceinline__ void cmp_swap(unsigned& a, unsigned& b) {
+  const unsigned lo = min(a, b);
+  b = max(a, b);
+  a = lo;
+}
+template <int Q, int O, int N>
+__device__ __forceinline__ void lane_bitonic(unsigned (&x)[Q]) {  // words O .. O + N - 1, bitonic (any order if N is odd)
+  if constexpr (N == 3) {
+    cmp_swap(x[O], x[O + 1]);
+    cmp_swap(x[O + 1], x[O + 2]);
+    cmp_swap(x[O], x[O + 1]);
+  } else if constexpr (N == 5) {
+    cmp_swap(x[O], x[O + 3]);
+    cmp_swap(x[O + 1], x[O + 4]);
+    cmp_swap(x[O], x[O + 2]);
+    cmp_swap(x[O + 1], x[O + 3]);
+    cmp_swap(x[O], x[O + 1]);
+    cmp_swap(x[O + 2], x[O + 4]);
+    cmp_swap(x[O + 1], x[O + 2]);
+    cmp_swap(x[O + 3], x[O + 4]);
+    cmp_swap(x[O + 2], x[O + 3]);
+  } else if constexpr (N > 1) {
+    static_assert(N % 2 == 0, "half-cleaner");
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) cmp_swap(x[O + i], x[O + N / 2 + i]);
+    lane_bitonic<Q, O, N / 2>(x);
+    lane_bitonic<Q, O + N / 2, N / 2>(x);
+  }
+}
+template <int Q, int O, int N>
+__device__ __forceinline__ void lane_sort(unsigned (&x)[Q]) {
+  if constexpr (N == 3 || N == 5) {
+    lane_bitonic<Q, O, N>(x);
+  } else if constexpr (N > 1) {
+    lane_sort<Q, O, N / 2>(x);
+    lane_sort<Q, O + N / 2, N / 2>(x);
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) cmp_swap(x[O + i], x[O + N - 1 - i]);
+    lane_bitonic<Q, O, N / 2>(x);
+    lane_bitonic<Q, O + N / 2, N / 2>(x);
+  }
+}
+template <int Q>
+__device__ __forceinline__ void warp_sort(unsigned (&x)[Q], int lane) {
+  lane_sort<Q, 0, Q>(x);
+#pragma unroll
+  for (int m = 1; m <= 5; ++m) {
+    {
+      const int d = (1 << m) - 1;
+      const bool low = (lane & (1 << (m - 1))) == 0;
+      unsigned v[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) v[q] = __shfl_xor_sync(0xffffffffu, x[Q - 1 - q], d);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) x[q] = low ? min(x[q], v[q]) : max(x[q], v[q]);
+    }
+#pragma unroll
+    for (int d = 1 << (m - 1) >> 1; d > 0; d >>= 1) {
+      const bool low = (lane & d) == 0;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const unsigned v = __shfl_xor_sync(0xffffffffu, x[q], d);
+        x[q] = low ? min(x[q], v) : max(x[q], v);
+      }
+    }
+    lane_bitonic<Q, 0, Q>(x);
+  }
+}
+
+// One 4x4 product, element lane = 4 r + c in lanes 0..15 (mm4's order).
+__device__ __forceinline__ float warp_mm4(float A, float B, int lane) {
+  const int r = (lane >> 2) & 3, c = lane & 3;
+  float s = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float t = __fmul_rn(__shfl_sync(0xffffffffu, A, 4 * r + k), __shfl_sync(0xffffffffu, B, 4 * k + c));
+    s = k == 0 ? t : __fadd_rn(s, t);
+  }
+  return s;
+}
+
+// Pairs of size class CLS: all scan keypoints against the n_items / ns model
+// keypoints in list, or, with a pair list, its pairs of this class.
+template <int CLS>
+__global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
     k_ref_distance_warp(const float4* __restrict__ mcloud, const float4* __restrict__ mkeys,
                         const int* __restrict__ moff, const int* __restrict__ midx, const float* __restrict__ mtdf,
+                        const RefKeyBox* __restrict__ boxes, const int* __restrict__ list,
                         const float4* __restrict__ skeys, int ns, const int* __restrict__ pair_m,
-                        const int* __restrict__ pair_s, long long n_pairs, float res, float half, RefRot rot,
+                        const int* __restrict__ pair_s, long long n_items, float res, float half, RefRot rot,
                         float* __restrict__ score, float* __restrict__ Tout, int* __restrict__ err) {
-  __shared__ unsigned s_bm[REFW_WARPS][REF_WIN * REF_WIN * REF_WIN / 32];
-  __shared__ long long s_ix[REFW_WARPS][3][REF_WIN];
-  __shared__ unsigned long long s_key[REFW_WARPS][REFW_PPT * 32];
-  __shared__ float s_val[REFW_WARPS][REFW_PPT * 32];
-  __shared__ int s_u[REFW_WARPS];
+  constexpr int Q = refw_rows(CLS);
+  constexpr bool TABLE = CLS >= 9;
+  __shared__ unsigned s_bm[REFW_WARPS][REF_WIN * REF_WIN];  // leaves of a cloud that reads no field value
+  __shared__ __align__(16) float s_v[REFW_WARPS][32 * Q];
+  __shared__ unsigned s_ord[REFW_WARPS][3][64];             // order code of a local key, by axis, above the point index
+  __shared__ int s_fld[TABLE ? REFW_WARPS : 1][3][64];      // its share of the field index
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned* bm = s_bm[w];
-  const float inv = __fdiv_rn(1.f, res);
-  for (int i = lane; i < REF_WIN * REF_WIN * REF_WIN / 32; i += 32) bm[i] = 0u;
-  __syncwarp();
+  long long p = (long long)blockIdx.x * REFW_WARPS + w;
+  if (p >= n_items) return;
+  int m, sk;
+  if (pair_m) {
+    m = pair_m[p], sk = pair_s[p];
+    const int np = moff[m + 1] - moff[m];
+    if (np > REFW_MAX || refw_class(np, boxes[m].table != 0) != CLS) return;
+  } else {
+    m = list[p / ns], sk = (int)(p % ns);
+    p = (long long)m * ns + sk;
+  }
+  const int beg = moff[m], n = moff[m + 1] - beg;
+  const float4 km = mkeys[m], ks = skeys[sk];
+  float* To = Tout + 16 * p;
+  if (!(isfinite(km.x) && isfinite(km.y) && isfinite(km.z) && isfinite(ks.x) && isfinite(ks.y) && isfinite(ks.z))) {
+    if (lane == 0) score[p] = __int_as_float(0x7fc00000);
+    if (lane < 16) To[lane] = (lane % 5) == 0 ? 1.f : 0.f;
+    return;
+  }
+  const RefKeyBox* kb = boxes + m;
+  const float lim = fminf(res * REFW_RANGE, 256.f);
+  const float tx = __fsub_rn(km.x, ks.x), ty = __fsub_rn(km.y, ks.y), tz = __fsub_rn(km.z, ks.z);
+  float px[Q], py[Q], pz[Q];
+  bool fine = kb->ok != 0;
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int j = lane + 32 * q;
+    px[q] = py[q] = pz[q] = 0.f;
+    if (n > 0) {  // rows past the cloud repeat its first point: the same leaf
+      const float4 c = mcloud[midx[beg + (j < n ? j : 0)]];
+      px[q] = __fadd_rn(c.x, tx), py[q] = __fadd_rn(c.y, ty), pz[q] = __fadd_rn(c.z, tz);
+      fine = fine && fabsf(c.x) <= lim && fabsf(c.y) <= lim && fabsf(c.z) <= lim && fabsf(px[q]) <= lim &&
+             fabsf(py[q]) <= lim && fabsf(pz[q]) <= lim;
+    }
+  }
+  if (!__all_sync(0xffffffffu, fine)) {
+    if (lane == 0) {
+      To[15] = __uint_as_float(REFW_REDO);
+      atomicAdd(err + 2, 1);
+    }
+    return;
+  }
+  const float* grid = mtdf + (size_t)m * REF_VOL;
   const double dres = (double)res;
-  for (long long p = (long long)blockIdx.x * REFW_WARPS + w; p < n_pairs; p += (long long)gridDim.x * REFW_WARPS) {
-    const int m = pair_m ? pair_m[p] : (int)(p / ns);
-    const int s = pair_s ? pair_s[p] : (int)(p % ns);
-    const float4 km = mkeys[m], ks = skeys[s];
-    float* To = Tout + 16 * p;
-    if (!(isfinite(km.x) && isfinite(km.y) && isfinite(km.z) && isfinite(ks.x) && isfinite(ks.y) &&
-          isfinite(ks.z))) {
-      if (lane == 0) {
-        score[p] = __int_as_float(0x7fc00000);
-        eye4(To);
-      }
-      continue;
-    }
-    const int beg = moff[m], n = moff[m + 1] - beg;
-    const float* grid = mtdf + (size_t)m * REF_VOL;
-    const float lo[3] = {__fsub_rn(km.x, half), __fsub_rn(km.y, half), __fsub_rn(km.z, half)};
-    const float hi[3] = {__fadd_rn(km.x, half), __fadd_rn(km.y, half), __fadd_rn(km.z, half)};
-    float Tm[16], T1[16], T3[16], M[16];
-    eye4(Tm);
-    Tm[3] = __fsub_rn(km.x, ks.x), Tm[7] = __fsub_rn(km.y, ks.y), Tm[11] = __fsub_rn(km.z, ks.z);
-    eye4(T1);
-    T1[3] = -km.x, T1[7] = -km.y;
-    eye4(T3);
-    T3[3] = km.x, T3[7] = km.y;
-    {
-      float Rs[16];
-      eye4(Rs);
-      Rs[0] = rot.c1, Rs[4] = rot.s1, Rs[1] = -rot.s1, Rs[5] = rot.c1;
-      mm4(T3, Rs, M);
-      mm4(M, T1, M);
-    }
-    float px[REFW_PPT], py[REFW_PPT], pz[REFW_PPT];
+  const float inv = __fdiv_rn(1.f, res);
+  const long long r64 = to_fix(res), eps64 = 1ll << 17;  // FLT_EPSILON = 2^-23
+  const int ax = lane % 3;                               // this lane's axis
+  const long long mn0 = kb->mn[ax], mx0 = kb->mx[ax];
+  const int J = kb->J[ax], stride = ax == 0 ? 1 : (ax == 1 ? REF_DIM : REF_DIM * REF_DIM);
+  const int J0 = kb->J[0], J1 = kb->J[1], J2 = kb->J[2];
+  const int depth0 = kb->depth;
+  const float m0 = kb->M[0], m1 = kb->M[1], m3 = kb->M[2], m4 = kb->M[3], m5 = kb->M[4], m7 = kb->M[5];
+  float zmn = pz[0], zmx = pz[0], far = 0.f;
 #pragma unroll
-    for (int q = 0; q < REFW_PPT; ++q) {
-      const int j = lane + 32 * q;
-      px[q] = py[q] = pz[q] = 0.f;
-      if (j < n) {
-        const float4 c = mcloud[midx[beg + j]];
-        px[q] = c.x, py[q] = c.y, pz[q] = c.z;
-        xf3(Tm, px[q], py[q], pz[q]);
+  for (int q = 0; q < Q; ++q) {
+    zmn = fminf(zmn, pz[q]), zmx = fmaxf(zmx, pz[q]);
+    far = fmaxf(far, fabsf(px[q] - km.x) + fabsf(py[q] - km.y));
+  }
+  zmn = warp_min(zmn), zmx = warp_max(zmx), far = warp_max(far);
+  // leaf coordinates: y = (p - mn0) / res - 1/2 by one FMA, off by at most
+  // 2^-22 (|c| + |y|); rounding it to a whole number gives the leaf (counted
+  // from the field cube's corner) unless y is more than `sure` from it
+  const float c_a = -(from_fix_rn(mn0) * inv) - 0.5f;
+  const float reach = ((ax == 0 ? fabsf(km.x) : (ax == 1 ? fabsf(km.y) : 0.f)) +
+                       (ax == 2 ? fmaxf(fabsf(zmn), fabsf(zmx)) : 1.01f * far)) * inv;
+  const float sure = 0.5f - warp_max((2.f * fabsf(c_a) + reach + 2.f) * 0x1p-22f + 2.5e-7f * inv);
+  const float c0 = __shfl_sync(0xffffffffu, c_a, 0), c1 = __shfl_sync(0xffffffffu, c_a, 1),
+              c2 = __shfl_sync(0xffffffffu, c_a, 2);
+  constexpr float MAGIC = 12582912.f;  // 1.5 * 2^23: adding it rounds to a whole number, in the low bits
+  constexpr int MBITS = 0x4b400000;
+  const float zfirst = __shfl_sync(0xffffffffu, pz[0], 0);
+  unsigned spread = 0;  // the lane's five bits, every third
+#pragma unroll
+  for (int i = 0; i < 5; ++i) spread |= ((unsigned)lane >> i & 1u) << (3 * i);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) s_ord[w][a][lane] = spread << (9 + 2 - a);
+  for (int i = lane; i < REF_WIN * REF_WIN; i += 32) s_bm[w][i] = 0u;
+  __syncwarp();
+  float dtf = 0.f, bestf = 100000000.f;
+  int best_i = 0;
+  bool bad = false;
+  for (int it = 0; it < 36; ++it) {
+    if (it != 0) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const float x = __fadd_rn(__fadd_rn(__fmul_rn(m0, px[q]), __fmul_rn(m1, py[q])), m3);
+        const float y = __fadd_rn(__fadd_rn(__fmul_rn(m4, px[q]), __fmul_rn(m5, py[q])), m7);
+        px[q] = x, py[q] = y;
       }
     }
-    OctBox b0;
-    oct_define(b0, lo, hi, dres);
-    OctBoxF bf0;
-    oct_float(b0, bf0);
-    float dtf = 0.f, bestf = 100000000.f;
-    int best_i = 0;
-    bool bad = false;
-    for (int it = 0; it < 36 && !bad; ++it) {
-      if (it != 0) {
+    int u = 0;
+    if (n > 0) {
+      float xmn = px[0], xmx = px[0], ymn = py[0], ymx = py[0];
 #pragma unroll
-        for (int q = 0; q < REFW_PPT; ++q)
-          if (lane + 32 * q < n) xf3(M, px[q], py[q], pz[q]);
+      for (int q = 1; q < Q; ++q) {
+        xmn = fminf(xmn, px[q]), xmx = fmaxf(xmx, px[q]);
+        ymn = fminf(ymn, py[q]), ymx = fmaxf(ymx, py[q]);
       }
-      OctBox b = b0;
-      OctBoxF bf = bf0;
-      for (int round = 0; round < 4 * REF_MAX_DEPTH + 4; ++round) {
-        int first = 0x7fffffff;
+      xmn = warp_min(xmn), xmx = warp_max(xmx), ymn = warp_min(ymn), ymx = warp_max(ymx);
+      const float amn = ax == 0 ? xmn : (ax == 1 ? ymn : zmn), amx = ax == 0 ? xmx : (ax == 1 ? ymx : zmx);
+      // this axis: leaves of the cloud's box; K, depth: the grown cube is
+      // leaves [-K, -K + 2^depth)
+      int kmn, kmx, K = 0, depth = depth0;
+      bool near;
+      {
+        const float y0 = __fmaf_rn(amn, inv, c_a), y1 = __fmaf_rn(amx, inv, c_a);
+        const float t0 = __fadd_rn(y0, MAGIC), t1 = __fadd_rn(y1, MAGIC);
+        kmn = __float_as_int(t0) - MBITS, kmx = __float_as_int(t1) - MBITS;
+        near = fabsf(__fsub_rn(y0, __fsub_rn(t0, MAGIC))) > sure || fabsf(__fsub_rn(y1, __fsub_rn(t1, MAGIC))) > sure;
+      }
+      near = __any_sync(0xffffffffu, near);
+      // growth: the first point outside (in index order) grows the cube until
+      // it fits, until no point is outside.  Away from whole numbers the
+      // leaves decide (the bounds are whole, up to the FLT_EPSILON that
+      // `sure` covers)
+      for (int round = 0; !near && round < 2 * REF_MAX_DEPTH; ++round) {
+        if (!__any_sync(0xffffffffu, kmn < -K || kmx >= (1 << depth) - K)) break;
+        float sx = __shfl_sync(0xffffffffu, px[0], 0), sy = __shfl_sync(0xffffffffu, py[0], 0), sz = zfirst;
+        float yp = __fmaf_rn(ax == 0 ? sx : (ax == 1 ? sy : sz), inv, c_a);
+        float tp = __fadd_rn(yp, MAGIC);
+        int ip = __float_as_int(tp) - MBITS;
+        if (!__any_sync(0xffffffffu, ip < -K || ip >= (1 << depth) - K)) {
+          // the first point that is outside or too near a bound to tell
+          const float flo = (float)-K - sure, fhi = (float)((1 << depth) - K) - 1.f + sure;
+          const float lo0 = __shfl_sync(0xffffffffu, flo, 0), lo1 = __shfl_sync(0xffffffffu, flo, 1),
+                      lo2 = __shfl_sync(0xffffffffu, flo, 2), hi0 = __shfl_sync(0xffffffffu, fhi, 0),
+                      hi1 = __shfl_sync(0xffffffffu, fhi, 1), hi2 = __shfl_sync(0xffffffffu, fhi, 2);
+          unsigned first = ~0u;
 #pragma unroll
-        for (int q = 0; q < REFW_PPT; ++q) {
-          const int j = lane + 32 * q;
-          if (j < n && first == 0x7fffffff && oct_outside_f(bf, px[q], py[q], pz[q])) first = j;
+          for (int q = Q - 1; q >= 0; --q) {
+            const float y0 = __fmaf_rn(px[q], inv, c0), y1 = __fmaf_rn(py[q], inv, c1), y2 = __fmaf_rn(pz[q], inv, c2);
+            if (y0 < lo0 || y0 > hi0 || y1 < lo1 || y1 > hi1 || y2 < lo2 || y2 > hi2) first = (unsigned)(lane + 32 * q);
+          }
+          first = __reduce_min_sync(0xffffffffu, first);
+          const unsigned q0 = first >> 5;
+#pragma unroll
+          for (int q = 0; q < Q; ++q)
+            if ((unsigned)q == q0) sx = px[q], sy = py[q], sz = pz[q];
+          const int src = (int)(first & 31u);
+          sx = __shfl_sync(0xffffffffu, sx, src);
+          sy = __shfl_sync(0xffffffffu, sy, src);
+          sz = __shfl_sync(0xffffffffu, sz, src);
+          yp = __fmaf_rn(ax == 0 ? sx : (ax == 1 ? sy : sz), inv, c_a);
+          tp = __fadd_rn(yp, MAGIC);
+          ip = __float_as_int(tp) - MBITS;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-        if (first == 0x7fffffff) break;
-        const int q0 = first >> 5, src = first & 31;
-        float sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll
-        for (int q = 0; q < REFW_PPT; ++q)
-          if (q == q0) sx = px[q], sy = py[q], sz = pz[q];
-        sx = __shfl_sync(0xffffffffu, sx, src);
-        sy = __shfl_sync(0xffffffffu, sy, src);
-        sz = __shfl_sync(0xffffffffu, sz, src);
-        if (!oct_fit(b, sx, sy, sz, dres)) {
-          bad = true;
-          break;
+        near = __any_sync(0xffffffffu, fabsf(__fsub_rn(yp, __fsub_rn(tp, MAGIC))) > sure);
+        while (!near && !bad) {
+          const bool up = ip >= (1 << depth) - K;
+          if (!__any_sync(0xffffffffu, up || ip < -K)) break;
+          if (!up) K += 1 << depth;
+          bad = ++depth > REF_MAX_DEPTH;
         }
-        oct_float(b, bf);
+        if (bad) break;
+      }
+      if (near && !bad) {
+        // some point decides the growth from close to a whole leaf: the same in
+        // whole units of 2^-40 m
+        long long mn = mn0, mx = mx0;
+        const long long bmn = to_fix(amn), bmx = to_fix(amx);
+        K = 0, depth = depth0;
+        for (int round = 0; !bad && round < 2 * REF_MAX_DEPTH && __any_sync(0xffffffffu, bmn < mn || bmx >= mx); ++round) {
+          const float fmn = from_fix_ru(mn), fmx = from_fix_ru(mx);
+          OctBoxF bf;
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            bf.mn_up[a] = __shfl_sync(0xffffffffu, fmn, a);
+            bf.mx_up[a] = __shfl_sync(0xffffffffu, fmx, a);
+          }
+          unsigned first = ~0u;
+#pragma unroll
+          for (int q = Q - 1; q >= 0; --q)
+            if (oct_outside_f(bf, px[q], py[q], pz[q])) first = (unsigned)(lane + 32 * q);
+          first = __reduce_min_sync(0xffffffffu, first);
+          const unsigned q0 = first >> 5;
+          float sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll
+          for (int q = 0; q < Q; ++q)
+            if ((unsigned)q == q0) sx = px[q], sy = py[q], sz = pz[q];
+          const int src = (int)(first & 31u);
+          sx = __shfl_sync(0xffffffffu, sx, src);
+          sy = __shfl_sync(0xffffffffu, sy, src);
+          sz = __shfl_sync(0xffffffffu, sz, src);
+          const long long P = to_fix(ax == 0 ? sx : (ax == 1 ? sy : sz));
+          while (!bad && __any_sync(0xffffffffu, P < mn || P >= mx)) {
+            if (P < mx) {
+              mn -= r64 << depth;
+              K += 1 << depth;
+            }
+            bad = ++depth > REF_MAX_DEPTH;
+            mx = mn + (r64 << depth) - eps64;
+          }
+        }
+        kmn = ref_key_exact(amn, mn, r64, dres, kmn + K) - K;
+        kmx = ref_key_exact(amx, mn, r64, dres, kmx + K) - K;
       }
       if (bad) break;
-      // keys packed 21 bits per axis; the Morton code only for the first leaf
-      unsigned long long pk[REFW_PPT];
-      unsigned long long mmin = ~0ull;
-      unsigned kmin[3] = {~0u, ~0u, ~0u}, kmax[3] = {0u, 0u, 0u};
-#pragma unroll
-      for (int q = 0; q < REFW_PPT; ++q) {
-        pk[q] = ~0ull;
-        if (lane + 32 * q < n) {
-          const unsigned kx = oct_key_f(b, bf, px[q], 0, dres, inv), ky = oct_key_f(b, bf, py[q], 1, dres, inv),
-                         kz = oct_key_f(b, bf, pz[q], 2, dres, inv);
-          pk[q] = (unsigned long long)kx | ((unsigned long long)ky << 21) | ((unsigned long long)kz << 42);
-          mmin = min(mmin, morton3(kx, ky, kz, b.depth));
-          kmin[0] = min(kmin[0], kx), kmin[1] = min(kmin[1], ky), kmin[2] = min(kmin[2], kz);
-          kmax[0] = max(kmax[0], kx), kmax[1] = max(kmax[1], ky), kmax[2] = max(kmax[2], kz);
+      if (__any_sync(0xffffffffu, kmx - kmn >= REF_WIN)) {
+        if (lane == 0) atomicOr(err, REF_ERR_WINDOW);
+      } else {
+        // the field index's range over the cloud's box: nothing to read when
+        // it lies outside the field, and then the leaves' order does not
+        // matter either (every value is 900)
+        int flo = kmn + J, fhi = kmx + J;
+        flo = (flo + (flo < 0)) * stride, fhi = (fhi + (fhi < 0)) * stride;
+        flo = lane < 3 ? flo : 0, fhi = lane < 3 ? fhi : 0;
+        const bool inside =
+            TABLE || (__reduce_add_sync(0xffffffffu, fhi) >= 0 && __reduce_add_sync(0xffffffffu, flo) < REF_VOL);
+        // local keys: from a multiple of 32 of the cube's keys at or below the
+        // lowest (0..63), or from the lowest (0..31)
+        const int base = inside ? ((kmn + K) & ~31) - K : kmn;
+        const int b0 = __shfl_sync(0xffffffffu, base, 0), b1 = __shfl_sync(0xffffffffu, base, 1),
+                  b2 = __shfl_sync(0xffffffffu, base, 2);
+        if (inside) {
+          const unsigned B = (unsigned)((kmn + K) >> 5), chg = B ^ (B + 1u);  // bits that a crossing changes
+          const unsigned cx = __shfl_sync(0xffffffffu, chg, 0), cy = __shfl_sync(0xffffffffu, chg, 1),
+                         cz = __shfl_sync(0xffffffffu, chg, 2);
+          s_ord[w][0][lane + 32] = (spread << 11) | (1u << (24 + (cx >= cy) + (cx >= cz)));
+          s_ord[w][1][lane + 32] = (spread << 10) | (1u << (24 + (cy > cx) + (cy >= cz)));
+          s_ord[w][2][lane + 32] = (spread << 9) | (1u << (24 + (cz > cx) + (cz > cy)));
+          if constexpr (TABLE) {
+#pragma unroll 1
+            for (int a = 0; a < 3; ++a) {
+              const int ba = a == 0 ? b0 : (a == 1 ? b1 : b2);
+              const int st = a == 0 ? 1 : (a == 1 ? REF_DIM : REF_DIM * REF_DIM);
+              const float lo = __fsub_rn(a == 0 ? km.x : (a == 1 ? km.y : km.z), half);
+              const double dmn = (double)__shfl_sync(0xffffffffu, mn0, a) * 0x1p-40;
+#pragma unroll 1
+              for (int l = lane; l < 64; l += 32) {
+                const float e = __double2float_rn(__dadd_rn(__dmul_rn(__dadd_rn((double)(ba + l), 0.5), dres), dmn));
+                s_fld[TABLE ? w : 0][a][l] = __float2int_rz(__fdiv_rn(__fsub_rn(e, lo), res)) * st;
+              }
+            }
+          }
+          __syncwarp();
         }
-      }
+        // one point: its sort word and squared field value, or its leaf's bit
+        const bool neg = __any_sync(0xffffffffu, kmn + J < 0);  // some field coordinate is truncated upward
+        auto place = [&](int j, int i0, int i1, int i2, float* sq) -> unsigned {
+          const int l0 = (i0 - b0) & 63, l1 = (i1 - b1) & 63, l2 = (i2 - b2) & 63;
+          int idx;
+          if constexpr (TABLE) {
+            idx = s_fld[TABLE ? w : 0][0][l0] + s_fld[TABLE ? w : 0][1][l1] + s_fld[TABLE ? w : 0][2][l2];
+          } else {
+            int f0 = i0 + J0, f1 = i1 + J1, f2 = i2 + J2;
+            if (neg) f0 += f0 < 0, f1 += f1 < 0, f2 += f2 < 0;
+            idx = f0 + REF_DIM * f1 + REF_DIM * REF_DIM * f2;
+          }
+          const float v = (unsigned)idx < (unsigned)REF_VOL ? __ldg(grid + idx) : 900.f;
+          *sq = __fmul_rn(v, v);
+          return j < n ? s_ord[w][0][l0] + s_ord[w][1][l1] + s_ord[w][2][l2] + (unsigned)j : ~0u;
+        };
+        auto mark = [&](int i0, int i1, int i2, bool* fresh) -> unsigned {
+          const unsigned wd = (unsigned)(((i1 - b1) & 31) + REF_WIN * ((i2 - b2) & 31)), bit = 1u << ((i0 - b0) & 31);
+          *fresh = (atomicOr(&s_bm[w][wd], bit) & bit) == 0u;
+          return wd;
+        };
+        unsigned word[Q], close = 0u;  // close: bit q, point too near a whole leaf
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        mmin = min(mmin, __shfl_xor_sync(0xffffffffu, mmin, o));
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          kmin[a] = min(kmin[a], __shfl_xor_sync(0xffffffffu, kmin[a], o));
-          kmax[a] = max(kmax[a], __shfl_xor_sync(0xffffffffu, kmax[a], o));
+        for (int q = 0; q < Q; ++q) {
+          const int j = lane + 32 * q;
+          const float y0 = __fmaf_rn(px[q], inv, c0), y1 = __fmaf_rn(py[q], inv, c1), y2 = __fmaf_rn(pz[q], inv, c2);
+          const float t0 = __fadd_rn(y0, MAGIC), t1 = __fadd_rn(y1, MAGIC), t2 = __fadd_rn(y2, MAGIC);
+          const bool c = fabsf(__fsub_rn(y0, __fsub_rn(t0, MAGIC))) > sure ||
+                         fabsf(__fsub_rn(y1, __fsub_rn(t1, MAGIC))) > sure ||
+                         fabsf(__fsub_rn(y2, __fsub_rn(t2, MAGIC))) > sure;
+          if (c && j < n) close |= 1u << q;
+          const int i0 = __float_as_int(t0) - MBITS, i1 = __float_as_int(t1) - MBITS, i2 = __float_as_int(t2) - MBITS;
+          if (inside) {
+            float sq;
+            word[q] = place(j, i0, i1, i2, &sq);
+            s_v[w][j] = sq;
+          } else {
+            bool fresh = false;
+            word[q] = 0u;
+            if (!c && j < n) word[q] = mark(i0, i1, i2, &fresh);
+            u += __popc(__ballot_sync(0xffffffffu, fresh));
+          }
         }
-      }
-      const bool window_ok = n == 0 || (kmax[0] - kmin[0] < (unsigned)REF_WIN &&
-                                        kmax[1] - kmin[1] < (unsigned)REF_WIN && kmax[2] - kmin[2] < (unsigned)REF_WIN);
-      if (!window_ok && lane == 0) atomicOr(err, REF_ERR_WINDOW);
-      // the field's integer coordinate of every leaf column of the window,
-      // one per lane and axis (a huge negative value where get_Distance's
-      // float quotient leaves the int range: the index is then out of range)
+        while (__any_sync(0xffffffffu, close != 0u)) {
+          const int qq = close ? __ffs(close) - 1 : Q;
+          float x = 0.f, y = 0.f, z = 0.f;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const float c = oct_centre(b, kmin[a] + (unsigned)lane, a, dres);
-        const float qv = __fdiv_rn(__fsub_rn(c, lo[a]), res);
-        s_ix[w][a][lane] = (qv > -2147483648.f && qv < 2147483648.f) ? (long long)__float2int_rz(qv)
-                                                                      : -(1ll << 50);
-      }
-      unsigned long long pk_first;
-      {
-        unsigned fx, fy, fz;
-        demorton3(mmin, b.depth, fx, fy, fz);
-        pk_first = (unsigned long long)fx | ((unsigned long long)fy << 21) | ((unsigned long long)fz << 42);
-      }
-      if (lane == 0) s_u[w] = 0;
-      __syncwarp();
-      // distinct leaves: the lane that sets a leaf's bit reads its field and
-      // lists (Morton code, value); the first leaf's value is never added
-      unsigned lw[REFW_PPT];
+          for (int q = 0; q < Q; ++q)
+            if (q == qq) x = px[q], y = py[q], z = pz[q];
+          int i[3];
 #pragma unroll
-      for (int q = 0; q < REFW_PPT; ++q) {
-        lw[q] = 0xffffffffu;
-        if (!window_ok || pk[q] == ~0ull) continue;
-        const unsigned kx = (unsigned)(pk[q] & 0x1fffffull), ky = (unsigned)((pk[q] >> 21) & 0x1fffffull),
-                       kz = (unsigned)(pk[q] >> 42);
-        const unsigned lx = kx - kmin[0], ly = ky - kmin[1], lz = kz - kmin[2];
-        const unsigned l = lx + REF_WIN * (ly + REF_WIN * lz);
-        lw[q] = l >> 5;
-        const unsigned bit = 1u << (l & 31u);
-        const unsigned old = atomicOr(&bm[l >> 5], bit);
-        if (old & bit) continue;
-        float v = 0.f;
-        if (pk[q] != pk_first) {
-          const long long idx = s_ix[w][1][ly] * REF_DIM + s_ix[w][2][lz] * (REF_DIM * REF_DIM) + s_ix[w][0][lx];
-          v = (idx >= 0 && idx < REF_VOL) ? __ldg(grid + idx) : 900.f;
+          for (int a = 0; a < 3; ++a) {
+            const long long mna = __shfl_sync(0xffffffffu, mn0 - (long long)K * r64, a);
+            const int ka = __shfl_sync(0xffffffffu, K, a);
+            const float pa = a == 0 ? x : (a == 1 ? y : z), ca = a == 0 ? c0 : (a == 1 ? c1 : c2);
+            i[a] = 0;
+            if (close) i[a] = ref_key_exact(pa, mna, r64, dres, __float2int_rn(__fmaf_rn(pa, inv, ca)) + ka) - ka;
+          }
+          bool fresh = false;
+          if (close) {
+            unsigned wd;
+            if (inside) {
+              float sq;
+              wd = place(lane + 32 * qq, i[0], i[1], i[2], &sq);
+              s_v[w][lane + 32 * qq] = sq;
+            } else {
+              wd = mark(i[0], i[1], i[2], &fresh);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q) word[q] = q == qq ? wd : word[q];
+          }
+          u += __popc(__ballot_sync(0xffffffffu, fresh));
+          close &= close - 1u;
         }
-        const int slot = atomicAdd(&s_u[w], 1);
-        s_key[w][slot] = morton3(kx, ky, kz, b.depth);
-        s_val[w][slot] = v;
-      }
-      __syncwarp();
-      const int u = s_u[w];
-      int P = 2;
-      while (P < u) P <<= 1;
-      for (int i = u + lane; i < P; i += 32) s_key[w][i] = ~0ull;
-      __syncwarp();
-      leaf_sort(s_key[w], s_val[w], P, lane, 32, WarpSync());
-      if (lane == 0) {
-        dtf = leaf_running_score(dtf, s_val[w], u);
-        if (dtf < bestf) {
-          bestf = dtf;
-          best_i = it;
-        }
-      }
-      __syncwarp();
+        if (!inside) {
+          __syncwarp();
 #pragma unroll
-      for (int q = 0; q < REFW_PPT; ++q)
-        if (lw[q] != 0xffffffffu) bm[lw[q]] = 0u;
-      __syncwarp();
+          for (int q = 0; q < Q; ++q) s_bm[w][word[q]] = 0u;
+#pragma unroll 8
+          for (int i = 1; i < u; ++i) dtf = __fadd_rn(dtf, 810000.f);
+        } else {
+          warp_sort<Q>(word, lane);
+          __syncwarp();
+          // distinct leaves after the first keep their value
+          const unsigned prev = __shfl_up_sync(0xffffffffu, word[Q - 1], 1);
+          float val[Q];
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const unsigned before = q == 0 ? prev : word[q > 0 ? q - 1 : 0];
+            const bool head = (q == 0 && lane == 0) || (word[q] >> 9) != (before >> 9);
+            const bool leaf = head && word[q] != ~0u;
+            u += __popc(__ballot_sync(0xffffffffu, leaf));
+            val[q] = leaf && !(q == 0 && lane == 0) ? s_v[w][word[q] & 511u] : 0.f;
+          }
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < Q; ++q) s_v[w][lane * Q + q] = val[q];
+          __syncwarp();
+          const float4* sv = reinterpret_cast<const float4*>(s_v[w]);
+          const int n4 = (n + 3) >> 2;
+#pragma unroll 4
+          for (int i = 0; i < n4; ++i) {
+            const float4 v = sv[i];
+            dtf = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(dtf, v.x), v.y), v.z), v.w);
+          }
+        }
+        __syncwarp();
+      }
     }
-    if (lane != 0) continue;
-    if (bad) {
-      score[p] = __int_as_float(0x7fc00000);
-      eye4(To);
-      continue;
+    dtf = __fdiv_rn(dtf, u == 0 ? 18446744073709551616.f : (float)(u - 1));
+    if (dtf < bestf) {
+      bestf = dtf;
+      best_i = it;
     }
-    score[p] = bestf;
-    float S[16], R2[16], A[16];
-    eye4(S);
-    const float cs = __fdiv_rn(km.z, ks.z);
-    S[0] = S[5] = S[10] = cs;
-    eye4(R2);
-    R2[0] = rot.c2[best_i], R2[4] = rot.s2[best_i], R2[1] = -rot.s2[best_i], R2[5] = rot.c2[best_i];
-    mm4(S, T3, A);
-    mm4(A, R2, A);
-    mm4(A, T1, A);
-    mm4(A, Tm, A);
-    for (int i = 0; i < 16; ++i) To[i] = A[i];
   }
+  if (bad) {  // past REF_MAX_DEPTH levels (REFW_RANGE keeps clouds far below it)
+    if (lane == 0) {
+      To[15] = __uint_as_float(REFW_REDO);
+      atomicAdd(err + 2, 1);
+    }
+    return;
+  }
+  if (lane == 0) score[p] = bestf;
+  // S T3 R2 T1 Tm, one element a lane
+  const int r = (lane >> 2) & 3, c = lane & 3;
+  const float one = r == c ? 1.f : 0.f;
+  const float cs = __fdiv_rn(km.z, ks.z);
+  float A = r == c && r < 3 ? cs : one;
+  A = warp_mm4(A, lane == 3 ? km.x : (lane == 7 ? km.y : one), lane);
+  const float rc = rot.c2[best_i], rs = rot.s2[best_i];
+  A = warp_mm4(A, lane == 0 || lane == 5 ? rc : (lane == 4 ? rs : (lane == 1 ? -rs : one)), lane);
+  A = warp_mm4(A, lane == 3 ? -km.x : (lane == 7 ? -km.y : one), lane);
+  A = warp_mm4(A, lane == 3 ? tx : (lane == 7 ? ty : (lane == 11 ? tz : one)), lane);
+  if (lane < 16) To[lane] = A;
 }
 
 __global__ void k_ref_sum_counts(const uint32_t* __restrict__ cnt, int n, unsigned long long* __restrict__ out) {
@@ -1199,15 +1607,27 @@ rtr_status rtr_ref_distance(rtr_context* ctx, const float* d_mcloud, const float
   cudaStream_t st = (cudaStream_t)stream;
   RTR_CUDA(cudaSetDevice(ctx->device));
   ScratchPlan plan;
-  const size_t o_err = plan.add<int>(4);
+  // err: [0] error bits, [1] largest cloud, [2] pairs the warp form leaves,
+  // [3..] model keypoints per size class
+  const size_t o_err = plan.add<int>(3 + REFW_CLASSES);
+  const size_t least = plan.bytes;  // without the warp form: every pair a CTA
+  const size_t o_box = plan.add<RefKeyBox>((size_t)n_model);
+  const size_t o_list = plan.add<int>((size_t)n_model * REFW_CLASSES);
+  const int warp_max = scratch_obtainable(ctx, plan.bytes, st) ? REFW_MAX : -1;
   Scratch s;
-  RTR_TRY(ensure_scratch(ctx, plan.bytes, st, &s));
+  RTR_TRY(ensure_scratch(ctx, warp_max < 0 ? least : plan.bytes, st, &s));
   int* err = reinterpret_cast<int*>(s.base + o_err);
-  RTR_CUDA(cudaMemsetAsync(err, 0, 4 * sizeof(int), st));
+  RefKeyBox* boxes = reinterpret_cast<RefKeyBox*>(s.base + o_box);
+  int* list = reinterpret_cast<int*>(s.base + o_list);
+  const RefRot rot = ref_rot_tables();
+  RTR_CUDA(cudaMemsetAsync(err, 0, (3 + REFW_CLASSES) * sizeof(int), st));
   k_ref_max_count<<<(n_model + 255) / 256, 256, 0, st>>>(d_moffsets, n_model, err + 1);
-  RTR_LAUNCHED(1);
-  int h[4];
-  RTR_TRY(ref_read_ints(ctx, err, 4, st, h));
+  if (warp_max >= 0)
+    k_ref_keybox<<<(n_model + 63) / 64, 64, 0, st>>>(reinterpret_cast<const float4*>(d_mkeys), d_moffsets, n_model,
+                                                     resolution, half_tdf, rot, boxes, list, err + 3);
+  RTR_LAUNCHED(warp_max >= 0 ? 2 : 1);
+  int h[3 + REFW_CLASSES];
+  RTR_TRY(ref_read_ints(ctx, err, 3 + REFW_CLASSES, st, h));
   const int nmax = h[1];
   if (nmax > 0) RTR_CHECK_ARG(d_mindices, "rtr_ref_distance: NULL indices");
   if (nmax > REF_PPT * 1024)
@@ -1223,32 +1643,54 @@ rtr_status rtr_ref_distance(rtr_context* ctx, const float* d_mcloud, const float
       RTR_CHECK_ARG(pm[(size_t)i] >= 0 && pm[(size_t)i] < n_model && ps_[(size_t)i] >= 0 && ps_[(size_t)i] < n_scan,
                     "rtr_ref_distance: pair %lld = (%d, %d) out of range", i, pm[(size_t)i], ps_[(size_t)i]);
   }
-  const RefRot rot = ref_rot_tables();
   ProfScope ps(ctx, st, "ref_distance");
   const float4* mc = reinterpret_cast<const float4*>(d_mcloud);
   const float4* mk = reinterpret_cast<const float4*>(d_mkeys);
   const float4* sk = reinterpret_cast<const float4*>(d_skeys);
   const unsigned nb = (unsigned)n_pairs;
-  if (nmax <= REFW_PPT * 32) {
-    const long long nbw = (n_pairs + REFW_WARPS - 1) / REFW_WARPS;
-    k_ref_distance_warp<<<(unsigned)nbw, 32 * REFW_WARPS, 0, st>>>(mc, mk, d_moffsets, d_mindices, d_mtdf, sk, n_scan,
-                                                                   d_pair_m, d_pair_s, n_pairs, resolution, half_tdf,
-                                                                   rot, d_score, d_T, err);
-  } else if (nmax <= REF_PPT * 256) {
+  // a launch per size class that has clouds, the largest first
+#define REF_WARP_CLASS(c)                                                                                            \
+  if (h[3 + (c)] > 0) {                                                                                              \
+    const long long items = all ? (long long)h[3 + (c)] * n_scan : n_pairs;                                          \
+    k_ref_distance_warp<c><<<(unsigned)((items + REFW_WARPS - 1) / REFW_WARPS), 32 * REFW_WARPS, 0, st>>>(           \
+        mc, mk, d_moffsets, d_mindices, d_mtdf, boxes, list + (size_t)(c) * n_model, sk, n_scan, d_pair_m, d_pair_s, \
+        items, resolution, half_tdf, rot, d_score, d_T, err);                                                        \
+    RTR_LAUNCHED(1);                                                                                                 \
+  }
+  REF_WARP_CLASS(10)
+  REF_WARP_CLASS(8)
+  REF_WARP_CLASS(7)
+  REF_WARP_CLASS(9)
+  REF_WARP_CLASS(6)
+  REF_WARP_CLASS(5)
+  REF_WARP_CLASS(4)
+  REF_WARP_CLASS(3)
+  REF_WARP_CLASS(2)
+  REF_WARP_CLASS(1)
+  REF_WARP_CLASS(0)
+#undef REF_WARP_CLASS
+  RTR_CUDA(cudaGetLastError());
+  if (nmax <= warp_max) {
+    RTR_TRY(ref_read_ints(ctx, err, 4, st, h));
+    RTR_TRY(ref_check_err(h[0], "rtr_ref_distance"));
+    if (h[2] == 0) return RTR_OK;
+  }
+  // larger clouds, and the pairs left: a CTA each
+  if (nmax <= REF_PPT * 256) {
     RTR_TRY(ref_distance_smem<256>());
     k_ref_distance<256><<<nb, 256, ref_leaf_smem(256), st>>>(mc, mk, d_moffsets, d_mindices, d_mtdf, sk, n_scan,
                                                              d_pair_m, d_pair_s, resolution, half_tdf, rot, d_score,
-                                                             d_T, err);
+                                                             d_T, err, warp_max);
   } else if (nmax <= REF_PPT * 512) {
     RTR_TRY(ref_distance_smem<512>());
     k_ref_distance<512><<<nb, 512, ref_leaf_smem(512), st>>>(mc, mk, d_moffsets, d_mindices, d_mtdf, sk, n_scan,
                                                              d_pair_m, d_pair_s, resolution, half_tdf, rot, d_score,
-                                                             d_T, err);
+                                                             d_T, err, warp_max);
   } else {
     RTR_TRY(ref_distance_smem<1024>());
     k_ref_distance<1024><<<nb, 1024, ref_leaf_smem(1024), st>>>(mc, mk, d_moffsets, d_mindices, d_mtdf, sk, n_scan,
                                                                 d_pair_m, d_pair_s, resolution, half_tdf, rot, d_score,
-                                                                d_T, err);
+                                                                d_T, err, warp_max);
   }
   RTR_LAUNCHED(1);
   RTR_CUDA(cudaGetLastError());

@@ -139,3 +139,79 @@ def test_bad_arguments_are_refused(ctx, rtr):
     with pytest.raises(rtr.RtrError):
         ctx.ref_distance(model, keys, mo, mi, tdf, keys, bad_m, bad_s)  # model index 7 of 4
     ctx.check()
+
+
+@pytest.mark.parametrize("res,half", [(0.01, 0.15), (0.01, 0.1525), (0.004, 0.0601)])
+def test_distance_by_cloud_size_and_position(ctx, res, half):
+    """get_Distance over the pair kernel's cases, each equal to the oracle:
+    clouds at the edges of its size classes (rows of 32 points up to 512,
+    beyond that a CTA per pair), points and offsets on whole leaves (keys
+    decided exactly), tiny coordinates, field cubes whose leaves do not meet
+    the field's voxels in their middles (half 0.1525, 0.0601), scan keypoints
+    near, far and beyond the range of the fixed-point form.  Field values are
+    random, so the order of the sums shows."""
+    rng = np.random.default_rng(int(res * 1e4) + int(half * 1e5))
+    sizes = [0, 1, 31, 32, 33, 64, 65, 96, 97, 128, 129, 160, 161, 192, 193, 256, 257, 384, 385, 512, 513, 700]
+    box = np.float32(half * 2 / 3 * 0.98)
+    keys, clouds = [], []
+    for i, n in enumerate(sizes):
+        k = np.zeros(4, np.float32) if i % 4 == 1 else np.append(rng.uniform(-1, 1, 3), 0).astype(np.float32)
+        c = np.zeros((n, 4), np.float32)
+        c[:, :3] = k[:3] + rng.uniform(-box, box, (n, 3)).astype(np.float32)
+        if i % 3 == 0 and n:  # whole leaves about the key
+            c[:, :3] = k[:3] + (np.float32(res) * rng.integers(-9, 10, (n, 3))).astype(np.float32)
+        if i % 4 == 1 and n:
+            c[:, :3] *= 10.0 ** rng.uniform(-9, 0, (n, 3)).astype(np.float32)
+        keys.append(k)
+        clouds.append(c)
+    km = np.stack(keys)
+    model = np.concatenate(clouds)
+    mo = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    mi = np.arange(model.shape[0], dtype=np.int32)
+    tdf = rng.uniform(0, 900, (len(sizes), 27000)).astype(np.float32)
+    off = np.array([[0, 0, 0], [3 * res, -2 * res, res], [0.013, 0.002, -0.02], [0.31, -0.2, 0.05], [-7.3, 4.1, 0.6],
+                    [0.0, 0.0, 0.2], [400.0, 0.0, 0.0]], np.float32)
+    ks = np.zeros((len(off) * 3, 4), np.float32)
+    for j, b in enumerate((1, 4, 7)):
+        ks[j * len(off):(j + 1) * len(off), :3] = km[b, :3] + off
+    rsc, rT = O.ref_distance(model, km, mo, mi, tdf, ks, res=res, half=half)
+    args = (_dev(model), _dev(km), _dev(mo), _dev(mi), _dev(tdf), _dev(ks))
+    sc, T = ctx.ref_distance(*args, resolution=res, half_tdf=half)
+    assert np.array_equal(sc.cpu().numpy(), rsc, equal_nan=True)
+    assert np.array_equal(T.cpu().numpy(), rT, equal_nan=True)
+    # the same as a pair list, shuffled
+    pm, ps = [x.ravel().astype(np.int32) for x in np.meshgrid(np.arange(len(sizes)), np.arange(len(ks)), indexing="ij")]
+    o = rng.permutation(pm.size)
+    sc, T = ctx.ref_distance(*args, _dev(pm[o]), _dev(ps[o]), resolution=res, half_tdf=half)
+    assert np.array_equal(sc.cpu().numpy(), rsc[o], equal_nan=True)
+    assert np.array_equal(T.cpu().numpy(), rT[o], equal_nan=True)
+
+
+def test_distance_without_room_for_its_tables(rtr):
+    """8,000 model keypoints under a 1 MiB scratch limit: the tables of the
+    warp form do not fit, every pair takes a CTA, same results."""
+    rng = np.random.default_rng(2)
+    nk = 8000
+    km = np.zeros((nk, 4), np.float32)
+    km[:, :3] = rng.uniform(-1, 1, (nk, 3))
+    cnt = rng.integers(0, 40, nk)
+    mo = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+    cloud = np.zeros((mo[-1], 4), np.float32)
+    cloud[:, :3] = np.repeat(km[:, :3], cnt, 0) + rng.uniform(-0.1, 0.1, (mo[-1], 3))
+    mi = np.arange(mo[-1], dtype=np.int32)
+    tdf = rng.uniform(0, 900, (nk, 27000)).astype(np.float32)
+    ks = km[:2] + np.float32(0.05)
+    ks[:, 3] = 0
+    import torch
+    args = (_dev(cloud), _dev(km), _dev(mo), _dev(mi), torch.from_numpy(tdf).cuda(), _dev(ks))
+    res = []
+    for mb in (0, 1):
+        c = rtr.Context(0)
+        try:
+            c.set_tuning("scratch_limit_mb", mb)
+            sc, T = c.ref_distance(*args)
+            res.append((sc.cpu().numpy(), T.cpu().numpy()))
+        finally:
+            c.close()
+    assert np.array_equal(res[0][0], res[1][0], equal_nan=True)
+    assert np.array_equal(res[0][1], res[1][1], equal_nan=True)
