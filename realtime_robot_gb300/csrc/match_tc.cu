@@ -6,7 +6,7 @@
 // lo.hi (three tcgen05.mma per K step), which leaves |err(q.b)| of order
 // 1e-4 |q| |b| (dropped lo.lo, the split's rounding, FP32 accumulation); the
 // certification uses TC_ERR * max(|q|, max |b|)^2, which covers that and the
-// FP32 norms with margin (unit-norm SHOT vectors: 1e-3).  Inf or NaN values
+// FP32 norms with margin (unit-norm SHOT vectors: 5e-4).  Inf or NaN values
 // make a query uncertified.  Per query the epilogue keeps the 8
 // smallest approximate distances; an exact FP32 re-rank (sequential sums, as
 // the oracle) picks the winner, and a query is certified when its 8th
@@ -49,8 +49,17 @@ constexpr int TC_BAND_Q = 16384;  // band pass: uncertified queries it takes (th
 constexpr int TC_A_BYTES = TC_BM * TC_KB * 2;   // 8 KB
 constexpr int TC_B_BYTES = TC_BN * TC_KB * 2;   // 16 KB
 constexpr int TC_STAGE_BYTES = 2 * TC_A_BYTES + 2 * TC_B_BYTES;  // 48 KB
+constexpr int TC_KTAIL = TC_DIM / TC_KB;         // the K-block that holds only the norm column (its first)
+constexpr int TC_RANGES = 8;                     // most database ranges of the first pass
 constexpr int TC_THREADS = 192;
-constexpr float TC_ERR = 1.0e-3f;  // conservative bound on |d~ - d| (see top)
+constexpr int TC_ROW = 36;  // floats a row in the epilogue's staging (16-byte stores of 8 rows meet 32 banks)
+// Bound on |d~ - d| over max(|q|, max |b|)^2, d the FP32 sequential sum.  The
+// dropped lo.lo and the split's rests: 2.3e-5; 68 accumulations of 16 products,
+// each term cut at 2^-23 of the largest: 2.8e-4; the sequential sum's own
+// rounding (352 terms, d up to 4): 8.4e-5; norms and the last step: 2e-6;
+// 3.9e-4 at worst.  Measured at most 2.2e-5 (SHOT rows of the room, Gaussian,
+// sparse, offset and badly scaled ones).
+constexpr float TC_ERR = 5.0e-4f;
 constexpr long long TC_SPIN_LIMIT = 1LL << 26;
 
 // ---------------------------------------------------------------------------
@@ -228,20 +237,20 @@ struct TcArgs {
   const float* qn;   // [nq_cap] |q|^2
   int* cand_idx;     // [nq_cap][8]; band pass: [nq_cap][TC_BAND] rows within the threshold
   float* cand_d;     // [nq_cap][8]
+  int* more_idx;     // [ranges - 1][nq_cap][8]: the lists of the database ranges after the first
+  float* more_d;
   int* status;
   const float* thr;  // band pass: [nq_cap] largest d~ a row may have and still tie the winner
   int* band_n;       // band pass: [nq_cap] rows listed (over TC_BAND: overflowed)
   long long spin_limit;  // tries per mbarrier wait (the context's wait budget)
 };
 
-// BAND = false: per query the 8 smallest d~ (the first pass).  BAND = true:
-// per query every row with d~ <= thr[q] (the band pass over uncertified
-// queries), the first TC_BAND of them listed in band_n[q] (zeroed by the
+// The band pass over the uncertified queries: per query every row with
+// d~ <= thr[q], the first TC_BAND of them listed in band_n[q] (zeroed by the
 // caller; a count over TC_BAND means the band overflowed and the row stops
-// counting); its grid splits the database into gridDim.y ranges so that a
+// counting); the grid splits the database into gridDim.y ranges so that a
 // few uncertified queries still fill the GPU.
-template <bool BAND>
-__global__ void __launch_bounds__(TC_THREADS, 1) k_match_tc(const __grid_constant__ CUtensorMap mq_hi,
+__global__ void __launch_bounds__(TC_THREADS, 1) k_match_band(const __grid_constant__ CUtensorMap mq_hi,
                                                             const __grid_constant__ CUtensorMap mq_lo,
                                                             const __grid_constant__ CUtensorMap mb_hi,
                                                             const __grid_constant__ CUtensorMap mb_lo, TcArgs a) {
@@ -339,12 +348,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_match_tc(const __grid_constan
     }
   } else {
     // ---------------- epilogue: warps 0-3, thread = query row ----------------
-    // The accumulator holds q.b - |b|^2 / 2, so the nearest rows are the
-    // largest values: one compare per element, d~ = |q|^2 - 2 acc at the end.
+    // The accumulator holds q.b - |b|^2 / 2.
     const int row = warp * 32 + lane;
     const int q = q0 + row;
     const float qn = q < nq ? a.qn[q] : 0.f;
-    if (BAND) {
+    {
       // rows past the live queries (stale scratch, any bits) list nothing
       const bool live = q < nq;
       const float thr = live ? a.thr[q] : 0.f;
@@ -379,7 +387,159 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_match_tc(const __grid_constan
         tc_fence_before();
         mbar_arrive(&acc_empty[buf]);
       }
-    } else {
+    }
+  }
+  // after an abort nothing of this CTA may still be in flight when it frees
+  // its TMEM and exits: the MMA issuer waits for every MMA it issued, the
+  // producer for the stage loads not yet seen complete (the last ones; each
+  // earlier load of a stage completed before the stage was reused)
+  __syncthreads();
+  if (abort_flag) {
+    if (warp == 5 && lane == 0) {
+      umma_commit(&drain_bar);
+      mbar_drain(&drain_bar, 0u);
+    }
+    if (warp == 4 && lane == 0)
+      for (int i = issued > TC_STAGES ? issued - TC_STAGES : 0; i < issued; ++i)
+        mbar_drain(&full_bar[i % TC_STAGES], (uint32_t)(i / TC_STAGES) & 1u);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (abort_flag && threadIdx.x == 0) atomicExch(a.status, (int)RTR_ERR_TIMEOUT);
+  if (warp == 5) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  }
+}
+
+// The first pass: per query the 8 smallest d~ (largest q.b - |b|^2 / 2) of each
+// database range (gridDim.y of them, contiguous tiles).
+// What bounds it: the tensor cores.  Its 68 MMAs of 128 x 256 x 16 a tile alone
+// (nothing loaded, nothing read back) take 401 us for the room's 111k x 3,001,
+// the library GEMM's rate; with everything 460 us.  766 us while the epilogue
+// inserted under divergence (3,072 columns a row, about 700 insertions a warp
+// at 45 instructions in a chain of compares; now about 220 a warp, all lanes at
+// once).  Tried and not better: two CTAs a cluster sharing a tile
+// (cta_group::2; 483 us against 495 with the same epilogue), eight epilogue
+// warps, the next accumulator columns loaded ahead, database boxes of 128 rows
+// (+20 us).
+__global__ void __launch_bounds__(TC_THREADS, 1) k_match_top(const __grid_constant__ CUtensorMap mq_hi,
+                                                            const __grid_constant__ CUtensorMap mq_lo,
+                                                            const __grid_constant__ CUtensorMap mb_hi,
+                                                            const __grid_constant__ CUtensorMap mb_lo, TcArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full_bar[TC_STAGES], empty_bar[TC_STAGES], acc_full[2], acc_empty[2], drain_bar;
+  __shared__ uint32_t tmem_base;
+  __shared__ int abort_flag;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nq = a.d_nq ? min(*a.d_nq, a.nq_cap) : a.nq_host;
+  const int q0 = blockIdx.x * TC_BM;
+  if (q0 >= nq) return;  // uniform per CTA, before any barrier or TMEM use
+  // database tiles of this CTA: all of them, or (band pass, gridDim.y > 1)
+  // one of gridDim.y contiguous ranges
+  const int n_all = (a.ndb + TC_BN - 1) / TC_BN;
+  const int t_lo = (int)((long long)blockIdx.y * n_all / gridDim.y);
+  const int t_hi = (int)((long long)(blockIdx.y + 1) * n_all / gridDim.y);
+  // every CTA starts at another tile, so that the CTAs, which run in step, do
+  // not all read the same rows at the same time (518 -> 495 us)
+  const int t_off = (int)(blockIdx.x % (unsigned)max(t_hi - t_lo, 1));
+  auto tile = [&](int t) {
+    const int r = t + t_off;
+    return r < t_hi ? r : r - (t_hi - t_lo);
+  };
+
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    for (int s = 0; s < TC_STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 128);
+    }
+    mbar_init(&drain_bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 5) {  // allocate 512 TMEM columns (two 128 x 256 FP32 accumulators)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base;
+  volatile int* abort = &abort_flag;
+  const long long lim = a.spin_limit;
+  int issued = 0;  // producer: stage loads issued
+
+  if (warp == 4) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0) {
+      int it = 0;
+      for (int t = t_lo; t < t_hi && !*abort; ++t) {
+        for (int kb = 0; kb < TC_NKB && !*abort; ++kb, ++it) {
+          const int s = it % TC_STAGES;
+          const uint32_t ph = (uint32_t)(it / TC_STAGES) & 1u;
+          if (it >= TC_STAGES && !mbar_wait(&empty_bar[s], ph ^ 1u, abort, lim)) break;
+          uint8_t* st = smem + s * TC_STAGE_BYTES;
+          mbar_expect_tx(&full_bar[s], TC_STAGE_BYTES);
+          tma_load_2d(st, &mq_hi, &full_bar[s], kb * TC_KB, q0);
+          tma_load_2d(st + TC_A_BYTES, &mq_lo, &full_bar[s], kb * TC_KB, q0);
+          tma_load_2d(st + 2 * TC_A_BYTES, &mb_hi, &full_bar[s], kb * TC_KB, tile(t) * TC_BN);
+          tma_load_2d(st + 2 * TC_A_BYTES + TC_B_BYTES, &mb_lo, &full_bar[s], kb * TC_KB, tile(t) * TC_BN);
+        }
+      }
+      issued = it;
+    }
+  } else if (warp == 5) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc();
+      int it = 0;
+      for (int t = t_lo; t < t_hi && !*abort; ++t) {
+        const int buf = (t - t_lo) & 1;
+        const uint32_t use = (uint32_t)((t - t_lo) >> 1);
+        if (t - t_lo >= 2 && !mbar_wait(&acc_empty[buf], (use - 1) & 1u, abort, lim)) break;
+        tc_fence_after();
+        const uint32_t dcol = tmem + (uint32_t)buf * TC_BN;
+        for (int kb = 0; kb < TC_NKB; ++kb, ++it) {
+          const int s = it % TC_STAGES;
+          const uint32_t ph = (uint32_t)(it / TC_STAGES) & 1u;
+          if (!mbar_wait(&full_bar[s], ph, abort, lim)) break;
+          tc_fence_after();
+          const uint32_t base = smem_u32(smem + s * TC_STAGE_BYTES);
+          const uint32_t ah = base, al = base + TC_A_BYTES, bh = base + 2 * TC_A_BYTES,
+                         bl = base + 2 * TC_A_BYTES + TC_B_BYTES;
+          // the tail block: one column that counts, and none in the queries' lo part
+          for (int k = 0; k < (kb == TC_KTAIL ? 1 : TC_KB / 16); ++k) {
+            const uint32_t off = (uint32_t)k * 32;  // 16 bf16 along K inside the swizzle row
+            const uint32_t acc0 = (kb > 0 || k > 0) ? 1u : 0u;
+            umma_f16(dcol, umma_desc(ah + off), umma_desc(bh + off), idesc, acc0);
+            umma_f16(dcol, umma_desc(ah + off), umma_desc(bl + off), idesc, 1u);
+            if (kb != TC_KTAIL) umma_f16(dcol, umma_desc(al + off), umma_desc(bh + off), idesc, 1u);
+          }
+          umma_commit(&empty_bar[s]);  // stage free once these MMAs have read it
+        }
+        umma_commit(&acc_full[buf]);  // accumulator ready
+      }
+    }
+  } else {
+    // ---------------- epilogue: warps 0-3, thread = query row ----------------
+    // The accumulator holds q.b - |b|^2 / 2, so the nearest rows are the
+    // largest values: one compare per element, d~ = |q|^2 - 2 acc at the end.
+    const int row = warp * 32 + lane;
+    const int q = q0 + row;
+    const float qn = q < nq ? a.qn[q] : 0.f;
+    {
+    // The list of 8 is ascending in d~.  A chunk of 32 columns is compared with
+    // the list's last value (a subtraction and a funnel shift collect a lane's
+    // hits as bits), staged in shared memory, and each lane takes its own hits
+    // in column order, all lanes at once: the warp runs as many insertions a
+    // chunk as its busiest lane has hits.  An insertion's slots are independent
+    // (the middle of the left neighbour, the new value and the slot).
     float ba[TC_TOP];
     int bi[TC_TOP];
 #pragma unroll
@@ -387,44 +547,55 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_match_tc(const __grid_constan
       ba[s] = -__int_as_float(0x7f800000);
       bi[s] = 0x7fffffff;
     }
+    float* stage = reinterpret_cast<float*>(smem + TC_STAGES * TC_STAGE_BYTES) + (size_t)row * TC_ROW;
     for (int t = t_lo; t < t_hi; ++t) {
       const int buf = (t - t_lo) & 1;
       const uint32_t use = (uint32_t)((t - t_lo) >> 1);
       if (!mbar_wait(&acc_full[buf], use & 1u, abort, lim)) break;
       tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * TC_BN;
-      const int valid = min(TC_BN, a.ndb - t * TC_BN);  // rows past the database read as zero
-      for (int c0 = 0; c0 < TC_BN; c0 += 32) {
+      const int valid = min(TC_BN, a.ndb - tile(t) * TC_BN);
+      for (int c0 = 0; c0 < valid; c0 += 32) {
         float v[32];
         tmem_ld32(taddr + (uint32_t)c0, v);
-        const int jb = t * TC_BN + c0;
-        const int lim = valid - c0;
+        uint32_t hits = 0;  // bit 31 - i: column i (NaN and ties with the last value: not taken)
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          if (v[i] > ba[TC_TOP - 1] && i < lim) {
-            ba[TC_TOP - 1] = v[i];
-            bi[TC_TOP - 1] = jb + i;
+        for (int i = 0; i < 32; ++i)
+          hits = __funnelshift_l(__float_as_uint(__fsub_rn(ba[TC_TOP - 1], v[i])), hits, 1);
+        if (valid - c0 < 32) hits &= ~(0xffffffffu >> (valid - c0));
+        if (!__any_sync(0xffffffffu, hits)) continue;
 #pragma unroll
-            for (int s = TC_TOP - 1; s > 0; --s) {
-              const bool gt = ba[s] > ba[s - 1];
-              const float x0 = ba[s], x1 = ba[s - 1];
-              const int y0 = bi[s], y1 = bi[s - 1];
-              ba[s] = gt ? x1 : x0;
-              ba[s - 1] = gt ? x0 : x1;
-              bi[s] = gt ? y1 : y0;
-              bi[s - 1] = gt ? y0 : y1;
-            }
+        for (int i = 0; i < 32; i += 4)
+          *reinterpret_cast<float4*>(stage + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        do {
+          const int i = hits ? __clz(hits) : 0;
+          float x = stage[i];
+          x = hits ? x : -__int_as_float(0x7f800000);
+          const int xi = tile(t) * TC_BN + c0 + i;
+          hits &= 0x7fffffffu >> i;  // (a lane without hits keeps none)
+          bool gt[TC_TOP];
+#pragma unroll
+          for (int s = 0; s < TC_TOP; ++s) gt[s] = x > ba[s];
+#pragma unroll
+          for (int s = TC_TOP - 1; s > 0; --s) {
+            bi[s] = gt[s - 1] ? bi[s - 1] : (gt[s] ? xi : bi[s]);
+            ba[s] = gt[s - 1] ? ba[s - 1] : (gt[s] ? x : ba[s]);
           }
-        }
+          bi[0] = gt[0] ? xi : bi[0];
+          ba[0] = gt[0] ? x : ba[0];
+        } while (__any_sync(0xffffffffu, hits));
       }
       tc_fence_before();
       mbar_arrive(&acc_empty[buf]);
     }
     if (q < nq) {
+      const size_t off = (size_t)a.nq_cap * TC_TOP * (blockIdx.y > 0 ? blockIdx.y - 1 : 0);
+      int* ci = blockIdx.y > 0 ? a.more_idx + off : a.cand_idx;
+      float* cd = blockIdx.y > 0 ? a.more_d + off : a.cand_d;
 #pragma unroll
       for (int s = 0; s < TC_TOP; ++s) {
-        a.cand_idx[(size_t)q * TC_TOP + s] = bi[s] == 0x7fffffff ? -1 : bi[s];
-        a.cand_d[(size_t)q * TC_TOP + s] = bi[s] == 0x7fffffff ? __int_as_float(0x7f800000) : qn - 2.f * ba[s];
+        ci[(size_t)q * TC_TOP + s] = bi[s] == 0x7fffffff ? -1 : bi[s];
+        cd[(size_t)q * TC_TOP + s] = bi[s] == 0x7fffffff ? __int_as_float(0x7f800000) : qn - 2.f * ba[s];
       }
     }
     }
@@ -481,74 +652,148 @@ __device__ __forceinline__ float exact_d2(const float* __restrict__ x, const flo
   return acc;
 }
 
-// Exact FP32 re-rank of the candidates that can still win and
-// certification; four queries per warp, one lane per candidate.  Uncertified
-// queries go to the redo list with their running minimum reset.
+// Exact FP32 re-rank of the candidates that can still win, and
+// certification.  Uncertified queries go to the redo list with their running
+// minimum reset.
+// A warp takes 16 queries, lists the candidates in doubt (one or two a query)
+// and handles eight of them at a time: the lanes read each candidate's and its
+// query's row together (whole lines, all eight in flight), the squared
+// differences go through shared memory, and a lane adds up one candidate's in
+// order.  Bound by latency (of the rows, then of the adds): 98 us for the
+// room's 111k queries with a lane reading its rows by itself, 67 us now.
+constexpr int RR_WARPS = 4;
+constexpr int RR_Q = 16;
+constexpr int RR_C = 8;
 template <bool V4>
-__global__ void __launch_bounds__(256) k_rerank(const float* __restrict__ q, int nq_host, const int* d_nq, int nq_cap,
-                                                const float* __restrict__ db, int ndb,
-                                                const int* __restrict__ cand_idx, const float* __restrict__ cand_d,
-                                                int* __restrict__ out_idx, float* __restrict__ out_d2,
-                                                int* __restrict__ redo, int* __restrict__ n_redo,
-                                                unsigned long long* __restrict__ redo_best,
-                                                float* __restrict__ redo_thr,
-                                                const float* __restrict__ qn, const float* __restrict__ db_max,
-                                                const unsigned long long* __restrict__ zero_best,
-                                                const unsigned char* __restrict__ qzero) {
+__global__ void __launch_bounds__(32 * RR_WARPS)
+    k_rerank(const float* __restrict__ q, int nq_host, const int* d_nq, int nq_cap, const float* __restrict__ db, int ndb,
+             const int* __restrict__ cand_idx, const float* __restrict__ cand_d, const int* __restrict__ more_idx,
+             const float* __restrict__ more_d, int ranges, int* __restrict__ out_idx, float* __restrict__ out_d2,
+             int* __restrict__ redo, int* __restrict__ n_redo, unsigned long long* __restrict__ redo_best,
+             float* __restrict__ redo_thr, const float* __restrict__ qn, const float* __restrict__ db_max,
+             const unsigned long long* __restrict__ zero_best, const unsigned char* __restrict__ qzero) {
+  __shared__ __align__(16) float s_term[RR_WARPS][RR_C][TC_DIM + 4];
+  __shared__ int s_cand[RR_WARPS][RR_Q * TC_TOP];
+  __shared__ unsigned char s_of[RR_WARPS][RR_Q * TC_TOP];
+  __shared__ unsigned long long s_best[RR_WARPS][RR_Q];
+  __shared__ float s_worst[RR_WARPS][RR_Q], s_bound[RR_WARPS][RR_Q];
   const int nq = d_nq ? min(*d_nq, nq_cap) : nq_host;
-  const int lane = threadIdx.x & 31, sub = lane >> 3, l8 = lane & 7;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4; base < nq; base += warps * 4) {
-    const int i = base + sub;
-    const bool valid = i < nq;
-    const bool zq = valid && qzero[i] != 0;  // (no early exit: the shuffles below need every lane)
-    int c = valid && !zq ? cand_idx[(size_t)i * TC_TOP + l8] : -1;
-    if (c >= ndb) c = -1;  // never read past the database, whatever the first pass left
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane >> 3, l8 = lane & 7;
+  const int warps = gridDim.x * RR_WARPS;
+  const float dbm = *db_max;
+  for (int base = (blockIdx.x * RR_WARPS + w) * RR_Q; base < nq; base += warps * RR_Q) {
+    if (lane < RR_Q) s_best[w][lane] = ~0ull;
     // |d~ - d| <= err: a candidate whose d~ exceeds the smallest d~ (the
-    // first, the list is ascending) by more than 2 err has an exact distance
-    // above that candidate's, so it can neither win nor tie: its exact
-    // distance is not computed
-    const float err_q = valid ? TC_ERR * fmaxf(qn[i], *db_max) : 0.f;
-    const bool need = c >= 0 && cand_d[(size_t)i * TC_TOP + l8] <= cand_d[(size_t)i * TC_TOP] + 2.f * err_q;
-    float d = __int_as_float(0x7f800000);
-    if (need) d = exact_d2<V4>(q + (size_t)i * TC_DIM, db + (size_t)c * TC_DIM);
-    int bi = need ? c : 0x7fffffff;
-    float bd = d;
+    // first of the ranges' ascending lists) by more than 2 err has an exact
+    // distance above that candidate's, so it can neither win nor tie: its
+    // exact distance is not computed
+    if (lane < RR_Q) {
+      const int i = base + lane;
+      float bound = -__int_as_float(0x7f800000), worst = __int_as_float(0x7f800000);
+      if (i < nq && qzero[i] == 0) {
+        float first = cand_d[(size_t)i * TC_TOP];
+        worst = cand_d[(size_t)i * TC_TOP + TC_TOP - 1];
+        for (int r = 0; r + 1 < ranges; ++r) {
+          const float* l = more_d + ((size_t)r * nq_cap + i) * TC_TOP;
+          first = fminf(first, l[0]);
+          worst = fminf(worst, l[TC_TOP - 1]);
+        }
+        bound = first + 2.f * (TC_ERR * fmaxf(qn[i], dbm));
+      }
+      s_bound[w][lane] = bound;
+      s_worst[w][lane] = worst;
+    }
+    __syncwarp();
+    for (int r = 0; r < ranges; ++r) {
+      const int* li = r > 0 ? more_idx + (size_t)(r - 1) * nq_cap * TC_TOP : cand_idx;
+      const float* ld = r > 0 ? more_d + (size_t)(r - 1) * nq_cap * TC_TOP : cand_d;
+      int cnt = 0;
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {  // within the aligned group of 8 lanes
-      const float od = __shfl_xor_sync(0xffffffffu, bd, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (od < bd || (od == bd && oi < bi)) {
-        bd = od;
-        bi = oi;
+      for (int q0 = 0; q0 < RR_Q; q0 += 4) {
+        const size_t at = (size_t)(base + q0 + sub) * TC_TOP + l8;
+        const bool live = base + q0 + sub < nq;
+        const int c = live ? li[at] : -1;
+        const float d = live ? ld[at] : 0.f;
+        // (never read past the database, whatever the first pass left)
+        const bool need = c >= 0 && c < ndb && d <= s_bound[w][q0 + sub];
+        const unsigned nb = __ballot_sync(0xffffffffu, need);
+        if (need) {
+          const int e = cnt + __popc(nb & ((1u << lane) - 1u));
+          s_cand[w][e] = c;
+          s_of[w][e] = (unsigned char)(q0 + sub);
+        }
+        cnt += __popc(nb);
+      }
+      __syncwarp();
+      for (int b0 = 0; b0 < cnt; b0 += RR_C) {
+        const int m = min(RR_C, cnt - b0);
+#pragma unroll 4
+        for (int j = 0; j < m; ++j) {
+          const float* x = q + (size_t)(base + s_of[w][b0 + j]) * TC_DIM;
+          const float* y = db + (size_t)s_cand[w][b0 + j] * TC_DIM;
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int v = lane + 32 * k;
+            if (v >= TC_DIM / 4) continue;
+            float4 a, b;
+            if (V4) {
+              a = __ldg(reinterpret_cast<const float4*>(x) + v);
+              b = __ldg(reinterpret_cast<const float4*>(y) + v);
+            } else {
+              a = make_float4(x[4 * v], x[4 * v + 1], x[4 * v + 2], x[4 * v + 3]);
+              b = make_float4(y[4 * v], y[4 * v + 1], y[4 * v + 2], y[4 * v + 3]);
+            }
+            a.x = __fsub_rn(a.x, b.x), a.y = __fsub_rn(a.y, b.y), a.z = __fsub_rn(a.z, b.z), a.w = __fsub_rn(a.w, b.w);
+            *reinterpret_cast<float4*>(&s_term[w][j][4 * v]) =
+                make_float4(__fmul_rn(a.x, a.x), __fmul_rn(a.y, a.y), __fmul_rn(a.z, a.z), __fmul_rn(a.w, a.w));
+          }
+        }
+        __syncwarp();
+        if (lane < m) {
+          float acc = 0.f;
+#pragma unroll 8
+          for (int k = 0; k < TC_DIM; k += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(&s_term[w][lane][k]);
+            acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, t.x), t.y), t.z), t.w);
+          }
+          // the least (distance, index) of each query; a NaN distance never wins
+          if (acc <= __int_as_float(0x7f800000))
+            atomicMin(&s_best[w][s_of[w][b0 + lane]],
+                      ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned)s_cand[w][b0 + lane]);
+        }
+        __syncwarp();
       }
     }
-    if (zq && l8 == 0) {
-      // an all-zero query ties (up to rounding) with every unit-norm row: its
-      // answer is the database's, the row of least exact sequential |b|^2
-      // (lowest index on ties), found when the database was split
-      const unsigned long long key = *zero_best;
-      out_idx[i] = key == ~0ull ? -1 : (int)(unsigned)(key & 0xffffffffull);
-      if (out_d2) out_d2[i] = key == ~0ull ? __int_as_float(0x7f800000) : __uint_as_float((unsigned)(key >> 32));
-    } else if (valid && l8 == 0) {
-      const float worst = cand_d[(size_t)i * TC_TOP + TC_TOP - 1];
-      const int nvalid = ndb < TC_TOP ? ndb : TC_TOP;
-      const bool all_seen = nvalid < TC_TOP;  // every descriptor was a candidate
-      // the bound scales with the norms: |err| <= TC_ERR * max(|q|, |b|max)^2
-      const float err = TC_ERR * fmaxf(qn[i], *db_max);
-      const bool certified = all_seen || (worst - err > bd);
-      if (certified) {
-        out_idx[i] = bi == 0x7fffffff ? -1 : bi;
-        if (out_d2) out_d2[i] = bd;
+    __syncwarp();
+    const int i = base + lane;
+    if (lane < RR_Q && i < nq) {
+      const unsigned long long best = s_best[w][lane];
+      if (qzero[i] != 0) {
+        // an all-zero query ties (up to rounding) with every unit-norm row: its
+        // answer is the database's, the row of least exact sequential |b|^2
+        // (lowest index on ties), found when the database was split
+        const unsigned long long key = *zero_best;
+        out_idx[i] = key == ~0ull ? -1 : (int)(unsigned)(key & 0xffffffffull);
+        if (out_d2) out_d2[i] = key == ~0ull ? __int_as_float(0x7f800000) : __uint_as_float((unsigned)(key >> 32));
       } else {
-        const int p = atomicAdd(n_redo, 1);
-        redo[p] = i;
-        redo_best[p] = ~0ull;
-        // a row that ties or beats the exact winner has d~ <= bd + err; the
-        // band pass lists rows up to twice that margin
-        redo_thr[p] = bd + 2.f * err;
+        const float bd = best == ~0ull ? __int_as_float(0x7f800000) : __uint_as_float((unsigned)(best >> 32));
+        const bool all_seen = ndb < TC_TOP;  // every descriptor was a candidate
+        // the bound scales with the norms: |err| <= TC_ERR * max(|q|, |b|max)^2
+        const float err = TC_ERR * fmaxf(qn[i], dbm);
+        if (all_seen || s_worst[w][lane] - err > bd) {
+          out_idx[i] = best == ~0ull ? -1 : (int)(unsigned)(best & 0xffffffffull);
+          if (out_d2) out_d2[i] = bd;
+        } else {
+          const int p = atomicAdd(n_redo, 1);
+          redo[p] = i;
+          redo_best[p] = ~0ull;
+          // a row that ties or beats the exact winner has d~ <= bd + err; the
+          // band pass lists rows up to twice that margin
+          redo_thr[p] = bd + 2.f * err;
+        }
       }
     }
+    __syncwarp();  // the lists are reused
   }
 }
 
@@ -557,17 +802,24 @@ __global__ void __launch_bounds__(256) k_rerank(const float* __restrict__ q, int
 // zero row), packed (d^2 bits, index) so that atomicMin keeps the lowest
 // index on ties.  Rows with an infinite or NaN sum never win.  It depends on
 // the database only: computed when the database is split.
-__global__ void k_zero_best(const float* __restrict__ db, int ndb, unsigned long long* __restrict__ best) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ndb; j += gridDim.x * blockDim.x) {
-    const float* y = db + (size_t)j * TC_DIM;
-    float acc = 0.f;
-    for (int k = 0; k < TC_DIM; ++k) {
-      const float t = __fsub_rn(0.f, y[k]);
-      acc = __fadd_rn(acc, __fmul_rn(t, t));
-    }
-    if (acc < __int_as_float(0x7f800000))
-      atomicMin(best, ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned)j);
+// A block takes 32 rows: all threads bring them to shared memory (coalesced),
+// one warp adds them up, a row a lane (rows 353 floats apart: no conflicts).
+constexpr int ZB_ROWS = 32;
+__global__ void __launch_bounds__(256) k_zero_best(const float* __restrict__ db, int ndb,
+                                                   unsigned long long* __restrict__ best) {
+  __shared__ float s_row[ZB_ROWS][TC_DIM + 1];
+  const int j0 = blockIdx.x * ZB_ROWS, rows = min(ZB_ROWS, ndb - j0);
+  for (int i = threadIdx.x; i < rows * TC_DIM; i += blockDim.x) s_row[i / TC_DIM][i % TC_DIM] = db[(size_t)j0 * TC_DIM + i];
+  __syncthreads();
+  if ((int)threadIdx.x >= rows) return;
+  float acc = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < TC_DIM; ++k) {
+    const float t = __fsub_rn(0.f, s_row[threadIdx.x][k]);
+    acc = __fadd_rn(acc, __fmul_rn(t, t));
   }
+  if (acc < __int_as_float(0x7f800000))
+    atomicMin(best, ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned)(j0 + threadIdx.x));
 }
 
 __global__ void k_band_gather(const uint4* __restrict__ qhi, const uint4* __restrict__ qlo,
@@ -725,6 +977,26 @@ static long long tc_spin_limit(const rtr_context* ctx) {
   return t < 1 ? 1 : t;
 }
 
+// Database ranges of the first pass: the fewest waves of CTAs times tiles of a
+// CTA (its start costs about half a tile), where a few queries would leave SMs
+// idle.  The lists of the ranges after the first have to fit in the band
+// pass's rows.
+static int match_ranges(int nqp, int ndb, int bq) {
+  const int sms = 152, tiles = (ndb + TC_BN - 1) / TC_BN;
+  const long long ctas = nqp / TC_BM;
+  int best = 1;
+  double cost = 0.0;
+  for (int r = 1; r <= TC_RANGES && r <= tiles; ++r) {
+    if ((long long)(r - 1) * nqp * TC_TOP * 2 > (long long)bq * TC_BAND) break;
+    const double c = (double)((ctas * r + sms - 1) / sms) * ((tiles + r - 1) / r + 0.6);
+    if (r == 1 || c < 0.97 * cost) {
+      best = r;
+      cost = c;
+    }
+  }
+  return best;
+}
+
 void match_tc_plan(ScratchPlan& p, int nq_cap, bool with_db, int ndb) {
   const int nqp = ((nq_cap + TC_BM - 1) / TC_BM) * TC_BM;
   p.add<__nv_bfloat16>((size_t)nqp * TC_KPAD);
@@ -764,8 +1036,7 @@ rtr_status match_tc_prepare_db(const float* db, int ndb, __nv_bfloat16* hi, __nv
   RTR_CUDA(cudaMemsetAsync(db_zero_key(norm2, ndb), 0xff, sizeof(unsigned long long), st));
   k_split_bf16<<<blocks, 256, 0, st>>>(db, ndb, nullptr, ndb, hi, lo, norm2, reinterpret_cast<unsigned*>(norm2 + ndb),
                                        true, nullptr);
-  const int zb = (ndb + 255) / 256 < 152 * 4 ? (ndb + 255) / 256 : 152 * 4;
-  k_zero_best<<<zb > 0 ? zb : 1, 256, 0, st>>>(db, ndb, db_zero_key(norm2, ndb));
+  k_zero_best<<<ndb > 0 ? (ndb + ZB_ROWS - 1) / ZB_ROWS : 1, 256, 0, st>>>(db, ndb, db_zero_key(norm2, ndb));
   RTR_LAUNCHED(2);
   RTR_CUDA(cudaGetLastError());
   return RTR_OK;
@@ -814,29 +1085,36 @@ rtr_status match_tc_dev(rtr_context* ctx, Scratch& s, const float* q, int nq_cap
       !make_map(&m_bl, db_lo, ndb, TC_BN) || !make_map(&m_qh2, hi2, bq, TC_BM) || !make_map(&m_ql2, lo2, bq, TC_BM))
     return fail(RTR_ERR_CUDA, "match_tc: cuTensorMapEncodeTiled failed");
   const size_t smem = (size_t)TC_STAGES * TC_STAGE_BYTES + 1024;
+  const size_t top_smem = smem + TC_BM * TC_ROW * sizeof(float);
   // per call: the attribute is per device, and calls may come from several threads
-  RTR_CUDA(cudaFuncSetAttribute(k_match_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  RTR_CUDA(cudaFuncSetAttribute(k_match_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  TcArgs a{nq_cap, d_nq, nq_cap, ndb, qn, cidx, cd, ctx->d_status, nullptr, nullptr, tc_spin_limit(ctx)};
+  RTR_CUDA(cudaFuncSetAttribute(k_match_top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)top_smem));
+  RTR_CUDA(cudaFuncSetAttribute(k_match_band, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // The lists of further ranges lie in the band pass's rows (written after
+  // the re-rank has read them).
+  const int ranges = match_ranges(nqp, ndb, bq);
+  int* more_idx = band_idx;
+  float* more_d = reinterpret_cast<float*>(band_idx + (size_t)(ranges - 1) * nq_cap * TC_TOP);
+  TcArgs a{nq_cap, d_nq, nq_cap, ndb, qn, cidx, cd, more_idx, more_d, ctx->d_status, nullptr, nullptr,
+           tc_spin_limit(ctx)};
   {
     ProfScope pg(ctx, st, "match_gemm");
-    k_match_tc<false><<<nqp / TC_BM, TC_THREADS, smem, st>>>(m_qh, m_ql, m_bh, m_bl, a);
+    k_match_top<<<dim3(nqp / TC_BM, ranges), TC_THREADS, top_smem, st>>>(m_qh, m_ql, m_bh, m_bl, a);
   }
   RTR_CUDA(cudaMemsetAsync(nredo, 0, 2 * sizeof(int), st));
-  int rb = (nq_cap + 31) / 32;
+  int rb = (nq_cap + RR_WARPS * RR_Q - 1) / (RR_WARPS * RR_Q);
   if (rb > 152 * 16) rb = 152 * 16;
   // block per uncertified query (grid-stride over the device-side count)
   const int wb = band_rows(nqp) < 152 * 8 ? band_rows(nqp) : 152 * 8;
   const bool v4 = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(db)) & 15u) == 0;
   // band pass over the uncertified queries: the GEMM again, listing every
   // row within the tie margin, then exact distances to those rows only
-  TcArgs ab{bq, nredo, bq, ndb, qn2, band_idx, nullptr, ctx->d_status, redo_thr, band_n, tc_spin_limit(ctx)};
+  TcArgs ab{bq, nredo, bq, ndb, qn2, band_idx, nullptr, nullptr, nullptr, ctx->d_status, redo_thr, band_n, tc_spin_limit(ctx)};
   ProfScope pr(ctx, st, "match_rerank");
   if (v4)
-    k_rerank<true><<<rb, 256, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, out_idx, out_d2, redo, nredo,
+    k_rerank<true><<<rb, 32 * RR_WARPS, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, more_idx, more_d, ranges, out_idx, out_d2, redo, nredo,
                                        redo_best, redo_thr, qn, db_n2 + ndb, db_zero_key(db_n2, ndb), qzero);
   else
-    k_rerank<false><<<rb, 256, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, out_idx, out_d2, redo, nredo,
+    k_rerank<false><<<rb, 32 * RR_WARPS, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, more_idx, more_d, ranges, out_idx, out_d2, redo, nredo,
                                         redo_best, redo_thr, qn, db_n2 + ndb, db_zero_key(db_n2, ndb), qzero);
   pr.end();
   ProfScope pu(ctx, st, "match_uncertified");
@@ -848,7 +1126,7 @@ rtr_status match_tc_dev(rtr_context* ctx, Scratch& s, const float* q, int nq_cap
     ProfScope pb(ctx, st, "match_band");
     const int n_tiles = (ndb + TC_BN - 1) / TC_BN;
     const dim3 grid(bq / TC_BM, n_tiles < 8 ? n_tiles : 8);
-    k_match_tc<true><<<grid, TC_THREADS, smem, st>>>(m_qh2, m_ql2, m_bh, m_bl, ab);
+    k_match_band<<<grid, TC_THREADS, smem, st>>>(m_qh2, m_ql2, m_bh, m_bl, ab);
   }
   if (v4) {
     k_band_rerank<true><<<wb, 256, 0, st>>>(q, db, redo, nredo, redo_thr, band_idx, band_n, bq, ndb, redo_best, full,

@@ -146,3 +146,31 @@ def test_match_tc_zero_and_nonfinite_queries(ctx, descs):
     assert np.array_equal(idx.cpu().numpy(), ri)
     assert np.array_equal(d2.cpu().numpy(), rd, equal_nan=True)
     assert ctx.match_full_scans() >= 3
+
+
+@pytest.mark.parametrize("nq", [1, 127, 129, 2500])
+@pytest.mark.parametrize("ndb", [7, 255, 257, 513, 2049, 2300])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_match_tc_database_ranges(ctx, descs, nq, ndb, aligned):
+    """Few queries take the database in up to eight ranges, each with its own
+    list of 8: a last range of a row or a few, rows of the first tiles repeated
+    at the end (ties across ranges go to the lowest index), rows that do not
+    start on 16 bytes, a zero query among them."""
+    import torch
+    md, sd = descs
+    db = np.concatenate([md, md])[:ndb].copy()
+    db[-(ndb // 3):] = db[: ndb // 3]
+    q = np.concatenate([sd, md])[:nq].copy()
+    q[nq // 2] = 0.0
+    if nq > 100:
+        q[50:100] = md[:50]  # exact hits and ties
+    dev = []
+    for a in (q, db):
+        flat = torch.empty(a.size + 4, dtype=torch.float32, device="cuda")
+        v = flat[0 if aligned else 1:][: a.size].view(a.shape)
+        v.copy_(torch.from_numpy(a))
+        dev.append(v)
+    idx, d2 = ctx.match(*dev)
+    ri, rd = O.match(q, db)
+    assert np.array_equal(idx.cpu().numpy(), ri)
+    assert np.array_equal(d2.cpu().numpy(), rd)
