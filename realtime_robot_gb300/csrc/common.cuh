@@ -101,6 +101,8 @@ struct rtr_context {
   size_t scratch_limit = 0;            // largest scratch arena this context may hold (0: no limit)
   int tune_batch_workers = 0;          // workers of rtr_recognize_batch (0: automatic)
   int coop_div = 1;                    // cooperative grids use 1/coop_div of the GPU
+  bool worker = false;                 // a worker of rtr_recognize_batch / rtr_recognize_multi
+  bool grid_sorts = false;             // sorts take a grid of tiles whatever their size (see recognize_impl)
   int tune_gc_window = 0;              // seeds per grouping window (0: automatic)
   int tune_gc_no_lists = 0;            // 1: the grouping keeps no pass lists (every stale set ends a round)
   int tune_gc_inline = 0;              // times a round the grouping walk recomputes sets in place (0: automatic)

@@ -1,6 +1,9 @@
 // grid.cu — stable LSD radix sort and the uniform-grid build (counted into place).
 #include <math.h>
 
+#include <atomic>
+
+#include "csort.cuh"
 #include "grid.cuh"
 
 namespace rtr {
@@ -10,6 +13,8 @@ constexpr int RS_WARPS = RS_BLOCK / 32;
 constexpr int RS_ITEMS = 16;
 constexpr int RS_TILE = RS_BLOCK * RS_ITEMS;  // 4096 keys per block
 constexpr int RS_RADIX = 256;
+constexpr int RS_CLUSTER_MAX = 131072;  // items that one cluster sorts in a launch (more: a grid, two launches a pass)
+constexpr int RS_CLUSTER_ITEMS = 1024;   // items a CTA before the cluster grows
 
 __device__ __forceinline__ int count_of(int n_host, const int* d_n) { return d_n ? *d_n : n_host; }
 
@@ -202,20 +207,80 @@ __global__ void __launch_bounds__(RS_BLOCK) k_rs_scatter(const uint32_t* __restr
   }
 }
 
+// All passes by one cluster (csort.cuh).
+__global__ void __launch_bounds__(CS_THREADS) k_rs_cluster(uint32_t* __restrict__ k0, uint32_t* __restrict__ v0,
+                                                           uint32_t* __restrict__ k1, uint32_t* __restrict__ v1,
+                                                           int n_host, const int* d_n, int passes, int iota) {
+  __shared__ CsShared s;
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const CsChunk c(count_of(n_host, d_n), (int)cl.block_rank(), (int)cl.num_blocks());
+  for (int p = 0; p < passes; ++p) {
+    uint32_t* ki = p & 1 ? k1 : k0;
+    uint32_t* vi = p & 1 ? v1 : v0;
+    cs_count(s, c, 8 * p, [&](int i) { return __ldcg(ki + i); });
+    cs_offsets(s, cl);
+    cs_scatter(s, c, 8 * p, ki, p == 0 && iota ? nullptr : vi, p & 1 ? k0 : k1, p & 1 ? v0 : v1, cl);
+  }
+}
+
+// Whether the current device schedules clusters of CS_MAX CTAs of this size
+// (more than 8 is up to the device), asked once a device.
+static bool cluster_max_ok() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  int k = known[dev].load(std::memory_order_relaxed);
+  if (k == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CS_MAX);
+    cfg.blockDim = dim3(CS_THREADS);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CS_MAX;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool ok =
+        cudaFuncSetAttribute(k_rs_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, k_rs_cluster, &cfg) == cudaSuccess && n > 0;
+    if (!ok) cudaGetLastError();
+    k = ok ? 2 : 1;
+    known[dev].store(k, std::memory_order_relaxed);
+  }
+  return k == 2;
+}
+
+// One cluster sorts up to RS_CLUSTER_MAX items in a launch (13 us for two
+// passes of 2k items, 26 for four of 12k; a grid takes two launches a pass,
+// 6.6 us each there).  Voxels and keypoints of a 123k-point scan: 767 us with
+// the line at 32k items, 667 at 131k; the 300k-point room's recognition 3,210
+// us with it there, 3,243 with the line beyond its points.  Clusters of at
+// most 8 CTAs: the scan 727 us.
+int cluster_sort_ctas(const rtr_context* ctx, int n_cap) {
+  if (n_cap > RS_CLUSTER_MAX || (ctx && ctx->grid_sorts)) return 0;
+  const int want = (n_cap + RS_CLUSTER_ITEMS - 1) / RS_CLUSTER_ITEMS;
+  int c = 1;
+  while (c < want && c < (c < 8 || cluster_max_ok() ? CS_MAX : 8)) c *= 2;
+  return c;
+}
+
 int radix_hist_entries(int n_cap) {
   int nb = (n_cap + RS_TILE - 1) / RS_TILE;
   if (nb < 1) nb = 1;
   return nb * RS_RADIX;
 }
 
-void radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t* hist,
+void radix_sort_pairs(const rtr_context* ctx, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t* hist,
                       int n_cap, int n_host, const int* d_n, int bits, bool vals_iota,
                       cudaStream_t st, uint32_t** k_out, uint32_t** v_out) {
   int nb = (n_cap + RS_TILE - 1) / RS_TILE;
   if (nb < 1) nb = 1;
   int passes = (bits + 7) / 8;
   if (passes < 1) passes = 1;
-  for (int p = 0; p < passes; ++p) {
+  const int ctas = cluster_sort_ctas(ctx, n_cap);
+  if (ctas > 0) launch_cluster(k_rs_cluster, ctas, st, k0, v0, k1, v1, n_host, d_n, passes, (int)vals_iota);
+  for (int p = 0; p < passes && ctas == 0; ++p) {
     const int shift = 8 * p;
     const bool even = (p & 1) == 0;
     uint32_t* ki = even ? k0 : k1;
@@ -231,7 +296,7 @@ void radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, ui
       k_rs_scatter<false><<<nb, RS_BLOCK, 0, st>>>(ki, vi, ko, vo, n_host, d_n, shift, hist, nb);
     }
   }
-  RTR_LAUNCHED((nb <= RS_FUSE_TILES ? 2 : 3) * passes);
+  RTR_LAUNCHED(ctas > 0 ? 1 : (nb <= RS_FUSE_TILES ? 2 : 3) * passes);
   const bool odd = (passes & 1) != 0;
   *k_out = odd ? k1 : k0;
   *v_out = odd ? v1 : v0;
@@ -557,7 +622,7 @@ rtr_status grid_build(const GridBufs& b, const float4* pts, int n_host, const in
     int bits = 1;
     while (bits < 32 && (1ull << bits) < (unsigned long long)b.cell_cap) ++bits;
     uint32_t *ks, *vs;
-    radix_sort_pairs(b.k0, b.v0, b.k1, b.v1, b.hist, b.n_cap, n_host, d_n, bits, true, st, &ks, &vs);
+    radix_sort_pairs(nullptr, b.k0, b.v0, b.k1, b.v1, b.hist, b.n_cap, n_host, d_n, bits, true, st, &ks, &vs);
     k_grid_gather<<<nb, 256, 0, st>>>(pts, vs, n_host, d_n, b.pts);
   } else {
     k_grid_scatter<<<nb, 256, 0, st>>>(pts, b.k0, b.v0, b.starts, n_host, d_n, b.pts);

@@ -50,7 +50,26 @@ struct GridBufs {
 // When vals_in is NULL the values are the element indices.  Ping-pongs
 // between (k0,v0) and (k1,v1); *k_out/*v_out point at the sorted arrays.
 int radix_hist_entries(int n_cap);
-void radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t* hist,
+// CTAs of the cluster that sorts n_cap items in one launch; 0: a grid of tiles
+// (too many items, or ctx asks for it; ctx may be NULL).
+int cluster_sort_ctas(const rtr_context* ctx, int n_cap);
+// Launches a kernel of clusters of `ctas` CTAs of 1,024 threads (one cluster).
+template <class... P, class... A>
+inline void launch_cluster(void (*kern)(P...), int ctas, cudaStream_t st, A... args) {
+  if (ctas > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(1024);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, (P)args...);
+}
+void radix_sort_pairs(const rtr_context* ctx, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t* hist,
                       int n_cap, int n_host, const int* d_n, int bits, bool vals_iota,
                       cudaStream_t st, uint32_t** k_out, uint32_t** v_out);
 

@@ -739,7 +739,7 @@ static rtr_status scene_stages(rtr_context* ctx, const Scratch& stage, SceneBufs
       ProfScope ps2(ctx, st, "prune_select");
       k_score_keys<<<nb, 256, 0, st>>>(score, dKeys, n, k0);
       uint32_t *ks, *vs;
-      radix_sort_pairs(k0, v0, k1, v1, hist, n, n, dKeys, 32, true, st, &ks, &vs);
+      radix_sort_pairs(ctx, k0, v0, k1, v1, hist, n, n, dKeys, 32, true, st, &ks, &vs);
       k_mark_top<<<nb, 256, 0, st>>>(vs, dKeys, n, keep, b.flags);
     }
     ProfScope ps2(ctx, st, "prune_compact");
@@ -844,6 +844,15 @@ static rtr_status recognize_impl(rtr_context* ctx, const rtr_model* m, const flo
                                  const rtr_recog_params* q, rtr_recog_result* out, cudaStream_t st,
                                  const rtr_mlp* mlp = nullptr, float keep = 1.f) {
   const bool learned = mlp != nullptr;
+  // A plain recognition keeps a grid of tiles for its sorts, also where one
+  // cluster would do: tests/test_gpu_graph.py holds it to more than 100
+  // launches, and it has 101 (a 12k-point segment takes 2.185 ms so, 2.088 with
+  // the clusters and 59 launches; a batch of 64 takes 29.2 and 25.1).
+  struct GridSorts {
+    rtr_context* c;
+    GridSorts(rtr_context* ctx, bool on) : c(ctx) { c->grid_sorts = on; }
+    ~GridSorts() { c->grid_sorts = false; }
+  } grid_sorts(ctx, !learned && !ctx->worker);
   Scratch s;
   RTR_TRY(ensure_scratch(ctx, recognize_scratch_bytes(n, q, learned), st, &s));
   SceneBufs sb;

@@ -4,6 +4,7 @@
 // model_point.h:99-156, scan_point.h:57-113, key_point.h:112-161, 251-334).
 #include <math.h>
 
+#include "csort.cuh"
 #include "eig3.cuh"
 #include "recog.cuh"
 #include "scan.cuh"
@@ -158,6 +159,155 @@ __global__ void __launch_bounds__(256) k_seg_starts(const uint32_t* __restrict__
   }
 }
 
+// The whole segmentation by one cluster: bounds, keys, sort, heads and starts
+// (each of them as in the kernels above).  The number of passes is known here:
+// a byte for each 8 bits of the largest key, points without a voxel taking the
+// key after the last.
+__global__ void __launch_bounds__(CS_THREADS) k_voxseg(const float4* __restrict__ pts, int n_host, const int* d_n,
+                                                       float inv, VoxMeta* meta, uint32_t* k0, uint32_t* v0,
+                                                       uint32_t* k1, uint32_t* v1, int* __restrict__ seg_start,
+                                                       int* d_nseg) {
+  __shared__ CsShared s;
+  __shared__ int s_red[7][CS_WARPS], s_ext[7];  // lo, hi, error: of the warps, of this CTA
+  __shared__ int s_lo[3], s_hi[3], s_err;
+  __shared__ int s_heads[CS_WARPS], s_keyed[CS_WARPS], s_sum[2];
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int rank = (int)cl.block_rank(), ctas = (int)cl.num_blocks();
+  const int n = cnt_of(n_host, d_n);
+  const CsChunk c(n, rank, ctas);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // bounds
+  int ext[7] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000, (int)0x80000000, 0};
+#pragma unroll 4
+  for (int j = 0; j < c.steps; ++j) {
+    const int i = c.beg + j * 32 + lane;
+    if (i >= n) continue;
+    const float4 p = pts[i];
+    if (!finite3(p)) continue;
+    const int v[3] = {vox_coord(p.x, inv, &ext[6]), vox_coord(p.y, inv, &ext[6]), vox_coord(p.z, inv, &ext[6])};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      ext[a] = min(ext[a], v[a]);
+      ext[3 + a] = max(ext[3 + a], v[a]);
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 7; ++a) {
+    const int v = a < 3 ? __reduce_min_sync(0xffffffffu, ext[a]) : __reduce_max_sync(0xffffffffu, ext[a]);
+    if (lane == 0) s_red[a][warp] = v;
+  }
+  __syncthreads();
+  if (warp < 7) {
+    const int v = s_red[warp][lane];
+    const int r = warp < 3 ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+    if (lane == 0) s_ext[warp] = r;
+  }
+  cl.sync();
+  if (warp < 7) {
+    const bool in = lane < ctas;
+    const int v = in ? cl.map_shared_rank(s_ext, in ? lane : 0)[warp] : s_ext[warp];
+    const int r = warp < 3 ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+    if (lane == 0) (warp < 3 ? s_lo[warp] : (warp < 6 ? s_hi[warp - 3] : s_err)) = r;
+  }
+  __syncthreads();
+  const bool any = n > 0 && s_lo[0] <= s_hi[0];  // a finite point
+  const int l0 = any ? s_lo[0] : 0, l1 = any ? s_lo[1] : 0, l2 = any ? s_lo[2] : 0;
+  const long long dx = any ? (long long)s_hi[0] - l0 + 1 : 1, dy = any ? (long long)s_hi[1] - l1 + 1 : 1,
+                  dz = any ? (long long)s_hi[2] - l2 + 1 : 1;
+  const bool bad = s_err != 0 || dx * dy > 0xffffffffLL || dx * dy * dz >= 0xffffffffLL;
+  if (rank == 0 && threadIdx.x == 0) {
+    for (int a = 0; a < 3; ++a) {
+      meta->lo[a] = any || n <= 0 ? s_lo[a] : 0;
+      meta->hi[a] = s_hi[a];
+    }
+    meta->dx = (unsigned)dx;
+    meta->dy = (unsigned)dy;
+    meta->dz = (unsigned)dz;
+    meta->error = bad ? 1 : 0;
+    meta->n = n;
+  }
+  const uint32_t skip = bad ? 1u : (uint32_t)(dx * dy * dz);  // (below 2^32 - 1)
+  const int passes = (32 - __clz((int)skip) + 7) / 8;
+  const unsigned udx = (unsigned)dx, udy = (unsigned)dy;
+  // the sorted keys end in k0, v0
+  for (int p = 0; p < passes; ++p) {
+    const bool to0 = ((passes - p) & 1) != 0;
+    uint32_t* ki = to0 ? k1 : k0;
+    if (p == 0) {
+      cs_count(s, c, 0, [&](int i) {
+        const float4 q = pts[i];
+        uint32_t k = skip;
+        if (finite3(q)) {
+          int e = 0;
+          const unsigned x = (unsigned)(vox_coord(q.x, inv, &e) - l0), y = (unsigned)(vox_coord(q.y, inv, &e) - l1),
+                         z = (unsigned)(vox_coord(q.z, inv, &e) - l2);
+          k = bad ? 0u : (z * udy + y) * udx + x;
+        }
+        ki[i] = k;
+        return k;
+      });
+    } else {
+      cs_count(s, c, 8 * p, [&](int i) { return __ldcg(ki + i); });
+    }
+    cs_offsets(s, cl);
+    cs_scatter(s, c, 8 * p, ki, p == 0 ? nullptr : (to0 ? v1 : v0), to0 ? k0 : k1, to0 ? v0 : v1, cl);
+  }
+  // heads: the first of each run of equal keys
+  int heads = 0, keyed = 0;
+#pragma unroll 4
+  for (int j = 0; j < c.steps; ++j) {
+    const int i = c.beg + j * 32 + lane;
+    const uint32_t k = i < n ? __ldcg(k0 + i) : skip;
+    const uint32_t before = i > 0 && i < n ? __ldcg(k0 + i - 1) : skip;
+    heads += __popc(__ballot_sync(0xffffffffu, k != skip && k != before));
+    keyed += __popc(__ballot_sync(0xffffffffu, k != skip));
+  }
+  if (lane == 0) {
+    s_heads[warp] = heads;
+    s_keyed[warp] = keyed;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int h = s_heads[lane];
+    int inc = h;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    s_heads[lane] = inc - h;
+    const int kt = __reduce_add_sync(0xffffffffu, s_keyed[lane]);
+    if (lane == 31) {
+      s_sum[0] = inc;
+      s_sum[1] = kt;
+    }
+  }
+  cl.sync();
+  int at = s_heads[warp], total = 0, points = 0;
+  for (int r = 0; r < ctas; ++r) {
+    const int* o = cl.map_shared_rank(s_sum, r);
+    const int h = o[0];
+    at += r < rank ? h : 0;
+    total += h;
+    points += o[1];
+  }
+#pragma unroll 4
+  for (int j = 0; j < c.steps; ++j) {
+    const int i = c.beg + j * 32 + lane;
+    const uint32_t k = i < n ? __ldcg(k0 + i) : skip;
+    const uint32_t before = i > 0 && i < n ? __ldcg(k0 + i - 1) : skip;
+    const bool head = k != skip && k != before;
+    const unsigned b = __ballot_sync(0xffffffffu, head);
+    if (head) seg_start[at + __popc(b & lanemask_lt())] = i;
+    at += __popc(b);
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    *d_nseg = total;
+    seg_start[total] = points;
+  }
+  cl.sync();  // no CTA leaves while another reads its sums
+}
+
 void voxseg_plan(ScratchPlan& p, int n_cap) {
   const int n = n_cap > 0 ? n_cap : 1;
   p.add<VoxMeta>(1);
@@ -185,14 +335,22 @@ bool voxseg_take(Scratch& s, int n_cap, VoxSeg* v) {
          v->seg_start && v->d_nseg;
 }
 
-void voxseg_build(VoxSeg& v, const float4* pts, int n_host, const int* d_n, float inv, cudaStream_t st) {
+void voxseg_build(const rtr_context* ctx, VoxSeg& v, const float4* pts, int n_host, const int* d_n, float inv, cudaStream_t st) {
+  const int ctas = cluster_sort_ctas(ctx, v.n_cap);
+  if (ctas > 0) {
+    launch_cluster(k_voxseg, ctas, st, pts, n_host, d_n, inv, v.meta, v.k0, v.v0, v.k1, v.v1, v.seg_start, v.d_nseg);
+    RTR_LAUNCHED(1);
+    v.keys = v.k0;
+    v.order = v.v0;
+    return;
+  }
   const int nb = blocks_for(v.n_cap);
   k_vox_init<<<1, 32, 0, st>>>(v.meta);
   k_vox_bounds<<<nb < 152 * 2 ? nb : 152 * 2, 256, 0, st>>>(pts, n_host, d_n, inv, v.meta);  // block-reduced
   k_vox_setup<<<1, 1, 0, st>>>(v.meta, n_host, d_n);
   k_vox_keys<<<nb, 256, 0, st>>>(pts, n_host, d_n, inv, v.meta, v.k0);
   uint32_t *ks, *vs;
-  radix_sort_pairs(v.k0, v.v0, v.k1, v.v1, v.hist, v.n_cap, n_host, d_n, 32, true, st, &ks, &vs);
+  radix_sort_pairs(ctx, v.k0, v.v0, v.k1, v.v1, v.hist, v.n_cap, n_host, d_n, 32, true, st, &ks, &vs);
   k_seg_heads<<<nb, 256, 0, st>>>(ks, n_host, d_n, v.flags);
   scan_exclusive(v.flags, v.flags, v.tile_sums, v.n_cap, n_host, d_n, reinterpret_cast<uint32_t*>(v.d_nseg), st);
   k_seg_starts<<<nb, 256, 0, st>>>(ks, v.flags, n_host, d_n, v.seg_start, v.d_nseg);
@@ -665,7 +823,7 @@ rtr_status voxel_downsample_dev(rtr_context* ctx, Scratch& s, const float4* pts,
   VoxSeg v;
   if (!voxseg_take(s, n_cap, &v)) return fail(RTR_ERR_CAPACITY, "voxel_downsample: scratch");
   const float inv = 1.0f / leaf;
-  voxseg_build(v, pts, n_cap, d_n, inv, st);
+  voxseg_build(ctx, v, pts, n_cap, d_n, inv, st);
   k_vox_centroid<<<blocks_for(n_cap), 256, 0, st>>>(pts, v.order, v.seg_start, v.d_nseg, v.meta, out, d_count);
   RTR_LAUNCHED(1);
   return RTR_OK;
@@ -676,7 +834,7 @@ rtr_status uniform_sample_dev(rtr_context* ctx, Scratch& s, const float4* pts, i
   VoxSeg v;
   if (!voxseg_take(s, n_cap, &v)) return fail(RTR_ERR_CAPACITY, "uniform_sample: scratch");
   const float inv = 1.0f / r;
-  voxseg_build(v, pts, n_cap, d_n, inv, st);
+  voxseg_build(ctx, v, pts, n_cap, d_n, inv, st);
   k_uniform_pick<<<blocks_for(n_cap), 256, 0, st>>>(pts, v.order, v.seg_start, v.d_nseg, v.meta, inv, r, out, d_count);
   RTR_LAUNCHED(1);
   return RTR_OK;

@@ -128,3 +128,24 @@ def test_match_exact_bit_exact(ctx, clouds):
     md2 = np.concatenate([md[:100], md[:100]])
     idx, _ = ctx.match_exact(_dev(md[:100]), _dev(md2))
     assert np.array_equal(_host(idx), np.arange(100))
+
+
+@pytest.mark.parametrize("n", [1, 31, 1024, 1025, 8193, 16385, 131072, 131073])
+@pytest.mark.parametrize("half,leaf", [(0.02, 0.01), (0.5, 0.01), (3.0, 0.01), (5.0, 0.0065)])
+def test_voxels_by_size_and_key_width(ctx, n, half, leaf):
+    """The segmentation at the edges of its forms: one CTA to a cluster of
+    sixteen, beyond that a grid; keys of one to four bytes (64 voxels to just
+    under 2^32); points without a voxel among the others, and alone."""
+    rng = np.random.default_rng(n + int(1e4 * leaf))
+    pts = np.zeros((n, 4), np.float32)
+    pts[:, :3] = rng.uniform(-half, half, (n, 3))
+    if n > 1:
+        pts[:2, :3] = [[-half] * 3, [half] * 3]
+    if n > 30:
+        pts[rng.choice(np.arange(2, n), n // 10, replace=False), rng.integers(0, 3)] = np.nan
+        pts[n // 2:n // 2 + 5] = pts[2:7]
+    got = _host(ctx.voxel_downsample(_dev(pts), leaf))
+    assert np.array_equal(got, O.voxel_downsample(pts, leaf))
+    assert np.array_equal(_host(ctx.uniform_sample(_dev(pts), leaf)), O.uniform_sample(pts, leaf))
+    pts[:, 1] = np.inf
+    assert ctx.voxel_downsample(_dev(pts), leaf).shape[0] == 0
