@@ -691,11 +691,10 @@ static rtr_status scene_stages(rtr_context* ctx, const Scratch& stage, SceneBufs
   {
     ProfScope ps(ctx, st, "normals");
     Scratch t = stage;
-    // 5 leaves: the k-NN of a voxel (k = 10 at 1 cm) mostly resolves in its
-    // own cell and the next ring; smaller cells cost more cell visits than
-    // the extra points of larger ones (0.71 ms at 2 leaves, 0.41 ms at 5 on
-    // the 213k-voxel room)
-    const float cell = ctx->tune_normals_grid_mm > 0 ? 1e-3f * (float)ctx->tune_normals_grid_mm : 5.f * q->voxel_leaf;
+    // 2 leaves: the k-NN of a voxel (k = 10 at 1 cm) mostly lies in the 27
+    // cells around it (on the 213k-voxel room 223 us with the grid at 2 and 3
+    // leaves, 286 at 5)
+    const float cell = ctx->tune_normals_grid_mm > 0 ? 1e-3f * (float)ctx->tune_normals_grid_mm : 2.f * q->voxel_leaf;
     RTR_TRY(normals_dev(ctx, t, b.sv, n, dV, q->normal_k, q->viewpoint, cell, b.sn, st));
     if (q->scene_outward) {
       k_orient_outward<<<nblocks(n, 8, 152 * 16), 256, 0, st>>>(b.sv, b.sn, n, dV, 0.01f * 0.01f, 0.005f, 1.0f);

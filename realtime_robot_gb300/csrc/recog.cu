@@ -421,17 +421,42 @@ __global__ void __launch_bounds__(256) k_uniform_pick(const float4* __restrict__
 // kNN order, exact Jacobi, smallest eigenvector flipped towards vp,
 // curvature l0 / (l0 + l1 + l2)
 // ---------------------------------------------------------------------------
+// A warp takes `per` (<= 32) consecutive points of the grid's order: searches
+// them one at a time (knn_warp), then a lane finishes each.
+// With a thread a point the kernel waited for its slowest threads: chains of
+// 50-100k cycles over a few hundred candidates, longer where a point lies far
+// from others.  With the grid build (7k points of a segment / 105k of a scan /
+// 213k of a room, cells of two voxel leaves): 166 / 322 / 302 us then, 54 / 134
+// / 223 now; cells of five leaves 220 / 260 / 300 then, 69 / 140 / 286 now.  A
+// warp takes few points so that the chip's share of the work evens out (32 a
+// warp: the scan 173, 16: 151, 8: 149, 4: 160), four where there are few.
+constexpr int NRM_WARPS = 4;
+constexpr int NRM_SMALL = 19456;  // points up to which a warp takes four (152 SMs, 32 warps each)
 template <int K>
-__global__ void __launch_bounds__(128) k_normals(GridDev gd, const float4* __restrict__ pts, int n_host,
-                                                 const int* d_n, float vx, float vy, float vz,
-                                                 float4* __restrict__ out) {
-  const GridView g = load_view(gd);
+__global__ void __launch_bounds__(32 * NRM_WARPS) k_normals(GridDev gd, const float4* __restrict__ pts, int n_host,
+                                                            const int* d_n, float vx, float vy, float vz, int per,
+                                                            float4* __restrict__ out) {
+  __shared__ int s_idx[NRM_WARPS][K][33];
+  const BoxView v = box_view(gd);
   const int n = cnt_of(n_host, d_n);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float4 p = pts[i];
-    float bd[K];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j0 = (blockIdx.x * NRM_WARPS + warp) * per; j0 < n; j0 += gridDim.x * NRM_WARPS * per) {
+    const int cnt = min(per, n - j0);
+    const float4 p = lane < cnt ? v.g.pts[j0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = 0; t < cnt; ++t) {
+      const float4 q = make_float4(__shfl_sync(0xffffffffu, p.x, t), __shfl_sync(0xffffffffu, p.y, t),
+                                   __shfl_sync(0xffffffffu, p.z, t), 0.f);
+      unsigned long long e = KNN_NONE;
+      if (finite3(q)) e = knn_warp<K>(v, q);  // (a point with a coordinate that is not finite has no neighbours)
+      if (lane < K) s_idx[warp][lane][t] = e == KNN_NONE ? INT_MAX : (int)(unsigned)e;
+    }
+    __syncwarp();
     int bi[K];
-    grid_knn<K>(g, p, bd, bi);
+#pragma unroll
+    for (int s = 0; s < K; ++s) bi[s] = s_idx[warp][s][lane];
+    __syncwarp();
+    if (lane >= cnt) continue;
+    const int i = pt_index(p);
     int m = 0;
     float mx = 0.f, my = 0.f, mz = 0.f;
 #pragma unroll
@@ -846,13 +871,14 @@ rtr_status normals_dev(rtr_context* ctx, Scratch& s, const float4* pts, int n_ca
   const unsigned cap = default_cell_cap(n_cap);
   if (!grid_take(s, n_cap, cap, &gb)) return fail(RTR_ERR_CAPACITY, "normals: scratch");
   RTR_TRY(grid_build(gb, pts, n_cap, d_n, cell, st));
-  const int nb = blocks_for(n_cap, 128);
+  const int per = n_cap < NRM_SMALL ? 4 : 8;
+  const int nb = blocks_for(n_cap, NRM_WARPS * per, 1 << 20);
   if (k <= 8)
-    k_normals<8><<<nb, 128, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], out);
+    k_normals<8><<<nb, 32 * NRM_WARPS, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], per, out);
   else if (k <= 10)
-    k_normals<10><<<nb, 128, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], out);
+    k_normals<10><<<nb, 32 * NRM_WARPS, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], per, out);
   else if (k <= 16)
-    k_normals<16><<<nb, 128, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], out);
+    k_normals<16><<<nb, 32 * NRM_WARPS, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], per, out);
   else
     return fail(RTR_ERR_INVALID_ARG, "normals: k must be 8, 10 or 16");
   RTR_LAUNCHED(1);

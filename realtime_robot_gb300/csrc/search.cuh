@@ -524,46 +524,203 @@ __device__ __forceinline__ bool grid_any_within(const BoxView& v, float4 q, floa
 }
 
 // Exact K-NN (K compile-time), sorted by (d^2, index).  The K nearest by that
-// order are unique, so any k <= K of them form the exact k-NN.
+// order are unique, so any k <= K of them form the exact k-NN.  The list holds
+// (d^2 bits, index) as one word each, ascending; an empty slot is (+inf, 0),
+// which no candidate at infinite or NaN d^2 goes below.  The slots of an
+// insertion are independent of each other.
+constexpr unsigned long long KNN_NONE = 0x7f800000ull << 32;
 template <int K>
-__device__ __forceinline__ void knn_insert(float (&bd)[K], int (&bi)[K], float d2, int id) {
-  // NaN and infinite d^2 never enter the list
-  if (!(d2 < bd[K - 1]) && !(d2 == bd[K - 1] && id < bi[K - 1] && d2 < __int_as_float(0x7f800000))) return;
-  bd[K - 1] = d2;
-  bi[K - 1] = id;
+__device__ __forceinline__ void knn_insert(unsigned long long (&list)[K], float4 q, float4 p) {
+  const unsigned long long c =
+      ((unsigned long long)__float_as_uint(dist2_exact(q, p)) << 32) | (unsigned)pt_index(p);
+  if (!(c < list[K - 1])) return;
+  bool lt[K];
 #pragma unroll
-  for (int s = K - 1; s > 0; --s) {
-    const bool lt = bd[s] < bd[s - 1] || (bd[s] == bd[s - 1] && bi[s] < bi[s - 1]);
-    const float da = bd[s], db = bd[s - 1];
-    const int ia = bi[s], ib = bi[s - 1];
-    bd[s] = lt ? db : da;
-    bd[s - 1] = lt ? da : db;
-    bi[s] = lt ? ib : ia;
-    bi[s - 1] = lt ? ia : ib;
+  for (int s = 0; s < K; ++s) lt[s] = c < list[s];
+#pragma unroll
+  for (int s = K - 1; s > 0; --s) list[s] = lt[s - 1] ? list[s - 1] : (lt[s] ? c : list[s]);
+  list[0] = lt[0] ? c : list[0];
+}
+template <int K>
+__device__ __forceinline__ float knn_worst(const unsigned long long (&list)[K]) {
+  return __uint_as_float((unsigned)(list[K - 1] >> 32));
+}
+
+// The nearest of the 27 cells around q's (cx, cy, cz) inside the grid: nine
+// rows, a run of points each, the nearest first.  True when nothing farther
+// can enter the list.
+template <int K>
+__device__ __forceinline__ bool knn_near(const GridView& g, float4 q, int cx, int cy, int cz,
+                                         unsigned long long (&list)[K]) {
+  const float margin = search_margin(g, q, 1);
+  const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.nx - 1);
+  const float ly = g.oy + (float)cy * g.h, lz = g.oz + (float)cz * g.h;  // the query's cell
+  const float ylo = fmaxf(q.y - ly, 0.f), yhi = fmaxf(ly + g.h - q.y, 0.f);
+  const float zlo = fmaxf(q.z - lz, 0.f), zhi = fmaxf(lz + g.h - q.z, 0.f);
+#pragma unroll 1
+  for (int r = 0; r < 9; ++r) {
+    // rows (0, 0), (-1, 0), (1, 0), (0, -1), (0, 1) and the corners: two bits each, plus one
+    const int dy = (int)((0x28161u >> (2 * r)) & 3u) - 1, dz = (int)((0x22215u >> (2 * r)) & 3u) - 1;
+    const int y = cy + dy, z = cz + dz;
+    if (y < 0 || y >= g.ny || z < 0 || z >= g.nz) continue;
+    const float ey = dy < 0 ? ylo : (dy > 0 ? yhi : 0.f), ez = dz < 0 ? zlo : (dz > 0 ? zhi : 0.f);
+    if (beyond(sqrtf(ey * ey + ez * ez), margin, knn_worst<K>(list))) continue;
+    const uint2 span = row_span(g, x0, x1, y, z);
+    for (unsigned j = span.x; j < span.y; ++j) knn_insert<K>(list, q, g.pts[j]);
+  }
+  return ring_covers(g, cx, cy, cz, 1) || beyond(ring_bound(g, q, cx, cy, cz, 1), margin, knn_worst<K>(list));
+}
+
+// The K (<= 32) nearest of a finite query by a whole warp, every lane with the
+// same q; lane s < K returns entry s (KNN_NONE: none).
+// Rows of a box of cells, 32 at a time, a lane a row's ends; their points as
+// one sequence, 32 at a time.  The list is held sorted across the lanes: a few
+// candidates below its last entry go in one by one, more of them are sorted and
+// merged.  The box: the 27 cells around the query's (its own cell where these
+// hold many points); once the list is full its last entry bounds the search,
+// and one more box, of the cells within that distance, settles it; boxes of 7,
+// 15, ... cells a side while it is not full.  So a point far from others costs
+// tens of steps, not a chain of single cells, and no lane waits for another
+// query's.
+__device__ __forceinline__ unsigned long long knn_stage(unsigned long long x, int d, bool low) {
+  const unsigned long long o = __shfl_xor_sync(0xffffffffu, x, d);
+  return (o < x) == low ? o : x;
+}
+struct KnnWarp {
+  unsigned long long mine, worst, limit;  // entry `lane`; entry K - 1; no entry of the result is above limit
+};
+// The points of the rows whose ends the lanes hold.
+template <int K>
+__device__ __forceinline__ void knn_rows(const GridView& g, float4 q, uint2 span, KnnWarp& w) {
+  const int lane = threadIdx.x & 31;
+  const int len = (int)(span.y - span.x);
+  int incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  const int first = (int)span.x - (incl - len);  // point t of the sequence, if in this lane's row: first + t
+  for (int t0 = 0; t0 < total; t0 += 32) {
+    const int t = t0 + lane;
+    int r = 0;  // rows that end at or before t
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, r + o - 1) <= t) r += o;
+    const int j = __shfl_sync(0xffffffffu, first, r & 31) + t;
+    unsigned long long c = ~0ull;
+    if (t < total) {
+      const float4 p = g.pts[j];
+      c = ((unsigned long long)__float_as_uint(dist2_exact(q, p)) << 32) | (unsigned)pt_index(p);
+    }
+    // (an entry of the last box's list may be the limit itself)
+    const bool in = c < w.worst && c <= w.limit && c < KNN_NONE;
+    unsigned m = __ballot_sync(0xffffffffu, in);
+    if (__popc(m) <= 6) {
+      for (; m; m &= m - 1) {
+        const unsigned long long x = __shfl_sync(0xffffffffu, c, __ffs(m) - 1);
+        const unsigned long long before = __shfl_up_sync(0xffffffffu, w.mine, 1);
+        if (x < w.mine) w.mine = lane > 0 && x < before ? before : x;
+      }
+    } else {
+      c = in ? c : KNN_NONE;
+#pragma unroll
+      for (int s = 2; s <= 32; s <<= 1)
+#pragma unroll
+        for (int d = s >> 1; d > 0; d >>= 1) c = knn_stage(c, d, ((lane & d) == 0) == ((lane & s) == 0));
+      if (__shfl_sync(0xffffffffu, w.mine, 0) == KNN_NONE) {
+        w.mine = c;  // the first candidates
+      } else {
+        const unsigned long long o = __shfl_sync(0xffffffffu, c, 31 - lane);
+        w.mine = o < w.mine ? o : w.mine;  // the 32 least of both, bitonic
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) w.mine = knn_stage(w.mine, d, (lane & d) == 0);
+      }
+    }
+    w.worst = __shfl_sync(0xffffffffu, w.mine, K - 1);
+  }
+}
+constexpr int KNN_DENSE = 128;  // points in 27 cells from which the query's own cell goes first
+template <int K>
+__device__ __forceinline__ unsigned long long knn_warp(const BoxView& v, float4 q) {
+  const GridView& g = v.g;
+  const int lane = threadIdx.x & 31;
+  const float margin = box_margin(v, q);
+  const int cx = min(max(q_cell(q.x, g.ox, g.inv_h), 0), g.nx - 1), cy = min(max(q_cell(q.y, g.oy, g.inv_h), 0), g.ny - 1),
+            cz = min(max(q_cell(q.z, g.oz, g.inv_h), 0), g.nz - 1);
+  KnnWarp w{KNN_NONE, KNN_NONE, KNN_NONE};
+  {
+    const int zi = lane / 3, y = cy + lane - 3 * zi - 1, z = cz + zi - 1;
+    uint2 span = make_uint2(0u, 0u);
+    if (lane < 9 && y >= 0 && y < g.ny && z >= 0 && z < g.nz)
+      span = row_span(g, max(cx - 1, 0), min(cx + 1, g.nx - 1), y, z);
+    bool own = false;
+    if (__reduce_add_sync(0xffffffffu, span.y - span.x) > KNN_DENSE) {
+      const uint2 c = cell_span(g, cx, cy, cz);
+      own = c.y - c.x >= (unsigned)K;
+      if (own) span = lane == 0 ? c : make_uint2(0u, 0u);
+    }
+    knn_rows<K>(g, q, span, w);
+    if (!own && (ring_covers(g, cx, cy, cz, 1) || beyond(ring_bound(g, q, cx, cy, cz, 1), margin,
+                                                         __uint_as_float((unsigned)(w.worst >> 32)))))
+      return w.mine;
+  }
+  for (int k = 3;; k = 2 * k + 1) {
+    // the cells within the list's last distance, or +-k cells
+    const bool full = w.worst < KNN_NONE;
+    CellBox c;
+    if (full) {
+      c = cell_box(v, q, sqrt_up(__uint_as_float((unsigned)(w.worst >> 32))) + margin);
+    } else {
+      c.x0 = max(cx - k, 0), c.x1 = min(cx + k, g.nx - 1), c.y0 = max(cy - k, 0), c.y1 = min(cy + k, g.ny - 1);
+      c.z0 = max(cz - k, 0), c.z1 = min(cz + k, g.nz - 1);
+    }
+    w.limit = w.worst;
+    w.mine = w.worst = KNN_NONE;
+    const int ny = c.y1 - c.y0 + 1, rows = ny * (c.z1 - c.z0 + 1);
+    for (int r0 = 0; r0 < rows; r0 += 32) {
+      uint2 span = make_uint2(0u, 0u);
+      if (r0 + lane < rows) {
+        const int zi = (r0 + lane) / ny, y = c.y0 + (r0 + lane) - zi * ny, z = c.z0 + zi;
+        const float fy = (float)y, fz = (float)z;
+        const float dy = fmaxf(fmaxf(fy - c.uy, c.uy - (fy + 1.f)), 0.f), dz = fmaxf(fmaxf(fz - c.uz, c.uz - (fz + 1.f)), 0.f);
+        if (!full || !(dy * dy + dz * dz > c.tc2)) span = row_span(g, c.x0, c.x1, y, z);
+      }
+      knn_rows<K>(g, q, span, w);
+    }
+    if (full || ring_covers(g, cx, cy, cz, k)) return w.mine;
+    if (beyond(ring_bound(g, q, cx, cy, cz, k), margin, __uint_as_float((unsigned)(w.worst >> 32)))) return w.mine;
   }
 }
 
+// A query inside the grid takes the 27 cells around it first; further rings,
+// and queries outside, go cell by cell.
 template <int K>
 __device__ __forceinline__ void grid_knn(const GridView& g, float4 q, float (&bd)[K], int (&bi)[K]) {
+  unsigned long long list[K];
 #pragma unroll
-  for (int s = 0; s < K; ++s) {
-    bd[s] = __int_as_float(0x7f800000);
-    bi[s] = INT_MAX;
-  }
+  for (int s = 0; s < K; ++s) list[s] = KNN_NONE;
   const int cx = q_cell(q.x, g.ox, g.inv_h), cy = q_cell(q.y, g.oy, g.inv_h),
             cz = q_cell(q.z, g.oz, g.inv_h);
-  for (int k = first_ring(g, cx, cy, cz);; ++k) {
+  int k = first_ring(g, cx, cy, cz);
+  bool done = false;
+  if (k == 0) {
+    done = knn_near<K>(g, q, cx, cy, cz, list);
+    k = 2;
+  }
+  for (; !done; ++k) {
     const float margin = search_margin(g, q, k);
     RTR_FOR_RING(g, cx, cy, cz, k, {
       const uint2 c = cell_span(g, x, y, z);
-      if (c.x < c.y && !beyond(cell_box_dist(g, q, x, y, z), margin, bd[K - 1])) {
-        for (unsigned j = c.x; j < c.y; ++j) {
-          const float4 p = g.pts[j];
-          knn_insert<K>(bd, bi, dist2_exact(q, p), pt_index(p));
-        }
-      }
+      if (c.x < c.y && !beyond(cell_box_dist(g, q, x, y, z), margin, knn_worst<K>(list)))
+        for (unsigned j = c.x; j < c.y; ++j) knn_insert<K>(list, q, g.pts[j]);
     })
-    if (ring_covers(g, cx, cy, cz, k)) break;
-    if (beyond(ring_bound(g, q, cx, cy, cz, k), margin, bd[K - 1])) break;
+    done = ring_covers(g, cx, cy, cz, k) || beyond(ring_bound(g, q, cx, cy, cz, k), margin, knn_worst<K>(list));
+  }
+#pragma unroll
+  for (int s = 0; s < K; ++s) {
+    bd[s] = __uint_as_float((unsigned)(list[s] >> 32));
+    bi[s] = list[s] == KNN_NONE ? INT_MAX : (int)(unsigned)list[s];
   }
 }

@@ -149,3 +149,29 @@ def test_voxels_by_size_and_key_width(ctx, n, half, leaf):
     assert np.array_equal(_host(ctx.uniform_sample(_dev(pts), leaf)), O.uniform_sample(pts, leaf))
     pts[:, 1] = np.inf
     assert ctx.voxel_downsample(_dev(pts), leaf).shape[0] == 0
+
+
+@pytest.mark.parametrize("k", [8, 10, 16])
+@pytest.mark.parametrize("cell", [0.003, 0.02, 0.2])
+def test_normals_sparse_dense_and_odd_points(ctx, k, cell):
+    """Neighbour searches at the edges of their forms: dense patches (own cell
+    first), single points far from others (boxes grown several times), fewer
+    points than k, lattice points (ties), coordinates that are not finite."""
+    rng = np.random.default_rng(5)
+    a = rng.uniform(-0.1, 0.1, (1500, 3))
+    a[:, 2] *= 0.05
+    lattice = np.stack(np.meshgrid(*[np.arange(7) * 0.01] * 3), -1).reshape(-1, 3) + [1.0, 0.0, 0.0]
+    far = rng.uniform(-3, 3, (40, 3))
+    pts = np.zeros((1500 + 343 + 40, 4), np.float32)
+    pts[:, :3] = np.concatenate([a, lattice, far])
+    pts = pts[rng.permutation(len(pts))]
+    for n in (len(pts), 129, 4, 1):
+        q = pts[:n]
+        got = _host(ctx.normals(_dev(q), k, (0.3, -1.0, 2.0), cell))
+        assert np.array_equal(got, O.normals(q, k, (0.3, -1.0, 2.0)), equal_nan=True), n
+    q = pts.copy()
+    q[7, 0] = np.nan
+    q[9, 2] = np.inf
+    got = _host(ctx.normals(_dev(q), k, (0.3, -1.0, 2.0), cell))
+    keep = np.isfinite(q[:, :3]).all(1)
+    assert np.array_equal(got[keep], O.normals(q[keep], k, (0.3, -1.0, 2.0)), equal_nan=True)
