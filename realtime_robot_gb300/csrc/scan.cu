@@ -40,11 +40,11 @@ __global__ void __launch_bounds__(SC_BLOCK) k_scan_sums(const uint32_t* __restri
                                                         const int* d_n, uint32_t* __restrict__ sums) {
   __shared__ uint32_t red[SC_BLOCK / 32];
   const int n = sc_count(n_host, d_n);
-  const int base = blockIdx.x * SC_TILE + threadIdx.x * SC_ITEMS;
+  const int base = blockIdx.x * SC_TILE + threadIdx.x;  // (a sum: any order, whole lines)
   uint32_t s = 0;
 #pragma unroll
   for (int j = 0; j < SC_ITEMS; ++j)
-    if (base + j < n) s += in[base + j];
+    if (base + j * SC_BLOCK < n) s += in[base + j * SC_BLOCK];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -94,20 +94,42 @@ __global__ void __launch_bounds__(1024) k_scan_top(uint32_t* __restrict__ h, int
 __global__ void __launch_bounds__(SC_BLOCK) k_scan_apply(const uint32_t* __restrict__ in,
                                                          uint32_t* __restrict__ out, int n_host,
                                                          const int* d_n, const uint32_t* __restrict__ sums) {
+  // whole lines in and out, a thread's 16 entries side by side in between (300k
+  // entries: 6.1 us with each thread walking its own 64 bytes, 3.4 so)
+  __shared__ uint32_t tile[SC_TILE + SC_TILE / 32];  // (one word of padding a row of 32)
   const int n = sc_count(n_host, d_n);
-  const int base = blockIdx.x * SC_TILE + threadIdx.x * SC_ITEMS;
+  const int base = blockIdx.x * SC_TILE;
   uint32_t v[SC_ITEMS];
+#pragma unroll
+  for (int j = 0; j < SC_ITEMS; ++j) {
+    const int i = j * SC_BLOCK + threadIdx.x;
+    v[j] = base + i < n ? in[base + i] : 0u;
+  }
+#pragma unroll
+  for (int j = 0; j < SC_ITEMS; ++j) {
+    const int i = j * SC_BLOCK + threadIdx.x;
+    tile[i + (i >> 5)] = v[j];
+  }
+  __syncthreads();
   uint32_t s = 0;
 #pragma unroll
   for (int j = 0; j < SC_ITEMS; ++j) {
-    v[j] = (base + j < n) ? in[base + j] : 0u;
+    const int i = threadIdx.x * SC_ITEMS + j;
+    v[j] = tile[i + (i >> 5)];
     s += v[j];
   }
   uint32_t run = block_excl_scan(s, nullptr) + sums[blockIdx.x];
 #pragma unroll
   for (int j = 0; j < SC_ITEMS; ++j) {
-    if (base + j < n) out[base + j] = run;
+    const int i = threadIdx.x * SC_ITEMS + j;
+    tile[i + (i >> 5)] = run;
     run += v[j];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < SC_ITEMS; ++j) {
+    const int i = j * SC_BLOCK + threadIdx.x;
+    if (base + i < n) out[base + i] = tile[i + (i >> 5)];
   }
 }
 
