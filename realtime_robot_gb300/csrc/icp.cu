@@ -80,8 +80,8 @@ __device__ __forceinline__ float centre_of(const GridMeta* m, int a) {
 // the kernel.  Per iteration of block 0, matching and sums before and now: two
 // 20k chairs 25 and 8 us; 102k points against a 285k-point frame 35 and 10 us;
 // 16 refinements of a 9.2k-voxel model in a room 24 and 10 us.
-template <int G>  // lanes cooperating on one source point's 1-NN search
-__global__ void __launch_bounds__(ICP_THREADS, 2) k_icp(const IcpDev* __restrict__ probs,
+template <int G, int OCC>  // lanes cooperating on one source point's 1-NN search; blocks wanted an SM
+__global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restrict__ probs,
                                                         const int* __restrict__ blk2prob) {
   const IcpDev& a = probs[blk2prob[blockIdx.x]];
   const int lb = (int)blockIdx.x - a.blk0;
@@ -478,23 +478,42 @@ __global__ void __launch_bounds__(256) k_gather_pts(const float4* __restrict__ p
   }
 }
 
+// Blocks an SM holds of the ICP kernel.  Two with all the registers that the
+// pose solve wants, where one call has the GPU: a solve an iteration is on its
+// critical path (two 20k chairs 1,295 us; 1,571 with three blocks an SM, 1,816
+// with four).  Four, the solve spilling, for the workers of a batch: other
+// pairs fill that wait, and the searches gain from the threads (64 pairs 22.9
+// ms with two, 20.4 with four, 21.8 with the share below).
+constexpr int ICP_OCC = 2, ICP_OCC_WORKER = 4;
+
 // Co-resident blocks of the ICP kernel (the smallest over the group sizes,
-// so a plan made for one group size fits every variant).
+// so a plan made for one group size fits every variant).  Workers run beside
+// each other's groupings, whose blocks take half an SM's registers, an ICP
+// block a quarter: with three quarters of the SMs' capacity shared out, every
+// cooperative launch finds its places however the others' blocks lie (k
+// workers with b = 3 S / n blocks each can make at most k b / 3 of S SMs unfit
+// for a grouping block, and the other SMs hold the other workers' shares).
 int icp_max_blocks(rtr_context* ctx) {
-  static std::atomic<int> cached[64];  // per device; 0 = not yet known
-  const int dev = ctx->device;
+  static std::atomic<int> cached[64][2];  // per device; 0 = not yet known
+  const int dev = ctx->device, kind = ctx->worker ? 1 : 0;
   if (dev >= 0 && dev < 64) {
-    const int v = cached[dev].load(std::memory_order_relaxed);
+    const int v = cached[dev][kind].load(std::memory_order_relaxed);
     if (v > 0) return v;
   }
   int a = 0, b = 0, c = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_icp<2>, ICP_THREADS, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icp<4>, ICP_THREADS, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_icp<8>, ICP_THREADS, 0);
+  if (kind) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_icp<2, ICP_OCC_WORKER>, ICP_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icp<4, ICP_OCC_WORKER>, ICP_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_icp<8, ICP_OCC_WORKER>, ICP_THREADS, 0);
+  } else {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_icp<2, ICP_OCC>, ICP_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icp<4, ICP_OCC>, ICP_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_icp<8, ICP_OCC>, ICP_THREADS, 0);
+  }
   int per_sm = a < b ? a : b;
   per_sm = per_sm < c ? per_sm : c;
-  const int v = per_sm * ctx->num_sms;
-  if (dev >= 0 && dev < 64) cached[dev].store(v, std::memory_order_relaxed);
+  const int v = (kind ? per_sm * 3 / 4 : per_sm) * ctx->num_sms;
+  if (dev >= 0 && dev < 64) cached[dev][kind].store(v, std::memory_order_relaxed);
   return v;
 }
 
@@ -512,6 +531,7 @@ int icp_pick_group(const rtr_context* ctx, long long total_pts, int blocks) {
   return per_block <= 128 ? 8 : (per_block <= 1024 ? 4 : 2);
 }
 
+template <int OCC>
 static rtr_status launch_icp(int G, const IcpDev* d_probs, const int* d_blk2prob, int blocks, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
@@ -524,11 +544,11 @@ static rtr_status launch_icp(int G, const IcpDev* d_probs, const int* d_blk2prob
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (G == 2)
-    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<2>, d_probs, d_blk2prob));
+    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<2, OCC>, d_probs, d_blk2prob));
   else if (G == 4)
-    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<4>, d_probs, d_blk2prob));
+    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<4, OCC>, d_probs, d_blk2prob));
   else
-    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<8>, d_probs, d_blk2prob));
+    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<8, OCC>, d_probs, d_blk2prob));
   RTR_LAUNCHED(1);
   return RTR_OK;
 }
@@ -647,7 +667,9 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
   RTR_CUDA(cudaGetLastError());
   long long total = 0;
   for (int i = 0; i < M; ++i) total += specs[i].dev.n_src;
-  return launch_icp(icp_pick_group(ctx, total, used), d_probs, d_b2p, used, st);
+  const int G = icp_pick_group(ctx, total, used);
+  return ctx->worker ? launch_icp<ICP_OCC_WORKER>(G, d_probs, d_b2p, used, st)
+                     : launch_icp<ICP_OCC>(G, d_probs, d_b2p, used, st);
 }
 
 }  // namespace rtr
