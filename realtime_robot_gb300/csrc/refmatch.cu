@@ -101,11 +101,6 @@ __device__ __forceinline__ void oct_define(OctBox& b, const float lo[3], const f
   b.depth = d;
 }
 
-__device__ __forceinline__ bool oct_outside(const OctBox& b, float x, float y, float z) {
-  return (double)x < b.mn[0] || (double)y < b.mn[1] || (double)z < b.mn[2] || (double)x >= b.mx[0] ||
-         (double)y >= b.mx[1] || (double)z >= b.mx[2];
-}
-
 // Grow until (x, y, z) fits; false past REF_MAX_DEPTH levels.
 __device__ bool oct_fit(OctBox& b, float x, float y, float z, double res) {
   const float p[3] = {x, y, z};
@@ -242,6 +237,26 @@ __device__ __forceinline__ void eye4(float* M) {
   for (int i = 0; i < 16; ++i) M[i] = (i % 5) == 0 ? 1.f : 0.f;
 }
 
+// A keypoint's cube for its CTA: worked out by one warp (FP64 is charged per
+// warp instruction, a division some 20 of them; with every warp defining the
+// cube and dividing for every key the occupancy of 573 keypoints took 86 us a
+// pass, 14 us so), keys from floats where they are certain.
+struct OctShared {
+  OctBox b;
+  OctBoxF f;
+};
+__device__ __forceinline__ void oct_share(OctShared& s, const float lo[3], const float hi[3], float res) {
+  if (threadIdx.x < 32) {
+    OctBox b;
+    oct_define(b, lo, hi, (double)res);
+    if (threadIdx.x == 0) {
+      s.b = b;
+      oct_float(b, s.f);
+    }
+  }
+  __syncthreads();
+}
+
 __device__ __forceinline__ bool in_box(float4 p, const float lo[3], const float hi[3]) {
   return p.x >= lo[0] && p.y >= lo[1] && p.z >= lo[2] && p.x <= hi[0] && p.y <= hi[1] && p.z <= hi[2];
 }
@@ -264,20 +279,23 @@ __global__ void __launch_bounds__(OCC_NT) k_ref_occ(const float4* __restrict__ c
   const float lo[3] = {__fsub_rn(kp.x, half), __fsub_rn(kp.y, half), __fsub_rn(kp.z, half)};
   const float hi[3] = {__fadd_rn(kp.x, half), __fadd_rn(kp.y, half), __fadd_rn(kp.z, half)};
   if (!fill) {
-    OctBox b;
-    oct_define(b, lo, hi, (double)res);
+    __shared__ OctShared s_box;
+    for (int i = tid; i < 1024; i += OCC_NT) s_bm[i] = 0u;
+    oct_share(s_box, lo, hi, res);
+    const OctBox& b = s_box.b;
+    const OctBoxF bf = s_box.f;
+    const float inv = __fdiv_rn(1.f, res);
     const bool deep = b.depth > REF_OCC_DEPTH;
     if (deep && tid == 0) atomicOr(err, REF_ERR_DEPTH);
-    for (int i = tid; i < 1024; i += OCC_NT) s_bm[i] = 0u;
-    __syncthreads();
     int c = 0;
     for (int i = tid; i < n; i += OCC_NT) {
       const float4 p = cloud[i];
       if (!in_box(p, lo, hi)) continue;
       ++c;
       if (deep) continue;
-      const unsigned long long m = morton3(oct_key1(b, p.x, 0, (double)res), oct_key1(b, p.y, 1, (double)res),
-                                           oct_key1(b, p.z, 2, (double)res), b.depth);
+      const unsigned long long m =
+          morton3(oct_key_f(b, bf, p.x, 0, (double)res, inv), oct_key_f(b, bf, p.y, 1, (double)res, inv),
+                  oct_key_f(b, bf, p.z, 2, (double)res, inv), b.depth);
       atomicOr(&s_bm[(unsigned)(m >> 5)], 1u << (unsigned)(m & 31ull));
     }
     __syncthreads();
@@ -335,8 +353,12 @@ __global__ void __launch_bounds__(OCC_NT) k_ref_tdf_cells(const float4* __restri
   const float4 kp = keys[k];
   const float lo[3] = {__fsub_rn(kp.x, half), __fsub_rn(kp.y, half), __fsub_rn(kp.z, half)};
   const float hi[3] = {__fadd_rn(kp.x, half), __fadd_rn(kp.y, half), __fadd_rn(kp.z, half)};
-  OctBox b;
-  oct_define(b, lo, hi, (double)res);
+  __shared__ OctShared s_box;
+  __shared__ int s_ix[3][1 << REF_OCC_DEPTH];  // the field coordinate of a leaf's key
+  oct_share(s_box, lo, hi, res);
+  const OctBox& b = s_box.b;
+  const OctBoxF bf = s_box.f;
+  const float inv = __fdiv_rn(1.f, res);
   if (b.depth > REF_OCC_DEPTH) {
     if (tid == 0) {
       atomicOr(err, REF_ERR_DEPTH);
@@ -344,18 +366,24 @@ __global__ void __launch_bounds__(OCC_NT) k_ref_tdf_cells(const float4* __restri
     }
     return;
   }
+  if (fill && tid < 3 << REF_OCC_DEPTH) {
+    const int a = tid >> REF_OCC_DEPTH;
+    const float c = oct_centre(b, (unsigned)(tid & ((1 << REF_OCC_DEPTH) - 1)), a, (double)res);
+    s_ix[a][tid & ((1 << REF_OCC_DEPTH) - 1)] = __double2int_rz(__ddiv_rn(__dsub_rn((double)c, (double)lo[a]), (double)res));
+  }
   for (int i = tid; i < 1024; i += OCC_NT) s_bm[i] = 0u;
   __syncthreads();
   const int beg = offsets[k], end = offsets[k + 1];
   bool grew = false;
   for (int j = beg + tid; j < end; j += OCC_NT) {
     const float4 p = cloud[indices[j]];
-    if (oct_outside(b, p.x, p.y, p.z)) {
+    if (oct_outside_f(bf, p.x, p.y, p.z)) {
       grew = true;
       continue;
     }
-    const unsigned long long m = morton3(oct_key1(b, p.x, 0, (double)res), oct_key1(b, p.y, 1, (double)res),
-                                         oct_key1(b, p.z, 2, (double)res), b.depth);
+    const unsigned long long m =
+        morton3(oct_key_f(b, bf, p.x, 0, (double)res, inv), oct_key_f(b, bf, p.y, 1, (double)res, inv),
+                oct_key_f(b, bf, p.z, 2, (double)res, inv), b.depth);
     atomicOr(&s_bm[(unsigned)(m >> 5)], 1u << (unsigned)(m & 31ull));
   }
   if (grew) atomicOr(err, REF_ERR_GROW);
@@ -400,10 +428,7 @@ __global__ void __launch_bounds__(OCC_NT) k_ref_tdf_cells(const float4* __restri
         const unsigned kk[3] = {kx, ky, kz};
         int* o = occ + 3 * (size_t)(out0 + rank - 1);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const float c = oct_centre(b, kk[a], a, (double)res);
-          o[a] = __double2int_rz(__ddiv_rn(__dsub_rn((double)c, (double)lo[a]), (double)res));
-        }
+        for (int a = 0; a < 3; ++a) o[a] = s_ix[a][kk[a]];
       }
       ++rank;
     }
