@@ -12,6 +12,7 @@
 // in FP64 (pose.cuh) and publishes it to the others.  Every wait is bounded by
 // a clock64 budget; a block that runs out writes RTR_ERR_TIMEOUT and leaves.
 #include <math.h>
+#include <algorithm>
 #include <atomic>
 #include <string.h>
 
@@ -75,17 +76,30 @@ __device__ __forceinline__ float centre_of(const GridMeta* m, int a) {
 //   2. G lanes per queued point: the search (grid_nn1_from), starting from
 //      the last neighbour; a queue keeps every lane busy where single points
 //      scattered over the warps would hold up 32 lanes each;
-//   3. a thread per point: the sums.
+//   3. S lanes per point, 16 / S of the sums each.
 // A search per point and iteration, each from the full bound, was over half of
 // the kernel.  Per iteration of block 0, matching and sums before and now: two
 // 20k chairs 25 and 8 us; 102k points against a 285k-point frame 35 and 10 us;
 // 16 refinements of a 9.2k-voxel model in a room 24 and 10 us.
-template <int G, int OCC>  // lanes cooperating on one source point's 1-NN search; blocks wanted an SM
+//
+// The sums.  Which points a block owns, and the order and the tree in which
+// they are added, depend on n, the number of blocks and S alone: point l of a
+// pass goes to the same S lanes however the matching is run.  A compensated
+// sum in another order differs in its last bits (1e-14), and where a pose's
+// small entries are rounded to FP32 for the next iteration that now and then
+// becomes an ulp, 1e-8 of the result; so a change of the matching, its lanes
+// or its queue leaves every bit of the sums where it was.
+// (Runs of eight points, mixed best over the blocks, and a thread per point's
+// sums gain nothing: two 20k chairs 1,227 us, 1,197 so; 102k points against a
+// 285k-point frame 1,105 and 1,120; 64 pairs 26.3 ms and 25.5.)
+// G: lanes cooperating on one source point's 1-NN search; S: lanes sharing a
+// point's sums (icp_pick_sum_lanes); OCC: blocks wanted an SM
+template <int G, int S, int OCC>
 __global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restrict__ probs,
                                                         const int* __restrict__ blk2prob) {
   const IcpDev& a = probs[blk2prob[blockIdx.x]];
   const int lb = (int)blockIdx.x - a.blk0;
-  __shared__ float s_red[ICP_WARPS][ICP_NV][2];
+  __shared__ float s_red[ICP_WARPS][ICP_NV][2], s_blk[2 * ICP_WARPS][ICP_NV][2];
   __shared__ int s_cnt[ICP_WARPS];
   __shared__ double s_sum[ICP_NV];
   __shared__ float s_T[12];
@@ -117,12 +131,14 @@ __global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restri
   float mag = 0.f;  // the size of the source's coordinates
 #pragma unroll
   for (int k = 0; k < 3; ++k) mag += fmaxf(fabsf(box_lo(a.src_meta, k)), fabsf(box_hi(a.src_meta, k)));
-  // point l of this block: groups of 8 points (whole lines) dealt out to the
-  // blocks in turn, which mixes regions with and without neighbours
-  const int groups = (a.n_src + 7) / 8;
-  const int n_loc = lb < groups ? ((groups - lb + B - 1) / B) * 8 : 0;
-  auto point_of = [&](int l) { return ((l >> 3) * B + lb) * 8 + (l & 7); };
-  const int lg = lane & (G - 1);
+  // point l of this block: runs of PPB points dealt out to the blocks in turn
+  constexpr int PPB = ICP_THREADS / S;  // points a block sums side by side
+  constexpr int NVL = ICP_NV / S;       // sums kept per lane
+  static_assert(ICP_CHUNK % PPB == 0, "a chunk is a whole number of passes of the sums");
+  const int groups = (a.n_src + PPB - 1) / PPB;
+  const int n_loc = lb < groups ? ((groups - lb + B - 1) / B) * PPB : 0;
+  auto point_of = [&](int l) { return ((l / PPB) * B + lb) * PPB + (l & (PPB - 1)); };
+  const int lg = lane & (G - 1), ls = lane & (S - 1);
   const unsigned gmask = ((1u << G) - 1u) << (lane & ~(G - 1));
 
   const bool prof0 = a.prof != nullptr && lb == 0 && tid == 0;
@@ -139,8 +155,10 @@ __global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restri
     const float4 cp = xform_exact(T, cs);
     // rounding of the search, and of a point's position then and now
     const float margin = bv.margin + 2.0e-6f * (mag + fabsf(T[3]) + fabsf(T[7]) + fabsf(T[11]));
-    float run_s = 0.f, run_c = 0.f;  // thread v < 16: the block's sum of value v so far
-    int run_n = 0;
+    KSum acc[NVL];  // values ls * NVL ... of the points tid / S, tid / S + PPB, ... in that order
+#pragma unroll
+    for (int k = 0; k < NVL; ++k) acc[k].init();
+    int cnt = 0;
     for (int c0 = 0; c0 < n_loc; c0 += ICP_CHUNK) {
       const int cn = min(ICP_CHUNK, n_loc - c0);
       if (c0 > 0) __syncthreads();  // the last chunk's places are free
@@ -198,83 +216,92 @@ __global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restri
       }
       __syncthreads();
       // 3. the sums: dp 0-2, dq 3-5, dp dq^T 6-14, d^2 15
-      KSum acc[ICP_NV];
-#pragma unroll
-      for (int k = 0; k < ICP_NV; ++k) acc[k].init();
-      int cnt = 0;
-      for (int l = tid; l < cn; l += ICP_THREADS) {
+      for (int l = tid / S; l < cn; l += PPB) {
         const int i = point_of(c0 + l), pos = s_pos[l];
-        if (i >= a.n_src) continue;
+        if (i >= a.n_src) break;  // and all after it
         if (pos >= 0) {
           const float4 p = xform_exact(T, a.src[i]), q = g.pts[pos];
           const float dp[3] = {__fsub_rn(p.x, cp.x), __fsub_rn(p.y, cp.y), __fsub_rn(p.z, cp.z)};
           const float dq[3] = {__fsub_rn(q.x, c[0]), __fsub_rn(q.y, c[1]), __fsub_rn(q.z, c[2])};
+          float val[ICP_NV];
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
-            acc[k].add(dp[k]);
-            acc[3 + k].add(dq[k]);
+            val[k] = dp[k];
+            val[3 + k] = dq[k];
 #pragma unroll
-            for (int m = 0; m < 3; ++m) acc[6 + 3 * k + m].add(__fmul_rn(dp[k], dq[m]));
+            for (int m = 0; m < 3; ++m) val[6 + 3 * k + m] = __fmul_rn(dp[k], dq[m]);
           }
-          acc[15].add(dist2_exact(p, q));
+          val[15] = dist2_exact(p, q);
+#pragma unroll
+          for (int k = 0; k < NVL; ++k) {
+            float x = val[k];
+#pragma unroll
+            for (int o = 1; o < S; ++o)
+              if (ls == o) x = val[o * NVL + k];
+            acc[k].add(x);
+          }
           ++cnt;
         }
-        if (a.trace_corr)
+        if (a.trace_corr && ls == 0)
           a.trace_corr[(size_t)it * (size_t)a.n_src + (size_t)(a.src_idx ? a.src_idx[i] : i)] =
               pos >= 0 ? pt_index(g.pts[pos]) : -1;
       }
-      // compensated sums over the warp, halving the values a lane
-      // holds with each exchange (lane bit 4 keeps values 0-7 or 8-15, ...), so
-      // 16 combinations a lane instead of 80; lane l ends with value l / 2
-      {
-        float s[ICP_NV], e[ICP_NV];
-#pragma unroll
-        for (int k = 0; k < ICP_NV; ++k) {
-          s[k] = acc[k].s;
-          e[k] = acc[k].c;
-        }
-#pragma unroll
-        for (int off = 16, nv = ICP_NV / 2; off >= 2; off >>= 1, nv >>= 1) {
-          const bool up = (lane & off) != 0;
-#pragma unroll
-          for (int k = 0; k < nv; ++k) {
-            const float ks = up ? s[k + nv] : s[k], ke = up ? e[k + nv] : e[k];
-            const float os = __shfl_xor_sync(0xffffffffu, up ? s[k] : s[k + nv], off);
-            const float oe = __shfl_xor_sync(0xffffffffu, up ? e[k] : e[k + nv], off);
-            float t, err;
-            two_sum(ks, os, t, err);
-            s[k] = t;
-            e[k] = __fadd_rn(__fadd_rn(ke, oe), err);
-          }
-        }
-        const float os = __shfl_xor_sync(0xffffffffu, s[0], 1), oe = __shfl_xor_sync(0xffffffffu, e[0], 1);
-        float t, err;
-        two_sum(s[0], os, t, err);
-        if ((lane & 1) == 0) {
-          s_red[warp][lane >> 1][0] = t;
-          s_red[warp][lane >> 1][1] = __fadd_rn(__fadd_rn(e[0], oe), err);
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-      if (lane == 0) s_cnt[warp] = cnt;
-      __syncthreads();
-      if (tid < ICP_NV) {
-        for (int w = 0; w < ICP_WARPS; ++w) {
-          float t, e;
-          two_sum(run_s, s_red[w][tid][0], t, e);
-          run_s = t;
-          run_c = __fadd_rn(__fadd_rn(run_c, s_red[w][tid][1]), e);
-        }
-      }
-      if (tid == 0)
-        for (int w = 0; w < ICP_WARPS; ++w) run_n += s_cnt[w];
     }
+    // compensated sums over the warp's points, halving the values a lane holds
+    // with each exchange (lane bit 4 keeps the lower or the upper half, ...):
+    // the tree of offsets 16 ... S over all values, at NVL combinations a lane
+    {
+      float s[NVL], e[NVL];
+      int v = ls * NVL;  // the value this lane ends with
+#pragma unroll
+      for (int k = 0; k < NVL; ++k) {
+        s[k] = acc[k].s;
+        e[k] = acc[k].c;
+      }
+#pragma unroll
+      for (int off = 16, nv = NVL / 2; nv >= 1; off >>= 1, nv >>= 1) {
+        const bool up = (lane & off) != 0;
+        if (up) v += nv;
+#pragma unroll
+        for (int k = 0; k < nv; ++k) {
+          const float ks = up ? s[k + nv] : s[k], ke = up ? e[k + nv] : e[k];
+          const float os = __shfl_xor_sync(0xffffffffu, up ? s[k] : s[k + nv], off);
+          const float oe = __shfl_xor_sync(0xffffffffu, up ? e[k] : e[k + nv], off);
+          float t, err;
+          two_sum(ks, os, t, err);
+          s[k] = t;
+          e[k] = __fadd_rn(__fadd_rn(ke, oe), err);
+        }
+      }
+      const float os = __shfl_xor_sync(0xffffffffu, s[0], S), oe = __shfl_xor_sync(0xffffffffu, e[0], S);
+      float t, err;
+      two_sum(s[0], os, t, err);
+      if ((lane & S) == 0) {
+        s_red[warp][v][0] = t;
+        s_red[warp][v][1] = __fadd_rn(__fadd_rn(e[0], oe), err);
+      }
+    }
+    cnt = ls == 0 ? cnt : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+    if (lane == 0) s_cnt[warp] = cnt;
+    __syncthreads();
     if (tid < ICP_NV) {
-      a.partial[lb * 32 + tid] = run_s;
-      a.partial[lb * 32 + ICP_NV + tid] = run_c;
+      float s = s_red[0][tid][0], cc = s_red[0][tid][1];
+      for (int w = 1; w < ICP_WARPS; ++w) {
+        float t, e;
+        two_sum(s, s_red[w][tid][0], t, e);
+        s = t;
+        cc = __fadd_rn(__fadd_rn(cc, s_red[w][tid][1]), e);
+      }
+      a.partial[lb * 32 + tid] = s;
+      a.partial[lb * 32 + ICP_NV + tid] = cc;
     }
-    if (tid == 0) a.pcount[lb] = run_n;
+    if (tid == 0) {
+      int tot = 0;
+      for (int w = 0; w < ICP_WARPS; ++w) tot += s_cnt[w];
+      a.pcount[lb] = tot;
+    }
     __syncthreads();
     if (tid == 0) {
       if (prof0) {
@@ -293,12 +320,13 @@ __global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restri
       // Cross-block reduction.  GB300 issues one FP64 warp-instruction per ~16
       // SM cycles, so the tree runs on compensated FP32 pairs (TwoSum, ~48-bit
       // significand) and FP64 closes it: one (double)hi + (double)lo per value.
-      // Thread (k, v) adds value v of blocks k, k + 16, ... (in that order, ten
-      // blocks' loads in flight, whole lines), then k is reduced away.
+      // 32 sums of every 32nd block (thread (k, v): value v of those of k and of
+      // k + 16, in order; ten blocks' loads in flight, whole lines), then a tree
+      // of offsets 16, 8, 4, 2, 1 over them.
       {
         constexpr int KG = ICP_THREADS / ICP_NV;
         const int v = tid & (ICP_NV - 1), kg = tid / ICP_NV;
-        float hs = 0.f, ls = 0.f;
+        float hs[2] = {0.f, 0.f}, lo[2] = {0.f, 0.f};
         int nloc = 0;
         for (int b0 = kg; b0 < B; b0 += 10 * KG) {
           float h[10], l[10];
@@ -312,35 +340,40 @@ __global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restri
 #pragma unroll
           for (int u = 0; u < 10; ++u) {
             float t, e;
-            two_sum(hs, h[u], t, e);
-            hs = t;
-            ls = __fadd_rn(__fadd_rn(ls, l[u]), e);
+            two_sum(hs[u & 1], h[u], t, e);
+            hs[u & 1] = t;
+            lo[u & 1] = __fadd_rn(__fadd_rn(lo[u & 1], l[u]), e);
           }
         }
-        {
-          const float os = __shfl_xor_sync(0xffffffffu, hs, 16), ol = __shfl_xor_sync(0xffffffffu, ls, 16);
-          float t, e;
-          two_sum(hs, os, t, e);
-          hs = t;
-          ls = __fadd_rn(__fadd_rn(ls, ol), e);
-        }
+        float t, e;
+        two_sum(hs[0], hs[1], t, e);
+        s_blk[kg][v][0] = t;
+        s_blk[kg][v][1] = __fadd_rn(__fadd_rn(lo[0], lo[1]), e);
         nloc += __shfl_xor_sync(0xffffffffu, nloc, 16);
-        if (lane < ICP_NV) {
-          s_red[warp][lane][0] = hs;
-          s_red[warp][lane][1] = ls;
-        }
         if (lane == 0) s_cnt[warp] = nloc;
       }
       __syncthreads();
       if (warp == 0) {
-        float hs = s_red[0][lane & (ICP_NV - 1)][0], ls = s_red[0][lane & (ICP_NV - 1)][1];
-        for (int w = 1; w < ICP_WARPS; ++w) {
-          float t, e;
-          two_sum(hs, s_red[w][lane & (ICP_NV - 1)][0], t, e);
-          hs = t;
-          ls = __fadd_rn(__fadd_rn(ls, s_red[w][lane & (ICP_NV - 1)][1]), e);
+        const int v = lane & (ICP_NV - 1), odd = lane / ICP_NV;
+        float h[ICP_WARPS], l[ICP_WARPS];
+#pragma unroll
+        for (int j = 0; j < ICP_WARPS; ++j) {
+          h[j] = s_blk[odd + 2 * j][v][0];
+          l[j] = s_blk[odd + 2 * j][v][1];
         }
-        if (lane < ICP_NV) s_sum[lane] = (double)hs + (double)ls;
+#pragma unroll
+        for (int off = ICP_WARPS / 2; off > 0; off >>= 1)
+#pragma unroll
+          for (int j = 0; j < off; ++j) {
+            float t, e;
+            two_sum(h[j], h[j + off], t, e);
+            h[j] = t;
+            l[j] = __fadd_rn(__fadd_rn(l[j], l[j + off]), e);
+          }
+        float hs, e;
+        two_sum(h[0], __shfl_xor_sync(0xffffffffu, h[0], 16), hs, e);
+        const float lo = __fadd_rn(__fadd_rn(l[0], __shfl_xor_sync(0xffffffffu, l[0], 16)), e);
+        if (lane < ICP_NV) s_sum[lane] = (double)hs + (double)lo;
         __syncwarp();
       }
       if (a.prof && tid == 0) atomicAdd(a.prof + 4, icp_timer() - t_s0);
@@ -486,6 +519,18 @@ __global__ void __launch_bounds__(256) k_gather_pts(const float4* __restrict__ p
 // ms with two, 20.4 with four, 21.8 with the share below).
 constexpr int ICP_OCC = 2, ICP_OCC_WORKER = 4;
 
+template <int G, int S, int OCC>
+static int icp_per_sm_of() {
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_icp<G, S, OCC>, ICP_THREADS, 0);
+  return n;
+}
+template <int OCC>
+static int icp_per_sm() {
+  return std::min(std::min(icp_per_sm_of<2, 2, OCC>(), icp_per_sm_of<4, 2, OCC>()),
+                  std::min(icp_per_sm_of<4, 4, OCC>(), icp_per_sm_of<8, 8, OCC>()));
+}
+
 // Co-resident blocks of the ICP kernel (the smallest over the group sizes,
 // so a plan made for one group size fits every variant).  Workers run beside
 // each other's groupings, whose blocks take half an SM's registers, an ICP
@@ -500,18 +545,7 @@ int icp_max_blocks(rtr_context* ctx) {
     const int v = cached[dev][kind].load(std::memory_order_relaxed);
     if (v > 0) return v;
   }
-  int a = 0, b = 0, c = 0;
-  if (kind) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_icp<2, ICP_OCC_WORKER>, ICP_THREADS, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icp<4, ICP_OCC_WORKER>, ICP_THREADS, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_icp<8, ICP_OCC_WORKER>, ICP_THREADS, 0);
-  } else {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_icp<2, ICP_OCC>, ICP_THREADS, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_icp<4, ICP_OCC>, ICP_THREADS, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_icp<8, ICP_OCC>, ICP_THREADS, 0);
-  }
-  int per_sm = a < b ? a : b;
-  per_sm = per_sm < c ? per_sm : c;
+  const int per_sm = kind ? icp_per_sm<ICP_OCC_WORKER>() : icp_per_sm<ICP_OCC>();
   const int v = (kind ? per_sm * 3 / 4 : per_sm) * ctx->num_sms;
   if (dev >= 0 && dev < 64) cached[dev][kind].store(v, std::memory_order_relaxed);
   return v;
@@ -531,8 +565,19 @@ int icp_pick_group(const rtr_context* ctx, long long total_pts, int blocks) {
   return per_block <= 128 ? 8 : (per_block <= 1024 ? 4 : 2);
 }
 
+// Lanes that share a point's sums: 8, 4 or 2, the most with which a block takes
+// at most four passes over its points (the tuning override sets both).  The
+// search's lanes are the same or more, so four pairs are compiled.
+static int icp_pick_sum_lanes(const rtr_context* ctx, long long total_pts, int blocks) {
+  const int t = ctx->tune_icp_group;
+  if (t == 2 || t == 4 || t == 8) return t;
+  const long long lanes = (long long)blocks * ICP_THREADS;
+  if (total_pts * 8 <= 4 * lanes) return 8;
+  return total_pts * 4 <= 4 * lanes ? 4 : 2;
+}
+
 template <int OCC>
-static rtr_status launch_icp(int G, const IcpDev* d_probs, const int* d_blk2prob, int blocks, cudaStream_t st) {
+static rtr_status launch_icp(int G, int S, const IcpDev* d_probs, const int* d_blk2prob, int blocks, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(ICP_THREADS);
@@ -543,12 +588,14 @@ static rtr_status launch_icp(int G, const IcpDev* d_probs, const int* d_blk2prob
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (G == 2)
-    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<2, OCC>, d_probs, d_blk2prob));
+  if (S == 8)  // then G is 8 too
+    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<8, 8, OCC>, d_probs, d_blk2prob));
+  else if (S == 4)
+    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<4, 4, OCC>, d_probs, d_blk2prob));
   else if (G == 4)
-    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<4, OCC>, d_probs, d_blk2prob));
+    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<4, 2, OCC>, d_probs, d_blk2prob));
   else
-    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<8, OCC>, d_probs, d_blk2prob));
+    RTR_CUDA(cudaLaunchKernelEx(&cfg, k_icp<2, 2, OCC>, d_probs, d_blk2prob));
   RTR_LAUNCHED(1);
   return RTR_OK;
 }
@@ -667,9 +714,9 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
   RTR_CUDA(cudaGetLastError());
   long long total = 0;
   for (int i = 0; i < M; ++i) total += specs[i].dev.n_src;
-  const int G = icp_pick_group(ctx, total, used);
-  return ctx->worker ? launch_icp<ICP_OCC_WORKER>(G, d_probs, d_b2p, used, st)
-                     : launch_icp<ICP_OCC>(G, d_probs, d_b2p, used, st);
+  const int G = icp_pick_group(ctx, total, used), S = icp_pick_sum_lanes(ctx, total, used);
+  return ctx->worker ? launch_icp<ICP_OCC_WORKER>(G, S, d_probs, d_b2p, used, st)
+                     : launch_icp<ICP_OCC>(G, S, d_probs, d_b2p, used, st);
 }
 
 }  // namespace rtr

@@ -163,7 +163,7 @@ def test_pose_inliers_equals_oracle(ctx, rtr):
 
 
 @pytest.mark.parametrize("n_src,n_tgt,max_dist,cell,shift", [
-    (7, 50, 0.05, 0.0, 0.0),        # one group of 8 points, most blocks idle
+    (7, 50, 0.05, 0.0, 0.0),        # few points: most blocks idle
     (4099, 3001, 0.02, 0.03, 0.03),  # most points without a neighbour at first
     (4099, 3001, 0.3, 0.0, 0.1),    # a bound far beyond the neighbours' distance
     (2500, 2500, 0.0, 0.0, 0.0),    # no bound
@@ -227,3 +227,38 @@ def test_recognition_refines_alike_without_room_for_the_matching_state(rtr):
     for x, y in zip(a["instances"], b["instances"]):
         assert x["hypothesis"] == y["hypothesis"] and x["score"] == y["score"]
         np.testing.assert_allclose(x["pose"], y["pose"], rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("n_src,group", [(3, 0), (31, 0), (33, 8), (257, 2), (20000, 4), (20001, 0), (60007, 0),
+                                         (90011, 0), (700001, 0)])
+def test_icp_sums_keep_every_point_once(ctx, rtr, n_src, group):
+    """The sums' lanes (8, 4 or 2 a point, by the points a block has or by the
+    tuning), ragged last passes and blocks of more than one chunk (2,048
+    points): the first pose equals the FP64 solve of the same FP32 terms to
+    1e-12 (compensated sums hold 2^-45 of the terms' magnitudes, the
+    covariance's condition is below 100)."""
+    src, tgt, _ = rtr.config0_pair(n_src, 20000)
+    rng = np.random.default_rng(n_src)
+    src = src[rng.integers(0, src.shape[0], n_src)].copy()
+    src[:, :3] += rng.normal(0, 0.01, (n_src, 3)).astype(np.float32)
+    ctx.set_tuning("icp_group", group)
+    try:
+        res, tp, tc = ctx.icp(_dev(src), _dev(tgt), 1, 0.0, trace=True)
+        r = ctx.parse_icp_result(res)
+    finally:
+        ctx.set_tuning("icp_group", 0)
+    assert r["status"] == 0 and r["n_corr"] == n_src
+    q = tgt[tc.cpu().numpy()[0], :3]
+    half = np.float32(0.5)
+    cp = half * (src[:, :3].min(0) + src[:, :3].max(0))
+    cq = half * (tgt[:, :3].min(0) + tgt[:, :3].max(0))
+    dp, dq = src[:, :3] - cp, q - cq
+    prod = (dp[:, :, None] * dq[:, None, :]).astype(np.float64)
+    mp, mq = dp.astype(np.float64).mean(0), dq.astype(np.float64).mean(0)
+    U, _, Vt = np.linalg.svd(prod.sum(0) - n_src * np.outer(mp, mq))
+    R = Vt.T @ np.diag([1.0, 1.0, np.sign(np.linalg.det(U @ Vt))]) @ U.T
+    want = np.eye(4)
+    want[:3, :3] = R
+    want[:3, 3] = (mq + cq) - R @ (mp + cp)
+    tol = 1e-12 if n_src > 100 else 1e-9  # a few points: worse conditioned
+    np.testing.assert_allclose(tp.cpu().numpy()[1].reshape(4, 4), want, rtol=0, atol=tol)
