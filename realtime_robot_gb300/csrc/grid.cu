@@ -433,7 +433,9 @@ __device__ __forceinline__ int cell_of(float v, float o, float inv_h) {
 // point's rank in its cell in the order the counts were taken.  Lanes with
 // the same cell are counted by one atomic: points that come in voxel order
 // share cells, and a cell holding the whole cloud would otherwise serialise
-// an atomic per point.
+// an atomic per point.  COUNT false: the cells alone (the ordered form counts
+// them once they are sorted).
+template <bool COUNT>
 __global__ void __launch_bounds__(256) k_grid_count(const float4* __restrict__ pts, int n_host, const int* d_n,
                                                     const GridMeta* __restrict__ m, uint32_t* __restrict__ keys,
                                                     uint32_t* __restrict__ rank, uint32_t* __restrict__ counts) {
@@ -451,6 +453,10 @@ __global__ void __launch_bounds__(256) k_grid_count(const float4* __restrict__ p
       const int cy = clampi(cell_of(p.y, oy, ih), 0, ny - 1);
       const int cz = clampi(cell_of(p.z, oz, ih), 0, nz - 1);
       key = ((uint32_t)cz * (uint32_t)ny + (uint32_t)cy) * (uint32_t)nx + (uint32_t)cx;
+    }
+    if (!COUNT) {
+      if (i < n) keys[i] = key;
+      continue;
     }
     const unsigned peers = __match_any_sync(0xffffffffu, key);
     const int leader = __ffs(peers) - 1;
@@ -563,15 +569,28 @@ __global__ void __launch_bounds__(256) k_grid_scatter(const float4* __restrict__
   }
 }
 
+// Points in sorted order, and the sorted cells counted into the table (which
+// starts zeroed): neighbours share a cell, so there is about an atomic a cell
+// and warp, where counting the points as they come takes an atomic per point
+// of a cloud in random order, many on one word when cells are large (300k
+// points at random in 2,400 cells, grid and 500 queries: 328 -> 310 us).
 __global__ void __launch_bounds__(256) k_grid_gather(const float4* __restrict__ pts,
+                                                     const uint32_t* __restrict__ keys,
                                                      const uint32_t* __restrict__ order, int n_host,
-                                                     const int* d_n, float4* __restrict__ out) {
-  const int n = count_of(n_host, d_n);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t o = order[i];
-    float4 p = pts[o];
-    p.w = __int_as_float((int)o);
-    out[i] = p;
+                                                     const int* d_n, uint32_t* __restrict__ counts,
+                                                     float4* __restrict__ out) {
+  const int n = count_of(n_host, d_n), lane = threadIdx.x & 31;
+  for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += gridDim.x * blockDim.x) {
+    const int i = i0 + lane;
+    const uint32_t key = i < n ? keys[i] : 0xffffffffu;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    if (i < n) {
+      if (lane == __ffs(peers) - 1) atomicAdd(&counts[key], (uint32_t)__popc(peers));
+      const uint32_t o = order[i];
+      float4 p = pts[o];
+      p.w = __int_as_float((int)o);
+      out[i] = p;
+    }
   }
 }
 
@@ -642,18 +661,19 @@ rtr_status grid_build(const GridBufs& b, const float4* pts, int n_host, const in
   const unsigned nt = table_tiles(b.cell_cap);
   RTR_CUDA(cudaMemsetAsync(b.meta, 0, table_bytes(b.cell_cap), st));
   k_bbox<true><<<bbox_blocks(b.n_cap), 256, 0, st>>>(pts, n_host, d_n, b.meta, h_req, b.cell_cap);
-  k_grid_count<<<nb, 256, 0, st>>>(pts, n_host, d_n, b.meta, b.k0, b.v0, b.starts);
-  k_cells_sums<<<nt, CT_BLOCK, 0, st>>>(b.starts, b.meta, b.tiles);
-  k_cells_scan<<<nt, CT_BLOCK, 0, st>>>(b.starts, b.meta, b.tiles);
   if (ordered) {
+    k_grid_count<false><<<nb, 256, 0, st>>>(pts, n_host, d_n, b.meta, b.k0, nullptr, nullptr);
     int bits = 1;
     while (bits < 32 && (1ull << bits) < (unsigned long long)b.cell_cap) ++bits;
     uint32_t *ks, *vs;
     radix_sort_pairs(nullptr, b.k0, b.v0, b.k1, b.v1, b.hist, b.n_cap, n_host, d_n, bits, true, st, &ks, &vs);
-    k_grid_gather<<<nb, 256, 0, st>>>(pts, vs, n_host, d_n, b.pts);
+    k_grid_gather<<<nb, 256, 0, st>>>(pts, ks, vs, n_host, d_n, b.starts, b.pts);
   } else {
-    k_grid_scatter<<<nb, 256, 0, st>>>(pts, b.k0, b.v0, b.starts, n_host, d_n, b.pts);
+    k_grid_count<true><<<nb, 256, 0, st>>>(pts, n_host, d_n, b.meta, b.k0, b.v0, b.starts);
   }
+  k_cells_sums<<<nt, CT_BLOCK, 0, st>>>(b.starts, b.meta, b.tiles);
+  k_cells_scan<<<nt, CT_BLOCK, 0, st>>>(b.starts, b.meta, b.tiles);
+  if (!ordered) k_grid_scatter<<<nb, 256, 0, st>>>(pts, b.k0, b.v0, b.starts, n_host, d_n, b.pts);
   RTR_LAUNCHED(5);
   RTR_CUDA(cudaGetLastError());
   return RTR_OK;
