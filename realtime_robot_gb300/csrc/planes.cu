@@ -472,6 +472,7 @@ __global__ void __launch_bounds__(512) k_pl_hull(const float2* __restrict__ su, 
       return make_float2(ordered_to_float((unsigned)(x >> 32)), ordered_to_float((unsigned)x));
     };
     const int h = pl_half(len, [&](int i) { return at(b + i); }, [&](int i) { return half + b + i; });
+    __syncwarp();  // every lane's run is written: the others read it below (shuffles order no memory)
     // close the runs up (a lane writes at or before its own run, after every
     // lane before it has read)
     int to = h;

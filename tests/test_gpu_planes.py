@@ -102,3 +102,21 @@ def test_plane_hulls_at_their_limits_equal_oracle(ctx, rtr):
     for pts in (disc, lattice, tiny, np.repeat(tiny, 700, 0), np.zeros((64, 4), np.float32), lattice[:1025]):
         ref, _ = O.plane_segment(pts)
         _same(ctx.plane_segment(_dev(pts)), ref)
+
+
+@pytest.mark.parametrize("n", [33, 64, 257, 700, 1023, 1500, 2047])
+def test_plane_hull_from_runs_of_unlike_length(ctx, n):
+    """All n points are hull vertices or nearly so, crowded along the axis that
+    the hull kernel sorts by: of its 32 runs some keep every point in their
+    half chains and some a few, so lanes write runs of very unlike length
+    before they read one another's.  Several clouds of each size."""
+    rng = np.random.default_rng(n)
+    for k in range(6):
+        a = np.sort(2 * np.pi * rng.beta(0.3, 0.6, n))
+        r = 3.0 * np.where(rng.uniform(size=n) < 0.3 * (k % 3), rng.uniform(0.99, 1.0, n), 1.0)
+        pts = np.zeros((n, 4), np.float32)
+        pts[:, 0], pts[:, 1] = r * np.cos(a), (1.0 if k % 2 else 0.01) * r * np.sin(a)
+        ref, _ = O.plane_segment(pts[rng.permutation(n)])
+        got = ctx.plane_segment(_dev(pts[rng.permutation(n)]))
+        assert [s.hull_vertices for s in got] == [s.hull_vertices for s in ref]
+        _same(ctx.plane_segment(_dev(pts)), O.plane_segment(pts)[0])
