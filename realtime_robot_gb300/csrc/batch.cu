@@ -10,8 +10,8 @@
 // replayed, which removes the per-launch host cost of the ~130 kernels of
 // every pair.
 //
-// Each worker's cooperative kernels (grouping, ICP) take 1/workers of the
-// co-resident blocks so they run side by side.  A pair's result is the
+// Each worker's cooperative kernels (grouping, ICP) take a share of the
+// co-resident blocks (coop_share.h) so they run side by side.  A pair's result is the
 // single-call result up to the FP32 rounding of ICP block sums over a
 // different block count.  rtr_batch_autotune picks the worker count and the
 // ICP lanes per point by timing the caller's batch.
@@ -33,7 +33,10 @@ struct rtr_batch_graph {
 
 namespace rtr {
 
-rtr_status batch_ensure_workers(rtr_context* ctx, int n) {
+int gc_blocks_per_sm(int C);
+
+// n workers side by side, scenes of up to max_points points.
+rtr_status batch_ensure_workers(rtr_context* ctx, int n, int max_points) {
   while ((int)ctx->workers.size() < n) {
     rtr_context* w = nullptr;
     RTR_TRY(rtr_context_create(ctx->device, &w));
@@ -41,10 +44,12 @@ rtr_status batch_ensure_workers(rtr_context* ctx, int n) {
   }
   RTR_CUDA(cudaSetDevice(ctx->device));
   if (!ctx->ev_fork) RTR_CUDA(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
+  const int gc_per_sm = n > 1 ? gc_blocks_per_sm(max_points > 0 ? max_points : 1) : 2;
   for (rtr_context* w : ctx->workers) {
     if (!w->ev_fork) RTR_CUDA(cudaEventCreateWithFlags(&w->ev_fork, cudaEventDisableTiming));
     w->worker = true;
-    w->coop_div = n;  // cooperative kernels of the n workers fit the GPU side by side
+    w->coop_div = n;
+    w->coop_gc_per_sm = gc_per_sm;
     w->auto_graph = 0;  // a worker's consecutive pairs differ; whole batches are graphed instead
     w->wait_budget_ms = ctx->wait_budget_ms;
     w->wait_budget_cycles = ctx->wait_budget_cycles;
@@ -66,7 +71,9 @@ int batch_worker_count(const rtr_context* ctx, int n_pairs) {
 static rtr_status enqueue_batch(rtr_context* ctx, const rtr_batch_pair* pairs, int n_pairs, const rtr_recog_params* p,
                                 const rtr_mlp* mlp, float keep, int nw, rtr_recog_result* d_results,
                                 cudaStream_t origin) {
-  RTR_TRY(batch_ensure_workers(ctx, nw));
+  int max_n = 0;
+  for (int i = 0; i < n_pairs; ++i) max_n = std::max(max_n, pairs[i].n);
+  RTR_TRY(batch_ensure_workers(ctx, nw, max_n));
   std::vector<int> order((size_t)n_pairs);
   for (int i = 0; i < n_pairs; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return pairs[a].n > pairs[b].n; });

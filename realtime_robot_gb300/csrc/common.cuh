@@ -100,14 +100,15 @@ struct rtr_context {
   int tune_icp_group = 0;              // lanes per ICP source point (0: automatic)
   size_t scratch_limit = 0;            // largest scratch arena this context may hold (0: no limit)
   int tune_batch_workers = 0;          // workers of rtr_recognize_batch (0: automatic)
-  int coop_div = 1;                    // cooperative grids use 1/coop_div of the GPU
+  int coop_div = 1;                    // workers whose cooperative grids share the GPU (coop_share.h)
+  int coop_gc_per_sm = 2;              // grouping blocks an SM holds, in the largest of the workers' scenes
   bool worker = false;                 // a worker of rtr_recognize_batch / rtr_recognize_multi
   bool grid_sorts = false;             // sorts take a grid of tiles whatever their size (see recognize_impl)
   int tune_gc_window = 0;              // seeds per grouping window (0: automatic)
   int tune_gc_no_lists = 0;            // 1: the grouping keeps no pass lists (every stale set ends a round)
   int tune_gc_inline = 0;              // times a round the grouping walk recomputes sets in place (0: automatic)
   int tune_scene_grid_mm = 0;          // cell edge of the recognition's scene grid (0: 1.5 ICP distances)
-  int tune_normals_grid_mm = 0;        // cell edge of the scene normals' k-NN grid (0: 5 voxel leaves)
+  int tune_normals_grid_mm = 0;        // cell edge of the scene normals' k-NN grid (0: 2 voxel leaves)
   std::vector<rtr_context*> workers;   // child contexts of the batch driver
   cudaEvent_t ev_fork = nullptr;       // fork/join event of the batch driver
   int gc_stats[8] = {};                // last grouping: rounds, walk end, sets, phase us, candidates
@@ -163,7 +164,7 @@ rtr_status side_stream_ready(rtr_context* ctx);
 // Worker contexts of a batch (batch.cu): make sure `n` exist and share the
 // GPU's co-resident blocks; how many a call of `n_items` uses; and their
 // status words after a synchronised batch.
-rtr_status batch_ensure_workers(rtr_context* ctx, int n);
+rtr_status batch_ensure_workers(rtr_context* ctx, int n, int max_points);
 int batch_worker_count(const rtr_context* ctx, int n_items);
 rtr_status batch_check_workers(rtr_context* ctx, int nw);
 

@@ -19,6 +19,7 @@
 // walk); the walk recomputes a set that lost a member in place, or stops there
 // and the next window starts with it.  No host round trip inside the grouping.
 #include "common.cuh"
+#include "coop_share.h"
 #include "pose.cuh"
 #include "grid.cuh"
 
@@ -1412,6 +1413,21 @@ size_t gc_scratch_bytes(int C, int max_clusters) {
   return plan.bytes;
 }
 
+// Blocks of the grouping of up to C correspondences that an SM holds (1 or 2).
+int gc_blocks_per_sm(int C) {
+  const size_t dyn = sizeof(unsigned) * (size_t)((C + 31) / 32);
+  const bool long_sets = gc_set_stride(C) > GC_MAXS;
+  auto kern = long_sets ? k_gc_coop<true> : k_gc_coop<false>;
+  int per_sm = 0;
+  if (dyn > GC_MAX_DYN_SMEM ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GC_MAX_DYN_SMEM) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GC_WARPS * 32, dyn) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  return per_sm >= 2 ? 2 : 1;
+}
+
 // The grouping up to the walk's end, without a host round trip.  C_cap
 // bounds the correspondences; with d_C the live count is read on the device.
 static rtr_status gc_launch(rtr_context* ctx, Scratch& s, const float* d_model_kp, const float* d_scene_kp,
@@ -1462,14 +1478,15 @@ static rtr_status gc_launch(rtr_context* ctx, Scratch& s, const float* d_model_k
   int per_sm = 0;
   RTR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GC_WARPS * 32, dyn));
   if (per_sm < 1) return fail(RTR_ERR_CAPACITY, "rtr_gc_group: grouping kernel does not fit an SM");
-  // enough warps for the work, and a share of the GPU when several contexts run
-  // at once.  A warp holds 32 candidates of the seed tests, so it takes few
+  // enough warps for the work, and a share of the GPU beside other workers.  A warp holds 32 candidates of the seed tests, so it takes few
   // correspondences to use every SM (256 / 128 / 64 / 32 of them a block: a
   // 12k-point segment's recognition 2,007 / 1,947 / 1,933 / 1,912 us, grouping of
   // a 20k-point room 1,011 / 741 / 597 / 553 us)
   int blocks = (per_sm < 2 ? per_sm : 2) * ctx->num_sms;
-  const int div = ctx->coop_div > 0 ? ctx->coop_div : 1;
-  blocks = blocks / div > 0 ? blocks / div : 1;
+  if (ctx->coop_div > 1) {
+    const int share = coop_share(ctx->num_sms, ctx->coop_div, ctx->coop_gc_per_sm).gc;
+    blocks = share > 0 ? share : 1;
+  }
   const int by_work = (C + 31) / 32;
   if (by_work < blocks) blocks = by_work > 4 ? by_work : 4;
   {

@@ -16,6 +16,7 @@
 #include <atomic>
 #include <string.h>
 
+#include "coop_share.h"
 #include "grid.cuh"
 #include "icp.cuh"
 #include "pose.cuh"
@@ -514,9 +515,11 @@ __global__ void __launch_bounds__(256) k_gather_pts(const float4* __restrict__ p
 // Blocks an SM holds of the ICP kernel.  Two with all the registers that the
 // pose solve wants, where one call has the GPU: a solve an iteration is on its
 // critical path (two 20k chairs 1,295 us; 1,571 with three blocks an SM, 1,816
-// with four).  Four, the solve spilling, for the workers of a batch: other
-// pairs fill that wait, and the searches gain from the threads (64 pairs 22.9
-// ms with two, 20.4 with four, 21.8 with the share below).
+// with four).  Four, the solve spilling, for workers side by side: other pairs
+// fill that wait, and the searches gain from the threads (64 pairs with learned
+// pruning 22.8 ms with two and half the SMs' places, 21.1 with four and the
+// shares of coop_share.h, which leave every launch its places; six models in
+// one room the other way, 28.6 and 30.9 ms).
 constexpr int ICP_OCC = 2, ICP_OCC_WORKER = 4;
 
 template <int G, int S, int OCC>
@@ -531,22 +534,20 @@ static int icp_per_sm() {
                   std::min(icp_per_sm_of<4, 4, OCC>(), icp_per_sm_of<8, 8, OCC>()));
 }
 
+// A worker beside others takes the small form (a worker alone has the GPU).
+static bool icp_shared(const rtr_context* ctx) { return ctx->worker && ctx->coop_div > 1; }
+
 // Co-resident blocks of the ICP kernel (the smallest over the group sizes,
-// so a plan made for one group size fits every variant).  Workers run beside
-// each other's groupings, whose blocks take half an SM's registers, an ICP
-// block a quarter: with three quarters of the SMs' capacity shared out, every
-// cooperative launch finds its places however the others' blocks lie (k
-// workers with b = 3 S / n blocks each can make at most k b / 3 of S SMs unfit
-// for a grouping block, and the other SMs hold the other workers' shares).
+// so a plan made for one group size fits every variant).
 int icp_max_blocks(rtr_context* ctx) {
   static std::atomic<int> cached[64][2];  // per device; 0 = not yet known
-  const int dev = ctx->device, kind = ctx->worker ? 1 : 0;
+  const int dev = ctx->device, kind = icp_shared(ctx) ? 1 : 0;
   if (dev >= 0 && dev < 64) {
     const int v = cached[dev][kind].load(std::memory_order_relaxed);
     if (v > 0) return v;
   }
   const int per_sm = kind ? icp_per_sm<ICP_OCC_WORKER>() : icp_per_sm<ICP_OCC>();
-  const int v = (kind ? per_sm * 3 / 4 : per_sm) * ctx->num_sms;
+  const int v = per_sm * ctx->num_sms;
   if (dev >= 0 && dev < 64) cached[dev][kind].store(v, std::memory_order_relaxed);
   return v;
 }
@@ -644,7 +645,8 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
   const int maxb = icp_max_blocks(ctx);
   if (M > maxb) return fail(RTR_ERR_CAPACITY, "icp: %d problems exceed the %d co-resident blocks", M, maxb);
   // a share of the GPU when several contexts run cooperative kernels at once
-  int budget = maxb / (ctx->coop_div > 0 ? ctx->coop_div : 1);
+  int budget = icp_shared(ctx) ? std::min(maxb, coop_share(ctx->num_sms, ctx->coop_div, ctx->coop_gc_per_sm).icp)
+                               : maxb;
   if (budget < M) budget = M;
   IcpDev* d_probs = s.take<IcpDev>(M);
   int* d_b2p = s.take<int>(maxb);
@@ -715,8 +717,8 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
   long long total = 0;
   for (int i = 0; i < M; ++i) total += specs[i].dev.n_src;
   const int G = icp_pick_group(ctx, total, used), S = icp_pick_sum_lanes(ctx, total, used);
-  return ctx->worker ? launch_icp<ICP_OCC_WORKER>(G, S, d_probs, d_b2p, used, st)
-                     : launch_icp<ICP_OCC>(G, S, d_probs, d_b2p, used, st);
+  return icp_shared(ctx) ? launch_icp<ICP_OCC_WORKER>(G, S, d_probs, d_b2p, used, st)
+                         : launch_icp<ICP_OCC>(G, S, d_probs, d_b2p, used, st);
 }
 
 }  // namespace rtr

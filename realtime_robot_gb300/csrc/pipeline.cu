@@ -888,7 +888,7 @@ static rtr_status recognize_multi_impl(rtr_context* ctx, const rtr_model* const*
   }
   RTR_TRY(scene_stages(ctx, s, sb, scene, n, q, mlp, keep, st));
   RTR_CUDA(cudaStreamWaitEvent(st, sb.grid_ready, 0));  // joined before the workers fork
-  RTR_TRY(batch_ensure_workers(ctx, nw));
+  RTR_TRY(batch_ensure_workers(ctx, nw, n));
   ScratchPlan mp;
   model_plan(mp, n, q);
   for (int wi = 0; wi < nw; ++wi) {  // sized before the fork: growing synchronises
