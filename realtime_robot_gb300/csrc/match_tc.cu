@@ -6,8 +6,9 @@
 // lo.hi (three tcgen05.mma per K step), which leaves |err(q.b)| of order
 // 1e-4 |q| |b| (dropped lo.lo, the split's rounding, FP32 accumulation); the
 // certification uses TC_ERR * max(|q|, max |b|)^2, which covers that and the
-// FP32 norms with margin (unit-norm SHOT vectors: 5e-4).  Inf or NaN values
-// make a query uncertified.  Per query the epilogue keeps the 8
+// FP32 norms with margin (unit-norm SHOT vectors: 5e-4).  Inf values, and NaN
+// in a query, make a query uncertified; a database row with a NaN never wins
+// and is left out.  Per query the epilogue keeps the 8
 // smallest approximate distances; an exact FP32 re-rank (sequential sums, as
 // the oracle) picks the winner, and a query is certified when its 8th
 // approximate distance minus the error bound is still above the exact winner,
@@ -223,7 +224,10 @@ __global__ void k_split_bf16(const float* __restrict__ x, int n_host, const int*
     }
     if (lane == 0) {
       norm2[r] = ss;
-      if (max_bits && r < n) atomicMax(max_bits, __float_as_uint(ss));  // ss >= 0 (or NaN: stays largest)
+      // the largest norm (ss >= 0), the scale of the error bound.  A row with a
+      // NaN never wins and is nowhere in the lists: it sets no scale (a maximum
+      // of NaN would leave the bound to the query's norm alone)
+      if (max_bits && r < n && ss == ss) atomicMax(max_bits, __float_as_uint(ss));
       if (zero_row) zero_row[r] = (r < n && !nz) ? 1 : 0;
     }
   }

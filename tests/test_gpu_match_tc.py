@@ -174,3 +174,34 @@ def test_match_tc_database_ranges(ctx, descs, nq, ndb, aligned):
     ri, rd = O.match(q, db)
     assert np.array_equal(idx.cpu().numpy(), ri)
     assert np.array_equal(d2.cpu().numpy(), rd)
+
+
+@pytest.mark.parametrize("bad", [0, 1, 3])
+@pytest.mark.parametrize("nq", [40, 700])
+def test_match_tc_nan_rows_leave_the_error_bound_alone(ctx, nq, bad):
+    """A database row with a NaN never wins, and must not take the error
+    bound's scale (the largest norm) with it: queries of norm 1 against rows
+    of norm 1,000 whose distances differ by parts in a million, far below the
+    16-bit products' error, which only the large norms' bound covers."""
+    import torch
+    rng = np.random.default_rng(nq + bad)
+    u = rng.normal(size=352)
+    u /= np.linalg.norm(u)
+
+    def high(norm):  # how much the two 16-bit parts of -|b|^2 / 2 put a distance too high
+        t = torch.tensor([-0.5 * norm * norm], dtype=torch.float32)
+        h = t.bfloat16().float()
+        return float(2 * (t - h - (t - h).bfloat16().float()))
+    norm = max(np.linspace(1000, 1010, 401), key=high)
+    db = (norm * u + 0.0001 * rng.normal(size=(300, 352))).astype(np.float32)
+    q = rng.normal(size=(nq, 352)).astype(np.float32)
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    big = q[: nq // 2] * np.float32(1000)  # and queries of the rows' norm
+    q[: nq // 2] = big
+    for k in range(bad):
+        db[17 + 90 * k, 5 + k] = np.nan
+    idx, d2 = ctx.match(_dev(q), _dev(db))
+    ri, rd = O.match(q, db)
+    assert np.array_equal(idx.cpu().numpy(), ri)
+    assert np.array_equal(d2.cpu().numpy(), rd)
+    assert not np.isin(ri, [17, 107, 197][:bad]).any()
