@@ -711,13 +711,14 @@ __global__ void __launch_bounds__(NT) k_ref_distance(const float4* __restrict__ 
 // What bounds it: issue (and the shuffle / shared-memory pipe next to it):
 // about 120 instructions per point and rotation, no FP64 among them.  The
 // chip's FP64 rate is low enough that a dozen double operations a rotation
-// cost more than everything else, so the cubes are kept in fixed point
-// (units of 2^-40 m), where the reference's double arithmetic is exact:
+// cost more than everything else, so the cubes are kept in fixed point (a unit
+// that follows the leaf, 2^-40 at 0.01; see RefUnit), where the reference's
+// double arithmetic is exact:
 //  - the bounds of a keypoint's field cube, the leaf edge and FLT_EPSILON are
-//    multiples of the unit and below 2^13 m, so every sum and difference of
-//    the growth rule has at most 53 bits and the doubles are never rounded
+//    multiples of the unit and below 2^53 of them, so every sum and difference
+//    of the growth rule has at most 53 bits and the doubles are never rounded
 //    (k_ref_keybox checks it; keypoints that fail, and clouds beyond
-//    REFW_RANGE leaves of the origin, are left to k_ref_distance);
+//    2^REFW_RANGE_LOG2 leaves of the origin, are left to k_ref_distance);
 //  - a float p >= c (c a whole number of units) exactly when floor(p) >= c;
 //  - a leaf key is floor((p - min) / res): from a float estimate where that is
 //    farther from a whole number than its error, else from whole-number
@@ -738,18 +739,45 @@ __global__ void __launch_bounds__(NT) k_ref_distance(const float4* __restrict__ 
 // read (half the rotations there).
 constexpr int REFW_WARPS = 4;
 constexpr int REFW_MAX = 512;                 // points of the largest cloud taken
-constexpr float REFW_RANGE = 16384.f;         // leaves; coordinates also below 256 m
+constexpr int REFW_RANGE_LOG2 = 17;           // leaves from the origin
+
+// The unit of the fixed point, 2^-e: a leaf has 2^33 .. 2^34 of them, so all 24
+// bits of the resolution are whole units, a coordinate at the end of the
+// range has at most 2^51 and a grown cube's bounds stay below 2^53; the
+// quotient of a point's offset and the leaf then stays 1 / leaf, more than a
+// double's rounding, off the whole numbers it does not meet.  FLT_EPSILON,
+// which the growth rule takes off a cube whatever the leaf, is 2^(e - 23) units
+// (so e is at least 23, with a shorter range) and has to be a small part of a
+// leaf.  A fixed unit of 2^-40 held clouds in metres only: 120 x 400 keypoints,
+// 48,000 pairs, took 1.96 ms in metres and 96 in centimetres or millimetres, a
+// CTA a pair; 1.9 in all three now (kilometres 3.4).
+struct RefUnit {
+  float up, down;  // 2^e, 2^-e
+  float lim;       // largest coordinate taken (negative: none)
+  long long eps;   // FLT_EPSILON in units
+};
+static RefUnit ref_unit(float res) {
+  RefUnit u{1.f, 1.f, -1.f, 0};
+  if (!(res >= 1.0e-6f && res <= 0x1p20f)) return u;
+  int e = 33 - ilogbf(res);
+  if (e < 23) e = 23;
+  u.up = ldexpf(1.f, e);
+  u.down = ldexpf(1.f, -e);
+  u.lim = fminf(ldexpf(res, REFW_RANGE_LOG2), ldexpf(1.f, 51 - e));
+  u.eps = 1ll << (e - 23);
+  return u;
+}
 
 struct RefKeyBox {
-  long long mn[3], mx[3];  // the field cube, 2^-40 m
+  long long mn[3], mx[3];  // the field cube, in units
   float M[6];              // the yaw step about the keypoint: x and y rows, columns 0, 1, 3
   int J[3];                // field coordinate of key k: k + J, truncated toward zero
   int depth, ok, table;    // table: J is not certain, coordinates come from doubles
 };
 
-__device__ __forceinline__ long long to_fix(float x) { return __float2ll_rd(x * 0x1p40f); }
-__device__ __forceinline__ float from_fix_rn(long long v) { return __ll2float_rn(v) * 0x1p-40f; }
-__device__ __forceinline__ float from_fix_ru(long long v) { return __ll2float_ru(v) * 0x1p-40f; }
+__device__ __forceinline__ long long to_fix(float x, const RefUnit& u) { return __float2ll_rd(x * u.up); }
+__device__ __forceinline__ float from_fix_rn(long long v, const RefUnit& u) { return __ll2float_rn(v) * u.down; }
+__device__ __forceinline__ float from_fix_ru(long long v, const RefUnit& u) { return __ll2float_ru(v) * u.down; }
 
 __device__ __forceinline__ float warp_min(float x) {
   float r;
@@ -781,19 +809,19 @@ __device__ __forceinline__ int refw_class(int n, bool table) {  // n <= REFW_MAX
 // Field cube, yaw step and field offsets of every model keypoint; the keys of
 // each size class into list[class][n], their number into cls[class].
 __global__ void k_ref_keybox(const float4* __restrict__ mkeys, const int* __restrict__ moff, int n, float res,
-                             float half, RefRot rot, RefKeyBox* __restrict__ out, int* __restrict__ list,
-                             int* __restrict__ cls) {
+                             float half, RefUnit un, RefRot rot, RefKeyBox* __restrict__ out,
+                             int* __restrict__ list, int* __restrict__ cls) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= n) return;
   const int np = moff[m + 1] - moff[m];
   const float4 km = mkeys[m];
   RefKeyBox k;
   const double dres = (double)res;
-  const float lim = fminf(res * REFW_RANGE, 256.f);
-  bool ok = res <= 0.25f && res >= 1.0e-4f && half <= lim && fabsf(km.x) <= lim && fabsf(km.y) <= lim &&
-            fabsf(km.z) <= lim;  // false for NaN
-  const long long r64 = ok ? to_fix(res) : 1;
-  ok = ok && from_fix_rn(r64) == res;
+  const float lim = un.lim;
+  const double up = (double)un.up, down = (double)un.down;
+  bool ok = half <= lim && fabsf(km.x) <= lim && fabsf(km.y) <= lim && fabsf(km.z) <= lim;  // false for NaN
+  const long long r64 = ok ? to_fix(res, un) : 1;
+  ok = ok && from_fix_rn(r64, un) == res;
   const float lo[3] = {__fsub_rn(km.x, half), __fsub_rn(km.y, half), __fsub_rn(km.z, half)};
   const float hi[3] = {__fadd_rn(km.x, half), __fadd_rn(km.y, half), __fadd_rn(km.z, half)};
   OctBox b;
@@ -804,14 +832,14 @@ __global__ void k_ref_keybox(const float4* __restrict__ mkeys, const int* __rest
     k.mn[a] = k.mx[a] = 0;
     k.J[a] = 0;
     if (!ok) continue;
-    k.mn[a] = __double2ll_rd(b.mn[a] * 0x1p40);
-    k.mx[a] = __double2ll_rd(b.mx[a] * 0x1p40);
-    ok = ok && (double)k.mn[a] * 0x1p-40 == b.mn[a] && (double)k.mx[a] * 0x1p-40 == b.mx[a] &&
-         from_fix_rn(to_fix(lo[a])) == lo[a] && llabs(k.mx[a] - k.mn[a] - (r64 << b.depth)) <= 1ll << 17;
+    k.mn[a] = __double2ll_rd(b.mn[a] * up);
+    k.mx[a] = __double2ll_rd(b.mx[a] * up);
+    ok = ok && (double)k.mn[a] * down == b.mn[a] && (double)k.mx[a] * down == b.mx[a] &&
+         from_fix_rn(to_fix(lo[a], un), un) == lo[a] && llabs(k.mx[a] - k.mn[a] - (r64 << b.depth)) <= un.eps;
     // the field coordinate (centre of leaf k - lo) / res = k + num / (2 res):
     // its whole part is certain while the fraction stays clear of 0 and 1
-    // (rounding moves it by less than 0.05 at REFW_RANGE)
-    const long long num = 2 * (k.mn[a] - to_fix(lo[a])) + r64, den = 2 * r64;
+    // (rounding moves it by less than 0.05 in the range)
+    const long long num = 2 * (k.mn[a] - to_fix(lo[a], un)) + r64, den = 2 * r64;
     long long q = num / den;
     if (q * den > num) --q;
     const long long fr = num - q * den;
@@ -841,15 +869,16 @@ __global__ void k_ref_keybox(const float4* __restrict__ mkeys, const int* __rest
 
 // floor((p - mn) / res) as the reference's doubles give it; est is within a
 // few of it.  p lies in the cube.
-__device__ __forceinline__ int ref_key_exact(float p, long long mn, long long r64, double dres, int est) {
-  const long long P = to_fix(p);
-  if (from_fix_rn(P) == p) {
+__device__ __forceinline__ int ref_key_exact(float p, long long mn, long long r64, double dres, int est,
+                                             const RefUnit& un) {
+  const long long P = to_fix(p, un);
+  if (from_fix_rn(P, un) == p) {
     long long r = P - mn - (long long)est * r64;
     while (r < 0) --est, r += r64;
     while (r >= r64) ++est, r -= r64;
     return est;
   }
-  return (int)__double2uint_rz(__ddiv_rn(__dsub_rn((double)p, (double)mn * 0x1p-40), dres));
+  return (int)__double2uint_rz(__ddiv_rn(__dsub_rn((double)p, (double)mn * (double)un.down), dres));
 }
 
 // Ascending sort of 32 Q words, word i = lane * Q + q: runs of Q sorted in
@@ -946,8 +975,8 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
                         const int* __restrict__ moff, const int* __restrict__ midx, const float* __restrict__ mtdf,
                         const RefKeyBox* __restrict__ boxes, const int* __restrict__ list,
                         const float4* __restrict__ skeys, int ns, const int* __restrict__ pair_m,
-                        const int* __restrict__ pair_s, long long n_items, float res, float half, RefRot rot,
-                        float* __restrict__ score, float* __restrict__ Tout, int* __restrict__ err) {
+                        const int* __restrict__ pair_s, long long n_items, float res, float half, RefUnit un,
+                        RefRot rot, float* __restrict__ score, float* __restrict__ Tout, int* __restrict__ err) {
   constexpr int Q = refw_rows(CLS);
   constexpr bool TABLE = CLS >= 9;
   __shared__ unsigned s_bm[REFW_WARPS][REF_WIN * REF_WIN];  // leaves of a cloud that reads no field value
@@ -975,7 +1004,7 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
     return;
   }
   const RefKeyBox* kb = boxes + m;
-  const float lim = fminf(res * REFW_RANGE, 256.f);
+  const float lim = un.lim;
   const float tx = __fsub_rn(km.x, ks.x), ty = __fsub_rn(km.y, ks.y), tz = __fsub_rn(km.z, ks.z);
   float px[Q], py[Q], pz[Q];
   bool fine = kb->ok != 0;
@@ -1000,7 +1029,7 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
   const float* grid = mtdf + (size_t)m * REF_VOL;
   const double dres = (double)res;
   const float inv = __fdiv_rn(1.f, res);
-  const long long r64 = to_fix(res), eps64 = 1ll << 17;  // FLT_EPSILON = 2^-23
+  const long long r64 = to_fix(res, un), eps64 = un.eps;
   const int ax = lane % 3;                               // this lane's axis
   const long long mn0 = kb->mn[ax], mx0 = kb->mx[ax];
   const int J = kb->J[ax], stride = ax == 0 ? 1 : (ax == 1 ? REF_DIM : REF_DIM * REF_DIM);
@@ -1017,7 +1046,7 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
   // leaf coordinates: y = (p - mn0) / res - 1/2 by one FMA, off by at most
   // 2^-22 (|c| + |y|); rounding it to a whole number gives the leaf (counted
   // from the field cube's corner) unless y is more than `sure` from it
-  const float c_a = -(from_fix_rn(mn0) * inv) - 0.5f;
+  const float c_a = -(from_fix_rn(mn0, un) * inv) - 0.5f;
   const float reach = ((ax == 0 ? fabsf(km.x) : (ax == 1 ? fabsf(km.y) : 0.f)) +
                        (ax == 2 ? fmaxf(fabsf(zmn), fabsf(zmx)) : 1.01f * far)) * inv;
   const float sure = 0.5f - warp_max((2.f * fabsf(c_a) + reach + 2.f) * 0x1p-22f + 2.5e-7f * inv);
@@ -1114,10 +1143,10 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
         // some point decides the growth from close to a whole leaf: the same in
         // whole units of 2^-40 m
         long long mn = mn0, mx = mx0;
-        const long long bmn = to_fix(amn), bmx = to_fix(amx);
+        const long long bmn = to_fix(amn, un), bmx = to_fix(amx, un);
         K = 0, depth = depth0;
         for (int round = 0; !bad && round < 2 * REF_MAX_DEPTH && __any_sync(0xffffffffu, bmn < mn || bmx >= mx); ++round) {
-          const float fmn = from_fix_ru(mn), fmx = from_fix_ru(mx);
+          const float fmn = from_fix_ru(mn, un), fmx = from_fix_ru(mx, un);
           OctBoxF bf;
 #pragma unroll
           for (int a = 0; a < 3; ++a) {
@@ -1138,7 +1167,7 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
           sx = __shfl_sync(0xffffffffu, sx, src);
           sy = __shfl_sync(0xffffffffu, sy, src);
           sz = __shfl_sync(0xffffffffu, sz, src);
-          const long long P = to_fix(ax == 0 ? sx : (ax == 1 ? sy : sz));
+          const long long P = to_fix(ax == 0 ? sx : (ax == 1 ? sy : sz), un);
           while (!bad && __any_sync(0xffffffffu, P < mn || P >= mx)) {
             if (P < mx) {
               mn -= r64 << depth;
@@ -1148,8 +1177,8 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
             mx = mn + (r64 << depth) - eps64;
           }
         }
-        kmn = ref_key_exact(amn, mn, r64, dres, kmn + K) - K;
-        kmx = ref_key_exact(amx, mn, r64, dres, kmx + K) - K;
+        kmn = ref_key_exact(amn, mn, r64, dres, kmn + K, un) - K;
+        kmx = ref_key_exact(amx, mn, r64, dres, kmx + K, un) - K;
       }
       if (bad) break;
       if (__any_sync(0xffffffffu, kmx - kmn >= REF_WIN)) {
@@ -1181,7 +1210,7 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
               const int ba = a == 0 ? b0 : (a == 1 ? b1 : b2);
               const int st = a == 0 ? 1 : (a == 1 ? REF_DIM : REF_DIM * REF_DIM);
               const float lo = __fsub_rn(a == 0 ? km.x : (a == 1 ? km.y : km.z), half);
-              const double dmn = (double)__shfl_sync(0xffffffffu, mn0, a) * 0x1p-40;
+              const double dmn = (double)__shfl_sync(0xffffffffu, mn0, a) * (double)un.down;
 #pragma unroll 1
               for (int l = lane; l < 64; l += 32) {
                 const float e = __double2float_rn(__dadd_rn(__dmul_rn(__dadd_rn((double)(ba + l), 0.5), dres), dmn));
@@ -1247,7 +1276,7 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
             const int ka = __shfl_sync(0xffffffffu, K, a);
             const float pa = a == 0 ? x : (a == 1 ? y : z), ca = a == 0 ? c0 : (a == 1 ? c1 : c2);
             i[a] = 0;
-            if (close) i[a] = ref_key_exact(pa, mna, r64, dres, __float2int_rn(__fmaf_rn(pa, inv, ca)) + ka) - ka;
+            if (close) i[a] = ref_key_exact(pa, mna, r64, dres, __float2int_rn(__fmaf_rn(pa, inv, ca)) + ka, un) - ka;
           }
           bool fresh = false;
           if (close) {
@@ -1306,7 +1335,7 @@ __global__ void __launch_bounds__(32 * REFW_WARPS, refw_blocks(CLS))
       best_i = it;
     }
   }
-  if (bad) {  // past REF_MAX_DEPTH levels (REFW_RANGE keeps clouds far below it)
+  if (bad) {  // past REF_MAX_DEPTH levels (the range keeps clouds below it)
     if (lane == 0) {
       To[15] = __uint_as_float(REFW_REDO);
       atomicAdd(err + 2, 1);
@@ -1645,11 +1674,12 @@ rtr_status rtr_ref_distance(rtr_context* ctx, const float* d_mcloud, const float
   RefKeyBox* boxes = reinterpret_cast<RefKeyBox*>(s.base + o_box);
   int* list = reinterpret_cast<int*>(s.base + o_list);
   const RefRot rot = ref_rot_tables();
+  const RefUnit un = ref_unit(resolution);
   RTR_CUDA(cudaMemsetAsync(err, 0, (3 + REFW_CLASSES) * sizeof(int), st));
   k_ref_max_count<<<(n_model + 255) / 256, 256, 0, st>>>(d_moffsets, n_model, err + 1);
   if (warp_max >= 0)
     k_ref_keybox<<<(n_model + 63) / 64, 64, 0, st>>>(reinterpret_cast<const float4*>(d_mkeys), d_moffsets, n_model,
-                                                     resolution, half_tdf, rot, boxes, list, err + 3);
+                                                     resolution, half_tdf, un, rot, boxes, list, err + 3);
   RTR_LAUNCHED(warp_max >= 0 ? 2 : 1);
   int h[3 + REFW_CLASSES];
   RTR_TRY(ref_read_ints(ctx, err, 3 + REFW_CLASSES, st, h));
@@ -1679,7 +1709,7 @@ rtr_status rtr_ref_distance(rtr_context* ctx, const float* d_mcloud, const float
     const long long items = all ? (long long)h[3 + (c)] * n_scan : n_pairs;                                          \
     k_ref_distance_warp<c><<<(unsigned)((items + REFW_WARPS - 1) / REFW_WARPS), 32 * REFW_WARPS, 0, st>>>(           \
         mc, mk, d_moffsets, d_mindices, d_mtdf, boxes, list + (size_t)(c) * n_model, sk, n_scan, d_pair_m, d_pair_s, \
-        items, resolution, half_tdf, rot, d_score, d_T, err);                                                        \
+        items, resolution, half_tdf, un, rot, d_score, d_T, err);                                                        \
     RTR_LAUNCHED(1);                                                                                                 \
   }
   REF_WARP_CLASS(10)

@@ -215,3 +215,58 @@ def test_distance_without_room_for_its_tables(rtr):
             c.close()
     assert np.array_equal(res[0][0], res[1][0], equal_nan=True)
     assert np.array_equal(res[0][1], res[1][1], equal_nan=True)
+
+
+def _unit_case(scale, seed=11):
+    """Keypoints up to 1 (metre) of the origin, clouds about them; scaled."""
+    rng = np.random.default_rng(seed)
+    sizes = [0, 1, 40, 90, 120, 200, 300]
+    km = np.zeros((len(sizes), 4), np.float32)
+    km[:, :3] = rng.uniform(-1, 1, (len(sizes), 3))
+    clouds = []
+    for k, n in zip(km, sizes):
+        c = np.zeros((n, 4), np.float32)
+        c[:, :3] = k[:3] + rng.uniform(-0.1, 0.1, (n, 3))
+        c[: n // 3, :3] = k[:3] + 0.01 * rng.integers(-9, 10, (n // 3, 3))
+        clouds.append(c)
+    ks = np.zeros((12, 4), np.float32)
+    ks[:, :3] = rng.uniform(-1, 1, (12, 3))
+    ks[:6, :3] = km[1:, :3] + np.float32([0.03, -0.02, 0.01])
+    mo = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    tdf = rng.uniform(0, 900, (len(sizes), 27000)).astype(np.float32)
+    sc = np.float32(scale)
+    return np.concatenate(clouds) * sc, km * sc, mo, np.arange(mo[-1], dtype=np.int32), tdf, ks * sc
+
+
+def _launches(ctx, rtr, case, res, half, off=0.0):
+    model, km, mo, mi, tdf, ks = case
+    model, km, ks = model.copy(), km.copy(), ks.copy()
+    for a in (model, km, ks):
+        a[:, 0] += np.float32(off)
+    ref = O.ref_distance(model, km, mo, mi, tdf, ks, res=res, half=half)
+    args = [_dev(x) for x in (model, km, mo, mi, tdf, ks)]
+    n0 = rtr.launch_count()
+    got = ctx.ref_distance(*args, resolution=res, half_tdf=half)
+    n1 = rtr.launch_count()
+    for g, r in zip(got, ref):
+        assert np.array_equal(g.cpu().numpy(), r, equal_nan=True), (res, off)
+    return n1 - n0
+
+
+@pytest.mark.parametrize("scale", [100.0, 1000.0, 0.001, 1.0e6, 3.7])
+def test_distance_in_other_units_takes_the_same_route(ctx, rtr, scale):
+    """Clouds in centimetres, millimetres, kilometres and micrometres: the
+    pair kernel takes them as it takes metres (no pair left to a CTA of its
+    own, which is a launch more), same scores and transforms as the oracle."""
+    metres = _launches(ctx, rtr, _unit_case(1.0), 0.01, 0.1525)
+    assert _launches(ctx, rtr, _unit_case(scale), 0.01 * scale, 0.1525 * scale) == metres
+
+
+def test_distance_far_from_the_origin(ctx, rtr):
+    """Up to 2^17 leaves from the origin the pair kernel takes every pair;
+    beyond, pairs are left to a CTA each; same results as the oracle at both."""
+    near = _launches(ctx, rtr, _unit_case(1.0), 0.01, 0.1525)
+    for off in (200.0, 1300.0):
+        assert _launches(ctx, rtr, _unit_case(1.0), 0.01, 0.1525, off) == near
+    assert _launches(ctx, rtr, _unit_case(1.0), 0.01, 0.1525, 1320.0) == near + 1
+    assert _launches(ctx, rtr, _unit_case(1.0e6), 1.0e4, 0.1525e6, 3.0e8) == near + 1
