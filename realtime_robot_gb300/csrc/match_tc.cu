@@ -54,12 +54,15 @@ constexpr int TC_KTAIL = TC_DIM / TC_KB;         // the K-block that holds only 
 constexpr int TC_RANGES = 8;                     // most database ranges of the first pass
 constexpr int TC_THREADS = 192;
 constexpr int TC_ROW = 36;  // floats a row in the epilogue's staging (16-byte stores of 8 rows meet 32 banks)
-// Bound on |d~ - d| over max(|q|, max |b|)^2, d the FP32 sequential sum.  The
-// dropped lo.lo and the split's rests: 2.3e-5; 68 accumulations of 16 products,
-// each term cut at 2^-23 of the largest: 2.8e-4; the sequential sum's own
-// rounding (352 terms, d up to 4): 8.4e-5; norms and the last step: 2e-6;
-// 3.9e-4 at worst.  Measured at most 2.2e-5 (SHOT rows of the room, Gaussian,
-// sparse, offset and badly scaled ones).
+// Bound on |d~ - d| over max(|q|, max |b|)^2, d the FP32 sequential sum.  BF16
+// keeps 8 significant bits: hi is within 2^-8 of x, hi + lo within 2^-16.  The
+// dropped lo.lo and the two rests, twice: 2 * 3 * 2^-16 = 9.2e-5; the norm
+// column's rest: 1.5e-5; 68 accumulations of 16 products, each term cut at 2^-23
+// of the largest: 2.8e-4 (how the tensor cores add is not documented: an
+// assumption, ten times what is measured); the sequential sum's own rounding
+// (352 terms, d up to 4): 8.4e-5; norms and the last step: 2e-6; 4.7e-4 at
+// worst.  Measured at most 2.2e-5 (SHOT rows of the room, Gaussian, sparse,
+// offset and badly scaled ones).
 constexpr float TC_ERR = 5.0e-4f;
 constexpr long long TC_SPIN_LIMIT = 1LL << 26;
 
@@ -444,8 +447,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_match_top(const __grid_consta
   const int nq = a.d_nq ? min(*a.d_nq, a.nq_cap) : a.nq_host;
   const int q0 = blockIdx.x * TC_BM;
   if (q0 >= nq) return;  // uniform per CTA, before any barrier or TMEM use
-  // database tiles of this CTA: all of them, or (band pass, gridDim.y > 1)
-  // one of gridDim.y contiguous ranges
+  // database tiles of this CTA: one of gridDim.y contiguous ranges
   const int n_all = (a.ndb + TC_BN - 1) / TC_BN;
   const int t_lo = (int)((long long)blockIdx.y * n_all / gridDim.y);
   const int t_hi = (int)((long long)(blockIdx.y + 1) * n_all / gridDim.y);
