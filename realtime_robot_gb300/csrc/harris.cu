@@ -19,7 +19,7 @@
 // radius) around the point and lists the points within the radius in
 // ascending index: hits set a bit each in the warp's bitmap of the cloud,
 // which is then read out in order (clouds of up to HR_BITS points; larger
-// ones append the hits and sort the list, 5 times the instructions).  A sum
+// ones append the hits and sort the list).  A sum
 // in that order is one chain per accumulator, so the terms of 32 neighbours
 // are formed by 32 lanes, staged, and each accumulator's lane adds its own:
 // the chains run side by side.  With one lane doing all of it (gather, terms
@@ -38,7 +38,13 @@ namespace rtr {
 
 constexpr int HR_WARPS = 4;
 constexpr int HR_CAP = 1024;  // neighbours of one point within the radius
-constexpr int HR_BITS = 131072;  // largest cloud whose bitmap (16 KB a warp) is used
+// Largest cloud whose bitmap is used.  The bitmap is read out whole for every
+// point, so its cost follows the cloud, the sort's the neighbours (whole call,
+// us, bitmap / sort; sparse: lattices of chairs, 60 neighbours; dense: one
+// chair, up to 1,000): sparse 20k 345 / 365, 30k 431 / 413, 40k 589 / 467, 60k
+// 852 / 564, 131k 3276 / 869; dense 20k 635 / 993, 30k 1032 / 1736, 40k 1675 /
+// 2577.
+constexpr int HR_BITS = 40960;
 
 struct HrArgs {
   GridDev grid;

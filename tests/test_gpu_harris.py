@@ -54,3 +54,35 @@ def test_harris_bitmap_edges(ctx, rtr, n, tile):
         pts[:, 1] += (2 * (k // 7)).astype(np.float32)
         pts = pts[np.random.default_rng(1).permutation(n)]
     _check(ctx, rtr, pts)
+
+
+def _lattice(rtr, n):
+    """Chairs of 3,000 points far apart."""
+    pts = np.concatenate([rtr.synth_shape(rtr.CHAIR, 3000, 5 + j) for j in range(-(-n // 3000))])[:n].copy()
+    j = np.arange(n) // 3000
+    pts[:, 0] += (2 * (j % 10)).astype(np.float32)
+    pts[:, 1] += (2 * (j // 10)).astype(np.float32)
+    return pts
+
+
+@pytest.mark.parametrize("n", [40960, 40961])
+def test_harris_on_both_sides_of_the_bitmap(ctx, rtr, n):
+    assert _check(ctx, rtr, _lattice(rtr, n)) > 0
+
+
+def test_harris_time_follows_the_cloud(ctx, rtr):
+    """No size of cloud is much slower than a larger one: the bitmap's cost is
+    its length, read out for every point."""
+    import torch
+
+    def time(n):
+        p, best = _dev(_lattice(rtr, n)), float("inf")
+        for k in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ctx.harris3d(p)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b)) if k else best
+        return best
+    assert max(time(n) for n in (100000, 131072)) < 2.0 * time(140000)
