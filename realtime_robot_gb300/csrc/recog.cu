@@ -421,6 +421,53 @@ __global__ void __launch_bounds__(256) k_uniform_pick(const float4* __restrict__
 // kNN order, exact Jacobi, smallest eigenvector flipped towards vp,
 // curvature l0 / (l0 + l1 + l2)
 // ---------------------------------------------------------------------------
+// Normal and curvature from the neighbours (INT_MAX: none), in their order.
+template <int K>
+__device__ __forceinline__ float4 normal_of(const float4* __restrict__ pts, const int (&bi)[K], float4 p, float vx,
+                                            float vy, float vz) {
+  int m = 0;
+  float mx = 0.f, my = 0.f, mz = 0.f;
+#pragma unroll
+  for (int s = 0; s < K; ++s) {
+    if (bi[s] == INT_MAX) continue;
+    const float4 q = pts[bi[s]];
+    mx = __fadd_rn(mx, q.x);
+    my = __fadd_rn(my, q.y);
+    mz = __fadd_rn(mz, q.z);
+    ++m;
+  }
+  const float fm = (float)m;
+  mx = __fdiv_rn(mx, fm);
+  my = __fdiv_rn(my, fm);
+  mz = __fdiv_rn(mz, fm);
+  float c00 = 0.f, c01 = 0.f, c02 = 0.f, c11 = 0.f, c12 = 0.f, c22 = 0.f;
+#pragma unroll
+  for (int s = 0; s < K; ++s) {
+    if (bi[s] == INT_MAX) continue;
+    const float4 q = pts[bi[s]];
+    const float dx = __fsub_rn(q.x, mx), dy = __fsub_rn(q.y, my), dz = __fsub_rn(q.z, mz);
+    c00 = __fadd_rn(c00, __fmul_rn(dx, dx));
+    c01 = __fadd_rn(c01, __fmul_rn(dx, dy));
+    c02 = __fadd_rn(c02, __fmul_rn(dx, dz));
+    c11 = __fadd_rn(c11, __fmul_rn(dy, dy));
+    c12 = __fadd_rn(c12, __fmul_rn(dy, dz));
+    c22 = __fadd_rn(c22, __fmul_rn(dz, dz));
+  }
+  const float A[9] = {c00, c01, c02, c01, c11, c12, c02, c12, c22};
+  float w[3], V[9];
+  eig3_exact(A, w, V);
+  float nx = V[0], ny = V[3], nz = V[6];
+  const float ux = __fsub_rn(vx, p.x), uy = __fsub_rn(vy, p.y), uz = __fsub_rn(vz, p.z);
+  const float dotv = __fadd_rn(__fadd_rn(__fmul_rn(ux, nx), __fmul_rn(uy, ny)), __fmul_rn(uz, nz));
+  if (dotv < 0.f) {
+    nx = -nx;
+    ny = -ny;
+    nz = -nz;
+  }
+  const float den = __fadd_rn(__fadd_rn(w[0], w[1]), w[2]);
+  return make_float4(nx, ny, nz, den != 0.f ? __fdiv_rn(w[0], den) : 0.f);
+}
+
 // A warp takes `per` (<= 32) consecutive points of the grid's order: searches
 // them one at a time (knn_warp), then a lane finishes each.
 // With a thread a point the kernel waited for its slowest threads: chains of
@@ -434,13 +481,15 @@ constexpr int NRM_WARPS = 4;
 constexpr int NRM_SMALL = 19456;  // points up to which a warp takes four (152 SMs, 32 warps each)
 template <int K>
 __global__ void __launch_bounds__(32 * NRM_WARPS) k_normals(GridDev gd, const float4* __restrict__ pts, int n_host,
-                                                            const int* d_n, float vx, float vy, float vz, int per,
-                                                            float4* __restrict__ out) {
+                                                            const int* d_n, const int* __restrict__ tiles, float vx,
+                                                            float vy, float vz, int per, float4* __restrict__ out) {
   __shared__ int s_idx[NRM_WARPS][K][33];
   const BoxView v = box_view(gd);
   const int n = cnt_of(n_host, d_n);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int j0 = (blockIdx.x * NRM_WARPS + warp) * per; j0 < n; j0 += gridDim.x * NRM_WARPS * per) {
+  const int total = tiles ? tiles[0] * 32 : n;  // tiles: their number, then the first points over 32
+  for (int t0 = (blockIdx.x * NRM_WARPS + warp) * per; t0 < total; t0 += gridDim.x * NRM_WARPS * per) {
+    const int j0 = tiles ? tiles[1 + (t0 >> 5)] * 32 + (t0 & 31) : t0;
     const int cnt = min(per, n - j0);
     const float4 p = lane < cnt ? v.g.pts[j0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
     for (int t = 0; t < cnt; ++t) {
@@ -457,47 +506,63 @@ __global__ void __launch_bounds__(32 * NRM_WARPS) k_normals(GridDev gd, const fl
     __syncwarp();
     if (lane >= cnt) continue;
     const int i = pt_index(p);
-    int m = 0;
-    float mx = 0.f, my = 0.f, mz = 0.f;
+    out[i] = normal_of<K>(pts, bi, p, vx, vy, vz);
+  }
+}
+
+// A thread a point, for large clouds: a warp whose 32 points all have some
+// candidates (points in the 27 cells around) but not many searches them side by
+// side, each lane its own; the others go on the list of tiles that k_normals
+// takes.  Where points are spread evenly the threads' chains are alike, and once
+// there are threads enough a warp a point is the dearer form; k points have to
+// be near, or one lane's search far out holds the others up.
+// From NRM_EVEN points (with the grid build, k_normals alone / with this; us):
+// 300k points in a volume, k = 8, automatic cell 487 / 267 (424 with a thread a
+// point and sorted grids); a wall's 253k voxels, k = 10, cells of two leaves 240
+// / 167 (219); a room's 216k 234 / 214; 1M points of a sofa's surface 1,573 /
+// 1,598.  At 100k even clouds gain too (a volume 222 / 178), but uneven ones
+// lose (a room 275 / 336).
+constexpr int NRM_EVEN = 200000;
+__host__ __device__ constexpr unsigned nrm_few(int K) { return K <= 10 ? 256u : 96u; }
+template <int K>
+__global__ void __launch_bounds__(128) k_normals_even(GridDev gd, const float4* __restrict__ pts, int n_host,
+                                                      const int* d_n, int* __restrict__ tiles, float vx, float vy,
+                                                      float vz, float4* __restrict__ out) {
+  const GridView g = load_view(gd);
+  const int n = cnt_of(n_host, d_n), lane = threadIdx.x & 31;
+  for (int j0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); j0 < n; j0 += gridDim.x * blockDim.x) {
+    const bool live = j0 + lane < n;
+    const float4 p = g.pts[min(j0 + lane, n - 1)];
+    const bool search = live && finite3(p);
+    bool few = true;
+    if (search) {
+      const int cx = min(max(q_cell(p.x, g.ox, g.inv_h), 0), g.nx - 1),
+                cy = min(max(q_cell(p.y, g.oy, g.inv_h), 0), g.ny - 1),
+                cz = min(max(q_cell(p.z, g.oz, g.inv_h), 0), g.nz - 1);
+      auto around = [&](int e) {  // points in the cells up to e from the point's
+        const int x0 = max(cx - e, 0), x1 = min(cx + e, g.nx - 1);
+        unsigned sum = 0;
+        for (int z = max(cz - e, 0); z <= min(cz + e, g.nz - 1); ++z)
+          for (int y = max(cy - e, 0); y <= min(cy + e, g.ny - 1); ++y) {
+            const uint2 s = row_span(g, x0, x1, y, z);
+            sum += s.y - s.x;
+          }
+        return sum;
+      };
+      const unsigned near = around(1);
+      few = near <= nrm_few(K) && (near >= (unsigned)K || (near >= (unsigned)(K / 2) && around(2) >= (unsigned)K));
+    }
+    if (!__all_sync(0xffffffffu, few)) {
+      if (lane == 0) tiles[1 + atomicAdd(tiles, 1)] = j0 >> 5;
+      continue;
+    }
+    if (!live) continue;
+    float bd[K];
+    int bi[K];
 #pragma unroll
-    for (int s = 0; s < K; ++s) {
-      if (bi[s] == INT_MAX) continue;
-      const float4 q = pts[bi[s]];
-      mx = __fadd_rn(mx, q.x);
-      my = __fadd_rn(my, q.y);
-      mz = __fadd_rn(mz, q.z);
-      ++m;
-    }
-    const float fm = (float)m;
-    mx = __fdiv_rn(mx, fm);
-    my = __fdiv_rn(my, fm);
-    mz = __fdiv_rn(mz, fm);
-    float c00 = 0.f, c01 = 0.f, c02 = 0.f, c11 = 0.f, c12 = 0.f, c22 = 0.f;
-#pragma unroll
-    for (int s = 0; s < K; ++s) {
-      if (bi[s] == INT_MAX) continue;
-      const float4 q = pts[bi[s]];
-      const float dx = __fsub_rn(q.x, mx), dy = __fsub_rn(q.y, my), dz = __fsub_rn(q.z, mz);
-      c00 = __fadd_rn(c00, __fmul_rn(dx, dx));
-      c01 = __fadd_rn(c01, __fmul_rn(dx, dy));
-      c02 = __fadd_rn(c02, __fmul_rn(dx, dz));
-      c11 = __fadd_rn(c11, __fmul_rn(dy, dy));
-      c12 = __fadd_rn(c12, __fmul_rn(dy, dz));
-      c22 = __fadd_rn(c22, __fmul_rn(dz, dz));
-    }
-    const float A[9] = {c00, c01, c02, c01, c11, c12, c02, c12, c22};
-    float w[3], V[9];
-    eig3_exact(A, w, V);
-    float nx = V[0], ny = V[3], nz = V[6];
-    const float ux = __fsub_rn(vx, p.x), uy = __fsub_rn(vy, p.y), uz = __fsub_rn(vz, p.z);
-    const float dotv = __fadd_rn(__fadd_rn(__fmul_rn(ux, nx), __fmul_rn(uy, ny)), __fmul_rn(uz, nz));
-    if (dotv < 0.f) {
-      nx = -nx;
-      ny = -ny;
-      nz = -nz;
-    }
-    const float den = __fadd_rn(__fadd_rn(w[0], w[1]), w[2]);
-    out[i] = make_float4(nx, ny, nz, den != 0.f ? __fdiv_rn(w[0], den) : 0.f);
+    for (int s = 0; s < K; ++s) bi[s] = INT_MAX;
+    if (search) grid_knn<K>(g, p, bd, bi);
+    out[pt_index(p)] = normal_of<K>(pts, bi, p, vx, vy, vz);
   }
 }
 
@@ -865,24 +930,34 @@ rtr_status uniform_sample_dev(rtr_context* ctx, Scratch& s, const float4* pts, i
   return RTR_OK;
 }
 
+template <int K>
+static rtr_status normals_launch(const GridBufs& gb, const float4* pts, int n_cap, const int* d_n, const float vp[3],
+                                 float cell, float4* out, cudaStream_t st) {
+  const int per = n_cap < NRM_SMALL ? 4 : 8;
+  int* tiles = nullptr;
+  if (n_cap >= NRM_EVEN) {
+    tiles = reinterpret_cast<int*>(gb.k0);  // (the points' cells, read by now; n_cap entries)
+    RTR_CUDA(cudaMemsetAsync(tiles, 0, sizeof(int), st));
+    k_normals_even<K><<<blocks_for(n_cap, 128, 1 << 20), 128, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, tiles, vp[0],
+                                                                      vp[1], vp[2], out);
+    RTR_LAUNCHED(1);
+  }
+  k_normals<K><<<blocks_for(n_cap, NRM_WARPS * per, 1 << 20), 32 * NRM_WARPS, 0, st>>>(
+      grid_dev(gb), pts, n_cap, d_n, tiles, vp[0], vp[1], vp[2], per, out);
+  RTR_LAUNCHED(1);
+  return RTR_OK;
+}
+
 rtr_status normals_dev(rtr_context* ctx, Scratch& s, const float4* pts, int n_cap, const int* d_n, int k,
                        const float vp[3], float cell, float4* out, cudaStream_t st) {
   GridBufs gb;
   const unsigned cap = default_cell_cap(n_cap);
   if (!grid_take(s, n_cap, cap, &gb)) return fail(RTR_ERR_CAPACITY, "normals: scratch");
   RTR_TRY(grid_build(gb, pts, n_cap, d_n, cell, st));
-  const int per = n_cap < NRM_SMALL ? 4 : 8;
-  const int nb = blocks_for(n_cap, NRM_WARPS * per, 1 << 20);
-  if (k <= 8)
-    k_normals<8><<<nb, 32 * NRM_WARPS, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], per, out);
-  else if (k <= 10)
-    k_normals<10><<<nb, 32 * NRM_WARPS, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], per, out);
-  else if (k <= 16)
-    k_normals<16><<<nb, 32 * NRM_WARPS, 0, st>>>(grid_dev(gb), pts, n_cap, d_n, vp[0], vp[1], vp[2], per, out);
-  else
-    return fail(RTR_ERR_INVALID_ARG, "normals: k must be 8, 10 or 16");
-  RTR_LAUNCHED(1);
-  return RTR_OK;
+  if (k <= 8) return normals_launch<8>(gb, pts, n_cap, d_n, vp, cell, out, st);
+  if (k <= 10) return normals_launch<10>(gb, pts, n_cap, d_n, vp, cell, out, st);
+  if (k <= 16) return normals_launch<16>(gb, pts, n_cap, d_n, vp, cell, out, st);
+  return fail(RTR_ERR_INVALID_ARG, "normals: k must be 8, 10 or 16");
 }
 
 // SHOT over a grid of the points already built with cell R (grid_build).
