@@ -53,6 +53,7 @@ rtr_status fail(rtr_status st, const char* fmt, ...) {
 rtr_status cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
   const char* base = strrchr(file, '/');
   set_error("%s failed: %s (%s:%d)", what, cudaGetErrorString(e), base ? base + 1 : file, line);
+  (void)cudaGetLastError();  // reported here: the next call does not find it again
   return e == cudaErrorMemoryAllocation ? RTR_ERR_OOM : RTR_ERR_CUDA;
 }
 

@@ -1445,7 +1445,7 @@ static rtr_status gc_launch(rtr_context* ctx, Scratch& s, const float* d_model_k
   ProfScope pso(ctx, st, "gc_sort");
   k_gc_keys<<<nb, 256, 0, st>>>(d_corr_d, C, d_C, b.k0);
   uint32_t *ks, *vs;
-  radix_sort_pairs(ctx, b.k0, b.v0, b.k1, b.v1, b.hist, C, C, d_C, 32, true, st, &ks, &vs);
+  RTR_TRY(radix_sort_pairs(ctx, b.k0, b.v0, b.k1, b.v1, b.hist, C, C, d_C, 32, true, st, &ks, &vs));
   k_gc_gather<<<nb, 256, 0, st>>>(reinterpret_cast<const float4*>(d_model_kp),
                                   reinterpret_cast<const float4*>(d_scene_kp), d_corr_m, d_corr_s, vs, C, d_C, b.pm,
                                   b.ps);
@@ -1462,7 +1462,7 @@ static rtr_status gc_launch(rtr_context* ctx, Scratch& s, const float* d_model_k
   k_gcg_setup<<<1, 32, 0, st>>>(b.sg, b.mbox, gc_size, C, d_C);
   k_gcg_keys<<<nb, 256, 0, st>>>(b.ps, C, d_C, b.sg, b.gk0);
   uint32_t *gks, *gvs;  // gks unused: the cell order is all the seed tests need
-  radix_sort_pairs(ctx, b.gk0, b.gv0, b.gk1, b.gv1, b.hist, C, C, d_C, 16, true, st, &gks, &gvs);
+  RTR_TRY(radix_sort_pairs(ctx, b.gk0, b.gv0, b.gk1, b.gv1, b.hist, C, C, d_C, 16, true, st, &gks, &gvs));
   k_gcg_gather<<<nb, 256, 0, st>>>(b.ps, b.pm, gvs, C, d_C, b.cpts, b.cpm, b.cbox);
   RTR_LAUNCHED(3);
   pgr.end();

@@ -1,8 +1,6 @@
 // grid.cu — stable LSD radix sort and the uniform-grid build (counted into place).
 #include <math.h>
 
-#include <atomic>
-
 #include "csort.cuh"
 #include "grid.cuh"
 
@@ -229,13 +227,12 @@ __global__ void __launch_bounds__(CS_THREADS) k_rs_cluster(uint32_t* __restrict_
   }
 }
 
-// Whether the current device schedules clusters of CS_MAX CTAs of this size
-// (more than 8 is up to the device), asked once a device.
-static bool cluster_max_ok() {
-  static std::atomic<int> known[64];
+// Whether the current device schedules clusters of CS_MAX CTAs of this kernel
+// (more than 8 is up to the device).
+static bool cluster_max_ok(const void* kern, ClusterFit& fit) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  int k = known[dev].load(std::memory_order_relaxed);
+  int k = fit.known[dev].load(std::memory_order_relaxed);
   if (k == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(CS_MAX);
@@ -248,11 +245,11 @@ static bool cluster_max_ok() {
     cfg.numAttrs = 1;
     int n = 0;
     const bool ok =
-        cudaFuncSetAttribute(k_rs_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n, k_rs_cluster, &cfg) == cudaSuccess && n > 0;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
     if (!ok) cudaGetLastError();
     k = ok ? 2 : 1;
-    known[dev].store(k, std::memory_order_relaxed);
+    fit.known[dev].store(k, std::memory_order_relaxed);
   }
   return k == 2;
 }
@@ -263,11 +260,11 @@ static bool cluster_max_ok() {
 // the line at 32k items, 667 at 131k; the 300k-point room's recognition 3,210
 // us with it there, 3,243 with the line beyond its points.  Clusters of at
 // most 8 CTAs: the scan 727 us.
-int cluster_sort_ctas(const rtr_context* ctx, int n_cap) {
+int cluster_sort_ctas(const rtr_context* ctx, int n_cap, const void* kern, ClusterFit& fit) {
   if (n_cap > RS_CLUSTER_MAX || (ctx && ctx->grid_sorts)) return 0;
   const int want = (n_cap + RS_CLUSTER_ITEMS - 1) / RS_CLUSTER_ITEMS;
   int c = 1;
-  while (c < want && c < (c < 8 || cluster_max_ok() ? CS_MAX : 8)) c *= 2;
+  while (c < want && c < (c < 8 || cluster_max_ok(kern, fit) ? CS_MAX : 8)) c *= 2;
   return c;
 }
 
@@ -277,15 +274,16 @@ int radix_hist_entries(int n_cap) {
   return nb * RS_RADIX;
 }
 
-void radix_sort_pairs(const rtr_context* ctx, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t* hist,
+rtr_status radix_sort_pairs(const rtr_context* ctx, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t* hist,
                       int n_cap, int n_host, const int* d_n, int bits, bool vals_iota,
                       cudaStream_t st, uint32_t** k_out, uint32_t** v_out) {
   int nb = (n_cap + RS_TILE - 1) / RS_TILE;
   if (nb < 1) nb = 1;
   int passes = (bits + 7) / 8;
   if (passes < 1) passes = 1;
-  const int ctas = cluster_sort_ctas(ctx, n_cap);
-  if (ctas > 0) launch_cluster(k_rs_cluster, ctas, st, k0, v0, k1, v1, n_host, d_n, passes, (int)vals_iota);
+  static ClusterFit fit;
+  const int ctas = cluster_sort_ctas(ctx, n_cap, reinterpret_cast<const void*>(k_rs_cluster), fit);
+  if (ctas > 0) RTR_TRY(launch_cluster(k_rs_cluster, ctas, st, k0, v0, k1, v1, n_host, d_n, passes, (int)vals_iota));
   for (int p = 0; p < passes && ctas == 0; ++p) {
     const int shift = 8 * p;
     const bool even = (p & 1) == 0;
@@ -306,6 +304,8 @@ void radix_sort_pairs(const rtr_context* ctx, uint32_t* k0, uint32_t* v0, uint32
   const bool odd = (passes & 1) != 0;
   *k_out = odd ? k1 : k0;
   *v_out = odd ? v1 : v0;
+  RTR_CUDA(cudaGetLastError());
+  return RTR_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -666,7 +666,7 @@ rtr_status grid_build(const GridBufs& b, const float4* pts, int n_host, const in
     int bits = 1;
     while (bits < 32 && (1ull << bits) < (unsigned long long)b.cell_cap) ++bits;
     uint32_t *ks, *vs;
-    radix_sort_pairs(nullptr, b.k0, b.v0, b.k1, b.v1, b.hist, b.n_cap, n_host, d_n, bits, true, st, &ks, &vs);
+    RTR_TRY(radix_sort_pairs(nullptr, b.k0, b.v0, b.k1, b.v1, b.hist, b.n_cap, n_host, d_n, bits, true, st, &ks, &vs));
     k_grid_gather<<<nb, 256, 0, st>>>(pts, ks, vs, n_host, d_n, b.starts, b.pts);
   } else {
     k_grid_count<true><<<nb, 256, 0, st>>>(pts, n_host, d_n, b.meta, b.k0, b.v0, b.starts);

@@ -7,6 +7,8 @@
 // the device, so a build can sit inside a captured CUDA graph; capacities
 // come from the host.
 #pragma once
+#include <atomic>
+
 #include "common.cuh"
 
 struct GridMeta {
@@ -50,13 +52,19 @@ struct GridBufs {
 // When vals_in is NULL the values are the element indices.  Ping-pongs
 // between (k0,v0) and (k1,v1); *k_out/*v_out point at the sorted arrays.
 int radix_hist_entries(int n_cap);
-// CTAs of the cluster that sorts n_cap items in one launch; 0: a grid of tiles
-// (too many items, or ctx asks for it; ctx may be NULL).
-int cluster_sort_ctas(const rtr_context* ctx, int n_cap);
+// Whether each device schedules a kernel's largest cluster: asked once a kernel
+// and device (0: not yet, 1: no, 2: yes).
+struct ClusterFit {
+  std::atomic<int> known[64] = {};
+};
+// CTAs of the cluster of `kern` (1,024 threads a CTA) that sorts n_cap items in
+// one launch; 0: a grid of tiles (too many items, or ctx asks for it; ctx may be
+// NULL).
+int cluster_sort_ctas(const rtr_context* ctx, int n_cap, const void* kern, ClusterFit& fit);
 // Launches a kernel of clusters of `ctas` CTAs of 1,024 threads (one cluster).
 template <class... P, class... A>
-inline void launch_cluster(void (*kern)(P...), int ctas, cudaStream_t st, A... args) {
-  if (ctas > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+inline rtr_status launch_cluster(void (*kern)(P...), int ctas, cudaStream_t st, A... args) {
+  if (ctas > 8) RTR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(1024);
@@ -67,11 +75,12 @@ inline void launch_cluster(void (*kern)(P...), int ctas, cudaStream_t st, A... a
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, (P)args...);
+  RTR_CUDA(cudaLaunchKernelEx(&cfg, kern, (P)args...));
+  return RTR_OK;
 }
-void radix_sort_pairs(const rtr_context* ctx, uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint32_t* hist,
-                      int n_cap, int n_host, const int* d_n, int bits, bool vals_iota,
-                      cudaStream_t st, uint32_t** k_out, uint32_t** v_out);
+[[nodiscard]] rtr_status radix_sort_pairs(const rtr_context* ctx, uint32_t* k0, uint32_t* v0, uint32_t* k1,
+                                          uint32_t* v1, uint32_t* hist, int n_cap, int n_host, const int* d_n, int bits,
+                                          bool vals_iota, cudaStream_t st, uint32_t** k_out, uint32_t** v_out);
 
 // ordered: the points of a cell in ascending original index (a stable sort by
 // cell); otherwise in any order (counted into place, a quarter of the time).

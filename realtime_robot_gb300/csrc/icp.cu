@@ -811,7 +811,7 @@ rtr_status rtr_icp(rtr_context* ctx, const float* d_src, int n_src, const float*
   int bits = 1;
   while (bits < 32 && (1ull << bits) < (unsigned long long)cell_cap) ++bits;
   uint32_t *ks, *vs;
-  radix_sort_pairs(ctx, k0, v0, k1, v1, hist, n_src, n_src, nullptr, bits, true, st, &ks, &vs);
+  RTR_TRY(radix_sort_pairs(ctx, k0, v0, k1, v1, hist, n_src, n_src, nullptr, bits, true, st, &ks, &vs));
   k_gather_pts<<<nb, 256, 0, st>>>(reinterpret_cast<const float4*>(d_src), vs, n_src, src_sorted,
                                    src_idx);
   RTR_LAUNCHED(2);

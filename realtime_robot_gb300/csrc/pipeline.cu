@@ -738,7 +738,7 @@ static rtr_status scene_stages(rtr_context* ctx, const Scratch& stage, SceneBufs
       ProfScope ps2(ctx, st, "prune_select");
       k_score_keys<<<nb, 256, 0, st>>>(score, dKeys, n, k0);
       uint32_t *ks, *vs;
-      radix_sort_pairs(ctx, k0, v0, k1, v1, hist, n, n, dKeys, 32, true, st, &ks, &vs);
+      RTR_TRY(radix_sort_pairs(ctx, k0, v0, k1, v1, hist, n, n, dKeys, 32, true, st, &ks, &vs));
       k_mark_top<<<nb, 256, 0, st>>>(vs, dKeys, n, keep, b.flags);
     }
     ProfScope ps2(ctx, st, "prune_compact");

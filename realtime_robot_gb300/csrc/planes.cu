@@ -685,15 +685,15 @@ rtr_status rtr_plane_segment(rtr_context* ctx, const float* d_pts, int n, const 
       const int nl = host->n_left;
       k_pl_keys_v<<<pl_blocks(nl), 256, 0, st>>>(su, nl, k0);
       uint32_t *ks, *vs;
-      radix_sort_pairs(ctx, k0, v0, k1, v1, hist, nl, nl, nullptr, 32, true, st, &ks, &vs);
+      RTR_TRY(radix_sort_pairs(ctx, k0, v0, k1, v1, hist, nl, nl, nullptr, 32, true, st, &ks, &vs));
       // second, stable pass by u over the first pass's order
       uint32_t* ka = ks == k0 ? k1 : k0;
       uint32_t* va = vs == v0 ? v1 : v0;
       k_pl_keys_u<<<pl_blocks(nl), 256, 0, st>>>(su, vs, nl, ka);
       RTR_CUDA(cudaMemcpyAsync(va, vs, sizeof(uint32_t) * (size_t)nl, cudaMemcpyDeviceToDevice, st));
       uint32_t *ks2, *vs2;
-      radix_sort_pairs(ctx, ka, va, ka == k0 ? k1 : k0, va == v0 ? v1 : v0, hist, nl, nl, nullptr, 32, false, st, &ks2,
-                       &vs2);
+      RTR_TRY(radix_sort_pairs(ctx, ka, va, ka == k0 ? k1 : k0, va == v0 ? v1 : v0, hist, nl, nl, nullptr, 32, false,
+                               st, &ks2, &vs2));
       k_pl_chain<<<1, 32, 0, st>>>(su, vs2, nl, hull, host);
       RTR_LAUNCHED(3);
       RTR_CUDA(cudaGetLastError());

@@ -335,14 +335,17 @@ bool voxseg_take(Scratch& s, int n_cap, VoxSeg* v) {
          v->seg_start && v->d_nseg;
 }
 
-void voxseg_build(const rtr_context* ctx, VoxSeg& v, const float4* pts, int n_host, const int* d_n, float inv, cudaStream_t st) {
-  const int ctas = cluster_sort_ctas(ctx, v.n_cap);
+rtr_status voxseg_build(const rtr_context* ctx, VoxSeg& v, const float4* pts, int n_host, const int* d_n, float inv,
+                        cudaStream_t st) {
+  static ClusterFit fit;
+  const int ctas = cluster_sort_ctas(ctx, v.n_cap, reinterpret_cast<const void*>(k_voxseg), fit);
   if (ctas > 0) {
-    launch_cluster(k_voxseg, ctas, st, pts, n_host, d_n, inv, v.meta, v.k0, v.v0, v.k1, v.v1, v.seg_start, v.d_nseg);
+    RTR_TRY(launch_cluster(k_voxseg, ctas, st, pts, n_host, d_n, inv, v.meta, v.k0, v.v0, v.k1, v.v1, v.seg_start,
+                           v.d_nseg));
     RTR_LAUNCHED(1);
     v.keys = v.k0;
     v.order = v.v0;
-    return;
+    return RTR_OK;
   }
   const int nb = blocks_for(v.n_cap);
   k_vox_init<<<1, 32, 0, st>>>(v.meta);
@@ -350,13 +353,14 @@ void voxseg_build(const rtr_context* ctx, VoxSeg& v, const float4* pts, int n_ho
   k_vox_setup<<<1, 1, 0, st>>>(v.meta, n_host, d_n);
   k_vox_keys<<<nb, 256, 0, st>>>(pts, n_host, d_n, inv, v.meta, v.k0);
   uint32_t *ks, *vs;
-  radix_sort_pairs(ctx, v.k0, v.v0, v.k1, v.v1, v.hist, v.n_cap, n_host, d_n, 32, true, st, &ks, &vs);
+  RTR_TRY(radix_sort_pairs(ctx, v.k0, v.v0, v.k1, v.v1, v.hist, v.n_cap, n_host, d_n, 32, true, st, &ks, &vs));
   k_seg_heads<<<nb, 256, 0, st>>>(ks, n_host, d_n, v.flags);
   scan_exclusive(v.flags, v.flags, v.tile_sums, v.n_cap, n_host, d_n, reinterpret_cast<uint32_t*>(v.d_nseg), st);
   k_seg_starts<<<nb, 256, 0, st>>>(ks, v.flags, n_host, d_n, v.seg_start, v.d_nseg);
   RTR_LAUNCHED(6);
   v.keys = ks;
   v.order = vs;
+  return RTR_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -913,9 +917,10 @@ rtr_status voxel_downsample_dev(rtr_context* ctx, Scratch& s, const float4* pts,
   VoxSeg v;
   if (!voxseg_take(s, n_cap, &v)) return fail(RTR_ERR_CAPACITY, "voxel_downsample: scratch");
   const float inv = 1.0f / leaf;
-  voxseg_build(ctx, v, pts, n_cap, d_n, inv, st);
+  RTR_TRY(voxseg_build(ctx, v, pts, n_cap, d_n, inv, st));
   k_vox_centroid<<<blocks_for(n_cap), 256, 0, st>>>(pts, v.order, v.seg_start, v.d_nseg, v.meta, out, d_count);
   RTR_LAUNCHED(1);
+  RTR_CUDA(cudaGetLastError());
   return RTR_OK;
 }
 
@@ -924,9 +929,10 @@ rtr_status uniform_sample_dev(rtr_context* ctx, Scratch& s, const float4* pts, i
   VoxSeg v;
   if (!voxseg_take(s, n_cap, &v)) return fail(RTR_ERR_CAPACITY, "uniform_sample: scratch");
   const float inv = 1.0f / r;
-  voxseg_build(ctx, v, pts, n_cap, d_n, inv, st);
+  RTR_TRY(voxseg_build(ctx, v, pts, n_cap, d_n, inv, st));
   k_uniform_pick<<<blocks_for(n_cap), 256, 0, st>>>(pts, v.order, v.seg_start, v.d_nseg, v.meta, inv, r, out, d_count);
   RTR_LAUNCHED(1);
+  RTR_CUDA(cudaGetLastError());
   return RTR_OK;
 }
 

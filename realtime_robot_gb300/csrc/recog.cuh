@@ -29,7 +29,7 @@ struct VoxSeg {
 
 void voxseg_plan(ScratchPlan& p, int n_cap);
 bool voxseg_take(Scratch& s, int n_cap, VoxSeg* v);
-void voxseg_build(const rtr_context* ctx, VoxSeg& v, const float4* pts, int n_host, const int* d_n, float inv_leaf,
-                  cudaStream_t st);
+[[nodiscard]] rtr_status voxseg_build(const rtr_context* ctx, VoxSeg& v, const float4* pts, int n_host,
+                                      const int* d_n, float inv_leaf, cudaStream_t st);
 
 }  // namespace rtr

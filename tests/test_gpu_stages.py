@@ -219,3 +219,35 @@ def test_normals_of_an_even_volume_cost_no_more_with_the_automatic_cell(ctx):
             best = min(best, a.elapsed_time(b)) if k > 1 else best
         return best
     assert time(0.0) < 1.35 * time(1.25 * 4.0 / n ** (1 / 3))
+
+
+@pytest.mark.parametrize("n", [5000, 200000])
+def test_launches_that_fail_are_reported(rtr, n):
+    """Voxels and keypoints on a stream whose capture has been invalidated (by
+    a synchronisation): no kernel can be launched there, by a cluster or a
+    grid, and the calls say so; the context stays usable."""
+    import ctypes
+
+    import torch
+    cu = ctypes.CDLL("libcuda.so.1")
+    pts = np.zeros((n, 4), np.float32)
+    pts[:, :3] = np.random.default_rng(n).uniform(-1, 1, (n, 3))
+    p, out = _dev(pts), torch.zeros((n, 4), dtype=torch.float32, device="cuda")
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    c = rtr.Context(0)
+    try:
+        ref = _host(c.voxel_downsample(p, 0.05))  # (sizes the scratch)
+        c.uniform_sample(p, 0.05)
+        torch.cuda.synchronize()
+        s, g = ctypes.c_void_p(), ctypes.c_void_p()
+        assert cu.cuStreamCreate(ctypes.byref(s), 1) == 0
+        assert cu.cuStreamBeginCapture_v2(s, 2) == 0
+        assert cu.cuStreamSynchronize(s) != 0
+        args = (c.h, p.data_ptr(), n, ctypes.c_float(0.05), out.data_ptr(), cnt.data_ptr(), s)
+        rv, ru = rtr.lib().rtr_voxel_downsample(*args), rtr.lib().rtr_uniform_sample(*args)
+        assert cu.cuStreamEndCapture(s, ctypes.byref(g)) != 0
+        assert cu.cuStreamDestroy_v2(s) == 0
+        assert rv != 0 and ru != 0, (rv, ru)
+        assert np.array_equal(_host(c.voxel_downsample(p, 0.05)), ref)
+    finally:
+        c.close()
