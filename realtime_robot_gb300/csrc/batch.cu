@@ -29,6 +29,7 @@ struct rtr_batch_graph {
   // graph holds their arena addresses, so it may run only while none of the
   // arenas has been reallocated since
   std::vector<unsigned> gens;
+  std::shared_ptr<int> alive;  // the context's count of its graphs
 };
 
 namespace rtr {
@@ -168,6 +169,8 @@ rtr_status rtr_batch_graph_create(rtr_context* ctx, const rtr_batch_pair* h_pair
   bg->exec = x;
   bg->gens.push_back(ctx->scratch_gen);
   for (int wi = 0; wi < nw; ++wi) bg->gens.push_back(ctx->workers[wi]->scratch_gen);
+  bg->alive = ctx->batch_graphs;
+  ++*bg->alive;
   *out = bg;
   return RTR_OK;
 }
@@ -187,6 +190,7 @@ rtr_status rtr_batch_graph_launch(rtr_batch_graph* bg, rtr_stream_t stream) {
 
 rtr_status rtr_batch_graph_destroy(rtr_batch_graph* bg) {
   if (!bg) return RTR_OK;
+  --*bg->alive;
   cudaSetDevice(bg->ctx->device);
   if (bg->exec) cudaGraphExecDestroy(bg->exec);
   if (bg->graph) cudaGraphDestroy(bg->graph);

@@ -43,6 +43,7 @@ rtr_status cuda_fail(cudaError_t e, const char* what, const char* file, int line
 // context (host) + scratch arena
 // ---------------------------------------------------------------------------
 #include <atomic>
+#include <memory>
 #include <vector>
 
 namespace rtr {
@@ -99,6 +100,8 @@ struct rtr_context {
   void* plane_host = nullptr;          // page-locked words of the plane segmentation (planes.cu)
   int tune_icp_group = 0;              // lanes per ICP source point (0: automatic)
   size_t scratch_limit = 0;            // largest scratch arena this context may hold (0: no limit)
+  size_t scratch_refused = 0;          // size that cudaMalloc last refused a call that could do with less (0: none)
+  std::shared_ptr<int> batch_graphs = std::make_shared<int>(0);  // alive: they hold the arenas' addresses
   int tune_batch_workers = 0;          // workers of rtr_recognize_batch (0: automatic)
   int coop_div = 1;                    // workers whose cooperative grids share the GPU (coop_share.h)
   int coop_gc_per_sm = 2;              // grouping blocks an SM holds, in the largest of the workers' scenes
@@ -152,9 +155,12 @@ struct Scratch {
 // Ensure the arena holds `bytes`; grows (synchronising) unless `stream` is
 // being captured, in which case RTR_ERR_CAPACITY is returned.
 rtr_status ensure_scratch(rtr_context* ctx, size_t bytes, cudaStream_t stream, Scratch* out);
-// Whether ensure_scratch may be asked for `bytes`: held already, or free to
-// grow (no capture, within the caller's limit).  For what a call can do without.
-bool scratch_obtainable(const rtr_context* ctx, size_t bytes, cudaStream_t stream);
+// For a call that can do with `least` and is faster with `want`: the larger one
+// where it is held or can be had, else the smaller one (out->cap tells).  It
+// does not grow during a capture, over the caller's limit, again after a
+// cudaMalloc of that size has failed, or under a batch graph, which holds the
+// arena's address, as long as `least` is held.
+rtr_status ensure_scratch_upto(rtr_context* ctx, size_t want, size_t least, cudaStream_t stream, Scratch* out);
 
 bool stream_is_capturing(cudaStream_t s);
 

@@ -70,11 +70,6 @@ rtr_status side_stream_ready(rtr_context* ctx) {
   return RTR_OK;
 }
 
-bool scratch_obtainable(const rtr_context* ctx, size_t bytes, cudaStream_t stream) {
-  return bytes <= ctx->arena_bytes ||
-         (!stream_is_capturing(stream) && (!ctx->scratch_limit || bytes <= ctx->scratch_limit));
-}
-
 rtr_status ensure_scratch(rtr_context* ctx, size_t bytes, cudaStream_t stream, Scratch* out) {
   if (bytes > ctx->arena_bytes) {
     if (stream_is_capturing(stream))
@@ -108,6 +103,17 @@ rtr_status ensure_scratch(rtr_context* ctx, size_t bytes, cudaStream_t stream, S
   out->off = 0;
   out->cap = ctx->arena_bytes;
   return RTR_OK;
+}
+
+rtr_status ensure_scratch_upto(rtr_context* ctx, size_t want, size_t least, cudaStream_t stream, Scratch* out) {
+  const bool keep = least <= ctx->arena_bytes &&
+                    (*ctx->batch_graphs > 0 || (ctx->scratch_refused && want >= ctx->scratch_refused));
+  if (want <= ctx->arena_bytes || !(keep || stream_is_capturing(stream))) {
+    const rtr_status r = ensure_scratch(ctx, want, stream, out);
+    if (r != RTR_ERR_OOM) return r;
+    if (!ctx->scratch_limit || want <= ctx->scratch_limit) ctx->scratch_refused = want;
+  }
+  return ensure_scratch(ctx, least, stream, out);
 }
 
 rtr_status ensure_io(rtr_context* ctx, size_t bytes) {

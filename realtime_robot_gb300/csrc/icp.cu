@@ -27,6 +27,7 @@ namespace rtr {
 constexpr int ICP_THREADS = 256;
 constexpr int ICP_WARPS = ICP_THREADS / 32;
 constexpr int ICP_NV = 16;  // dp(3) dq(3) dp*dq^T(9) d^2(1)
+constexpr size_t ICP_STATE_MAX = size_t(50) << 20;  // points whose matching state a call asks scratch for (1 GB)
 constexpr int ICP_CHUNK = 2048;  // points a block matches between two barriers
 
 __device__ __forceinline__ unsigned long long icp_timer() {
@@ -656,14 +657,20 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
   int* pcount = s.take<int>(maxb);
   unsigned* sync = s.take<unsigned>(M);
   if (!sync) return fail(RTR_ERR_CAPACITY, "icp: scratch carve");
-  // the matching state, when the scratch at hand holds it (the plans of the
-  // single-cloud entry points include it; a recognition's stages leave far
-  // more): without it every point is searched in every iteration
+  // the matching state, of as many problems as the scratch at hand holds it for
+  // (the plans of the single-cloud entry points include it up to ICP_STATE_MAX
+  // points; a recognition's stages leave far more): without it every point is
+  // searched in every iteration
+  auto state_fits = [&](size_t n) {
+    Scratch t = s;
+    return t.take<float4>(n) && t.take<int>(n);
+  };
+  int with_state = 0;
   size_t n_state = 0;
-  for (int i = 0; i < M; ++i) n_state += (size_t)specs[i].dev.n_src;
+  while (with_state < M && state_fits(n_state + specs[with_state].dev.n_src))
+    n_state += specs[with_state++].dev.n_src;
   float4* anchor = s.take<float4>(n_state);
   int* last = s.take<int>(n_state);
-  if (!last) anchor = nullptr;
   // apportion blocks: want_i = ceil(n_i * G / threads), scaled to fit
   long long want_total = 0;
   std::vector<long long> want(M);
@@ -689,9 +696,9 @@ rtr_status icp_multi(rtr_context* ctx, Scratch& s, std::vector<IcpSpec>& specs, 
     d.partial = partial + (size_t)blk * 32;
     d.pcount = pcount + blk;
     d.arrive = sync + i;
-    d.anchor = anchor;
-    d.last = last;
-    if (anchor) {
+    d.anchor = i < with_state ? anchor : nullptr;
+    d.last = i < with_state ? last : nullptr;
+    if (i < with_state) {
       anchor += d.n_src;
       last += d.n_src;
     }
@@ -764,9 +771,9 @@ rtr_status rtr_icp(rtr_context* ctx, const float* d_src, int n_src, const float*
   plan.add<GridMeta>(1);
   ScratchPlan least = plan;  // without the matching state
   icp_multi_plan(least, 1, maxb, 0);
-  icp_multi_plan(plan, 1, maxb, n_src);
+  icp_multi_plan(plan, 1, maxb, std::min((size_t)n_src, ICP_STATE_MAX));
   Scratch s;
-  RTR_TRY(ensure_scratch(ctx, scratch_obtainable(ctx, plan.bytes, st) ? plan.bytes : least.bytes, st, &s));
+  RTR_TRY(ensure_scratch_upto(ctx, plan.bytes, least.bytes, st, &s));
   GridBufs gb;
   if (!grid_take(s, n_tgt, cell_cap, &gb)) return fail(RTR_ERR_CAPACITY, "rtr_icp: scratch carve");
   float4* src_sorted = s.take<float4>(n_src);
@@ -842,9 +849,9 @@ rtr_status rtr_icp_multi(rtr_context* ctx, const float* d_src, int n_src, const 
   plan.add<GridMeta>(1);
   ScratchPlan least = plan;  // without the matching state
   icp_multi_plan(least, n_problems, maxb, 0);
-  icp_multi_plan(plan, n_problems, maxb, (size_t)n_problems * n_src);
+  icp_multi_plan(plan, n_problems, maxb, std::min((size_t)n_problems * n_src, ICP_STATE_MAX));
   Scratch s;
-  RTR_TRY(ensure_scratch(ctx, scratch_obtainable(ctx, plan.bytes, st) ? plan.bytes : least.bytes, st, &s));
+  RTR_TRY(ensure_scratch_upto(ctx, plan.bytes, least.bytes, st, &s));
   GridBufs gb;
   if (!grid_take(s, n_tgt, cell_cap, &gb)) return fail(RTR_ERR_CAPACITY, "rtr_icp_multi: scratch carve");
   GridMeta* src_meta = s.take<GridMeta>(1);

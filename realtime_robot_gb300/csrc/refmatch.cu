@@ -1667,9 +1667,9 @@ rtr_status rtr_ref_distance(rtr_context* ctx, const float* d_mcloud, const float
   const size_t least = plan.bytes;  // without the warp form: every pair a CTA
   const size_t o_box = plan.add<RefKeyBox>((size_t)n_model);
   const size_t o_list = plan.add<int>((size_t)n_model * REFW_CLASSES);
-  const int warp_max = scratch_obtainable(ctx, plan.bytes, st) ? REFW_MAX : -1;
   Scratch s;
-  RTR_TRY(ensure_scratch(ctx, warp_max < 0 ? least : plan.bytes, st, &s));
+  RTR_TRY(ensure_scratch_upto(ctx, plan.bytes, least, st, &s));
+  const int warp_max = s.cap >= plan.bytes ? REFW_MAX : -1;
   int* err = reinterpret_cast<int*>(s.base + o_err);
   RefKeyBox* boxes = reinterpret_cast<RefKeyBox*>(s.base + o_box);
   int* list = reinterpret_cast<int*>(s.base + o_list);

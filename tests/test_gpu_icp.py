@@ -262,3 +262,79 @@ def test_icp_sums_keep_every_point_once(ctx, rtr, n_src, group):
     want[:3, 3] = (mq + cq) - R @ (mp + cp)
     tol = 1e-12 if n_src > 100 else 1e-9  # a few points: worse conditioned
     np.testing.assert_allclose(tp.cpu().numpy()[1].reshape(4, 4), want, rtol=0, atol=tol)
+
+
+def test_icp_without_its_matching_state(rtr):
+    """Under a scratch limit that leaves no room for the matching state of a
+    large source (8 MB), every point is searched in every iteration: the same
+    correspondences, poses and result, bit for bit."""
+    src, tgt, _ = rtr.config0_pair(4, 400000)
+    tgt = tgt[:3000].copy()
+    out = []
+    for mb in (0, 19):
+        c = rtr.Context(0)
+        try:
+            c.set_tuning("scratch_limit_mb", mb)
+            res, tp, tc = c.icp(_dev(src), _dev(tgt), 12, 0.05, trace=True)
+            out.append((c.parse_icp_result(res), tp.cpu().numpy(), tc.cpu().numpy(), c.scratch_bytes()))
+        finally:
+            c.close()
+    (ra, pa, ca, na), (rb, pb, cb, nb) = out
+    assert na >= nb + 4000000 and nb <= 19 << 20  # with the state, and without it
+    assert ra["n_corr"] == rb["n_corr"] and ra["iterations"] == rb["iterations"] == 12
+    assert np.array_equal(pa, pb) and np.array_equal(ca, cb)
+
+
+def test_icp_multi_with_the_state_of_some_problems(rtr):
+    """64 problems of 20,000 points under a limit that holds the matching state
+    of a few: the same results as with all of it, bit for bit."""
+    src, tgt, _ = rtr.config0_pair(5, 20000)
+    inits = np.repeat(np.eye(4)[None], 64, 0)
+    inits[:, 0, 3] = np.linspace(-0.02, 0.02, 64)
+    out = []
+    for mb in (0, 5):
+        c = rtr.Context(0)
+        try:
+            c.set_tuning("scratch_limit_mb", mb)
+            out.append((c.icp_multi(_dev(src), _dev(tgt), inits, 12, 0.05), c.scratch_bytes()))
+        finally:
+            c.close()
+    (a, na), (b, nb) = out
+    assert na >= 64 * 20000 * 20 and nb <= 5 << 20
+    for x, y in zip(a, b):
+        assert np.array_equal(x["pose"], y["pose"]) and x["n_corr"] == y["n_corr"] and x["fitness"] == y["fitness"]
+
+
+def test_icp_multi_bounds_its_scratch_and_leaves_batch_graphs_alone(rtr):
+    """The matching state is asked for up to a gigabyte (300 problems of 300,000
+    points would take 1.8); and not at all while a batch graph holds the arena's
+    address and the call can do without: the graph stays good."""
+    src, tgt, _ = rtr.config0_pair(3, 300000)
+    tgt = tgt[:3000].copy()
+    inits = np.repeat(np.eye(4)[None], 300, 0)
+    c = rtr.Context(0)
+    try:
+        r = c.icp_multi(_dev(src), _dev(tgt), inits, 1, 0.05)
+        assert len(r) == 300 and all(x["status"] == 0 and x["n_corr"] == r[0]["n_corr"] for x in r)
+        assert c.scratch_bytes() < 1500000000
+    finally:
+        c.close()
+    prm = rtr.recog_default_params(scene_outward=1)
+    c = rtr.Context(0)
+    try:
+        m = rtr.Model(c, _dev(rtr.synth_shape(rtr.CHAIR, 20000, 3)), prm)
+        scene = rtr.synth_transform_noise(rtr.synth_shape(rtr.CHAIR, 6000, 4), rtr.synth_rigid(5, 20.0, 0.2), 0.002, 6)
+        scenes = [_dev(scene), _dev(scene)]
+        ref = [rtr.parse_recog_result(x) for x in rtr.recognize_batch(c, [m, m], scenes, prm)]
+        g = rtr.BatchGraph(c, [m, m], scenes, prm)
+        held = c.scratch_bytes()
+        n = 2 * held // (64 * 20) + 1000  # points whose state the arena cannot hold
+        big = np.repeat(src, -(-n // src.shape[0]), 0)[:n]
+        assert len(c.icp_multi(_dev(big), _dev(tgt), inits[:64], 2, 0.05)) == 64
+        assert c.scratch_bytes() == held
+        got = [rtr.parse_recog_result(x) for x in g.launch()]
+        assert [len(x["instances"]) for x in got] == [len(x["instances"]) for x in ref]
+        g.close()
+        m.close()
+    finally:
+        c.close()
