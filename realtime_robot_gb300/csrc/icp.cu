@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(ICP_THREADS, OCC) k_icp(const IcpDev* __restri
     return;
   }
   const int B = a.nblk;
-  const BoxView bv = box_view(a.grid);
+  BoxView bv = box_view(a.grid);
+  if (G <= 4) bv.dense = grid_dense(a.grid, bv.g);
   const GridView& g = bv.g;
   const float r = sqrt_up(a.r2max);
   // Centring: target terms about the target box centre c, source terms about

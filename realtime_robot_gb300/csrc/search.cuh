@@ -253,6 +253,7 @@ struct BoxView {
   float margin;
   float nxm, nym, nzm;  // last cell of each axis
   float hx, hy, hz;     // upper corner
+  bool dense;           // many points a cell: large boxes are walked outwards (box_points_ordered)
 };
 __device__ __forceinline__ BoxView box_view(const GridDev& gd) {
   BoxView b;
@@ -266,6 +267,7 @@ __device__ __forceinline__ BoxView box_view(const GridDev& gd) {
   b.hz = g.oz + (float)g.nz * g.h;
   float s = fmaxf(fmaxf(fabsf(g.ox), fabsf(g.oy)), fabsf(g.oz));
   s = fmaxf(s, fmaxf(fmaxf(fabsf(b.hx), fabsf(b.hy)), fabsf(b.hz)));
+  b.dense = false;
   b.margin = 8.0e-6f * (1.0f + s + (float)(max(max(g.nx, g.ny), g.nz) + 3) * g.h);
   return b;
 }
@@ -281,13 +283,13 @@ __device__ __forceinline__ float sqrt_up(float x) {  // >= sqrt(x), by a few par
 
 // The cells meeting the box q -+ t (t > 0 includes the margin), in cell units.
 struct CellBox {
-  float uy, uz, tc2;
+  float ux, uy, uz, tc2;
   int x0, x1, y0, y1, z0, z1;
 };
 __device__ __forceinline__ CellBox cell_box(const BoxView& v, float4 q, float t) {
   const GridView& g = v.g;
-  const float ux = (q.x - g.ox) * g.inv_h;
   CellBox c;
+  const float ux = c.ux = (q.x - g.ox) * g.inv_h;
   c.uy = (q.y - g.oy) * g.inv_h;
   c.uz = (q.z - g.oz) * g.inv_h;
   const float tc = t * g.inv_h;
@@ -350,16 +352,98 @@ __device__ __forceinline__ void near2_take(float4 p, unsigned j, float4 q, Near2
   }
 }
 
-// Calls take(p, j) for the points of the box's rows, spread over the G lanes
-// of the group.  Up to 4 lanes walk the rows one after another, striding
-// through each row's points: fewest instructions, for kernels with enough
-// queries in flight to hide that every row is a dependent load.  With 8 lanes
-// and more each lane fetches one row's span, a prefix sum over the rows
-// numbers their points, and the lanes stride through the numbers, four loads
-// in flight each: a few round trips in all, for kernels whose queries are few
-// and wait on one another.  Uniform in the group.
-template <int G, typename F>
-__device__ __forceinline__ void box_points(const BoxView& v, const CellBox& c, int lg, unsigned gmask, F take) {
+// Whether a cell with a point in it holds more than DENSE_CELL on average: 32
+// points of the grid asked, a lane each.  Where cells hold many, a box scanned
+// whole costs far more than its nearest rows: two 400k chairs within 5 cm, cells
+// of 1 cm, 20 iterations 20.2 ms, 6.9 walked outwards (13.4 with rings of
+// cells); a million points a chair 85 and 26 (36), cells of 2.5 cm 180 and 128
+// (120); two 60k desks within 10 cm, 50 iterations, 4.7 and 3.5.  Where they hold
+// few, walking outwards is a longer chain: 60k points on 10k 2.9 and 4.0 ms, a
+// 640 x 480 frame 1.15 and 1.20 (1.14 with the line at 24 points, 1.21 at 16).
+constexpr unsigned DENSE_CELL = 24;
+__device__ __forceinline__ bool grid_dense(const GridDev& gd, const GridView& g) {
+  const int n = gd.meta->n, lane = threadIdx.x & 31;
+  unsigned cnt = 0;
+  if (n > 0) {
+    const float4 p = g.pts[(int)(((long long)n * lane) >> 5)];
+    const int cx = min(max(q_cell(p.x, g.ox, g.inv_h), 0), g.nx - 1), cy = min(max(q_cell(p.y, g.oy, g.inv_h), 0), g.ny - 1),
+              cz = min(max(q_cell(p.z, g.oz, g.inv_h), 0), g.nz - 1);
+    const uint2 s = cell_span(g, cx, cy, cz);
+    cnt = min(s.y - s.x, 8u * DENSE_CELL);
+  }
+  return __reduce_add_sync(0xffffffffu, cnt) > 32u * DENSE_CELL;
+}
+
+// Cell k of lo .. hi in the order centre, centre - 1, centre + 1, ...
+__device__ __forceinline__ int cell_outward(int lo, int hi, int centre, int k) {
+  const int a = centre - lo, b = hi - centre, m = min(a, b);
+  return centre + (k <= 2 * m ? ((k & 1) ? -(k + 1) / 2 : k / 2) : (a > b ? m - k : k - m));
+}
+
+// The rows of a larger box from the query outwards, each cut to the cells
+// within the second nearest distance that the lane has seen so far: what is
+// left out lies beyond it.  Lane lg takes the points j with j mod G = lg,
+// whatever its cuts.
+template <int G>
+__device__ __forceinline__ void box_points_ordered(const BoxView& v, const CellBox& c, float4 q, float margin, int lg,
+                                                   Near2& n) {
+  const GridView& g = v.g;
+  const int yc = min(max(__float2int_rd(c.uy), c.y0), c.y1), zc = min(max(__float2int_rd(c.uz), c.z0), c.z1);
+  const int ey = c.y1 - c.y0 + 1, ez = c.z1 - c.z0 + 1;
+  float lim2 = c.tc2;
+  for (int kz = 0; kz < ez; ++kz) {
+    const int z = cell_outward(c.z0, c.z1, zc, kz);
+    const float dz = fmaxf(fmaxf((float)z - c.uz, c.uz - ((float)z + 1.f)), 0.f);
+    if (dz * dz > lim2) continue;
+    for (int k0 = 0; k0 < ey; k0 += 4) {
+      uint2 s[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        s[u] = make_uint2(0u, 0u);
+        if (k0 + u < ey) {
+          const int y = cell_outward(c.y0, c.y1, yc, k0 + u);
+          const float dy = fmaxf(fmaxf((float)y - c.uy, c.uy - ((float)y + 1.f)), 0.f);
+          const float rest = lim2 - (dy * dy + dz * dz);
+          if (rest >= 0.f) {
+            const float w = sqrt_up(rest);
+            const int x0 = max(c.x0, __float2int_rd(fmaxf(c.ux - w, 0.f)));
+            const int x1 = min(c.x1, __float2int_rd(fminf(c.ux + w, v.nxm)));
+            if (x0 <= x1) s[u] = row_span(g, x0, x1, y, z);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        unsigned j = s[u].x + (((unsigned)lg - s[u].x) & (G - 1));
+        for (; j + G < s[u].y; j += 2 * G) {
+          const float4 p0 = g.pts[j], p1 = g.pts[j + G];
+          near2_take(p0, j, q, n);
+          near2_take(p1, j + G, q, n);
+        }
+        if (j < s[u].y) near2_take(g.pts[j], j, q, n);
+      }
+      const float t = (sqrt_up(n.sd) + margin) * g.inv_h;
+      lim2 = fminf(c.tc2, t * t * 1.00001f);
+    }
+  }
+}
+
+// The points of the box's rows into n, spread over the G lanes of the group.
+// Up to 4 lanes walk the rows one after another, striding through each row's
+// points: fewest instructions, for kernels with enough queries in flight to
+// hide that every row is a dependent load (larger boxes over dense cells:
+// box_points_ordered).  With 8 lanes and more each lane fetches one row's span,
+// a prefix sum over the rows numbers their points, and the lanes stride through
+// the numbers, four loads in flight each: a few round trips in all, for kernels
+// whose queries are few and wait on one another.  Uniform in the group.
+template <int G>
+__device__ __forceinline__ void box_points(const BoxView& v, const CellBox& c, float4 q, float margin, int lg,
+                                           unsigned gmask, Near2& n) {
+  auto take = [&](float4 p, unsigned j) { near2_take(p, j, q, n); };
+  if (G <= 4 && v.dense && (c.y1 - c.y0 + 1) * (c.z1 - c.z0 + 1) > 4) {
+    box_points_ordered<G>(v, c, q, margin, lg, n);
+    return;
+  }
   if (G <= 4) {
     box_rows(v, c, [&](uint2 s) {
       unsigned j = s.x + (unsigned)lg;
@@ -463,7 +547,7 @@ __device__ __forceinline__ int grid_nn1_from(const BoxView& v, float4 q, float r
   for (;;) {
     const CellBox c = cell_box(v, q, t);
     n = Near2{inf, inf, INT_MAX, -1};
-    box_points<G>(v, c, lg, gmask, [&](float4 p, unsigned j) { near2_take(p, j, q, n); });
+    box_points<G>(v, c, q, margin, lg, gmask, n);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
       const float od = __shfl_xor_sync(gmask, n.bd, o), os = __shfl_xor_sync(gmask, n.sd, o);

@@ -338,3 +338,53 @@ def test_icp_multi_bounds_its_scratch_and_leaves_batch_graphs_alone(rtr):
         m.close()
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("group", [2, 4])
+@pytest.mark.parametrize("n_tgt,max_dist,cell,shift", [
+    (6000, 0.3, 0.06, 0.1),    # boxes of many rows over cells of some 30 points
+    (6000, 0.3, 0.2, 0.15),    # hundreds of points a cell
+    (6000, 0.0, 0.1, 0.3),     # no bound
+    (3000, 0.05, 0.3, 0.02),   # everything in a few cells
+])
+def test_icp_in_dense_cells_equals_a_search_from_scratch(ctx, rtr, group, n_tgt, max_dist, cell, shift):
+    """Targets with many points a cell, whose larger boxes are walked from the
+    query outwards and cut by what has been seen: every iteration's
+    correspondences equal the oracle's search.  Duplicates tie to the lowest
+    index, and one point is not finite."""
+    src, tgt, _ = rtr.config0_pair(6, 8000)
+    src, tgt = src[:3001].copy(), tgt[:n_tgt].copy()
+    src[:, 0] += np.float32(shift)
+    tgt[100:140] = tgt[:40]
+    tgt[9, 0] = np.nan
+    ctx.set_tuning("icp_group", group)
+    try:
+        res, tp, tc = ctx.icp(_dev(src), _dev(tgt), 15, max_dist, cell_size=cell, trace=True)
+        n_it = ctx.parse_icp_result(res)["iterations"]
+    finally:
+        ctx.set_tuning("icp_group", 0)
+    poses, corr = tp.cpu().numpy(), tc.cpu().numpy()
+    for k in range(n_it):
+        ri, _ = O.nn1(O.transform_f32(poses[k].reshape(4, 4), src), tgt, max_dist, "brute")
+        assert np.array_equal(corr[k], ri), k
+
+
+def test_icp_of_dense_clouds_costs_what_its_neighbours_do(ctx, rtr):
+    """Two iterations of two 400,000-point chairs: a bound of 5 cells may cost
+    up to three times one of 2 (6.0 with every box scanned whole, 1.8 walked
+    outwards)."""
+    import torch
+    src, tgt, _ = rtr.config0_pair(4, 400000)
+    s, t = _dev(src), _dev(tgt)
+
+    def time(max_dist):
+        best = float("inf")
+        for k in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ctx.icp(s, t, 2, max_dist, cell_size=0.01)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b)) if k else best
+        return best
+    assert time(0.05) < 3.0 * time(0.02)
