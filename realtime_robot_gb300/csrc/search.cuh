@@ -587,8 +587,11 @@ __device__ __forceinline__ int grid_nn1_from(const BoxView& v, float4 q, float r
 }
 
 // Whether any point lies within sqrt(r2) of q (d^2 <= r2, finite r2), G lanes
-// per query; the same answer as grid_nn1_group finding a neighbour.  Every
-// lane stops once the group has found one.
+// per query; the same answer as grid_nn1_group finding a neighbour.  The own
+// cell first, then rows; every lane stops once the group has found one.  (Rows
+// alone begin in a corner of the box, which costs where cells hold many: 20,000
+// points of a wall against a million within 10 cm 1,110 us, 230 so, and 128
+// instead of 122 where cells hold few.)
 template <int G>
 __device__ __forceinline__ bool grid_any_within(const BoxView& v, float4 q, float r2, int lg, unsigned gmask) {
   const GridView& g = v.g;
@@ -596,6 +599,12 @@ __device__ __forceinline__ bool grid_any_within(const BoxView& v, float4 q, floa
   if (g.ox - q.x > r || q.x - v.hx > r || g.oy - q.y > r || q.y - v.hy > r || g.oz - q.z > r || q.z - v.hz > r)
     return false;
   bool found = false;
+  const int cx = q_cell(q.x, g.ox, g.inv_h), cy = q_cell(q.y, g.oy, g.inv_h), cz = q_cell(q.z, g.oz, g.inv_h);
+  if (cx >= 0 && cy >= 0 && cz >= 0 && cx < g.nx && cy < g.ny && cz < g.nz) {
+    const uint2 s = cell_span(g, cx, cy, cz);
+    for (unsigned j = s.x + (unsigned)lg; j < s.y && !found; j += G) found = dist2_exact(q, g.pts[j]) <= r2;
+    if (G > 1 ? __any_sync(gmask, found) != 0 : found) return true;
+  }
   int left = 4;
   box_rows(v, cell_box(v, q, r), [&](uint2 s) {
     for (unsigned j = s.x + (unsigned)lg; j < s.y && !found; j += G) found = dist2_exact(q, g.pts[j]) <= r2;

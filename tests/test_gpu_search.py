@@ -149,3 +149,29 @@ def test_grid_counted_into_place_on_uneven_clouds(ctx, kind):
     ki, _ = ctx.knn(_dev(q[:50]), _dev(t), 8)
     first = O.nn1(q[:50], t, 0.0, "brute")[0]
     assert np.array_equal(ki.cpu().numpy()[:, 0], first)
+
+
+def test_pose_inliers_cost_follows_the_hits_not_the_cells(ctx):
+    """A wall of a million points: with a radius of 10 cm a cell holds
+    thousands, and every query has a hit in its own; no more than 2.5 times the
+    2 cm count (5 with the box's corner first, 1.5 with the own cell first)."""
+    import torch
+    rng = np.random.default_rng(1)
+    w = np.zeros((1000000, 4), np.float32)
+    w[:, :2] = rng.uniform(0, 4, (1000000, 2))
+    w[:, 2] = rng.uniform(0, 0.004, 1000000)
+    scene, model = _dev(w), _dev(w[::50])
+    poses = np.repeat(np.eye(4)[None], 8, 0)
+    poses[:, 0, 3] = np.linspace(0, 0.05, 8)
+
+    def time(radius):
+        best = float("inf")
+        for k in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ctx.pose_inliers(model, scene, poses, radius)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b)) if k else best
+        return best
+    assert time(0.1) < 2.5 * time(0.02)
