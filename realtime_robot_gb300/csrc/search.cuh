@@ -639,26 +639,34 @@ __device__ __forceinline__ float knn_worst(const unsigned long long (&list)[K]) 
   return __uint_as_float((unsigned)(list[K - 1] >> 32));
 }
 
-// The nearest of the 27 cells around q's (cx, cy, cz) inside the grid: nine
-// rows, a run of points each, the nearest first.  True when nothing farther
-// can enter the list.
+// The nearest of the 27 cells around q's (cx, cy, cz) inside the grid: the own
+// cell, those beside it, then eight rows, a run of points each, the nearest
+// first and cut to the cells that can still hold an entry.  (The own row as one
+// run costs where cells hold many: 50,000 queries in a million points of a room,
+// k = 16 1,865 us, 1,170 now.)  True when nothing farther can enter the list.
 template <int K>
 __device__ __forceinline__ bool knn_near(const GridView& g, float4 q, int cx, int cy, int cz,
                                          unsigned long long (&list)[K]) {
   const float margin = search_margin(g, q, 1);
-  const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.nx - 1);
-  const float ly = g.oy + (float)cy * g.h, lz = g.oz + (float)cz * g.h;  // the query's cell
+  const float lx = g.ox + (float)cx * g.h, ly = g.oy + (float)cy * g.h, lz = g.oz + (float)cz * g.h;  // the query's cell
+  const float xlo = fmaxf(q.x - lx, 0.f), xhi = fmaxf(lx + g.h - q.x, 0.f);
   const float ylo = fmaxf(q.y - ly, 0.f), yhi = fmaxf(ly + g.h - q.y, 0.f);
   const float zlo = fmaxf(q.z - lz, 0.f), zhi = fmaxf(lz + g.h - q.z, 0.f);
 #pragma unroll 1
-  for (int r = 0; r < 9; ++r) {
-    // rows (0, 0), (-1, 0), (1, 0), (0, -1), (0, 1) and the corners: two bits each, plus one
+  for (int k = 0; k < 11; ++k) {
+    // rows (0, 0) in three parts, (-1, 0), (1, 0), (0, -1), (0, 1) and the corners: two bits each, plus one
+    const int r = max(k - 2, 0);
     const int dy = (int)((0x28161u >> (2 * r)) & 3u) - 1, dz = (int)((0x22215u >> (2 * r)) & 3u) - 1;
     const int y = cy + dy, z = cz + dz;
     if (y < 0 || y >= g.ny || z < 0 || z >= g.nz) continue;
     const float ey = dy < 0 ? ylo : (dy > 0 ? yhi : 0.f), ez = dz < 0 ? zlo : (dz > 0 ? zhi : 0.f);
-    if (beyond(sqrtf(ey * ey + ez * ez), margin, knn_worst<K>(list))) continue;
-    const uint2 span = row_span(g, x0, x1, y, z);
+    const float e2 = ey * ey + ez * ez, worst = knn_worst<K>(list);
+    if (r > 0 && beyond(sqrtf(e2), margin, worst)) continue;
+    const bool left = cx > 0 && k != 0 && k != 2 && !beyond(sqrtf(e2 + xlo * xlo), margin, worst);
+    const bool right = cx < g.nx - 1 && k > 1 && !beyond(sqrtf(e2 + xhi * xhi), margin, worst);
+    const int xa = k == 2 ? cx + 1 : (left ? cx - 1 : cx), xb = k == 1 ? cx - 1 : (right ? cx + 1 : cx);
+    if (xa > xb || (k == 1 && !left)) continue;
+    const uint2 span = row_span(g, xa, xb, y, z);
     for (unsigned j = span.x; j < span.y; ++j) knn_insert<K>(list, q, g.pts[j]);
   }
   return ring_covers(g, cx, cy, cz, 1) || beyond(ring_bound(g, q, cx, cy, cz, 1), margin, knn_worst<K>(list));

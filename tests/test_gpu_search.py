@@ -151,6 +151,30 @@ def test_grid_counted_into_place_on_uneven_clouds(ctx, kind):
     assert np.array_equal(ki.cpu().numpy()[:, 0], first)
 
 
+@pytest.mark.parametrize("k", [1, 5, 8, 16, 32])
+def test_knn_in_dense_cells_equals_brute_force(ctx, k):
+    """Clouds whose automatic cells hold dozens of points, lattices (ties) and
+    single points: every entry by (FP32 distance, index)."""
+    rng = np.random.default_rng(k)
+    n = 4000
+    t = _rand(rng, n, 1.0)
+    t[:2000, :3] = t[:2000, :3] * 0.02
+    t[2000:3000, :3] = np.float32(0.25) + np.float32(0.015625) * rng.integers(0, 8, (1000, 3)).astype(np.float32)
+    t[11, 0], t[12, 1] = np.nan, np.inf
+    q = np.concatenate([t[:300], t[2000:2300] + np.float32(0.0078125), t[3000:3200], _rand(rng, 50, 3.0)])
+    q = q[np.isfinite(q[:, :3]).all(1)].copy()
+    q[:, 3] = 0
+    idx, d2 = ctx.knn(_dev(q), _dev(t), k)
+    with np.errstate(all="ignore"):
+        d = q[:, None, :3] - t[None, :, :3]
+        d = d * d
+        ref = (d[..., 0] + d[..., 1]) + d[..., 2]
+    ref = np.where(np.isfinite(ref), ref, np.float32(np.inf))
+    o = np.argsort(ref, axis=1, kind="stable")[:, :k]
+    assert np.array_equal(idx.cpu().numpy(), o)
+    assert np.array_equal(d2.cpu().numpy(), np.take_along_axis(ref, o, 1))
+
+
 def test_pose_inliers_cost_follows_the_hits_not_the_cells(ctx):
     """A wall of a million points: with a radius of 10 cm a cell holds
     thousands, and every query has a hit in its own; no more than 2.5 times the
