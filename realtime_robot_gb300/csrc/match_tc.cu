@@ -664,7 +664,7 @@ __device__ __forceinline__ float exact_d2(const float* __restrict__ x, const flo
 // Exact FP32 re-rank of the candidates that can still win, and
 // certification.  Uncertified queries go to the redo list with their running
 // minimum reset.
-// A warp takes 16 queries, lists the candidates in doubt (one or two a query)
+// A warp takes `per` (4 .. 16) queries, lists the candidates in doubt (one or two a query)
 // and handles eight of them at a time: the lanes read each candidate's and its
 // query's row together (whole lines, all eight in flight), the squared
 // differences go through shared memory, and a lane adds up one candidate's in
@@ -673,11 +673,17 @@ __device__ __forceinline__ float exact_d2(const float* __restrict__ x, const flo
 constexpr int RR_WARPS = 4;
 constexpr int RR_Q = 16;
 constexpr int RR_C = 8;
+// Queries a warp takes: 16, fewer where a warp would have its chain of
+// candidates and others nothing (whole call, us, 4 / 8 / 16 a warp; rows of a
+// room: 50 queries 96 / 98 / 104, 6,000 124 / 128 / 134, 111k 668 / 651 / 650;
+// every row nine times in the database: 50 118 / 133 / 161, 6,000 135 / 150 /
+// 172, 20,000 227 / 235 / 232).
+static int rr_queries(int nq) { return nq <= 8000 ? 4 : (nq <= 16000 ? 8 : RR_Q); }
 template <bool V4>
 __global__ void __launch_bounds__(32 * RR_WARPS)
     k_rerank(const float* __restrict__ q, int nq_host, const int* d_nq, int nq_cap, const float* __restrict__ db, int ndb,
              const int* __restrict__ cand_idx, const float* __restrict__ cand_d, const int* __restrict__ more_idx,
-             const float* __restrict__ more_d, int ranges, int* __restrict__ out_idx, float* __restrict__ out_d2,
+             const float* __restrict__ more_d, int ranges, int per, int* __restrict__ out_idx, float* __restrict__ out_d2,
              int* __restrict__ redo, int* __restrict__ n_redo, unsigned long long* __restrict__ redo_best,
              float* __restrict__ redo_thr, const float* __restrict__ qn, const float* __restrict__ db_max,
              const unsigned long long* __restrict__ zero_best, const unsigned char* __restrict__ qzero) {
@@ -690,13 +696,13 @@ __global__ void __launch_bounds__(32 * RR_WARPS)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane >> 3, l8 = lane & 7;
   const int warps = gridDim.x * RR_WARPS;
   const float dbm = *db_max;
-  for (int base = (blockIdx.x * RR_WARPS + w) * RR_Q; base < nq; base += warps * RR_Q) {
-    if (lane < RR_Q) s_best[w][lane] = ~0ull;
+  for (int base = (blockIdx.x * RR_WARPS + w) * per; base < nq; base += warps * per) {
+    if (lane < per) s_best[w][lane] = ~0ull;
     // |d~ - d| <= err: a candidate whose d~ exceeds the smallest d~ (the
     // first of the ranges' ascending lists) by more than 2 err has an exact
     // distance above that candidate's, so it can neither win nor tie: its
     // exact distance is not computed
-    if (lane < RR_Q) {
+    if (lane < per) {
       const int i = base + lane;
       float bound = -__int_as_float(0x7f800000), worst = __int_as_float(0x7f800000);
       if (i < nq && qzero[i] == 0) {
@@ -719,6 +725,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS)
       int cnt = 0;
 #pragma unroll
       for (int q0 = 0; q0 < RR_Q; q0 += 4) {
+        if (q0 >= per) break;
         const size_t at = (size_t)(base + q0 + sub) * TC_TOP + l8;
         const bool live = base + q0 + sub < nq;
         const int c = live ? li[at] : -1;
@@ -775,7 +782,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS)
     }
     __syncwarp();
     const int i = base + lane;
-    if (lane < RR_Q && i < nq) {
+    if (lane < per && i < nq) {
       const unsigned long long best = s_best[w][lane];
       if (qzero[i] != 0) {
         // an all-zero query ties (up to rounding) with every unit-norm row: its
@@ -1110,7 +1117,8 @@ rtr_status match_tc_dev(rtr_context* ctx, Scratch& s, const float* q, int nq_cap
     k_match_top<<<dim3(nqp / TC_BM, ranges), TC_THREADS, top_smem, st>>>(m_qh, m_ql, m_bh, m_bl, a);
   }
   RTR_CUDA(cudaMemsetAsync(nredo, 0, 2 * sizeof(int), st));
-  int rb = (nq_cap + RR_WARPS * RR_Q - 1) / (RR_WARPS * RR_Q);
+  const int per = rr_queries(nq_cap);
+  int rb = (nq_cap + RR_WARPS * per - 1) / (RR_WARPS * per);
   if (rb > 152 * 16) rb = 152 * 16;
   // block per uncertified query (grid-stride over the device-side count)
   const int wb = band_rows(nqp) < 152 * 8 ? band_rows(nqp) : 152 * 8;
@@ -1120,11 +1128,13 @@ rtr_status match_tc_dev(rtr_context* ctx, Scratch& s, const float* q, int nq_cap
   TcArgs ab{bq, nredo, bq, ndb, qn2, band_idx, nullptr, nullptr, nullptr, ctx->d_status, redo_thr, band_n, tc_spin_limit(ctx)};
   ProfScope pr(ctx, st, "match_rerank");
   if (v4)
-    k_rerank<true><<<rb, 32 * RR_WARPS, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, more_idx, more_d, ranges, out_idx, out_d2, redo, nredo,
-                                       redo_best, redo_thr, qn, db_n2 + ndb, db_zero_key(db_n2, ndb), qzero);
+    k_rerank<true><<<rb, 32 * RR_WARPS, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, more_idx, more_d, ranges,
+                                                 per, out_idx, out_d2, redo, nredo, redo_best, redo_thr, qn,
+                                                 db_n2 + ndb, db_zero_key(db_n2, ndb), qzero);
   else
-    k_rerank<false><<<rb, 32 * RR_WARPS, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, more_idx, more_d, ranges, out_idx, out_d2, redo, nredo,
-                                        redo_best, redo_thr, qn, db_n2 + ndb, db_zero_key(db_n2, ndb), qzero);
+    k_rerank<false><<<rb, 32 * RR_WARPS, 0, st>>>(q, nq_cap, d_nq, nq_cap, db, ndb, cidx, cd, more_idx, more_d, ranges,
+                                                  per, out_idx, out_d2, redo, nredo, redo_best, redo_thr, qn,
+                                                  db_n2 + ndb, db_zero_key(db_n2, ndb), qzero);
   pr.end();
   ProfScope pu(ctx, st, "match_uncertified");
   k_band_gather<<<(bq + 7) / 8 < 152 * 2 ? (bq + 7) / 8 : 152 * 2, 256, 0, st>>>(reinterpret_cast<const uint4*>(qhi), reinterpret_cast<const uint4*>(qlo),

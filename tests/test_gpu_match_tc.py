@@ -205,3 +205,20 @@ def test_match_tc_nan_rows_leave_the_error_bound_alone(ctx, nq, bad):
     assert np.array_equal(idx.cpu().numpy(), ri)
     assert np.array_equal(d2.cpu().numpy(), rd)
     assert not np.isin(ri, [17, 107, 197][:bad]).any()
+
+
+@pytest.mark.parametrize("nq", [3, 5, 4001, 8000, 8001, 16001])
+def test_match_tc_rerank_shares_and_ties(ctx, descs, nq):
+    """Queries dealt to the re-rank's warps by 4, 8 and 16, ragged at the end,
+    with every database row nine times (eight candidates a query in doubt, ties
+    to the lowest index) and zero queries among them."""
+    md, sd = descs
+    db = np.concatenate([md[:60]] * 9)
+    q = np.concatenate([sd] * (nq // len(sd) + 1))[:nq].copy()
+    q[::101] = 0.0
+    q[1::7] = md[np.arange(len(q[1::7])) % 60]
+    idx, d2 = ctx.match(_dev(q), _dev(db))
+    ri, rd = O.match(q, db)
+    assert np.array_equal(idx.cpu().numpy(), ri)
+    assert np.array_equal(d2.cpu().numpy(), rd)
+    assert ri.max() < 60
