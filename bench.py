@@ -345,7 +345,7 @@ def run_ours(args):
     kern = {
         # one FP32-equivalent GEMM: 2 * scene keypoints * model keypoints * 352
         "match_gemm": ("tensor", 2.0 * Ks * Km * 352, "k_match_top (tcgen05 BF16 hi/lo split, FP32 accumulate, top-8)",
-                       "three BF16 MMAs per K step; two 96 KB TMA stages per CTA"),
+                       "three BF16 MMAs per K step (two in the tail block); four 48 KB TMA stages per CTA"),
         # the unique bytes the walk must move: both endpoints (32 B) of every
         # correspondence; everything else (C x sets consistency checks over
         # those endpoints, the pass masks, the sets) lives in L2

@@ -401,8 +401,9 @@ rtr_status rtr_pose_inliers(rtr_context* ctx, const float* d_model, int n_model,
  * One persistent cooperative kernel runs all iterations: per iteration it
  * transforms the source, finds the exact 1-NN in the target grid, rejects
  * pairs beyond max_corr_dist, accumulates the centred 3x3 cross-covariance in
- * FP32 with compensated (Kahan) sums, reduces the block partials in FP64 and
- * solves the pose in FP64 (Umeyama, Jacobi SVD). */
+ * FP32 with compensated (Kahan) sums, reduces the block partials in the same
+ * way (closed in FP64) and solves the pose (Umeyama's rotation: an FP32 start,
+ * then Newton steps with an FP64 residual to FP64 accuracy). */
 typedef struct rtr_icp_params {
   int    max_iterations;         /* PCL default 10                                */
   float  max_corr_dist;          /* metres; <= 0 = unbounded (PCL default)        */

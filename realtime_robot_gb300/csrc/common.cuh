@@ -242,19 +242,6 @@ struct KSum {
   }
 };
 
-// Warp-level compensated reduction of (s, c) pairs; lane 0 holds the result.
-__device__ __forceinline__ void warp_ksum(float& s, float& c) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    float s2 = __shfl_down_sync(0xffffffffu, s, off);
-    float c2 = __shfl_down_sync(0xffffffffu, c, off);
-    float t, e;
-    two_sum(s, s2, t, e);
-    s = t;
-    c = __fadd_rn(__fadd_rn(c, c2), e);
-  }
-}
-
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
   asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -265,10 +252,6 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-
-__device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // Float <-> order-preserving unsigned (for atomicMin/Max on floats).

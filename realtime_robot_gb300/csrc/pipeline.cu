@@ -1103,7 +1103,7 @@ rtr_status rtr_pose_inliers(rtr_context* ctx, const float* d_model, int n_model,
   float* score = s.take<float>(n_poses);
   if (!score) return fail(RTR_ERR_CAPACITY, "rtr_pose_inliers: scratch");
   ProfScope ps(ctx, st, "pose_inliers");
-  // a cell 1.5 x the radius: the counts take the 27-cell existence search
+  // a cell 1.5 x the radius: a query's box meets 8 to 27 cells
   RTR_TRY(grid_build(gb, reinterpret_cast<const float4*>(d_scene), n_scene, nullptr, 1.5f * radius, st));
   RTR_TRY(hv_score(grid_dev(gb), reinterpret_cast<const float4*>(d_model), n_model, 1, d_poses, n_poses, nullptr,
                    radius * radius, d_counts, score, st));
