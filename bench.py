@@ -355,9 +355,9 @@ def run_ours(args):
                     f"each seed's reach; stale sets recomputed in place); the 32 B x C endpoints stay in L2"),
         # per hypothesis and iteration: each model voxel (16 B) and its matched scene point (16 B)
         "icp_refine": ("hbm", 32.0 * M_ref * prm.icp_iterations * m.n_voxels, "k_icp (multi-problem refinement)",
-                       "latency- and barrier-bound: per iteration a 27-cell 1-NN per source point (own cell, "
-                       "then only the neighbours within reach; grid and voxels stay in L2), a per-hypothesis "
-                       "barrier and the FP64 pose solve"),
+                       "latency- and barrier-bound: per iteration each source point shows that its last neighbour "
+                       "still is the nearest or is searched from it (grid and voxels stay in L2), then a "
+                       "per-hypothesis barrier and the FP64 pose solve"),
     }
     kern = {k: v for k, v in kern.items() if k in stage_ms}
     top = max(kern, key=lambda k: stage_ms[k])

@@ -845,8 +845,9 @@ static rtr_status recognize_impl(rtr_context* ctx, const rtr_model* m, const flo
   const bool learned = mlp != nullptr;
   // A plain recognition keeps a grid of tiles for its sorts, also where one
   // cluster would do: tests/test_gpu_graph.py holds it to more than 100
-  // launches, and it has 101 (a 12k-point segment takes 2.185 ms so, 2.088 with
-  // the clusters and 59 launches; a batch of 64 takes 29.2 and 25.1).
+  // launches, and it has 101 (a 12k-point segment takes 1.73 ms so, 1.65 with
+  // the clusters and 59 launches; scenes of over 131,072 points sort by tiles
+  // anyway).
   struct GridSorts {
     rtr_context* c;
     GridSorts(rtr_context* ctx, bool on) : c(ctx) { c->grid_sorts = on; }

@@ -64,3 +64,17 @@ def test_tdf_batch_row_split_edges(ctx, n_keys, dim):
     out = ctx.tdf_batch(torch.from_numpy(occ).cuda(), torch.from_numpy(offs).cuda(), dim).cpu().numpy()
     for k in range(n_keys) if n_keys < 1000 else (0, 1, 65534, 65535, 65536, n_keys - 1):
         assert np.array_equal(out[k], O.tdf(occ[k * per:(k + 1) * per], dim)), k
+
+
+@pytest.mark.parametrize("n_keys,dim", [(28, 30), (29, 30), (6, 32), (8, 16), (114, 16), (115, 16)])
+def test_tdf_batch_on_both_sides_of_the_row_split(ctx, n_keys, dim):
+    """The two row splits meet where whole rows alone give three CTAs to every
+    two SMs (228 on 152): 28 and 29 keypoints of 30 cells an edge, 114 and 115
+    of 16."""
+    import torch
+    rng = np.random.default_rng(n_keys * dim)
+    occ = rng.integers(-3, dim + 3, size=(n_keys * 61, 3)).astype(np.int32)
+    offs = (np.arange(n_keys + 1) * 61).astype(np.int32)
+    out = ctx.tdf_batch(torch.from_numpy(occ).cuda(), torch.from_numpy(offs).cuda(), dim).cpu().numpy()
+    for k in range(n_keys):
+        assert np.array_equal(out[k], O.tdf(occ[k * 61:(k + 1) * 61], dim)), k
